@@ -651,12 +651,21 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
                     if (active) {
                         unsigned va[16], vb[16];
                         tc_ld_2x16x256b_x4_wait(tbase + (unsigned)(32 * pass), va, vb);
-                        if (a.out_unsigned)
-                            perm_block<4, false, CLAMP, false, EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, cbase + 32 * pass, region_off, rb,
-                                                                                          0, lane, 0, 0, 0u);
-                        else
-                            perm_block<4, false, CLAMP, false, EF_PERM>(va, vb, par_off, cbase + 32 * pass, region_off, rb, 0, lane,
-                                                                        0, 0, 0u);
+                        const int pc = cbase + 32 * pass;
+                        switch (a.ef & (EF_OUT_UNSIGNED | EF_WIDE | EF_FLOAT)) {
+                        case 0: perm_block<4, false, CLAMP, false, EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
+                        case EF_OUT_UNSIGNED:
+                            perm_block<4, false, CLAMP, false, EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
+                            break;
+                        case EF_WIDE: perm_block<4, false, false, false, EF_WIDE | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
+                        case EF_WIDE | EF_OUT_UNSIGNED:
+                            perm_block<4, false, false, false, EF_WIDE | EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
+                            break;
+                        case EF_FLOAT: perm_block<4, false, CLAMP, false, EF_FLOAT | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
+                        default:
+                            perm_block<4, false, CLAMP, false, EF_FLOAT | EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
+                            break;
+                        }
                     }
                     if (pass == 1) {
                         // the accumulator is drained: hand it back before the store goes out
@@ -974,7 +983,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     a.dp_a_signed = fast.dp_a_signed;
     const bool t_unsigned = fast.dp4a ? fast.dp_t_unsigned : (fast.t_lo == 0);
     a.ef = (fast.out_unsigned ? EF_OUT_UNSIGNED : 0) | (r.is_unsigned ? EF_RES_UNSIGNED : 0)
-         | (t_unsigned ? EF_T_UNSIGNED : 0) | (fast.dp_a_signed ? EF_DP_A_SIGNED : 0) | (fast.wide ? EF_WIDE : 0);
+         | (t_unsigned ? EF_T_UNSIGNED : 0) | (fast.dp_a_signed ? EF_DP_A_SIGNED : 0) | fast.form;
     const bool use_fast = igemm_uses_fast_epilogue(plan, fast, r.ptr != nullptr, out_dtype);
     // the weights of a cell on the 32-bit epilogue are stored permuted (and only those)
     if (use_fast != (plan.perm != 0)) return cudaErrorInvalidConfiguration;
@@ -1004,7 +1013,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     if (a.b_resident && tiles > grid && a.num_n_tiles > 1 && grid % a.num_n_tiles != 0) return cudaErrorInvalidConfiguration;
     a.step_m = grid / a.num_n_tiles;
     a.step_n = grid % a.num_n_tiles;
-    if (plan.pair && use_fast && !r.ptr && !fast.wide) {
+    if (plan.pair && use_fast && !r.ptr) {
         typedef void (*PairKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const IgemmArgs);
         static const PairKernel pair_kernels[2] = {igemm_pair_i8_tcgen05_kernel<false>, igemm_pair_i8_tcgen05_kernel<true>};
         static std::atomic<bool> pair_attr_set[64];

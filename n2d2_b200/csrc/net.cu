@@ -313,6 +313,38 @@ static bool build_wide_quant(const QuantHost& q, int cpad, long long x_bound, st
     return true;
 }
 
+// Floating-point scaling: y = round(clamp(float(acc + bias), lo, hi) * factor), the final pack saturates.  Clipping to [0, clip]
+// (to [clip, 0] for clip <= 0) before the rescale is the clamp: a sum inside the bound converts to a float that is not
+// beyond it, one outside converts to the bound or further.  A ReLU in front of a signed output is the lower bound 0, which
+// needs factors that are not negative; the sum has to stay inside 32 bits.  Rows: lo, hi, factor (floats), bias, unused.
+static bool build_float_quant(const QuantHost& q, int cpad, long long x_bound, std::vector<int32_t>& out, bool* need_clamp)
+{
+    if (q.mode != SC_FLOAT_MULT || q.out_bits != 8 || q.act == ACT_SATURATION) return false;
+    const bool relu_clamp = q.act == ACT_RECTIFIER && !q.out_unsigned;
+    if (q.is_clipped || relu_clamp) *need_clamp = true;
+    out.assign((size_t)5 * cpad, 0);
+    for (int c = 0; c < q.nb_channels; ++c) {
+        const float factor = q.fscale[c];
+        if (!std::isfinite(factor) || !(factor >= 0.0f)) return false;
+        const long long b = q.has_bias ? q.bias[c] : 0;
+        if (std::llabs(b) + x_bound > (1ll << 31) - 1) return false;
+        float lo = -INFINITY, hi = INFINITY;
+        if (q.is_clipped) {
+            lo = std::min(q.clip_f[c], 0.0f);
+            hi = std::max(q.clip_f[c], 0.0f);
+        }
+        if (relu_clamp) {
+            lo = std::max(lo, 0.0f);
+            hi = std::max(hi, 0.0f);
+        }
+        memcpy(&out[(size_t)0 * cpad + c], &lo, 4);
+        memcpy(&out[(size_t)1 * cpad + c], &hi, 4);
+        memcpy(&out[(size_t)2 * cpad + c], &factor, 4);
+        out[(size_t)3 * cpad + c] = (int32_t)b;
+    }
+    return true;
+}
+
 static bool build_fast_quant(const QuantHost& q, int cpad, long long x_bound, std::vector<int32_t>& out, int* eff_lo,
                              int* eff_hi, bool* need_clamp)
 {
@@ -387,7 +419,15 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
     const long long acc_bound = (long long)c.geom.kH * c.geom.kW * c.geom.Cg * 255ll * (w4 ? 8ll : 128ll);
     if (acc_bound * (w4 ? 16 : 1) > (1ll << 30)) return 0;
     bool need_clamp = false, wide = false;
-    if (!build_fast_quant(c.q, cpad, acc_bound, f1, &lo1, &hi1, &need_clamp)) {
+    const bool with_res = c.residual >= 0;
+    const bool flt = c.q.mode == SC_FLOAT_MULT;
+    if (flt) {
+        // both stages of a residual cell share one form
+        if (!build_float_quant(c.q, cpad, acc_bound, f1, &need_clamp)) return 0;
+        if (with_res && !build_float_quant(c.q2, cpad, 512, f2, &need_clamp)) return 0;
+        lo1 = c.q.out_unsigned ? 0 : (c.q.act == ACT_RECTIFIER ? 0 : -128);
+        hi1 = c.q.out_unsigned ? 255 : 127;
+    } else if (!build_fast_quant(c.q, cpad, acc_bound, f1, &lo1, &hi1, &need_clamp)) {
         // eff range etc. were set before the failing channel; retry in 64 bits
         need_clamp = false;
         if (c.q.out_bits != 8 || c.q.act == ACT_SATURATION
@@ -400,8 +440,7 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
         hi1 = c.q.out_unsigned ? 255 : 127;
         if (c.q.act == ACT_RECTIFIER && lo1 < 0) lo1 = 0;
     }
-    bool with_res = c.residual >= 0;
-    if (with_res && !build_fast_quant(c.q2, cpad, 512, f2, &lo2, &hi2, &need_clamp)) return 0;
+    if (with_res && !flt && !build_fast_quant(c.q2, cpad, 512, f2, &lo2, &hi2, &need_clamp)) return 0;
     if (wide && need_clamp) return 0;   // the 64-bit form has no clamps
     // Dot-product form of the residual stage (see perm_block): every multiplier of the sum's scaling fits a byte,
     // both operands have a native 8-bit range and no clamp is needed.  The four bytes [t, t', r, r'] of a dot
@@ -412,7 +451,7 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
     bool dp4a = false, dp_t_unsigned = false;
     unsigned dp_xor = 0;
     int dp_a_signed = 1;
-    if (with_res && !need_clamp && !wide && residual_dtype_i8) {
+    if (with_res && !need_clamp && !wide && !flt && residual_dtype_i8) {
         const bool t_uns = (lo1 == 0 && hi1 == 255), t_sig = (lo1 == -128 && hi1 == 127);
         const bool r_uns = residual_unsigned != 0;
         bool ok = t_uns || t_sig;
@@ -454,7 +493,7 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
     c.fast.t_hi = hi1;
     c.fast.out_unsigned = with_res ? c.q2.out_unsigned : c.q.out_unsigned;
     c.fast.need_clamp = need_clamp;
-    c.fast.wide = wide;
+    c.fast.form = wide ? EF_WIDE : (flt ? EF_FLOAT : 0);
     c.fast.dp4a = dp4a;
     c.fast.dp_t_unsigned = dp_t_unsigned;
     c.fast.dp_xor = dp_xor;
@@ -1660,7 +1699,7 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     switch (net->cells[cell].engine) {
     case ENG_TCGEN05: {
         const CellRec& c = net->cells[cell];
-        const bool pair = c.plan.pair && c.fast.enabled && !c.fast.wide && c.residual < 0
+        const bool pair = c.plan.pair && c.fast.enabled && c.residual < 0
                           && net->tensors[c.output].dtype == DT_I8 && c.geom.O % 32 == 0;
         if (c.geom.groups > 1) return "depthwise-tcgen05";
         return pair ? "tcgen05-pair" : (c.plan.w4 ? "tcgen05-w4" : "tcgen05");

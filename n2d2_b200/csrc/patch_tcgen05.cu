@@ -57,7 +57,6 @@ struct PatchArgs {
     const int* fq;
     int cpad;
     int out_unsigned;
-    int wide;               // 64-bit first rescale (see EF_WIDE)
 };
 
 // The MMAs of one tile with compile-time tap counts: a straight run of address adds and MMAs.  The issuing
@@ -94,8 +93,10 @@ __device__ __forceinline__ void issue_tap(int ksteps, unsigned d_tmem, unsigned 
     else issue_tap_n<1>(d_tmem, a_lo, b_lo, desc_hi, idesc, first, issue);
 }
 
-// SHAPE: 0 = any filter (loops), 1 / 2 / 3 = 3x3 filter with 32 / 64 / 128 channels (unrolled issue)
-template <bool CLAMP, int SHAPE>
+// SHAPE: 0 = any filter (loops), 1 / 2 / 3 = 3x3 filter with 32 / 64 / 128 channels (unrolled issue).  FORM: EF_WIDE or
+// EF_FLOAT, the form of the rescale (0: 32-bit); a template because a choice per 32-column block inside the epilogue
+// cost 2 % of a MobileNet
+template <bool CLAMP, int SHAPE, int FORM>
 __global__ void __launch_bounds__(P_THREADS, 1)
 patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PatchArgs a)
 {
@@ -326,11 +327,8 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                 for (int cb = 0; cb < a.N; cb += 32) {
                     unsigned va[16], vb[16];
                     tc_ld_2x16x256b_x4_wait(tbase + (unsigned)cb, va, vb);
-                    if (a.wide) {
-                        if (a.out_unsigned) perm_block_global<false, EF_WIDE | EF_OUT_UNSIGNED>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
-                        else perm_block_global<false, EF_WIDE>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
-                    } else if (a.out_unsigned) perm_block_global<CLAMP, EF_OUT_UNSIGNED>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
-                    else perm_block_global<CLAMP, 0>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
+                    if (a.out_unsigned) perm_block_global<CLAMP, FORM | EF_OUT_UNSIGNED>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
+                    else perm_block_global<CLAMP, FORM>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
                 }
                 // the accumulator is drained: hand it back
                 tc_fence_before();
@@ -544,12 +542,12 @@ cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, 
     a.fq = fast.fq;
     a.cpad = fast.cpad;
     a.out_unsigned = fast.out_unsigned;
-    a.wide = fast.wide ? 1 : 0;
     typedef void (*PatchKernel)(const CUtensorMap, const CUtensorMap, const PatchArgs);
-    static const PatchKernel variants[8] = {
-        patch_conv_tcgen05_kernel<false, 0>, patch_conv_tcgen05_kernel<false, 1>, patch_conv_tcgen05_kernel<false, 2>,
-        patch_conv_tcgen05_kernel<false, 3>, patch_conv_tcgen05_kernel<true, 0>,  patch_conv_tcgen05_kernel<true, 1>,
-        patch_conv_tcgen05_kernel<true, 2>,  patch_conv_tcgen05_kernel<true, 3>};
+#define N2D2B_PATCH(C, F) patch_conv_tcgen05_kernel<C, 0, F>, patch_conv_tcgen05_kernel<C, 1, F>, \
+                          patch_conv_tcgen05_kernel<C, 2, F>, patch_conv_tcgen05_kernel<C, 3, F>
+    static const PatchKernel variants[20] = {N2D2B_PATCH(false, 0), N2D2B_PATCH(true, 0), N2D2B_PATCH(false, EF_FLOAT),
+                                             N2D2B_PATCH(true, EF_FLOAT), N2D2B_PATCH(false, EF_WIDE)};   // the wide form has no clamps
+#undef N2D2B_PATCH
     static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
     int dev = 0;
     cudaGetDevice(&dev);
@@ -565,7 +563,7 @@ cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, 
     const long long per_group = plan.num_sms / plan.G > 0 ? plan.num_sms / plan.G : 1;
     const int grid = (int)((items < per_group ? items : per_group) * plan.G);
     const int shape = (g.kH == 3 && g.kW == 3 && !plan.b_stream) ? (g.C == 32 ? 1 : (g.C == 64 ? 2 : 3)) : 0;
-    return launch_pdl(variants[(fast.need_clamp ? 4 : 0) + shape], grid, P_THREADS, plan.smem_bytes, s, plan.tmA, plan.tmB, a);
+    return launch_pdl(variants[(fast.form == EF_WIDE ? 16 : (fast.form == EF_FLOAT ? 8 : 0) + (fast.need_clamp ? 4 : 0)) + shape], grid, P_THREADS, plan.smem_bytes, s, plan.tmA, plan.tmB, a);
 }
 
 }  // namespace n2d2b

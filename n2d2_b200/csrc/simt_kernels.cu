@@ -299,7 +299,7 @@ cudaError_t launch_conv_depthwise(const void* in, int in_unsigned, const int8_t*
     // 3x3 filters whose rescale has the proved 32-bit form take the dot-product kernel
     const int cw = g.C / 4;
     const bool idx32 = (long long)g.B * g.H * g.W * cw < (1ll << 31) && (long long)g.B * g.oH * g.oW * cw < (1ll << 31);
-    if (fast.enabled && !fast.wide && g.kH == 3 && g.kW == 3 && 256 % cw == 0 && idx32) {
+    if (fast.enabled && fast.form == 0 && g.kH == 3 && g.kW == 3 && 256 % cw == 0 && idx32) {
         const long long rows = (long long)g.B * g.oH;
         if (rows == 0 || g.oW == 0) return cudaSuccess;
         // few, long-lived blocks: a thread's weights and constants (29 loads) are fetched once and serve many rows

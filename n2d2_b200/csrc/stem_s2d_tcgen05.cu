@@ -62,7 +62,6 @@ struct S2dArgs {
     const int* fq;
     int cpad;
     int out_unsigned;
-    int wide;               // 64-bit first rescale (see EF_WIDE)
 };
 
 // [B][H][W][C] (C <= 4) -> [B][Hs][Ws][2][2][4]: block (dy, dx) of pixel (Y, X) = input pixel
@@ -147,7 +146,8 @@ __device__ __forceinline__ void s2d_drain(unsigned tbase, unsigned par_off, unsi
 }
 
 // SHAPE: 0 = any filter (loops), 1 = 4 x 4 (a 7x7/2 or 8x8/2 filter), 2 = 2 x 2 (a 3x3/2 filter)
-template <bool CLAMP, int SHAPE, bool POOL>
+// FORM: EF_WIDE or EF_FLOAT, the form of the rescale (0: 32-bit)
+template <bool CLAMP, int SHAPE, bool POOL, int FORM>
 __global__ void __launch_bounds__(Z_THREADS, 1)
 stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a)
 {
@@ -300,11 +300,8 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
                     // this warp's 32 positions of the tile, at their place in the band buffer (a multiple of 32 rows
                     // from its start, so the swizzle term of a row is the one the staging regions use)
                     const unsigned dst_off = cbuf_off + (unsigned)((t * ZBM + quad * 32) * a.BN);
-                    if (a.wide) {
-                        if (a.out_unsigned) s2d_drain<false, EF_WIDE | EF_OUT_UNSIGNED>(tbase, par_off, dst_off, a.BN, lane);
-                        else s2d_drain<false, EF_WIDE>(tbase, par_off, dst_off, a.BN, lane);
-                    } else if (a.out_unsigned) s2d_drain<CLAMP, EF_OUT_UNSIGNED>(tbase, par_off, dst_off, a.BN, lane);
-                    else s2d_drain<CLAMP, 0>(tbase, par_off, dst_off, a.BN, lane);
+                    if (a.out_unsigned) s2d_drain<CLAMP, FORM | EF_OUT_UNSIGNED>(tbase, par_off, dst_off, a.BN, lane);
+                    else s2d_drain<CLAMP, FORM>(tbase, par_off, dst_off, a.BN, lane);
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(tempty0 + 8u * group);
@@ -369,11 +366,8 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
                 for (int cb = 0; cb < a.N; cb += 32) {
                     unsigned va[16], vb[16];
                     tc_ld_2x16x256b_x4_wait(tbase + (unsigned)cb, va, vb);
-                    if (a.wide) {
-                        if (a.out_unsigned) perm_block_global<false, EF_WIDE | EF_OUT_UNSIGNED>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
-                        else perm_block_global<false, EF_WIDE>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
-                    } else if (a.out_unsigned) perm_block_global<CLAMP, EF_OUT_UNSIGNED>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
-                    else perm_block_global<CLAMP, 0>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
+                    if (a.out_unsigned) perm_block_global<CLAMP, FORM | EF_OUT_UNSIGNED>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
+                    else perm_block_global<CLAMP, FORM>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane);
                 }
                 // the accumulator is drained: hand it back
                 tc_fence_before();
@@ -610,14 +604,13 @@ cudaError_t launch_stem_s2d(const StemS2dPlan& plan, const ConvGeom& g, int n_ba
     a.fq = fast.fq;
     a.cpad = fast.cpad;
     a.out_unsigned = fast.out_unsigned;
-    a.wide = fast.wide ? 1 : 0;
     typedef void (*Kernel)(const CUtensorMap, const S2dArgs);
-    static const Kernel variants[12] = {stem_s2d_tcgen05_kernel<false, 0, false>, stem_s2d_tcgen05_kernel<false, 1, false>,
-                                        stem_s2d_tcgen05_kernel<false, 2, false>, stem_s2d_tcgen05_kernel<true, 0, false>,
-                                        stem_s2d_tcgen05_kernel<true, 1, false>,  stem_s2d_tcgen05_kernel<true, 2, false>,
-                                        stem_s2d_tcgen05_kernel<false, 0, true>,  stem_s2d_tcgen05_kernel<false, 1, true>,
-                                        stem_s2d_tcgen05_kernel<false, 2, true>,  stem_s2d_tcgen05_kernel<true, 0, true>,
-                                        stem_s2d_tcgen05_kernel<true, 1, true>,   stem_s2d_tcgen05_kernel<true, 2, true>};
+#define N2D2B_S2D(C, F) stem_s2d_tcgen05_kernel<C, 0, false, F>, stem_s2d_tcgen05_kernel<C, 1, false, F>, \
+                        stem_s2d_tcgen05_kernel<C, 2, false, F>, stem_s2d_tcgen05_kernel<C, 0, true, F>,  \
+                        stem_s2d_tcgen05_kernel<C, 1, true, F>,  stem_s2d_tcgen05_kernel<C, 2, true, F>
+    static const Kernel variants[30] = {N2D2B_S2D(false, 0), N2D2B_S2D(true, 0), N2D2B_S2D(false, EF_FLOAT), N2D2B_S2D(true, EF_FLOAT),
+                                        N2D2B_S2D(false, EF_WIDE)};   // the wide form has no clamps
+#undef N2D2B_S2D
     static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
     int dev = 0;
     cudaGetDevice(&dev);
@@ -631,7 +624,7 @@ cudaError_t launch_stem_s2d(const StemS2dPlan& plan, const ConvGeom& g, int n_ba
     const long long items = (long long)a.B * a.bands;
     const int grid = (int)(items < plan.num_sms ? items : plan.num_sms);
     const int shape = (plan.KH == 4 && plan.KWp == 4) ? 1 : ((plan.KH == 2 && plan.KWp == 2) ? 2 : 0);
-    return launch_pdl(variants[(plan.P ? 6 : 0) + (fast.need_clamp ? 3 : 0) + shape], grid, Z_THREADS, plan.smem_bytes, s, plan.tmA, a);
+    return launch_pdl(variants[(fast.form == EF_WIDE ? 24 : (fast.form == EF_FLOAT ? 12 : 0) + (fast.need_clamp ? 6 : 0)) + (plan.P ? 3 : 0) + shape], grid, Z_THREADS, plan.smem_bytes, s, plan.tmA, a);
 }
 
 }  // namespace n2d2b

@@ -352,6 +352,7 @@ static constexpr int EF_DP_A_SIGNED = 8;    // DP: the packed (t, r) bytes are r
 static constexpr int EF_WIDE = 16;          // first rescale in 64 bits: x * mult + (row 0 : row 3 as a 64-bit addend) >> shift
 static constexpr int EF_DP_XOR = 32;        // DP: some of the packed (t, r) bytes are flipped between unsigned and signed (dp_xor)
 static constexpr int EF_PERM = 64;          // weights stored with permuted output channels (perm_block)
+static constexpr int EF_FLOAT = 256;        // floating-point scaling: row 2 = factor, row 3 = bias, rows 0 and 1 = clamp of the converted value
 static constexpr int EF_W4 = 128;           // the accumulator holds 16 x the sum (packed 4-bit weights, see expand_int4_x16)
 
 // NG 8-column groups (NG = 4: 32 columns, NG = 2: 16) of a warp's 32 accumulator rows in the fragment layout
@@ -382,6 +383,37 @@ __device__ __forceinline__ void frag_rowbase(unsigned* rb, int wb, int lane)
         const unsigned xm = ((ro >> 7) & (unsigned)(wb / 16 - 1)) << 4;
         rb[k] = ro + ((unsigned)tc ^ xm);
     }
+}
+
+// Floating-point scaling of an integer value: the float product rounded half away from zero, as roundf does.  The sum with
+// +-0.5 rounds toward zero, so it never crosses an integer that the exact sum does not reach (a rounded-to-nearest sum
+// turns 0.5 - 2^-25 into 1), and its truncation is the wanted integer for every float.  Values outside 32 bits
+// saturate in the conversion, values outside 8 bits in the pack that follows.
+__device__ __forceinline__ int float_round_scaled(float f, float factor)
+{
+    const float v = __fmul_rn(f, factor);
+    return __float2int_rz(__fadd_rz(v, copysignf(0.5f, v)));
+}
+
+// One value through the rescale a cell's constants describe (see build_fast_quant, build_wide_quant and
+// build_float_quant for what the five rows hold in each form).
+template <bool CLAMP, int EF>
+__device__ __forceinline__ int rescale(int x, int lo, int hi, int mult, int add, int shift)
+{
+    if (EF & EF_FLOAT) {
+        float f = __int2float_rn(x + add);
+        if (CLAMP) f = fminf(fmaxf(f, __int_as_float(lo)), __int_as_float(hi));
+        return float_round_scaled(f, __int_as_float(mult));
+    }
+    if (CLAMP) x = min(max(x, lo), hi);
+    if (EF & EF_WIDE) {
+        // fixed-point scalings with many fractional bits: the product needs more than 32 bits, the shifted result does not
+        // (proved on the host, as is shift <= 31: the low word of the shifted pair is one funnel shift); no clamps in this
+        // form, the pack saturates
+        const long long p = (long long)x * mult + (long long)(((unsigned long long)(unsigned)lo << 32) | (unsigned)add);
+        return (int)__funnelshift_r((unsigned)p, (unsigned)((unsigned long long)p >> 32), (unsigned)shift);
+    }
+    return (x * mult + add) >> shift;
 }
 
 template <int NG, bool RES, bool CLAMP, bool DP, int EF>
@@ -437,23 +469,8 @@ __device__ __forceinline__ void frag_block(const unsigned* vA, const unsigned* v
 #pragma unroll
         for (int k = 0; k < NK; ++k) {   // rows tr + 8k
             const unsigned* v = (k < 2) ? vA : vB;
-            int x0 = (int)v[4 * i + 2 * (k & 1)], x1 = (int)v[4 * i + 2 * (k & 1) + 1];
-            if (CLAMP) {
-                x0 = min(max(x0, lo.x), hi.x);
-                x1 = min(max(x1, lo.y), hi.y);
-            }
-            int y0, y1;
-            if (EF & EF_WIDE) {
-                // fixed-point scalings with many fractional bits: the product needs more than 32 bits, the
-                // shifted result does not (proved on the host); no clamps in this form, the pack saturates
-                const long long p0 = (long long)x0 * mu.x + (long long)(((unsigned long long)(unsigned)lo.x << 32) | (unsigned)ad.x);
-                const long long p1 = (long long)x1 * mu.y + (long long)(((unsigned long long)(unsigned)lo.y << 32) | (unsigned)ad.y);
-                y0 = (int)(p0 >> sh.x);
-                y1 = (int)(p1 >> sh.y);
-            } else {
-                y0 = (x0 * mu.x + ad.x) >> sh.x;
-                y1 = (x1 * mu.y + ad.y) >> sh.y;
-            }
+            int y0 = rescale<CLAMP, EF>((int)v[4 * i + 2 * (k & 1)], lo.x, hi.x, mu.x, ad.x, sh.x);
+            int y1 = rescale<CLAMP, EF>((int)v[4 * i + 2 * (k & 1) + 1], lo.y, hi.y, mu.y, ad.y, sh.y);
             if (RES && DP) {
                 const unsigned rw = rres[i][k];   // two residual bytes, replaced below
                 unsigned a4;
@@ -481,14 +498,8 @@ __device__ __forceinline__ void frag_block(const unsigned* vA, const unsigned* v
                     r0 = byte_extend(rw, 0, false);
                     r1 = byte_extend(rw, 1, false);
                 }
-                int u0 = min(max(y0, t_lo), t_hi) + r0;
-                int u1 = min(max(y1, t_lo), t_hi) + r1;
-                if (CLAMP) {
-                    u0 = min(max(u0, lo2.x), hi2.x);
-                    u1 = min(max(u1, lo2.y), hi2.y);
-                }
-                y0 = (u0 * mu2.x + ad2.x) >> sh2.x;
-                y1 = (u1 * mu2.y + ad2.y) >> sh2.y;
+                y0 = rescale<CLAMP, EF & ~EF_WIDE>(min(max(y0, t_lo), t_hi) + r0, lo2.x, hi2.x, mu2.x, ad2.x, sh2.x);
+                y1 = rescale<CLAMP, EF & ~EF_WIDE>(min(max(y1, t_lo), t_hi) + r1, lo2.y, hi2.y, mu2.y, ad2.y, sh2.y);
             }
             unsigned d;
             // the third operand fills the upper half of d, which the 16-bit store drops: any live register will do
@@ -599,13 +610,7 @@ __device__ __forceinline__ void perm_block(const unsigned* vA, const unsigned* v
                 // thread channel 4h + c = 2i + e  ->  group i = 2h + c / 2, element e = c % 2
                 int x = (int)v[4 * (2 * h + (c >> 1)) + 2 * (k & 1) + (c & 1)];
                 if (EF & EF_W4) x >>= 4;   // a multiple of 16: exact
-                if (CLAMP) x = min(max(x, lov[c]), hiv[c]);
-                if (EF & EF_WIDE) {
-                    const long long p = (long long)x * muv[c] + (long long)(((unsigned long long)(unsigned)lov[c] << 32) | (unsigned)adv[c]);
-                    y[c] = (int)(p >> shv[c]);
-                } else {
-                    y[c] = (x * muv[c] + adv[c]) >> shv[c];
-                }
+                y[c] = rescale<CLAMP, EF>(x, lov[c], hiv[c], muv[c], adv[c], shv[c]);
             }
             if (RES && DP) {
                 // [t, t', r, r'] per column pair: the saturating pack of the cell's own output also places the two
@@ -636,9 +641,7 @@ __device__ __forceinline__ void perm_block(const unsigned* vA, const unsigned* v
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const int r = byte_extend(rw, c, (EF & EF_RES_UNSIGNED) != 0);
-                    int u = min(max(y[c], t_lo), t_hi) + r;
-                    if (CLAMP) u = min(max(u, lo2v[c]), hi2v[c]);
-                    y[c] = (u * mu2v[c] + ad2v[c]) >> sh2v[c];
+                    y[c] = rescale<CLAMP, EF & ~EF_WIDE>(min(max(y[c], t_lo), t_hi) + r, lo2v[c], hi2v[c], mu2v[c], ad2v[c], sh2v[c]);
                 }
             }
             outw[k][h] = pack4_sat(y[0], y[1], y[2], y[3], (EF & EF_OUT_UNSIGNED) != 0);
@@ -685,14 +688,7 @@ __device__ __forceinline__ void perm_block_global(const unsigned* vA, const unsi
             int y[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                int x = (int)v[4 * (2 * h + (c >> 1)) + 2 * (k & 1) + (c & 1)];
-                if (CLAMP) x = min(max(x, lov[c]), hiv[c]);
-                if (EF & EF_WIDE) {
-                    const long long p = (long long)x * muv[c] + (long long)(((unsigned long long)(unsigned)lov[c] << 32) | (unsigned)adv[c]);
-                    y[c] = (int)(p >> shv[c]);
-                } else {
-                    y[c] = (x * muv[c] + adv[c]) >> shv[c];
-                }
+                y[c] = rescale<CLAMP, EF>((int)v[4 * (2 * h + (c >> 1)) + 2 * (k & 1) + (c & 1)], lov[c], hiv[c], muv[c], adv[c], shv[c]);
             }
             outw[k][h] = pack4_sat(y[0], y[1], y[2], y[3], (EF & EF_OUT_UNSIGNED) != 0);
         }
@@ -797,18 +793,24 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
         const unsigned tbase = e.tmem_acc + ((unsigned)(quad * 32) << 16) + (unsigned)cbase;
         // one branch per tile selects the arithmetic variant; inside, nothing depends on a run-time flag
         if (!RES) {
-            switch (e.ef & (EF_OUT_UNSIGNED | EF_WIDE)) {
+            switch (e.ef & (EF_OUT_UNSIGNED | EF_WIDE | EF_FLOAT)) {
             case 0: epi_drain<RES, CLAMP, DP, (0) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_OUT_UNSIGNED: epi_drain<RES, CLAMP, DP, (EF_OUT_UNSIGNED) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_WIDE: epi_drain<RES, false, DP, (EF_WIDE) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_FLOAT: epi_drain<RES, CLAMP, DP, (EF_FLOAT) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_FLOAT | EF_OUT_UNSIGNED: epi_drain<RES, CLAMP, DP, (EF_FLOAT | EF_OUT_UNSIGNED) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             default: epi_drain<RES, false, DP, (EF_WIDE | EF_OUT_UNSIGNED) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             }
         } else if (!DP) {
-            switch (e.ef & (EF_OUT_UNSIGNED | EF_RES_UNSIGNED | EF_WIDE)) {
+            switch (e.ef & (EF_OUT_UNSIGNED | EF_RES_UNSIGNED | EF_WIDE | EF_FLOAT)) {
             case 0: epi_drain<RES, CLAMP, DP, (0) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case 1: epi_drain<RES, CLAMP, DP, (1) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case 2: epi_drain<RES, CLAMP, DP, (2) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case 3: epi_drain<RES, CLAMP, DP, (3) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_FLOAT | 0: epi_drain<RES, CLAMP, DP, (EF_FLOAT | 0) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_FLOAT | 1: epi_drain<RES, CLAMP, DP, (EF_FLOAT | 1) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_FLOAT | 2: epi_drain<RES, CLAMP, DP, (EF_FLOAT | 2) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_FLOAT | 3: epi_drain<RES, CLAMP, DP, (EF_FLOAT | 3) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_WIDE | 0: epi_drain<RES, false, DP, (EF_WIDE | 0) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_WIDE | 1: epi_drain<RES, false, DP, (EF_WIDE | 1) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_WIDE | 2: epi_drain<RES, false, DP, (EF_WIDE | 2) | P>(e, tbase, cbase, region_off, st.rb, lane); break;

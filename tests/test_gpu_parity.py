@@ -687,3 +687,34 @@ def test_networks_with_two_bit_and_one_bit_weights():
         net = netdesc.resnet18(size=32, classes=10, weight_bits=bits, scaling='double')
         n, eng = compare_net(net, 3, flags=0)
         assert 'fused' in eng
+
+
+# (C, H, O, k, stride, pad, flags, wanted engine): every kernel with the 32-bit-width epilogue, at tile edges and remainders
+FLOAT_CASES = [
+    (3, 37, 64, 7, 2, 3, 0, 'stem-tcgen05'), (4, 19, 32, 3, 1, 1, 0, 'stem-tcgen05'), (64, 13, 64, 3, 1, 1, 0, 'patch-tcgen05'),
+    (128, 9, 96, 3, 1, 1, 0, 'patch-tcgen05'), (64, 11, 256, 1, 1, 0, 0, 'tcgen05'), (256, 7, 72, 3, 2, 1, 0, 'tcgen05'),
+    (512, 15, 512, 1, 1, 0, R.FORCE_PAIR, 'tcgen05-pair'),
+]
+
+
+@pytest.mark.parametrize('case', FLOAT_CASES, ids=lambda c: 'C%d_%d_O%d_k%d_s%d' % c[:5])
+@pytest.mark.parametrize('form', ['plain', 'clipped', 'clipped_below', 'ties', 'signed_relu'])
+def test_floating_point_scaling_in_the_fused_epilogues(case, form):
+    C, H, O, k, s, p, flags, engine = case
+    net = single_conv_net(C, H, H, O, k, s, p, act='relu' if form == 'signed_relu' else 'linear', mode='float',
+                          unsigned_relu=form != 'signed_relu', seed=31)
+    q = net['layers'][0]['quant']
+    rng = np.random.default_rng(3)
+    if form == 'ties':        # powers of two: many products end in exactly one half
+        q['fscale'] = np.full(O, 2.0 ** np.floor(np.log2(q['fscale'].mean())), np.float32)
+    if form.startswith('clipped'):
+        q['is_clipped'] = True
+        q['clip'] = (rng.uniform(0.3, 2.0, O) * 40.0 / q['fscale'] * (-1 if form == 'clipped_below' else 1)).astype(np.float32)
+    compare_net(net, 3, flags=KEEP | flags, want_engine=engine)
+
+
+@pytest.mark.parametrize('unsigned', [True, False])
+@pytest.mark.parametrize('pack', [8, 4])
+def test_floating_point_scaling_with_fused_residual_sums(unsigned, pack):
+    net = netdesc.resnet18(size=64, classes=100, scaling='float', weight_bits=pack, unsigned_relu=unsigned, width=32)
+    compare_net(net, 3, flags=0)
