@@ -47,6 +47,11 @@ cudaError_t launch_pool(const void* in, int in_unsigned, const PoolGeom& g, void
 cudaError_t launch_pool_i32(const void* in, const PoolGeom& g, void* out, cudaStream_t s);
 cudaError_t launch_elemwise_sum(const SumInputs& ins, size_t pixels, int C, const QuantDev& q,
                                 void* out, int out_dtype, cudaStream_t s);
+// Stand-alone rescale of int32 [pixels][C] to 8 bits.  words: host constants, [5][C] of the 32-bit form (form 0, with valid
+// clamps) or the floating-point form (1), or [7][C] bias, p0, p1, fscale, clip_thr, clip_val, clip_f (form 2, exact 64-bit);
+// q: the scalar fields of QuantDev (its pointers are not used)
+cudaError_t launch_rescale_i32(const int32_t* in, void* out, size_t pixels, int C, int form, const int32_t* words, const QuantDev& q,
+                               cudaStream_t s);
 // Top-1 class per pixel (first maximum wins) of [pixels][C] scores; values may be nullptr.
 // [rows][ld] bytes -> [rows][C] bytes (C <= ld): drops the zero columns a padded cell computed
 cudaError_t launch_drop_padded_columns(const uint8_t* src, int ld, uint8_t* dst, int C, size_t rows, cudaStream_t s);

@@ -238,11 +238,11 @@ static void quant_output_type(const QuantHost& q, int* dtype, int* is_unsigned)
     }
 }
 
-static int upload_quant(QuantHost& q)
+// The exact form's per-channel words [7][C]
+static std::vector<int32_t> exact_words(const QuantHost& q)
 {
     const int C = q.nb_channels;
-    const size_t words = (size_t)C * 7;
-    std::vector<int32_t> blob(words);
+    std::vector<int32_t> blob((size_t)C * 7);
     memcpy(&blob[0 * C], q.bias.data(), C * 4);
     memcpy(&blob[1 * C], q.p0.data(), C * 4);
     memcpy(&blob[2 * C], q.p1.data(), C * 4);
@@ -250,10 +250,12 @@ static int upload_quant(QuantHost& q)
     memcpy(&blob[4 * C], q.clip_thr.data(), C * 4);
     memcpy(&blob[5 * C], q.clip_val.data(), C * 4);
     memcpy(&blob[6 * C], q.clip_f.data(), C * 4);
-    CUDA_TRY(cudaMalloc(&q.d_blob, words * 4 + 16));
-    CUDA_TRY(cudaMemcpy(q.d_blob, blob.data(), words * 4, cudaMemcpyHostToDevice));
-    int32_t* d = (int32_t*)q.d_blob;
-    QuantDev& v = q.dev;
+    return blob;
+}
+
+// The scalar fields of the device view
+static void fill_quant_scalars(const QuantHost& q, QuantDev& v)
+{
     v.mode = q.mode;
     v.act = q.act;
     v.saturate = (q.mode != SC_NONE) ? 1 : 0;
@@ -261,6 +263,17 @@ static int upload_quant(QuantHost& q)
     else { v.out_lo = -(1 << (q.out_bits - 1)); v.out_hi = (1 << (q.out_bits - 1)) - 1; }
     v.is_clipped = q.is_clipped;
     v.sat_thr = q.sat_thr;
+}
+
+static int upload_quant(QuantHost& q)
+{
+    const int C = q.nb_channels;
+    const std::vector<int32_t> blob = exact_words(q);
+    CUDA_TRY(cudaMalloc(&q.d_blob, blob.size() * 4 + 16));
+    CUDA_TRY(cudaMemcpy(q.d_blob, blob.data(), blob.size() * 4, cudaMemcpyHostToDevice));
+    int32_t* d = (int32_t*)q.d_blob;
+    QuantDev& v = q.dev;
+    fill_quant_scalars(q, v);
     v.bias = q.has_bias ? d + 0 * C : nullptr;
     v.p0 = d + 1 * C;
     v.p1 = d + 2 * C;
@@ -379,6 +392,9 @@ static bool build_fast_quant(const QuantHost& q, int cpad, long long x_bound, st
             H = ceil_div((out_hi << s) - half, m);
             L = ceil_div(((out_lo + 1) << s) - half, m) - 1;
         }
+        // a threshold is met exactly only if the rescale of the bound gives it (a scale above 1 can step over it; the
+        // native 8-bit bounds are the final pack's)
+        if (q.act == ACT_SATURATION && m > 0 && (((H * m + half) >> s) > out_hi || ((L * m + half) >> s) < out_lo)) return false;
         if (q.is_clipped) {
             if (!(q.clip_f[c] > 0.0f)) return false;
             L = std::max(L, 0ll);
@@ -1725,14 +1741,22 @@ int n2d2b_scaling_propagate(int device, const int32_t* d_in, void* d_out, size_t
     CUDA_TRY(cudaSetDevice(device));
     QuantHost q;
     if (int rc = validate_quant(quant, quant->scaling.nb_channels, false, q, nullptr)) return rc;
-    if (int rc = upload_quant(q)) return rc;
-    SumInputs ins{};
-    ins.n = 1;
-    ins.ptr[0] = d_in;
-    ins.dtype[0] = DT_I32;
-    cudaError_t e = launch_elemwise_sum(ins, nb_pixels, q.nb_channels, q.dev, d_out, DT_I8, (cudaStream_t)stream);
+    // the 32-bit or floating-point form where it is proved exact for every 32-bit input, the 64-bit one otherwise
+    std::vector<int32_t> words;
+    int form = 0, lo = 0, hi = 0;
+    bool need_clamp = false;
+    const long long any32 = (1ll << 31) - 1;
+    if (!build_fast_quant(q, q.nb_channels, any32, words, &lo, &hi, &need_clamp)) {
+        form = 1;
+        if (!build_float_quant(q, q.nb_channels, any32, words, &need_clamp)) {
+            form = 2;
+            words = exact_words(q);
+        }
+    }
+    QuantDev scalars{};
+    fill_quant_scalars(q, scalars);
+    cudaError_t e = launch_rescale_i32(d_in, d_out, nb_pixels, q.nb_channels, form, words.data(), scalars, (cudaStream_t)stream);
     cudaError_t e2 = cudaStreamSynchronize((cudaStream_t)stream);
-    cudaFree(q.d_blob);
     if (e != cudaSuccess) return fail(N2D2B_ERR_CUDA, "scaling kernel launch failed: %s", cudaGetErrorString(e));
     if (e2 != cudaSuccess) return fail(N2D2B_ERR_CUDA, "scaling kernel failed: %s", cudaGetErrorString(e2));
     return 0;

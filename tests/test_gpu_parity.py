@@ -718,3 +718,33 @@ def test_floating_point_scaling_in_the_fused_epilogues(case, form):
 def test_floating_point_scaling_with_fused_residual_sums(unsigned, pack):
     net = netdesc.resnet18(size=64, classes=100, scaling='float', weight_bits=pack, unsigned_relu=unsigned, width=32)
     compare_net(net, 3, flags=0)
+
+
+@pytest.mark.parametrize('shape', [(1, 1, 1, 1), (5, 1, 24, 24), (3, 3, 31, 33), (2, 3, 64, 64), (2, 4, 17, 19), (1, 12, 5, 7), (2, 16, 6, 5)],
+                         ids=lambda s: '%dx%dx%dx%d' % s)
+def test_stimuli_quantization_shapes(shape):
+    import torch
+    x = np.random.default_rng(5).uniform(-0.1, 1.1, shape).astype(np.float32)
+    d_in = torch.from_numpy(x).cuda()
+    d_out = torch.full(shape, 77, dtype=torch.uint8, device='cuda')
+    runtime.quantize_stimuli(d_in.data_ptr(), *shape, d_out.data_ptr(), 8, True)
+    want = np.clip(np.trunc(x * np.float32(255.0)), 0, 255).astype(np.uint8).transpose(0, 2, 3, 1)
+    assert np.array_equal(d_out.cpu().numpy().reshape(want.shape), want)
+
+
+# few levels: large groups of equal scores, so queues fill blocks of 32 classes, turn while partly filled and wrap around
+@pytest.mark.parametrize('classes,top_n', [(2, 2), (31, 31), (32, 7), (33, 33), (65, 40), (257, 200), (1000, 300)])
+@pytest.mark.parametrize('levels', [1, 2, 6])
+def test_top_n_with_large_groups_of_equal_scores(classes, top_n, levels):
+    rng = np.random.default_rng(classes + levels)
+    B = 5
+    scores = rng.integers(0, levels, (B, 1, 1, classes)).astype(np.int64) - levels // 2
+    want_l, want_v = oracle.estimated_labels_topn(scores.reshape(B, classes), top_n)
+    qn = runtime.QuantizedNet(_identity_scores_net(classes, 1, 1), B)
+    try:
+        qn.forward_host(scores.astype(np.int8))
+        got_l, got_v = qn.estimated_labels_topn_host(B, top_n)
+        assert np.array_equal(got_v.reshape(B, top_n), want_v)
+        assert np.array_equal(got_l.reshape(B, top_n), want_l)
+    finally:
+        qn.close()

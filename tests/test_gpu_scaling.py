@@ -45,3 +45,30 @@ def test_scaling_known_answers_on_gpu():
         q = dict(q, out_bits=8, out_unsigned=unsigned, act='linear')
         x = np.array(xs).reshape(len(xs), 1, 1, 1)
         assert _gpu_scaling(x, q).reshape(-1).tolist() == want
+
+
+# channel counts whose constants repeat over 1, 2 or 4 pixels, the limits of one launch, several launches; odd pixel counts
+@pytest.mark.parametrize('channels,pixels', [(1, 7), (3, 1001), (37, 23), (128, 5000), (150, 33), (150, 64), (1000, 9), (1024, 3),
+                                             (1025, 5), (2048, 17), (2500, 2)])
+@pytest.mark.parametrize('mode', ['single', 'double', 'fixed32', 'fixed_exact', 'float', 'float_clipped', 'saturation'])
+def test_scaling_shapes_and_forms(channels, pixels, mode):
+    from oracle import oracle
+    rng = np.random.default_rng(channels * 31 + pixels)
+    q = {'mode': mode.split('_')[0], 'act': 'relu', 'out_bits': 8, 'out_unsigned': True}
+    if mode in ('single', 'saturation'):
+        q.update(mode='single', shift0=rng.integers(0, 12, channels).astype(np.uint8))
+    elif mode == 'double':
+        q.update(shift0=rng.integers(1, 5, channels).astype(np.uint8), shift1=rng.integers(8, 15, channels).astype(np.uint8))
+    elif mode.startswith('fixed'):
+        # 2^23: the 32-bit form; 2^30: products only the 64-bit one holds
+        q.update(mode='fixed32', mult=rng.integers(1 << 14, 1 << 15, channels).astype(np.int32), frac_bits=23 if mode == 'fixed32' else 30)
+    else:
+        q['fscale'] = (rng.uniform(0.5, 2.0, channels) / 300.0).astype(np.float32)
+        if mode == 'float_clipped':
+            q.update(is_clipped=True, clip=(rng.uniform(-1.0, 3.0, channels) * 20000.0).astype(np.float32), act='linear', out_unsigned=False)
+    if mode == 'saturation':
+        q.update(act='saturation', sat_thr=5, out_unsigned=False)
+    x = np.rint(rng.normal(0.0, 20000.0, (1, channels, 1, pixels)) * rng.choice([1.0, 1.0, 1e4], (1, channels, 1, pixels)))
+    x.reshape(-1)[:3] = [-2.0 ** 31, 2.0 ** 31 - 1, 0][:x.size]
+    x = x.astype(np.int64)
+    assert np.array_equal(_gpu_scaling(x, q), np.asarray(oracle.scaling(x, q, 'i64')).astype(np.int64))
