@@ -3,7 +3,7 @@
 //   D[M x N] (int32, in TMEM) = A[M x K] (u8 or s8 activations, NHWC) * B[N x K]^T (s8 weights, OHWI)
 //   M = output pixels (batch * oH * oW), N = output channels, K = taps * Cin walked tap by tap.
 //
-// One persistent CTA per SM loops over 128 x BN output tiles.  Warp 0 issues TMA loads into a
+// One persistent CTA per SM loops over 128 x BN output tiles.  Three warps issue TMA loads into a
 // multi-stage shared-memory ring (A tile through a 2-D tiled map for a plain GEMM, or through an
 // im2col map that applies stride / padding / dilation and zero-fills the halo; B tile through a 2-D
 // map, or once into a resident block when the layer's weights are small), warp 1 issues
@@ -17,9 +17,9 @@
 // (src/Cell/ConvCell_Frame_CUDA.cpp:1169-1270) and its cublasGemm FC
 // (src/Cell/FcCell_Frame_CUDA.cpp:308-427).
 //
-// The kernel is launched with programmatic stream serialization: barriers, TMEM, constants and
-// resident weights are set up while the previous kernel drains; activations are touched only after
-// griddepcontrol.wait.
+// The kernel is launched with programmatic stream serialization: barriers, TMEM, constants, tensor maps,
+// resident weights and the first ring fill of streamed ones are set up while the previous kernel drains;
+// activations are touched only after griddepcontrol.wait.
 //
 // Every wait on an mbarrier is bounded: a wait that does not complete within about a second sets
 // *status_word and makes the whole CTA drain and exit, so a wrong descriptor cannot hang the GPU.
@@ -35,8 +35,12 @@ static constexpr int BM = 128;
 static constexpr int EPI_WARP0 = 2;
 static constexpr int NUM_EPI_WARPS = 16;      // four per TMEM lane quadrant, a quarter of the columns each
 static constexpr int REGION_BYTES = 2048;     // staging per epilogue warp: 32 rows x up to 64 bytes
-static constexpr int NUM_THREADS = 32 * (EPI_WARP0 + NUM_EPI_WARPS);
+static constexpr int NUM_PRODUCERS = 3;       // warps that issue TMA loads: warp 0 and the last two of the CTA
+static constexpr int NUM_THREADS = 32 * (EPI_WARP0 + NUM_EPI_WARPS + NUM_PRODUCERS - 1);
 static constexpr int W4_UNPACK_WARPS = 4;     // extra warps of the packed-int4 variant
+
+// A number of output pixels as (columns, rows, images)
+struct PixelStep { int x, y, n; };
 
 struct IgemmArgs {
     int M, N, Cin, taps, BK, BN, stages, a_im2col;
@@ -46,6 +50,7 @@ struct IgemmArgs {
     int b_resident;     // the CTA's whole weight block stays in shared memory (its column block never changes)
     int oW, oH, kW, sX, sY, pL, pT, dX, dY;
     int num_m_tiles, num_n_tiles;
+    PixelStep adv_tiles, adv_one;   // the step in m (step_m tiles or tile pairs) and one 128-row tile, in pixel coordinates
     int step_m, step_n;   // gridDim.x / num_n_tiles and gridDim.x % num_n_tiles: one persistent-loop step in tile coordinates
     int ef;               // EF_* switches of the 32-bit epilogue
     unsigned idesc;
@@ -63,6 +68,26 @@ struct IgemmArgs {
     int out_unsigned;   // final 8-bit range: 1 = [0,255], 0 = [-128,127]
     unsigned dp_xor;    // dot-product form of the residual stage: byte flips and operand signedness
     int dp_a_signed;
+};
+
+// Position of an output pixel in its image batch, walked without divisions
+struct PixelPos {
+    int ox, oy, n;
+    __device__ __forceinline__ void start(const IgemmArgs& a, int m)
+    {
+        const int t = m / a.oW;
+        ox = m - t * a.oW;
+        n = t / a.oH;
+        oy = t - n * a.oH;
+    }
+    __device__ __forceinline__ void advance(const IgemmArgs& a, const PixelStep& d)
+    {
+        ox += d.x;
+        oy += d.y;
+        n += d.n;
+        if (ox >= a.oW) { ox -= a.oW; ++oy; }
+        if (oy >= a.oH) { oy -= a.oH; ++n; }
+    }
 };
 
 // ----------------------------------------------------------------------------- the kernel
@@ -123,25 +148,28 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     // [2 buffers][2 quant sets][FAST_NP][256], 16-byte aligned for vector loads
     int* epi_params = (int*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
+    // the producer this warp is, or -1
+    constexpr int LAST_PRODUCERS = EPI_WARP0 + NUM_EPI_WARPS + (W4 ? W4_UNPACK_WARPS : 0);
+    const int producer = warp == 0 ? 0 : (warp >= LAST_PRODUCERS ? warp - LAST_PRODUCERS + 1 : -1);
     pdl_launch_dependents();
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < a.stages; ++s) {
-            mbar_init(full0 + 8u * s, 1);
-            mbar_init(empty0 + 8u * s, 1);
+    if (warp == 0) {
+        // one barrier per lane and pass: 80 of them in turn on one thread delayed the whole CTA
+        const int nb = 2 * a.stages + 6 + 4 * NUM_EPI_WARPS + 1;
+        for (int i = lane; i < nb; i += 32) {
+            const int j = i - (2 * a.stages + 2);   // tmem_empty[2] and params_ready[2] collect the epilogue warps
+            mbar_init(full0 + 8u * i, j >= 0 && j < 4 ? NUM_EPI_WARPS : (i == nb - 1 ? NUM_PRODUCERS : 1));   // the last one: resident weights
         }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(tfull0 + 8u * s, 1);
-            mbar_init(tempty0 + 8u * s, NUM_EPI_WARPS);
-            mbar_init(pready0 + 8u * s, NUM_EPI_WARPS);
+        if (W4 && lane < a.stages) mbar_init(bready0 + 8u * lane, W4_UNPACK_WARPS);
+        if (lane == 0) {
+            *abort_flag = 0;
+            prefetch_tensor_map(&tmA);
+            prefetch_tensor_map(&tmB);
+            if (FAST) prefetch_tensor_map(&tmO);
+            if (RES) prefetch_tensor_map(&tmR);
         }
-        for (int w = 0; w < 4 * NUM_EPI_WARPS; ++w) mbar_init(rbar0 + 8u * w, 1);
-        mbar_init(bfull, 1);
-        if (W4)
-            for (int s = 0; s < a.stages; ++s) mbar_init(bready0 + 8u * s, W4_UNPACK_WARPS);
-        *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -157,114 +185,146 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 
     const int num_tiles = a.num_m_tiles * a.num_n_tiles;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            unsigned it = 0;
-            bool ok = true;
-            if (a.b_resident && (int)blockIdx.x < num_tiles) {
-                // the launch keeps every CTA on one column block: its weights are fetched once
-                const int n0 = ((int)blockIdx.x % a.num_n_tiles) * a.BN;
-                mbar_expect_tx(bfull, (unsigned)(num_kb * b_stage_bytes));
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    const int tap = kb / kchunks;
-                    const int kc = kb - tap * kchunks;
-                    tma_load_2d(smem_u32(res_b + (size_t)kb * b_stage_bytes), &tmB, bfull, tap * a.Cin + kc * a.BK, n0);
+    if (producer >= 0) {
+        // ------------------------------------------------------------------ TMA producers
+        // A ring slot costs its producer 300-500 cycles (a wait, an expect_tx, one or two loads and the counters around
+        // them, in one warp's instruction latencies), a K block of the tensor pipe 200 (64 columns) to 512 (256): with
+        // one producer the loads, not the bandwidth behind them, bounded every streamed layer.  Three take every third
+        // ring fill each - never more producers than slots: a producer may be one phase of a slot's barrier ahead, which
+        // its own previous fill guarantees as long as that lies at most a whole ring back, and two phases ahead look like
+        // none to a parity wait.  Whatever does not depend on the previous kernel's output - the coordinates of the first tile, the first fill
+        // of streamed weights - comes before the wait: cold parameters and divisions cost 0.7 us there.
+        bool ok = true;
+        const int first = (int)blockIdx.x;
+        int m_tile = first / a.num_n_tiles, n_tile = first - m_tile * a.num_n_tiles;
+        int m0 = a.m_base + m_tile * BM, n0 = n_tile * a.BN;
+        PixelPos px;
+        px.start(a, m0);
+        int iw0 = px.ox * a.sX - a.pL, ih0 = px.oy * a.sY - a.pT, in0 = px.n;
+        const int takers = a.stages < NUM_PRODUCERS ? a.stages : NUM_PRODUCERS;
+        const int my_turn = producer < takers ? producer : 0x40000000;   // ring fills until this producer's first one (never, if idle)
+        unsigned pre = 0;   // ring fills whose weights are issued before the wait
+        if (first < num_tiles) {
+            if (!a.b_resident) pre = (unsigned)(num_kb < a.stages ? num_kb : a.stages);
+            const int nload = a.b_resident ? num_kb : (int)pre;
+            if (elect_one()) {
+                // resident: the launch keeps every CTA on one column block, its weights are fetched once.  Streamed: the
+                // first fill of the ring needs nothing of the previous kernel either.
+                int own = 0;
+                if (a.b_resident) {
+                    for (int i = my_turn; i < num_kb; i += takers) own += b_stage_bytes;
+                    mbar_expect_tx(bfull, (unsigned)own);
                 }
-            }
-            pdl_wait();   // weights are constants; the activations are the previous kernel's output
-            // The loops below keep ring slot, phase, tap and channel-chunk as running counters: a single
-            // thread pays the full latency of every dependent instruction, so an integer division per K
-            // block costs more than the load it prepares.
-            int s = 0;
-            unsigned ph = 0;
-            int m_tile = (int)blockIdx.x / a.num_n_tiles, n_tile = (int)blockIdx.x % a.num_n_tiles;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const int m0 = a.m_base + m_tile * BM, n0 = n_tile * a.BN;
-                m_tile += a.step_m;
-                n_tile += a.step_n;
-                if (n_tile >= a.num_n_tiles) { n_tile -= a.num_n_tiles; ++m_tile; }
-                int iw0 = 0, ih0 = 0, in0 = 0;
-                if (a.a_im2col) {
-                    const int ox = m0 % a.oW;
-                    const int t = m0 / a.oW;
-                    const int oy = t % a.oH;
-                    in0 = t / a.oH;
-                    iw0 = ox * a.sX - a.pL;
-                    ih0 = oy * a.sY - a.pT;
-                }
-                int kx = 0, ky = 0, kc = 0, kcoord = 0;   // kcoord = tap * Cin + kc * BK
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    if (!mbar_wait(empty0 + 8u * s, ph ^ 1u, abort_flag, a.status, 1)) { ok = false; break; }
-                    const unsigned bar = full0 + 8u * s;
-                    const unsigned dstA = tiles_s + (unsigned)(s * stage_bytes);
-                    mbar_expect_tx(bar, (unsigned)tx_bytes);
-                    if (a.a_im2col) {
-                        tma_load_im2col_4d(dstA, &tmA, bar, kc * a.BK + (a.grouped ? n0 : 0), iw0, ih0, in0,
-                                           (unsigned short)(kx * a.dX), (unsigned short)(ky * a.dY));
-                    } else {
-                        tma_load_2d(dstA, &tmA, bar, kcoord, m0);
+                int kc = 0, kcoord = 0, turn = my_turn;
+                for (int i = 0; i < nload; ++i) {
+                    if (turn == 0) {
+                        turn = takers;
+                        if (a.b_resident) {
+                            tma_load_2d(res_b_s + (unsigned)(i * b_stage_bytes), &tmB, bfull, kcoord, n0);
+                        } else {
+                            const unsigned bar = full0 + 8u * i, dst = tiles_s + (unsigned)(i * stage_bytes + a_stage_bytes);
+                            mbar_expect_tx(bar, (unsigned)tx_bytes);
+                            if (W4) tma_load_2d(dst + b_stage_bytes, &tmB, bar, kcoord >> 1, n0);   // packed: two per byte
+                            else tma_load_2d(dst, &tmB, bar, kcoord, n0);
+                        }
                     }
-                    if (W4) tma_load_2d(dstA + a_stage_bytes + b_stage_bytes, &tmB, bar, kcoord >> 1, n0);   // packed: two per byte
-                    else if (!a.b_resident) tma_load_2d(dstA + a_stage_bytes, &tmB, bar, kcoord, n0);
-                    if (++s == a.stages) { s = 0; ph ^= 1u; }
+                    --turn;
                     if (++kc == kchunks) {
                         kc = 0;
                         kcoord += a.Cin - (kchunks - 1) * a.BK;
-                        if (++kx == a.kW) { kx = 0; ++ky; }
                     } else {
                         kcoord += a.BK;
                     }
                 }
             }
+            __syncwarp();
+        }
+        pdl_wait();   // weights are constants; the activations are the previous kernel's output
+        const bool im2col = a.a_im2col != 0, load_b = !a.b_resident;
+        const unsigned ring_end = full0 + 8u * a.stages, to_empty = 8u * a.stages;
+        unsigned bar = full0, dst = tiles_s, ph = 1u, it = 0;
+        int turn = my_turn;    // ring fills until this producer's next one
+        for (int tile = first; tile < num_tiles && ok; tile += gridDim.x) {
+            int kx = 0, ky = 0, kc = 0, kcoord = 0;   // kcoord = tap * Cin + kc * BK
+            const int c0 = a.grouped ? n0 : 0;
+            for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                if (turn == 0) {
+                    turn = takers;
+                    if (!mbar_wait_issuer(bar + to_empty, ph, abort_flag, a.status, 1)) { ok = false; break; }
+                    if (elect_one()) {
+                        const bool weights = it >= pre;   // else they are on their way
+                        if (weights) mbar_expect_tx(bar, (unsigned)tx_bytes);
+                        if (im2col) tma_load_im2col_4d(dst, &tmA, bar, kc * a.BK + c0, iw0, ih0, in0, (unsigned short)(kx * a.dX), (unsigned short)(ky * a.dY));
+                        else tma_load_2d(dst, &tmA, bar, kcoord, m0);
+                        if (weights && load_b) {
+                            if (W4) tma_load_2d(dst + (unsigned)(a_stage_bytes + b_stage_bytes), &tmB, bar, kcoord >> 1, n0);
+                            else tma_load_2d(dst + (unsigned)a_stage_bytes, &tmB, bar, kcoord, n0);
+                        }
+                    }
+                    __syncwarp();
+                }
+                --turn;
+                bar += 8u;
+                dst += (unsigned)stage_bytes;
+                if (bar == ring_end) { bar = full0; dst = tiles_s; ph ^= 1u; }
+                if (++kc == kchunks) {
+                    kc = 0;
+                    kcoord += a.Cin - (kchunks - 1) * a.BK;
+                    if (++kx == a.kW) { kx = 0; ++ky; }
+                } else {
+                    kcoord += a.BK;
+                }
+            }
+            m_tile += a.step_m;
+            n_tile += a.step_n;
+            px.advance(a, a.adv_tiles);
+            if (n_tile >= a.num_n_tiles) { n_tile -= a.num_n_tiles; ++m_tile; px.advance(a, a.adv_one); }
+            m0 = a.m_base + m_tile * BM;
+            n0 = n_tile * a.BN;
+            iw0 = px.ox * a.sX - a.pL;
+            ih0 = px.oy * a.sY - a.pT;
+            in0 = px.n;
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        // The issuing thread pays the latency of every instruction it executes, so what surrounds a short
-        // MMA is kept to 32-bit adds on running descriptor words and an unrolled K loop.
-        if (lane == 0) {
-            unsigned acc_it = 0;
-            bool ok = true;
-            if (a.b_resident && (int)blockIdx.x < num_tiles) ok = mbar_wait(bfull, 0, abort_flag, a.status, 8);
-            int s = 0;
-            unsigned ph = 0;
-            // upper descriptor word: stride between 8-row groups, version, swizzle; lower word: address / 16
-            const unsigned desc_hi = (unsigned)(make_smem_desc(0u, a.BK) >> 32);
-            const unsigned a_lo0 = (tiles_s & 0x3ffffu) >> 4, b_res0 = (res_b_s & 0x3ffffu) >> 4;
-            const unsigned stage16 = (unsigned)(stage_bytes >> 4), a16 = (unsigned)(a_stage_bytes >> 4);
-            const unsigned b16 = (unsigned)(b_stage_bytes >> 4);
-            unsigned a_lo = a_lo0;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++acc_it) {
-                const unsigned as = acc_it & 1u;
-                const unsigned aph = (acc_it >> 1) & 1u;
-                if (!mbar_wait(tempty0 + 8u * as, aph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
+        unsigned acc_it = 0;
+        bool ok = true;
+        if (a.b_resident && (int)blockIdx.x < num_tiles) ok = mbar_wait_issuer(bfull, 0, abort_flag, a.status, 8);
+        int s = 0;
+        unsigned ph = 0;
+        // upper descriptor word: stride between 8-row groups, version, swizzle; lower word: address / 16
+        const unsigned desc_hi = (unsigned)(make_smem_desc(0u, a.BK) >> 32);
+        const unsigned a_lo0 = (tiles_s & 0x3ffffu) >> 4, b_res0 = (res_b_s & 0x3ffffu) >> 4;
+        const unsigned stage16 = (unsigned)(stage_bytes >> 4), a16 = (unsigned)(a_stage_bytes >> 4);
+        const unsigned b16 = (unsigned)(b_stage_bytes >> 4);
+        unsigned a_lo = a_lo0;
+        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++acc_it) {
+            const unsigned as = acc_it & 1u;
+            const unsigned aph = (acc_it >> 1) & 1u;
+            if (!mbar_wait_issuer(tempty0 + 8u * as, aph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
+            const unsigned d_tmem = tmem_base + as * (unsigned)a.BN;
+            unsigned b_res = b_res0;
+            for (int kb = 0; kb < num_kb; ++kb) {
+                if (!mbar_wait_issuer(full0 + 8u * s, ph, abort_flag, a.status, 3)) { ok = false; break; }
+                if (W4 && !mbar_wait_issuer(bready0 + 8u * s, ph, abort_flag, a.status, 11)) { ok = false; break; }
                 tc_fence_after();
-                const unsigned d_tmem = tmem_base + as * (unsigned)a.BN;
-                unsigned b_res = b_res0;
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(full0 + 8u * s, ph, abort_flag, a.status, 3)) { ok = false; break; }
-                    if (W4 && !mbar_wait(bready0 + 8u * s, ph, abort_flag, a.status, 11)) { ok = false; break; }
-                    tc_fence_after();
-                    const unsigned b_lo = a.b_resident ? b_res : a_lo + a16;
-                    const unsigned acc = kb ? 1u : 0u;
+                const unsigned al = a_lo, b_lo = a.b_resident ? b_res : a_lo + a16;
+                const unsigned acc = kb ? 1u : 0u, ebar = empty0 + 8u * s;
+                a_lo += stage16;
+                b_res += b16;
+                if (++s == a.stages) { s = 0; ph ^= 1u; a_lo = a_lo0; }
+                if (elect_one()) {
                     // advancing K by 32 bytes inside the swizzle span = +2 in the 16-byte address field
+                    tc_mma_i8_lohi(d_tmem, al, b_lo, desc_hi, a.idesc, acc);
+                    if (a.BK >= 64) tc_mma_i8_lohi(d_tmem, al + 2u, b_lo + 2u, desc_hi, a.idesc, 1u);
                     if (a.BK == 128) {
-                        tc_mma_i8_lohi(d_tmem, a_lo, b_lo, desc_hi, a.idesc, acc);
-                        tc_mma_i8_lohi(d_tmem, a_lo + 2u, b_lo + 2u, desc_hi, a.idesc, 1u);
-                        tc_mma_i8_lohi(d_tmem, a_lo + 4u, b_lo + 4u, desc_hi, a.idesc, 1u);
-                        tc_mma_i8_lohi(d_tmem, a_lo + 6u, b_lo + 6u, desc_hi, a.idesc, 1u);
-                    } else if (a.BK == 64) {
-                        tc_mma_i8_lohi(d_tmem, a_lo, b_lo, desc_hi, a.idesc, acc);
-                        tc_mma_i8_lohi(d_tmem, a_lo + 2u, b_lo + 2u, desc_hi, a.idesc, 1u);
-                    } else {
-                        tc_mma_i8_lohi(d_tmem, a_lo, b_lo, desc_hi, a.idesc, acc);
+                        tc_mma_i8_lohi(d_tmem, al + 4u, b_lo + 4u, desc_hi, a.idesc, 1u);
+                        tc_mma_i8_lohi(d_tmem, al + 6u, b_lo + 6u, desc_hi, a.idesc, 1u);
                     }
-                    tc_commit(empty0 + 8u * s);  // frees the stage once these MMAs have read it
-                    a_lo += stage16;
-                    b_res += b16;
-                    if (++s == a.stages) { s = 0; ph ^= 1u; a_lo = a_lo0; }
+                    tc_commit(ebar);  // frees the stage once these MMAs have read it
+                    if (kb + 1 == num_kb) tc_commit(tfull0 + 8u * as);
                 }
-                if (ok) tc_commit(tfull0 + 8u * as);
+                __syncwarp();
             }
         }
     } else if (W4 && warp >= EPI_WARP0 + NUM_EPI_WARPS) {
@@ -300,7 +360,6 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         }
     } else {
         // ------------------------------------------------------------------ epilogue warps
-        pdl_wait();   // residual loads and output stores touch tensors the previous kernel reads or writes
         const int quad = warp & 3;                       // TMEM lane quadrant this warp may read
         const int part = (warp - EPI_WARP0) >> 2;        // 0..3 within the quadrant: a quarter of the columns (32-bit epilogue)
         const int row = quad * 32 + lane;
@@ -314,6 +373,28 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         int staged_n_tile = -1;
         int* par = epi_params;
         bool ok = true;
+        const int bn_shift = 31 - __clz(a.BN);
+        // Stages a column block's per-channel constants (once per CTA when the grid is a multiple of the number of column
+        // blocks).  Two buffers: the other one may still be read by slower warps, this one is free once everybody
+        // passed the previous barrier.
+        auto stage_constants = [&](int n_tile) -> bool {
+            par = epi_params + (size_t)(stage_it & 1u) * (2 * FAST_NP * 256);
+            const int per_set = FAST_NP << bn_shift, all = a.fq2 ? 2 * per_set : per_set;
+            for (int i = epi_tid; i < all; i += 32 * NUM_EPI_WARPS) {
+                const int set = i >= per_set ? 1 : 0;
+                const int prm = (i - set * per_set) >> bn_shift, c = i & (a.BN - 1);
+                par[(set * FAST_NP + prm) * 256 + c] = __ldg((set ? a.fq2 : a.fq) + (size_t)prm * a.cpad + n_tile * a.BN + c);
+            }
+            const unsigned pb = pready0 + 8u * (stage_it & 1u);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(pb);
+            if (!mbar_wait_warp(pb, (stage_it >> 1) & 1u, abort_flag, a.status, 5, lane)) return false;
+            staged_n_tile = n_tile;
+            ++stage_it;
+            return true;
+        };
+        if (FAST && (int)blockIdx.x < num_tiles) ok = stage_constants((int)blockIdx.x % a.num_n_tiles);   // constants: before the wait
+        pdl_wait();   // residual loads and output stores touch tensors the previous kernel reads or writes
         int m_next = (int)blockIdx.x / a.num_n_tiles, n_next = (int)blockIdx.x % a.num_n_tiles;
         // residual loads run ahead of the tiles: pf_* walk the same tile sequence, res_slots - 1 tiles in front
         int pf_tile = blockIdx.x, pf_m = m_next, pf_n = n_next;
@@ -330,29 +411,10 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             const int m0 = a.m_base + m_tile * BM, n0 = n_tile * a.BN;
             const unsigned as = acc_it & 1u;
             const unsigned aph = (acc_it >> 1) & 1u;
-            if (FAST && n_tile != staged_n_tile) {
-                // stage this column block's per-channel constants (once per CTA when the grid is a
-                // multiple of the number of column blocks).  Two buffers: the other one may still be
-                // read by slower warps, this one is free once everybody passed the previous barrier.
-                par = epi_params + (size_t)(stage_it & 1u) * (2 * FAST_NP * 256);
-                const int nq = a.fq2 ? 2 : 1;
-                for (int i = epi_tid; i < nq * FAST_NP * a.BN; i += 32 * NUM_EPI_WARPS) {
-                    const int set = i / (FAST_NP * a.BN);
-                    const int rem = i - set * FAST_NP * a.BN;
-                    const int prm = rem / a.BN, c = rem - prm * a.BN;
-                    const int* src = set ? a.fq2 : a.fq;
-                    par[(set * FAST_NP + prm) * 256 + c] = __ldg(src + (size_t)prm * a.cpad + n0 + c);
-                }
-                const unsigned pb = pready0 + 8u * (stage_it & 1u);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(pb);
-                if (!mbar_wait_warp(pb, (stage_it >> 1) & 1u, abort_flag, a.status, 5, lane)) { ok = false; break; }
-                staged_n_tile = n_tile;
-                ++stage_it;
-            }
+            if (FAST && n_tile != staged_n_tile)
+                if (!stage_constants(n_tile)) { ok = false; break; }
             const int m = m0 + row;
             const bool m_ok = m < a.m_base + a.M;
-            const int nchunks = cols_per_warp / 32;
             const int cbase = part * cols_per_warp;
             if (FAST) {
                 // fragment-layout epilogue with swizzled staging, TMA store and TMA residual load
@@ -441,8 +503,8 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty0 + 8u * as);
         }
-        // no bulk store may still be reading this CTA's shared memory when it exits
-        if (FAST && lane == 0) bulk_wait_all();
+        // no bulk store may still be reading this CTA's shared memory when it exits (its writes complete with the grid)
+        if (FAST && lane == 0) bulk_wait_read_all();
     }
 
     tc_fence_before();
@@ -462,6 +524,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 // 32-bit epilogue only; the staging regions are 1 KB (32 rows x 32 columns, two passes per warp) to make
 // room for three 64 KB stages.
 static constexpr int PAIR_STAGES = 3;
+static_assert(NUM_PRODUCERS <= PAIR_STAGES, "a producer may be at most one ring ahead of the issuer (see the producers above)");
 static constexpr int PAIR_REGION = 1024;
 
 template <bool CLAMP>
@@ -485,8 +548,9 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     int* par = (int*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);   // [FAST_NP][256]
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
+    const int producer = warp == 0 ? 0 : (warp >= EPI_WARP0 + NUM_EPI_WARPS ? warp - (EPI_WARP0 + NUM_EPI_WARPS) + 1 : -1);
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < PAIR_STAGES; ++s) {
@@ -516,99 +580,133 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
     const int num_kb = a.taps * kchunks;
     const int m_end = a.m_base + a.M;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            pdl_wait();
-            int s = 0;
-            unsigned ph = 0;
-            bool ok = true;
-            int m_pair = (int)blockIdx.x / a.num_n_tiles, n_tile = (int)blockIdx.x % a.num_n_tiles;
-            for (int pt = blockIdx.x; pt < num_pt && ok; pt += gridDim.x) {
-                const int n0 = n_tile * 256;
-                int m0[2], iw0[2] = {0, 0}, ih0[2] = {0, 0}, in0[2] = {0, 0};
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    m0[h] = a.m_base + (2 * m_pair + h) * BM;
-                    if (a.a_im2col) {
-                        const int ox = m0[h] % a.oW;
-                        const int t = m0[h] / a.oW;
-                        const int oy = t % a.oH;
-                        in0[h] = t / a.oH;
-                        iw0[h] = ox * a.sX - a.pL;
-                        ih0[h] = oy * a.sY - a.pT;
-                    }
+    if (producer >= 0) {
+        // ------------------------------------------------------------------ TMA producers (as in the kernel above)
+        bool ok = true;
+        int m_pair = (int)blockIdx.x / a.num_n_tiles, n_tile = (int)blockIdx.x - m_pair * a.num_n_tiles;
+        int m0 = a.m_base + 2 * m_pair * BM, n0 = n_tile * 256;
+        PixelPos px;
+        px.start(a, m0);
+        const unsigned tiles_s = smem_u32(tiles);
+        unsigned pre = 0;
+        if ((int)blockIdx.x < num_pt) {
+            pre = (unsigned)(num_kb < PAIR_STAGES ? num_kb : PAIR_STAGES);
+            if (elect_one()) {
+                if (producer == 0) {
+                    prefetch_tensor_map(&tmA);
+                    prefetch_tensor_map(&tmO32);
                 }
-                m_pair += a.step_m;
-                n_tile += a.step_n;
-                if (n_tile >= a.num_n_tiles) { n_tile -= a.num_n_tiles; ++m_pair; }
-                int kx = 0, ky = 0, kc = 0, kcoord = 0;
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(empty0 + 8u * s, ph ^ 1u, abort_flag, a.status, 1)) { ok = false; break; }
-                    const unsigned bar = full0 + 8u * s;
-                    const unsigned dst = smem_u32(tiles) + (unsigned)(s * STAGE_BYTES);
-                    mbar_expect_tx(bar, (unsigned)STAGE_BYTES);
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        if (a.a_im2col)
-                            tma_load_im2col_4d(dst + h * A_BYTES, &tmA, bar, kc * 128, iw0[h], ih0[h], in0[h],
-                                               (unsigned short)(kx * a.dX), (unsigned short)(ky * a.dY));
-                        else
-                            tma_load_2d(dst + h * A_BYTES, &tmA, bar, kcoord, m0[h]);
+                int kc = 0, kcoord = 0, turn = producer;
+                for (unsigned i = 0; i < pre; ++i) {
+                    if (turn == 0) {
+                        turn = NUM_PRODUCERS;
+                        mbar_expect_tx(full0 + 8u * i, (unsigned)STAGE_BYTES);
+                        tma_load_2d(tiles_s + i * (unsigned)STAGE_BYTES + 2u * A_BYTES, &tmB, full0 + 8u * i, kcoord, n0);
                     }
-                    tma_load_2d(dst + 2 * A_BYTES, &tmB, bar, kcoord, n0);
-                    if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; }
+                    --turn;
                     if (++kc == kchunks) {
                         kc = 0;
                         kcoord += a.Cin - (kchunks - 1) * 128;
-                        if (++kx == a.kW) { kx = 0; ++ky; }
                     } else {
                         kcoord += 128;
                     }
                 }
             }
+            __syncwarp();
+        }
+        pdl_wait();
+        const bool im2col = a.a_im2col != 0;
+        unsigned bar = full0, dst = tiles_s, ph = 1u, it = 0;
+        int turn = producer;
+        for (int pt = blockIdx.x; pt < num_pt && ok; pt += gridDim.x) {
+            PixelPos p2 = px;
+            p2.advance(a, a.adv_one);
+            const int iw0 = px.ox * a.sX - a.pL, ih0 = px.oy * a.sY - a.pT, in0 = px.n;
+            const int iw1 = p2.ox * a.sX - a.pL, ih1 = p2.oy * a.sY - a.pT, in1 = p2.n;
+            int kx = 0, ky = 0, kc = 0, kcoord = 0;
+            for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                if (turn == 0) {
+                    turn = NUM_PRODUCERS;
+                    if (!mbar_wait_issuer(bar + 8u * PAIR_STAGES, ph, abort_flag, a.status, 1)) { ok = false; break; }
+                    if (elect_one()) {
+                        const bool weights = it >= pre;
+                        if (weights) mbar_expect_tx(bar, (unsigned)STAGE_BYTES);
+                        if (im2col) {
+                            const unsigned short ox = (unsigned short)(kx * a.dX), oy = (unsigned short)(ky * a.dY);
+                            tma_load_im2col_4d(dst, &tmA, bar, kc * 128, iw0, ih0, in0, ox, oy);
+                            tma_load_im2col_4d(dst + A_BYTES, &tmA, bar, kc * 128, iw1, ih1, in1, ox, oy);
+                        } else {
+                            tma_load_2d(dst, &tmA, bar, kcoord, m0);
+                            tma_load_2d(dst + A_BYTES, &tmA, bar, kcoord, m0 + BM);
+                        }
+                        if (weights) tma_load_2d(dst + 2 * A_BYTES, &tmB, bar, kcoord, n0);
+                    }
+                    __syncwarp();
+                }
+                --turn;
+                bar += 8u;
+                dst += (unsigned)STAGE_BYTES;
+                if (bar == full0 + 8u * PAIR_STAGES) { bar = full0; dst = tiles_s; ph ^= 1u; }
+                if (++kc == kchunks) {
+                    kc = 0;
+                    kcoord += a.Cin - (kchunks - 1) * 128;
+                    if (++kx == a.kW) { kx = 0; ++ky; }
+                } else {
+                    kcoord += 128;
+                }
+            }
+            m_pair += a.step_m;
+            n_tile += a.step_n;
+            px.advance(a, a.adv_tiles);
+            if (n_tile >= a.num_n_tiles) {
+                n_tile -= a.num_n_tiles;
+                ++m_pair;
+                px.advance(a, a.adv_one);
+                px.advance(a, a.adv_one);
+            }
+            m0 = a.m_base + 2 * m_pair * BM;
+            n0 = n_tile * 256;
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const unsigned desc_hi = (unsigned)(make_smem_desc(0u, 128) >> 32);
-            const unsigned t_lo0 = (smem_u32(tiles) & 0x3ffffu) >> 4;
-            const unsigned stage16 = (unsigned)(STAGE_BYTES >> 4), a16 = (unsigned)(A_BYTES >> 4);
-            int s = 0;
-            unsigned ph = 0, pit = 0, a_lo = t_lo0;
-            bool ok = true;
-            for (int pt = blockIdx.x; pt < num_pt && ok; pt += gridDim.x, ++pit) {
-                const unsigned aph = pit & 1u;
-                if (!mbar_wait(tempty0, aph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
-                if (!mbar_wait(tempty0 + 8u, aph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
+        const unsigned desc_hi = (unsigned)(make_smem_desc(0u, 128) >> 32);
+        const unsigned t_lo0 = (smem_u32(tiles) & 0x3ffffu) >> 4;
+        const unsigned stage16 = (unsigned)(STAGE_BYTES >> 4), a16 = (unsigned)(A_BYTES >> 4);
+        int s = 0;
+        unsigned ph = 0, pit = 0, a_lo = t_lo0;
+        bool ok = true;
+        for (int pt = blockIdx.x; pt < num_pt && ok; pt += gridDim.x, ++pit) {
+            const unsigned aph = pit & 1u;
+            if (!mbar_wait_issuer(tempty0, aph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
+            if (!mbar_wait_issuer(tempty0 + 8u, aph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
+            for (int kb = 0; kb < num_kb; ++kb) {
+                if (!mbar_wait_issuer(full0 + 8u * s, ph, abort_flag, a.status, 3)) { ok = false; break; }
                 tc_fence_after();
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(full0 + 8u * s, ph, abort_flag, a.status, 3)) { ok = false; break; }
-                    tc_fence_after();
-                    const unsigned b_lo = a_lo + 2u * a16;
-                    const unsigned acc = kb ? 1u : 0u;
+                const unsigned al0 = a_lo, b_lo = a_lo + 2u * a16;
+                const unsigned acc = kb ? 1u : 0u, ebar = empty0 + 8u * s;
+                a_lo += stage16;
+                if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; a_lo = t_lo0; }
+                if (elect_one()) {
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const unsigned d_tmem = tmem_base + (unsigned)(h * 256);
-                        const unsigned al = a_lo + (unsigned)h * a16;
+                        const unsigned al = al0 + (unsigned)h * a16;
                         tc_mma_i8_lohi(d_tmem, al, b_lo, desc_hi, a.idesc, acc);
                         tc_mma_i8_lohi(d_tmem, al + 2u, b_lo + 2u, desc_hi, a.idesc, 1u);
                         tc_mma_i8_lohi(d_tmem, al + 4u, b_lo + 4u, desc_hi, a.idesc, 1u);
                         tc_mma_i8_lohi(d_tmem, al + 6u, b_lo + 6u, desc_hi, a.idesc, 1u);
                     }
-                    tc_commit(empty0 + 8u * s);
-                    a_lo += stage16;
-                    if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; a_lo = t_lo0; }
+                    tc_commit(ebar);
+                    if (kb + 1 == num_kb) {
+                        tc_commit(tfull0);
+                        tc_commit(tfull0 + 8u);
+                    }
                 }
-                if (ok) {
-                    tc_commit(tfull0);
-                    tc_commit(tfull0 + 8u);
-                }
+                __syncwarp();
             }
         }
     } else {
         // ------------------------------------------------------------------ epilogue warps
-        pdl_wait();
         const int ew = warp - EPI_WARP0;
         const int quad = warp & 3;
         const int part = ew >> 2;                        // a quarter of the 256 columns
@@ -627,6 +725,7 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
         __syncwarp();
         if (lane == 0) mbar_arrive(pready);
         bool ok = mbar_wait_warp(pready, 0, abort_flag, a.status, 5, lane);
+        pdl_wait();
         unsigned pit = 0;
         int m_pair = (int)blockIdx.x / a.num_n_tiles;
         const int gx = n0 + cbase;
@@ -682,7 +781,7 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
                 }
             }
         }
-        if (lane == 0) bulk_wait_all();
+        if (lane == 0) bulk_wait_read_all();
     }
 
     tc_fence_before();
@@ -1011,8 +1110,17 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     if (tiles > grid && a.num_n_tiles > 1 && grid > a.num_n_tiles) grid -= grid % a.num_n_tiles;
     // resident weights rely on exactly that (or on one tile per CTA)
     if (a.b_resident && tiles > grid && a.num_n_tiles > 1 && grid % a.num_n_tiles != 0) return cudaErrorInvalidConfiguration;
+    auto pixels = [&](long long m) {
+        PixelStep d;
+        d.x = (int)(m % a.oW);
+        d.y = (int)(m / a.oW % a.oH);
+        d.n = (int)(m / a.oW / a.oH);
+        return d;
+    };
     a.step_m = grid / a.num_n_tiles;
     a.step_n = grid % a.num_n_tiles;
+    a.adv_tiles = pixels((long long)a.step_m * BM);
+    a.adv_one = pixels(BM);
     if (plan.pair && use_fast && !r.ptr) {
         typedef void (*PairKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const IgemmArgs);
         static const PairKernel pair_kernels[2] = {igemm_pair_i8_tcgen05_kernel<false>, igemm_pair_i8_tcgen05_kernel<true>};
@@ -1030,6 +1138,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
         if (pair_tiles <= pgrid || a.num_n_tiles == 1 || pgrid % a.num_n_tiles == 0) {
             a.step_m = pgrid / a.num_n_tiles;
             a.step_n = pgrid % a.num_n_tiles;
+            a.adv_tiles = pixels(2ll * a.step_m * BM);
             return launch_pdl(pair_kernels[fast.need_clamp ? 1 : 0], pgrid, NUM_THREADS, plan.pair_smem_bytes, s, plan.tmA,
                               plan.tmB, plan.tmO32, a);
         }

@@ -64,7 +64,7 @@ struct PatchArgs {
 // short MMA (one of 128 x 64 x 32 takes about 60 cycles of the tensor pipe) would cost more than the MMA.
 template <int KH, int KW, int KS>
 __device__ __forceinline__ void issue_tile(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned desc_hi, unsigned idesc,
-                                           unsigned row_step, unsigned col_step, unsigned btap, unsigned issue)
+                                           unsigned row_step, unsigned col_step, unsigned btap)
 {
 #pragma unroll
     for (int ky = 0; ky < KH; ++ky)
@@ -72,25 +72,24 @@ __device__ __forceinline__ void issue_tile(unsigned d_tmem, unsigned a_lo, unsig
         for (int kx = 0; kx < KW; ++kx)
 #pragma unroll
             for (int k = 0; k < KS; ++k)
-                tc_mma_i8_lohi_p(d_tmem, a_lo + ky * row_step + kx * col_step + 2u * k, b_lo + (ky * KW + kx) * btap + 2u * k,
-                                 desc_hi, idesc, (ky | kx | k) ? 1u : 0u, issue);
+                tc_mma_i8_lohi(d_tmem, a_lo + ky * row_step + kx * col_step + 2u * k, b_lo + (ky * KW + kx) * btap + 2u * k,
+                               desc_hi, idesc, (ky | kx | k) ? 1u : 0u);
 }
 
 // The MMAs of one filter tap of one tile (C / 32 K steps), unrolled for the channel counts the kernel takes
 template <int KS>
-__device__ __forceinline__ void issue_tap_n(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned desc_hi, unsigned idesc, unsigned first,
-                                            unsigned issue)
+__device__ __forceinline__ void issue_tap_n(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned desc_hi, unsigned idesc, unsigned first)
 {
-    tc_mma_i8_lohi_p(d_tmem, a_lo, b_lo, desc_hi, idesc, first, issue);
+    tc_mma_i8_lohi(d_tmem, a_lo, b_lo, desc_hi, idesc, first);
 #pragma unroll
-    for (int k = 1; k < KS; ++k) tc_mma_i8_lohi_p(d_tmem, a_lo + 2u * k, b_lo + 2u * k, desc_hi, idesc, 1u, issue);
+    for (int k = 1; k < KS; ++k) tc_mma_i8_lohi(d_tmem, a_lo + 2u * k, b_lo + 2u * k, desc_hi, idesc, 1u);
 }
 __device__ __forceinline__ void issue_tap(int ksteps, unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned desc_hi, unsigned idesc,
-                                          unsigned first, unsigned issue)
+                                          unsigned first)
 {
-    if (ksteps == 4) issue_tap_n<4>(d_tmem, a_lo, b_lo, desc_hi, idesc, first, issue);
-    else if (ksteps == 2) issue_tap_n<2>(d_tmem, a_lo, b_lo, desc_hi, idesc, first, issue);
-    else issue_tap_n<1>(d_tmem, a_lo, b_lo, desc_hi, idesc, first, issue);
+    if (ksteps == 4) issue_tap_n<4>(d_tmem, a_lo, b_lo, desc_hi, idesc, first);
+    else if (ksteps == 2) issue_tap_n<2>(d_tmem, a_lo, b_lo, desc_hi, idesc, first);
+    else issue_tap_n<1>(d_tmem, a_lo, b_lo, desc_hi, idesc, first);
 }
 
 // SHAPE: 0 = any filter (loops), 1 / 2 / 3 = 3x3 filter with 32 / 64 / 128 channels (unrolled issue).  FORM: EF_WIDE or
@@ -166,7 +165,16 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0 && cta < items) {
-            if (!a.b_stream) {
+            prefetch_tensor_map(&tmA);
+            prefetch_tensor_map(&tmB);
+            unsigned pre = 0, wt = 0;   // ring fills issued before the wait, ring fills so far
+            if (a.b_stream) {
+                pre = (unsigned)(taps < a.bring ? taps : a.bring);
+                for (unsigned t = 0; t < pre; ++t) {
+                    mbar_expect_tx(rfull0 + 8u * t, (unsigned)b_tap_bytes);
+                    tma_load_2d(smem_u32(res_b + (size_t)t * b_tap_bytes), &tmB, rfull0 + 8u * t, (int)t * a.C, ch0);
+                }
+            } else {
                 mbar_expect_tx(bfull, (unsigned)(taps * b_tap_bytes));
                 for (int t = 0; t < taps; ++t)
                     tma_load_2d(smem_u32(res_b + (size_t)t * b_tap_bytes), &tmB, bfull, t * a.C, ch0);
@@ -186,7 +194,11 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                             band * a.R - a.pT, a.n_base + n);
                 if (a.b_stream) {
                     // every item walks all taps once: its weights follow the patch through the ring
-                    for (int t = 0; t < taps && ok; ++t) {
+                    for (int t = 0; t < taps && ok; ++t, ++wt) {
+                        if (wt < pre) {
+                            if (++rs == a.bring) { rs = 0; rph ^= 1u; }
+                            continue;
+                        }
                         if (!mbar_wait(rempty0 + 8u * rs, rph ^ 1u, abort_flag, a.status, 5)) { ok = false; break; }
                         mbar_expect_tx(rfull0 + 8u * rs, (unsigned)b_tap_bytes);
                         tma_load_2d(smem_u32(res_b + (size_t)rs * b_tap_bytes), &tmB, rfull0 + 8u * rs, t * a.C, ch0);
@@ -203,9 +215,8 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         // ------------------------------------------------------------------ MMA issuers
         // Issuing a tile costs one thread about 100 cycles per MMA, the tensor pipe about 60: two threads take
         // alternate tiles (each tile has its own accumulator, so their MMAs are independent).
-        // every lane of the warp runs the loop; `issue` selects the lane whose MMAs and commits take effect
+        // every lane of the warp runs the loop, an elected one issues (see elect_one)
         const unsigned me = (unsigned)__shfl_sync(0xffffffffu, warp - 1, 0);
-        const unsigned issue = lane == 0 ? 1u : 0u;
         if (cta < items) {
             bool ok = a.b_stream ? true : mbar_wait_uniform(bfull, 0, abort_flag, a.status, 8);
             const unsigned desc_hi = (unsigned)(make_smem_desc(0u, a.C) >> 32);
@@ -244,18 +255,24 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                             if (!mbar_wait_uniform(rfull0 + 8u * rs, rph, abort_flag, a.status, 6)) { ok = false; break; }
                             tc_fence_after();
                             const unsigned bt = res_b_lo + (unsigned)rs * btap;
-                            if (mine0) issue_tap(ksteps, d0, ac, bt, desc_hi, a.idesc, first, issue);
-                            if (mine1) issue_tap(ksteps, d1, ac + tile2, bt, desc_hi, a.idesc, first, issue);
+                            if (elect_one()) {
+                                if (mine0) issue_tap(ksteps, d0, ac, bt, desc_hi, a.idesc, first);
+                                if (mine1) issue_tap(ksteps, d1, ac + tile2, bt, desc_hi, a.idesc, first);
+                                tc_commit(rempty0 + 8u * rs);
+                            }
+                            __syncwarp();
                             first = 1u;
-                            tc_commit_p(rempty0 + 8u * rs, issue);
                             if (++rs == a.bring) { rs = 0; rph ^= 1u; }
                         }
                     }
                     if (!ok) break;
-                    if (mine0) tc_commit_p(tfull0 + 8u * slot0, issue);
-                    if (mine1) tc_commit_p(tfull0 + 8u * slot1, issue);
+                    if (elect_one()) {
+                        if (mine0) tc_commit(tfull0 + 8u * slot0);
+                        if (mine1) tc_commit(tfull0 + 8u * slot1);
+                        tc_commit(pempty0 + 8u * pb);
+                    }
+                    __syncwarp();
                     seq += (unsigned)T;
-                    tc_commit_p(pempty0 + 8u * pb, issue);
                     band += step_b;
                     if (band >= a.bands) band -= a.bands;
                     continue;
@@ -269,23 +286,27 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                     // The operand of a tap starts at an arbitrary pixel row.  The swizzle is a function of the
                     // absolute shared-memory address, so the descriptor needs nothing but that address
                     // (measured: with the base-offset field left 0 every start row gives exact results).
-                    if (SHAPE == 1) issue_tile<3, 3, 1>(d_tmem, a_lo, res_b_lo, desc_hi, a.idesc, row_step, col_step, btap, issue);
-                    else if (SHAPE == 2) issue_tile<3, 3, 2>(d_tmem, a_lo, res_b_lo, desc_hi, a.idesc, row_step, col_step, btap, issue);
-                    else if (SHAPE == 3) issue_tile<3, 3, 4>(d_tmem, a_lo, res_b_lo, desc_hi, a.idesc, row_step, col_step, btap, issue);
-                    else {
-                        unsigned ar = a_lo, bt = res_b_lo, first = 0;
-                        for (int ky = 0; ky < a.taps_y; ++ky, ar += row_step) {
-                            unsigned ac = ar;
-                            for (int kx = 0; kx < a.taps_x; ++kx, ac += col_step, bt += btap)
-                                for (int k = 0; k < ksteps; ++k) {
-                                    tc_mma_i8_lohi_p(d_tmem, ac + 2u * k, bt + 2u * k, desc_hi, a.idesc, first, issue);
-                                    first = 1u;
-                                }
+                    if (elect_one()) {
+                        if (SHAPE == 1) issue_tile<3, 3, 1>(d_tmem, a_lo, res_b_lo, desc_hi, a.idesc, row_step, col_step, btap);
+                        else if (SHAPE == 2) issue_tile<3, 3, 2>(d_tmem, a_lo, res_b_lo, desc_hi, a.idesc, row_step, col_step, btap);
+                        else if (SHAPE == 3) issue_tile<3, 3, 4>(d_tmem, a_lo, res_b_lo, desc_hi, a.idesc, row_step, col_step, btap);
+                        else {
+                            unsigned ar = a_lo, bt = res_b_lo, first = 0;
+                            for (int ky = 0; ky < a.taps_y; ++ky, ar += row_step) {
+                                unsigned ac = ar;
+                                for (int kx = 0; kx < a.taps_x; ++kx, ac += col_step, bt += btap)
+                                    for (int k = 0; k < ksteps; ++k) {
+                                        tc_mma_i8_lohi(d_tmem, ac + 2u * k, bt + 2u * k, desc_hi, a.idesc, first);
+                                        first = 1u;
+                                    }
+                            }
                         }
+                        tc_commit(tfull0 + 8u * slot);
                     }
-                    tc_commit_p(tfull0 + 8u * slot, issue);
+                    __syncwarp();
                 }
-                if (ok) tc_commit_p(pempty0 + 8u * pb, issue);   // the patch is free once both issuers' MMAs have read it
+                if (ok && elect_one()) tc_commit(pempty0 + 8u * pb);   // the patch is free once every issuer's MMAs have read it
+                __syncwarp();
                 band += step_b;
                 if (band >= a.bands) band -= a.bands;
             }

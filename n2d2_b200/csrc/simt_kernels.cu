@@ -39,6 +39,8 @@ __global__ void conv_direct_kernel(const uint8_t* __restrict__ in, int in_unsign
                                    const int8_t* __restrict__ w, ConvGeom g, QuantDev q,
                                    Residual r, void* __restrict__ out, size_t total)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const bool vec4 = (g.Cg % 4 == 0);
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -91,9 +93,9 @@ cudaError_t launch_conv_direct(const void* in, int in_unsigned, const int8_t* w,
     const int block = 256;
     const unsigned grid = grid_for(total, block);
     if (out_dtype == DT_I8)
-        conv_direct_kernel<int8_t><<<grid, block, 0, s>>>((const uint8_t*)in, in_unsigned, w, g, q, r, out, total);
+        launch_pdl(conv_direct_kernel<int8_t>, grid, block, 0, s, (const uint8_t*)in, in_unsigned, w, g, q, r, out, total);
     else
-        conv_direct_kernel<int32_t><<<grid, block, 0, s>>>((const uint8_t*)in, in_unsigned, w, g, q, r, out, total);
+        launch_pdl(conv_direct_kernel<int32_t>, grid, block, 0, s, (const uint8_t*)in, in_unsigned, w, g, q, r, out, total);
     return cudaGetLastError();
 }
 
@@ -128,6 +130,8 @@ __global__ void conv_depthwise_kernel(const uint8_t* __restrict__ in, int in_uns
                                       const int8_t* __restrict__ w_hwc, ConvGeom g, QuantDev q,
                                       uint8_t* __restrict__ out, size_t total_vec)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const int cv = g.C / 16;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total_vec;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -187,6 +191,8 @@ __global__ void __launch_bounds__(256)
 conv_depthwise3x3_dp4a_kernel(const uint8_t* __restrict__ in, const int8_t* __restrict__ w_hwc, ConvGeom g,
                               const int* __restrict__ fq, int cpad, uint8_t* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const int cw = g.C / 4;                        // channel words per pixel
     // blockDim.x is a multiple of cw: a thread keeps its channel word over the whole launch.  A thread's four
     // pixels are adjacent, so most of its input words are shared between them (spreading a thread's pixels for
@@ -314,8 +320,8 @@ cudaError_t launch_conv_depthwise(const void* in, int in_unsigned, const int8_t*
         const bool s1 = g.sX == 1 && g.dX == 1;
 #define N2D2B_DW(U, C, O)                                                                                         \
     do {                                                                                                          \
-        if (s1) conv_depthwise3x3_dp4a_kernel<U, C, O, true><<<grid, threads, 0, s>>>(ip, w_hwc, g, fast.fq, fast.cpad, op); \
-        else conv_depthwise3x3_dp4a_kernel<U, C, O, false><<<grid, threads, 0, s>>>(ip, w_hwc, g, fast.fq, fast.cpad, op);   \
+        if (s1) launch_pdl(conv_depthwise3x3_dp4a_kernel<U, C, O, true>, grid, threads, 0, s, ip, w_hwc, g, fast.fq, fast.cpad, op); \
+        else launch_pdl(conv_depthwise3x3_dp4a_kernel<U, C, O, false>, grid, threads, 0, s, ip, w_hwc, g, fast.fq, fast.cpad, op);   \
     } while (0)
         const int v = (in_unsigned ? 4 : 0) | (fast.need_clamp ? 2 : 0) | (fast.out_unsigned ? 1 : 0);
         switch (v) {
@@ -335,7 +341,7 @@ cudaError_t launch_conv_depthwise(const void* in, int in_unsigned, const int8_t*
     const size_t total = (size_t)g.B * g.oH * g.oW * (g.C / 16);
     if (total == 0) return cudaSuccess;
     const int block = 256;
-    conv_depthwise_kernel<<<grid_for(total, block), block, 0, s>>>((const uint8_t*)in, in_unsigned, w_hwc, g, q,
+    launch_pdl(conv_depthwise_kernel, grid_for(total, block), block, 0, s, (const uint8_t*)in, in_unsigned, w_hwc, g, q,
                                                                    (uint8_t*)out, total);
     return cudaGetLastError();
 }
@@ -348,6 +354,8 @@ cudaError_t launch_conv_depthwise(const void* in, int in_unsigned, const int8_t*
 __global__ void pool_vec_kernel(const uint8_t* __restrict__ in, int in_unsigned, PoolGeom g,
                                 uint8_t* __restrict__ out, size_t total_vec)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const int cv = g.C / 16;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total_vec;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -394,6 +402,8 @@ __global__ void pool_vec_kernel(const uint8_t* __restrict__ in, int in_unsigned,
 template <bool UNSIGNED>
 __global__ void pool_max_row_kernel(const uint8_t* __restrict__ in, PoolGeom g, uint8_t* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const int cv = g.C / 16;
     for (int row = blockIdx.x; row < g.B * g.oH; row += gridDim.x) {
         const int b = row / g.oH, oy = row - b * g.oH;
@@ -458,6 +468,8 @@ template <typename ElemT>
 __global__ void pool_scalar_kernel(const void* __restrict__ in, int in_unsigned, PoolGeom g,
                                    void* __restrict__ out, size_t total)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
         const int c = (int)(idx % g.C);
@@ -498,6 +510,8 @@ template <bool UNSIGNED>
 __global__ void pool_global_avg_kernel(const uint8_t* __restrict__ in, int pixels, int C, size_t total_words,
                                        uint8_t* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const int cw = C / 4;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total_words; idx += (size_t)gridDim.x * blockDim.x) {
         const size_t b = idx / cw;
@@ -532,24 +546,24 @@ cudaError_t launch_pool(const void* in, int in_unsigned, const PoolGeom& g, void
         const int items = g.oW * (g.C / 16);
         const int threads = items >= 256 ? 256 : ((items + 31) / 32) * 32;
         const unsigned grid = (unsigned)(rows < (1ll << 20) ? rows : (1ll << 20));
-        if (in_unsigned) pool_max_row_kernel<true><<<grid, threads, 0, s>>>((const uint8_t*)in, g, (uint8_t*)out);
-        else pool_max_row_kernel<false><<<grid, threads, 0, s>>>((const uint8_t*)in, g, (uint8_t*)out);
+        if (in_unsigned) launch_pdl(pool_max_row_kernel<true>, grid, threads, 0, s, (const uint8_t*)in, g, (uint8_t*)out);
+        else launch_pdl(pool_max_row_kernel<false>, grid, threads, 0, s, (const uint8_t*)in, g, (uint8_t*)out);
     } else if (!g.is_max && g.C % 4 == 0 && g.pH == g.H && g.pW == g.W && g.padY == 0 && g.padX == 0 && g.oH == 1 && g.oW == 1
                && g.H * g.W <= 257 && ((uintptr_t)in & 3) == 0 && ((uintptr_t)out & 3) == 0) {
         const size_t total = (size_t)g.B * (g.C / 4);
         if (total == 0) return cudaSuccess;
         if (in_unsigned)
-            pool_global_avg_kernel<true><<<grid_for(total, block), block, 0, s>>>((const uint8_t*)in, g.H * g.W, g.C, total, (uint8_t*)out);
+            launch_pdl(pool_global_avg_kernel<true>, grid_for(total, block), block, 0, s, (const uint8_t*)in, g.H * g.W, g.C, total, (uint8_t*)out);
         else
-            pool_global_avg_kernel<false><<<grid_for(total, block), block, 0, s>>>((const uint8_t*)in, g.H * g.W, g.C, total, (uint8_t*)out);
+            launch_pdl(pool_global_avg_kernel<false>, grid_for(total, block), block, 0, s, (const uint8_t*)in, g.H * g.W, g.C, total, (uint8_t*)out);
     } else if (g.C % 16 == 0) {
         const size_t total = (size_t)g.B * g.oH * g.oW * (g.C / 16);
         if (total == 0) return cudaSuccess;
-        pool_vec_kernel<<<grid_for(total, block), block, 0, s>>>((const uint8_t*)in, in_unsigned, g, (uint8_t*)out, total);
+        launch_pdl(pool_vec_kernel, grid_for(total, block), block, 0, s, (const uint8_t*)in, in_unsigned, g, (uint8_t*)out, total);
     } else {
         const size_t total = (size_t)g.B * g.oH * g.oW * g.C;
         if (total == 0) return cudaSuccess;
-        pool_scalar_kernel<int8_t><<<grid_for(total, block), block, 0, s>>>(in, in_unsigned, g, out, total);
+        launch_pdl(pool_scalar_kernel<int8_t>, grid_for(total, block), block, 0, s, in, in_unsigned, g, out, total);
     }
     return cudaGetLastError();
 }
@@ -558,7 +572,7 @@ cudaError_t launch_pool_i32(const void* in, const PoolGeom& g, void* out, cudaSt
 {
     const size_t total = (size_t)g.B * g.oH * g.oW * g.C;
     if (total == 0) return cudaSuccess;
-    pool_scalar_kernel<int32_t><<<grid_for(total, 256), 256, 0, s>>>(in, 0, g, out, total);
+    launch_pdl(pool_scalar_kernel<int32_t>, grid_for(total, 256), 256, 0, s, in, 0, g, out, total);
     return cudaGetLastError();
 }
 
@@ -569,6 +583,8 @@ cudaError_t launch_pool_i32(const void* in, const PoolGeom& g, void* out, cudaSt
 template <typename OutT>
 __global__ void elemwise_sum_kernel(SumInputs ins, size_t total, int C, QuantDev q, void* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
         const int c = (int)(idx % C);
@@ -587,6 +603,8 @@ __global__ void elemwise_sum2_vec_kernel(const uint8_t* __restrict__ a, int a_un
                                          const uint8_t* __restrict__ b, int b_unsigned, size_t total_vec,
                                          int C, QuantDev q, uint8_t* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total_vec;
          idx += (size_t)gridDim.x * blockDim.x) {
         const uint4 av = *(const uint4*)(a + idx * 16);
@@ -609,13 +627,13 @@ cudaError_t launch_elemwise_sum(const SumInputs& ins, size_t pixels, int C, cons
     const int block = 256;
     if (ins.n == 2 && out_dtype == DT_I8 && ins.dtype[0] == DT_I8 && ins.dtype[1] == DT_I8 && C % 16 == 0
         && !q.bias) {
-        elemwise_sum2_vec_kernel<<<grid_for(total / 16, block), block, 0, s>>>(
+        launch_pdl(elemwise_sum2_vec_kernel, grid_for(total / 16, block), block, 0, s, 
             (const uint8_t*)ins.ptr[0], ins.is_unsigned[0], (const uint8_t*)ins.ptr[1], ins.is_unsigned[1],
             total / 16, C, q, (uint8_t*)out);
     } else if (out_dtype == DT_I8) {
-        elemwise_sum_kernel<int8_t><<<grid_for(total, block), block, 0, s>>>(ins, total, C, q, out);
+        launch_pdl(elemwise_sum_kernel<int8_t>, grid_for(total, block), block, 0, s, ins, total, C, q, out);
     } else {
-        elemwise_sum_kernel<int32_t><<<grid_for(total, block), block, 0, s>>>(ins, total, C, q, out);
+        launch_pdl(elemwise_sum_kernel<int32_t>, grid_for(total, block), block, 0, s, ins, total, C, q, out);
     }
     return cudaGetLastError();
 }
@@ -775,6 +793,8 @@ __global__ void fc_direct_kernel(const uint8_t* __restrict__ in, int in_unsigned
                                  const int8_t* __restrict__ w, int B, int K, int O, QuantDev q,
                                  void* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const int lane = threadIdx.x & 31;
     const size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
     const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -802,9 +822,9 @@ cudaError_t launch_fc_direct(const void* in, int in_unsigned, const int8_t* w, i
     const int block = 256;
     const unsigned grid = grid_for(total * 32, block);
     if (out_dtype == DT_I8)
-        fc_direct_kernel<int8_t><<<grid, block, 0, s>>>((const uint8_t*)in, in_unsigned, w, B, K, O, q, out);
+        launch_pdl(fc_direct_kernel<int8_t>, grid, block, 0, s, (const uint8_t*)in, in_unsigned, w, B, K, O, q, out);
     else
-        fc_direct_kernel<int32_t><<<grid, block, 0, s>>>((const uint8_t*)in, in_unsigned, w, B, K, O, q, out);
+        launch_pdl(fc_direct_kernel<int32_t>, grid, block, 0, s, (const uint8_t*)in, in_unsigned, w, B, K, O, q, out);
     return cudaGetLastError();
 }
 
@@ -817,6 +837,8 @@ cudaError_t launch_fc_direct(const void* in, int in_unsigned, const int8_t* w, i
 template <typename V>
 __global__ void drop_padded_columns_kernel(const V* __restrict__ src, int ld, V* __restrict__ dst, int C, size_t rows)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const size_t total = rows * (size_t)C;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t r = i / (size_t)C;
@@ -832,9 +854,9 @@ cudaError_t launch_drop_padded_columns(const uint8_t* src, int ld, uint8_t* dst,
     const int threads = 256;
     const int blocks = (int)std::min<size_t>((total + threads - 1) / threads, 148 * 8);
     if (vec)
-        drop_padded_columns_kernel<uint2><<<blocks, threads, 0, s>>>((const uint2*)src, ld / 8, (uint2*)dst, C / 8, rows);
+        launch_pdl(drop_padded_columns_kernel<uint2>, blocks, threads, 0, s, (const uint2*)src, ld / 8, (uint2*)dst, C / 8, rows);
     else
-        drop_padded_columns_kernel<uint8_t><<<blocks, threads, 0, s>>>(src, ld, dst, C, rows);
+        launch_pdl(drop_padded_columns_kernel<uint8_t>, blocks, threads, 0, s, src, ld, dst, C, rows);
     return cudaGetLastError();
 }
 
@@ -842,6 +864,8 @@ template <typename T>
 __global__ void argmax_kernel(const T* __restrict__ scores, size_t pixels, int C, int32_t* __restrict__ labels,
                               int32_t* __restrict__ values)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     const int lane = threadIdx.x & 31;
     const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);
     for (size_t p = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < pixels; p += warps) {
@@ -869,9 +893,9 @@ cudaError_t launch_argmax(const void* scores, int dtype, int is_unsigned, size_t
     if (pixels == 0 || C == 0) return cudaSuccess;
     const int block = 256;
     const unsigned grid = grid_for(pixels * 32, block);
-    if (dtype == DT_I32) argmax_kernel<int32_t><<<grid, block, 0, s>>>((const int32_t*)scores, pixels, C, labels, values);
-    else if (is_unsigned) argmax_kernel<uint8_t><<<grid, block, 0, s>>>((const uint8_t*)scores, pixels, C, labels, values);
-    else argmax_kernel<int8_t><<<grid, block, 0, s>>>((const int8_t*)scores, pixels, C, labels, values);
+    if (dtype == DT_I32) launch_pdl(argmax_kernel<int32_t>, grid, block, 0, s, (const int32_t*)scores, pixels, C, labels, values);
+    else if (is_unsigned) launch_pdl(argmax_kernel<uint8_t>, grid, block, 0, s, (const uint8_t*)scores, pixels, C, labels, values);
+    else launch_pdl(argmax_kernel<int8_t>, grid, block, 0, s, (const int8_t*)scores, pixels, C, labels, values);
     return cudaGetLastError();
 }
 
@@ -894,6 +918,8 @@ template <typename T>
 __global__ void topn_kernel(const T* __restrict__ scores, size_t pixels, size_t hw, int C, int topN, int32_t* __restrict__ labels,
                             int32_t* __restrict__ values)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     extern __shared__ int topn_smem[];
     int* val = topn_smem;
     int* ids = val + C;
@@ -1023,7 +1049,7 @@ cudaError_t launch_topn(const void* scores, int dtype, int is_unsigned, size_t p
     do {                                                                                                                \
         cudaError_t e = cudaFuncSetAttribute(topn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
         if (e != cudaSuccess) return e;                                                                                 \
-        topn_kernel<T><<<grid, 32, smem, s>>>((const T*)scores, pixels, hw, C, topN, labels, values);                   \
+        launch_pdl(topn_kernel<T>, grid, 32, smem, s, (const T*)scores, pixels, hw, C, topN, labels, values);                   \
     } while (0)
     if (dtype == DT_I32) N2D2B_TOPN(int32_t);
     else if (is_unsigned) N2D2B_TOPN(uint8_t);

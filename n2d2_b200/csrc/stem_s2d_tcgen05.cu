@@ -69,6 +69,8 @@ struct S2dArgs {
 __global__ void s2d_image_kernel(const uint8_t* __restrict__ in, int C, int H, int W, int Hs, int Ws, int P, int rows,
                                  uint4* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     for (int row = blockIdx.x; row < rows; row += gridDim.x) {
         const int n = row / Hs, Y = row - n * Hs;
         const uint8_t* img = in + (size_t)n * H * W * C;
@@ -226,9 +228,9 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
         }
     } else if (warp < Z_EPI_WARP0) {
         // ------------------------------------------------------------------ MMA issuers (alternate tiles)
-        const unsigned me = (unsigned)(warp - 1);
-        if (lane == 0 && (int)blockIdx.x < items) {
-            bool ok = mbar_wait(bfull, 0, abort_flag, a.status, 8);
+        const unsigned me = (unsigned)__shfl_sync(0xffffffffu, warp - 1, 0);
+        if ((int)blockIdx.x < items) {   // the whole warp runs the loop, an elected lane issues (see elect_one)
+            bool ok = mbar_wait_issuer(bfull, 0, abort_flag, a.status, 8);
             // activations: rows of 16 bytes, next K chunk = next pixel (16 bytes), next 8 rows 128 bytes on
             const unsigned a_hi = noswz_hi(128u);
             const unsigned band_lo = noswz_lo(smem_u32(band0), 16u);
@@ -244,28 +246,32 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
             for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
                 const unsigned pb = it & 1u, ph = (it >> 1) & 1u;
                 const int T = band_tiles(band);
-                if (!mbar_wait(pfull0 + 8u * pb, ph, abort_flag, a.status, 3)) { ok = false; break; }
+                if (!mbar_wait_issuer(pfull0 + 8u * pb, ph, abort_flag, a.status, 3)) { ok = false; break; }
                 tc_fence_after();
                 unsigned a_lo = band_lo + pb * (unsigned)(a.band_alloc >> 4);
                 for (int t = 0; t < T; ++t, ++seq, a_lo += tile_step) {
                     if ((seq & (Z_ISSUERS - 1)) != me) continue;
                     const unsigned slot = seq & (Z_SLOTS - 1), sph = (seq / Z_SLOTS) & 1u;
-                    if (!mbar_wait(tempty0 + 8u * slot, sph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
+                    if (!mbar_wait_issuer(tempty0 + 8u * slot, sph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
                     tc_fence_after();
                     const unsigned d_tmem = tmem_base + slot * (unsigned)a.BN;
-                    if (SHAPE == 1) s2d_issue_tile<4, 2>(d_tmem, a_lo, a_hi, b_lo0, b_hi, a.idesc, row_step, b_row_step);
-                    else if (SHAPE == 2) s2d_issue_tile<2, 1>(d_tmem, a_lo, a_hi, b_lo0, b_hi, a.idesc, row_step, b_row_step);
-                    else {
-                        unsigned ar = a_lo, br = b_lo0, first = 0;
-                        for (int ky = 0; ky < a.KH; ++ky, ar += row_step, br += b_row_step)
-                            for (int j = 0; 2 * j < a.KWp; ++j) {
-                                tc_mma_i8_words(d_tmem, ar + 2u * j, a_hi, br + 16u * j, b_hi, a.idesc, first);
-                                first = 1u;
-                            }
+                    if (elect_one()) {
+                        if (SHAPE == 1) s2d_issue_tile<4, 2>(d_tmem, a_lo, a_hi, b_lo0, b_hi, a.idesc, row_step, b_row_step);
+                        else if (SHAPE == 2) s2d_issue_tile<2, 1>(d_tmem, a_lo, a_hi, b_lo0, b_hi, a.idesc, row_step, b_row_step);
+                        else {
+                            unsigned ar = a_lo, br = b_lo0, first = 0;
+                            for (int ky = 0; ky < a.KH; ++ky, ar += row_step, br += b_row_step)
+                                for (int j = 0; 2 * j < a.KWp; ++j) {
+                                    tc_mma_i8_words(d_tmem, ar + 2u * j, a_hi, br + 16u * j, b_hi, a.idesc, first);
+                                    first = 1u;
+                                }
+                        }
+                        tc_commit(tfull0 + 8u * slot);
                     }
-                    tc_commit(tfull0 + 8u * slot);
+                    __syncwarp();
                 }
-                if (ok) tc_commit(pempty0 + 8u * pb);   // the band is free once the item's MMAs have read it
+                if (ok && elect_one()) tc_commit(pempty0 + 8u * pb);   // the band is free once the item's MMAs have read it
+                __syncwarp();
                 band += step_b;
                 if (band >= a.bands) band -= a.bands;
             }
@@ -490,7 +496,7 @@ cudaError_t launch_s2d_image(const void* in, const ConvGeom& g, int batch, void*
     if (rows == 0) return cudaSuccess;
     const unsigned grid = (unsigned)(rows < (1ll << 20) ? rows : (1ll << 20));
     const int threads = Ws >= 128 ? 128 : ((Ws + 31) / 32) * 32;
-    s2d_image_kernel<<<grid, threads, 0, s>>>((const uint8_t*)in, g.C, g.H, g.W, Hs, Ws, P, (int)rows, (uint4*)out);
+    launch_pdl(s2d_image_kernel, grid, threads, 0, s, (const uint8_t*)in, g.C, g.H, g.W, Hs, Ws, P, (int)rows, (uint4*)out);
     return cudaGetLastError();
 }
 

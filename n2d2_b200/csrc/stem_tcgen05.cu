@@ -51,6 +51,8 @@ static constexpr int PAD_ROWS = 4;
 __global__ void pad_image_kernel(const uint8_t* __restrict__ in, int C, int H, int W, int Hp, int Wp, int pT, int pL,
                                  int rows, uint32_t* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
     for (int row0 = blockIdx.x * PAD_ROWS; row0 < rows; row0 += gridDim.x * PAD_ROWS) {
         const uint8_t* irow[PAD_ROWS];
 #pragma unroll
@@ -99,7 +101,7 @@ cudaError_t launch_pad_image(const void* in, const ConvGeom& g, int batch, void*
     const long long blocks = (rows + PAD_ROWS - 1) / PAD_ROWS;
     const unsigned grid = (unsigned)(blocks < (1ll << 20) ? blocks : (1ll << 20));
     const int threads = Wp >= 256 ? 256 : ((Wp + 31) / 32) * 32;
-    pad_image_kernel<<<grid, threads, 0, s>>>((const uint8_t*)in, g.C, g.H, g.W, Hp, Wp, g.pT, g.pL, (int)rows,
+    launch_pdl(pad_image_kernel, grid, threads, 0, s, (const uint8_t*)in, g.C, g.H, g.W, Hp, Wp, g.pT, g.pL, (int)rows,
                                              (uint32_t*)out);
     return cudaGetLastError();
 }

@@ -18,6 +18,8 @@ static constexpr int FAST_NP = 5;             // words per channel of a fast req
 // activations or writes outputs sits behind that wait, directly or through the kernel's own barriers.
 // pdl_launch_dependents, at the start of a kernel, lets the next one begin that early.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A tensor map is read through a cache of its own; fetching it ahead takes that miss (about half a microsecond) off the first load
+__device__ __forceinline__ void prefetch_tensor_map(const CUtensorMap* tm) { asm volatile("prefetch.tensormap [%0];" ::"l"(tm) : "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... P, typename... A>
@@ -60,6 +62,21 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity)
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
+}
+// How the producer and issuer loops are written.  One warp's instruction latencies, not bandwidth, bound them (measured on one
+// warp, cycles): a wait on a phase that has completed 70-100, a TMA load 50, an MMA of 128 x 64 x 32 that the whole warp
+// predicates 66 against 48 under elect.sync (its own time on the tensor pipe; code under `lane == 0` computes the
+// operands in vector registers and moves them over one by one), a commit 71 / 19.  A ring slot that took a wait, an
+// expect_tx and a load in turn cost 290-320 cycles, 45-57 bytes per clock with 16 KB boxes where the memory side
+// delivers 71 to every SM at once and 114 to one.  So the whole warp runs these loops and one elected lane issues.
+__device__ __forceinline__ bool elect_one()
+{
+    unsigned p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ unsigned long long globaltimer_ns()
 {
@@ -107,6 +124,27 @@ __device__ __forceinline__ bool mbar_wait_uniform(unsigned bar, unsigned parity,
     const unsigned long long t0 = globaltimer_ns();
     while (true) {
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+        if (__any_sync(0xffffffffu, globaltimer_ns() - t0 > WAIT_LIMIT_NS)) {
+            *abort_flag = 1;
+            atomicCAS(status, 0, code);
+            return false;
+        }
+    }
+}
+
+// The same for a warp that issues tensor-core or copy instructions: after a few tight polls it sleeps between polls, so that
+// a long wait leaves the issue slots to the warps that work.
+__device__ __forceinline__ bool mbar_wait_issuer(unsigned bar, unsigned parity, volatile int* abort_flag, int* status, int code)
+{
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const unsigned long long t0 = globaltimer_ns();
+    unsigned rounds = 0;
+    while (true) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (++rounds > 8) __nanosleep(128);
         if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
         if (__any_sync(0xffffffffu, globaltimer_ns() - t0 > WAIT_LIMIT_NS)) {
             *abort_flag = 1;
@@ -185,29 +223,6 @@ __device__ __forceinline__ void tc_mma_i8_lohi(unsigned d_tmem, unsigned a_lo, u
         "setp.ne.b32 p, %5, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}"
         ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
-}
-// Forms for an issuing WARP: every lane runs the loop (uniform control flow lets the compiler keep descriptor
-// words, counters and barrier addresses in uniform registers, where the MMA wants them; a loop under
-// `if (lane == 0)` computes them in vector registers and pays a move per operand per MMA), and `issue`
-// (true on one lane) predicates the instruction itself.
-__device__ __forceinline__ void tc_mma_i8_lohi_p(unsigned d_tmem, unsigned a_lo, unsigned b_lo, unsigned desc_hi, unsigned idesc,
-                                                 unsigned accumulate, unsigned issue)
-{
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-        "mov.b64 da, {%1, %3};\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(issue) : "memory");
-}
-__device__ __forceinline__ void tc_commit_p(unsigned bar, unsigned issue)
-{
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "setp.ne.b32 q, %1, 0;\n\t"
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(issue) : "memory");
 }
 __device__ __forceinline__ void tc_commit(unsigned bar)
 {
