@@ -142,6 +142,9 @@ struct n2d2b_net {
     bool pipe_busy[2] = {false, false};
     cudaStream_t pipe_stream[2] = {nullptr, nullptr};   // the stream each slot's work was queued on
     unsigned pipe_next = 0;
+    // the whole network as one kernel (small chains of convolutions, poolings and fully-connected cells)
+    SmallNetPlan small;
+    void* d_small = nullptr;
 };
 
 static int validate_quant(const n2d2b_quant* qu, int channels, bool accumulators_have_bias, QuantHost& q,
@@ -420,6 +423,19 @@ static bool build_fast_quant(const QuantHost& q, int cpad, long long x_bound, st
     return true;
 }
 
+// The constants of a rescale without a residual, in the first form proved exact for |x| <= x_bound: 0 (32-bit, with valid
+// clamps), EF_FLOAT, EF_WIDE; -1 when only the exact 64-bit evaluation is.
+static int build_rescale(const QuantHost& q, int cpad, long long x_bound, std::vector<int32_t>& words)
+{
+    int lo = 0, hi = 0;
+    bool need_clamp = false;
+    if (build_fast_quant(q, cpad, x_bound, words, &lo, &hi, &need_clamp)) return 0;
+    if (build_float_quant(q, cpad, x_bound, words, &need_clamp)) return EF_FLOAT;
+    const bool integer = q.mode == SC_SINGLE_SHIFT || q.mode == SC_DOUBLE_SHIFT || q.mode == SC_FIXED_MULT16 || q.mode == SC_FIXED_MULT32;
+    if (integer && q.out_bits == 8 && x_bound < (1ll << 30) && build_wide_quant(q, cpad, x_bound, words)) return EF_WIDE;
+    return -1;
+}
+
 // w4: the cell's weights are 4-bit values (|w| <= 8), which tightens the accumulator bound
 static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8 = false, int residual_unsigned = 0,
                        bool w4 = false)
@@ -631,6 +647,7 @@ void n2d2b_net_destroy(n2d2b_net* net)
         cudaFree(c.d_colpad);
     }
     cudaFree(net->d_status);
+    cudaFree(net->d_small);
     cudaFree(net->d_labels_scratch);
     cudaFree(net->d_stage_in);
     cudaFree(net->d_stage_out);
@@ -958,6 +975,48 @@ static int final_tensor_of(const n2d2b_net* net)
     return -1;
 }
 
+// A chain of convolutions, poolings and fully-connected cells whose weights fit one SM's shared memory runs as one kernel
+// (small_net.cu).  The bound on the arithmetic keeps out what the tensor cores do better: 2^20 multiply-accumulates
+// take an SM about 8 us there, and a batch of b images b / 148 times that.
+static int plan_small_net(n2d2b_net* net)
+{
+    if (net->flags & (N2D2B_KEEP_ALL_OUTPUTS | N2D2B_NO_FUSION | N2D2B_FORCE_SIMT | N2D2B_FORCE_IM2COL | N2D2B_EXACT64_EPILOGUE
+                      | N2D2B_FORCE_PAIR))
+        return 0;
+    long long macs = 0, weights = 0;
+    int tensor = 0;
+    for (const CellRec& c : net->cells) {
+        if (c.skipped || c.residual >= 0 || c.inputs.size() != 1 || c.inputs[0] != tensor) return 0;
+        if (c.type != CELL_CONV && c.type != CELL_FC && c.type != CELL_POOL) return 0;
+        if (net->tensors[tensor].dtype != DT_I8 || net->tensors[c.output].dtype != DT_I8) return 0;
+        if (c.type != CELL_POOL) {
+            if (c.geom.groups != 1 || c.geom.dX != 1) return 0;
+            macs += (long long)c.geom.oH * c.geom.oW * c.geom.O * c.geom.kH * c.geom.kW * c.geom.C;
+            weights += (long long)c.weights.size();
+        }
+        if ((long long)net->tensors[c.output].elems() * net->tensors[c.output].C >= (1ll << 32)) return 0;   // exact quotients
+        tensor = c.output;
+    }
+    if (macs > (1 << 20) || weights > 160 * 1024 || net->cells.size() > SMALL_NET_CELLS) return 0;
+    SmallNetPlan p;
+    for (const CellRec& c : net->cells) {
+        const int in_u = net->tensors[c.inputs[0]].is_unsigned, out_u = net->tensors[c.output].is_unsigned;
+        if (c.type == CELL_POOL) {
+            small_net_add_pool(&p, c.pgeom, in_u);
+            continue;
+        }
+        std::vector<int32_t> words;
+        const int form = build_rescale(c.q, c.geom.O, (long long)c.geom.kH * c.geom.kW * c.geom.C * 255ll * 128ll, words);
+        small_net_add_conv(&p, c.geom, in_u, out_u, c.weights.data(), form, words.data(), c.geom.O, c.q.dev);
+    }
+    if (!small_net_finish(&p, (int)net->tensors[tensor].bytes_per_image())) return 0;
+    CUDA_TRY(cudaMalloc(&net->d_small, p.blob.size()));
+    CUDA_TRY(cudaMemcpy(net->d_small, p.blob.data(), p.blob.size(), cudaMemcpyHostToDevice));
+    p.blob.shrink_to_fit();
+    net->small = std::move(p);
+    return 0;
+}
+
 int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
 {
     if (!net) return fail(N2D2B_ERR_INVALID, "net must not be NULL");
@@ -1193,6 +1252,8 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
             }
         }
     }
+    if (int rc = plan_small_net(net)) return rc;
+    if (net->d_small) net->launches = 1;
     CUDA_TRY(cudaMalloc(&net->d_stage_in, net->tensors[0].bytes_per_image() * (size_t)max_batch + 256));
     CUDA_TRY(cudaMalloc(&net->d_stage_out,
                         net->tensors[final_tensor_of(net)].bytes_per_image() * (size_t)max_batch + 256));
@@ -1395,6 +1456,12 @@ static int forward_impl(n2d2b_net* net, const void* d_input, int batch, void* d_
     if (batch == 0) return 0;
     if (!d_input) return fail(N2D2B_ERR_INVALID, "d_input must not be NULL");
     CUDA_TRY(cudaSetDevice(net->device));
+    if (net->d_small && !ms && first_cell == 0) {
+        CUDA_TRY(launch_small_net(net->small, net->d_small, d_input, batch, tensor_ptr(net, final_tensor_of(net), d_input), d_output,
+                                  net->num_sms, s));
+        net->last_input = d_input;
+        return 0;
+    }
     std::vector<cudaEvent_t> ev;
     if (ms) {
         if (nb_cells != (int)net->cells.size())
@@ -1743,16 +1810,9 @@ int n2d2b_scaling_propagate(int device, const int32_t* d_in, void* d_out, size_t
     if (int rc = validate_quant(quant, quant->scaling.nb_channels, false, q, nullptr)) return rc;
     // the 32-bit or floating-point form where it is proved exact for every 32-bit input, the 64-bit one otherwise
     std::vector<int32_t> words;
-    int form = 0, lo = 0, hi = 0;
-    bool need_clamp = false;
-    const long long any32 = (1ll << 31) - 1;
-    if (!build_fast_quant(q, q.nb_channels, any32, words, &lo, &hi, &need_clamp)) {
-        form = 1;
-        if (!build_float_quant(q, q.nb_channels, any32, words, &need_clamp)) {
-            form = 2;
-            words = exact_words(q);
-        }
-    }
+    const int proved = build_rescale(q, q.nb_channels, (1ll << 31) - 1, words);
+    const int form = proved == 0 ? 0 : (proved == EF_FLOAT ? 1 : 2);
+    if (form == 2) words = exact_words(q);
     QuantDev scalars{};
     fill_quant_scalars(q, scalars);
     cudaError_t e = launch_rescale_i32(d_in, d_out, nb_pixels, q.nb_channels, form, words.data(), scalars, (cudaStream_t)stream);

@@ -748,3 +748,45 @@ def test_top_n_with_large_groups_of_equal_scores(classes, top_n, levels):
         assert np.array_equal(got_l.reshape(B, top_n), want_l)
     finally:
         qn.close()
+
+
+def _small_chain(kind, mode, unsigned=True):
+    b = netdesc.NetBuilder(kind, {'lenet': 3, 'wide': 5, 'fc': 4}.get(kind, 1), 17 if kind == 'lenet' else 24, 19 if kind == 'lenet' else 24, 41, mode,
+                           unsigned_relu=unsigned, input_unsigned=unsigned)
+    if kind == 'mnist':
+        x = b.conv(-1, 16, 4, stride=2)
+        x = b.conv(x, 24, 5, stride=2)
+        b.fc(b.fc(x, 150, act='relu'), 10)
+    elif kind == 'lenet':          # padding, odd channel counts, both poolings
+        x = b.conv(-1, 7, 3, pad=1)
+        x = b.pool(x, 'max', 2, 2)
+        x = b.conv(x, 10, 3, stride=1, pad=2)
+        x = b.pool(x, 'avg', 3, 2, pad=1)
+        b.fc(x, 33)
+    elif kind == 'wide':           # runs of 15 bytes, more outputs than threads, a convolution as the last cell
+        x = b.conv(-1, 9, 3, stride=3)
+        b.conv(x, 21, 2, pad=1, act='linear')
+    else:                          # fully connected on the network input
+        b.fc(b.fc(-1, 31, act='relu'), 5)
+    return b.net
+
+
+# one image per CTA, a group that is not full, more groups than CTAs
+@pytest.mark.parametrize('batch', [1, 5, 150, 301, 1203])
+@pytest.mark.parametrize('kind,mode', [('mnist', 'single'), ('mnist', 'float'), ('lenet', 'double'), ('lenet', 'fixed'), ('wide', 'single'), ('fc', 'double')])
+def test_small_networks_as_one_kernel(kind, mode, batch):
+    net = _small_chain(kind, mode, unsigned=kind != 'wide')
+    x = netdesc.make_input(net, batch, seed=batch)
+    picks = sorted({0, batch - 1, batch // 2, min(batch - 1, 3), min(batch - 1, 4)})
+    ref = oracle.run_net(net, x[picks], 'i64')[-1].reshape(len(picks), -1)
+    qn = runtime.QuantizedNet(net, batch)
+    other = runtime.QuantizedNet(net, batch, flags=R.NO_FUSION)      # cell by cell
+    try:
+        assert qn.launches_per_forward() == 1 and other.launches_per_forward() > 1
+        out = qn.forward_host(x)
+        assert np.array_equal(out[picks].astype(np.int64), ref)
+        assert np.array_equal(out, other.forward_host(x))
+        assert np.array_equal(qn.read_layer(len(net['layers']) - 1, batch).reshape(batch, -1), out)
+    finally:
+        qn.close()
+        other.close()
