@@ -47,6 +47,7 @@ struct IgemmArgs {
     int grouped;        // block-diagonal layer (depthwise as groups of BN channels): a column block reads its own input channels
     int res_slots;          // staging regions per epilogue warp of a residual cell (2 or 4)
     int m_base;         // first output row of this call within the tensors (a batch slice starts at image img0)
+    int late_weights;   // weights only after the dependency wait
     int b_resident;     // the CTA's whole weight block stays in shared memory (its column block never changes)
     int oW, oH, kW, sX, sY, pL, pT, dX, dY;
     int num_m_tiles, num_n_tiles;
@@ -204,6 +205,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         const int takers = a.stages < NUM_PRODUCERS ? a.stages : NUM_PRODUCERS;
         const int my_turn = producer < takers ? producer : 0x40000000;   // ring fills until this producer's first one (never, if idle)
         unsigned pre = 0;   // ring fills whose weights are issued before the wait
+        if (a.late_weights) pdl_wait();
         if (first < num_tiles) {
             if (!a.b_resident) pre = (unsigned)(num_kb < a.stages ? num_kb : a.stages);
             const int nload = a.b_resident ? num_kb : (int)pre;
@@ -589,6 +591,7 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
         px.start(a, m0);
         const unsigned tiles_s = smem_u32(tiles);
         unsigned pre = 0;
+        if (a.late_weights) pdl_wait();
         if ((int)blockIdx.x < num_pt) {
             pre = (unsigned)(num_kb < PAIR_STAGES ? num_kb : PAIR_STAGES);
             if (elect_one()) {
@@ -1035,6 +1038,45 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
     return 0;
 }
 
+// Eight weights per thread; at most a few megabytes that stay in L2
+__global__ void __launch_bounds__(256) widen_int4_kernel(const uint8_t* __restrict__ packed, int rows_src, int ng_src, int8_t* __restrict__ dst, int rows,
+                                                         int ng_dst, unsigned words)
+{
+    pdl_launch_dependents();
+    pdl_wait();   // the destination may still be read by the previous kernel
+    const unsigned total = (unsigned)rows * words;   // 8-byte words of the destination
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const unsigned n = i / words, w = i - n * words;
+        const int real = perm_real_channel((int)n, ng_dst);
+        uint2 o = make_uint2(0u, 0u);
+        if (real < rows_src) {
+            int src = real;
+            if (ng_src) {   // where the packed rows hold this channel (the inverse of perm_real_channel)
+                const int j = real % (8 * ng_src), q = j / (2 * ng_src), r = j - q * 2 * ng_src;
+                src = real - j + 8 * (r >> 1) + 2 * q + (r & 1);
+            }
+            unsigned lo, hi;
+            expand_int4_x16(__ldg((const unsigned*)packed + (size_t)src * words + w), lo, hi);
+            auto down = [](unsigned x) {   // 16 x the value in every byte -> the value
+                const unsigned t = (x >> 4) & 0x0f0f0f0fu;
+                return t | ((t & 0x08080808u) * 0x1eu);
+            };
+            o = make_uint2(down(lo), down(hi));
+        }
+        ((uint2*)dst)[i] = o;
+    }
+}
+
+cudaError_t launch_widen_int4(const uint8_t* packed, int rows_src, int ng_src, int8_t* dst, int rows, int ng_dst, size_t row_bytes, cudaStream_t s)
+{
+    const unsigned words = (unsigned)(row_bytes / 8);
+    const unsigned long long total = (unsigned long long)rows * words;
+    if (total == 0) return cudaSuccess;
+    if (total >= (1ull << 31)) return cudaErrorInvalidValue;
+    const unsigned long long blocks = (total + 255) / 256;
+    return launch_pdl(widen_int4_kernel, (int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, s, packed, rows_src, ng_src, dst, rows, ng_dst, words);
+}
+
 bool igemm_uses_fast_epilogue(const IgemmPlan& plan, const FastQuant& fast, bool has_residual, int out_dtype)
 {
     return fast.enabled && out_dtype == DT_I8 && (plan.N % 32 == 0) && (!has_residual || fast.fq2) && plan.has_out_maps;
@@ -1057,6 +1099,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     a.m_base = m_base;
     a.M = plan.M; a.N = plan.N; a.Cin = plan.Cin; a.taps = plan.taps; a.BK = plan.BK; a.BN = plan.BN;
     a.b_resident = plan.b_resident;
+    a.late_weights = plan.late_weights;
     a.stages = plan.stages; a.a_im2col = plan.a_im2col;
     a.grouped = plan.grouped;
     a.res_slots = plan.res_slots ? plan.res_slots : 2;

@@ -125,6 +125,7 @@ struct PatchPlan {
     int stage_cols;       // columns an epilogue warp stages per pass
     int in_unsigned;
     int num_sms;
+    int late_weights;     // the weights are the previous kernel's output (see IgemmPlan)
     int G;                // channel groups: 1, or the block-diagonal groups of a depthwise layer
     size_t smem_bytes;
 };
@@ -166,6 +167,7 @@ struct IgemmPlan {
     // im2col geometry
     int oW, oH, kW, sX, sY, pL, pT, dX, dY;
     int grid;             // CTAs to launch
+    int late_weights;     // the weights are the previous kernel's output: not before griddepcontrol.wait
     size_t smem_bytes;
 };
 // depthwise layers the kernel takes as block-diagonal groups (channels a multiple of 64, or 32): channels per group,
@@ -187,6 +189,11 @@ void igemm_permute_weights(const int8_t* w, int8_t* dst, int N, size_t row_bytes
 // residual stay the tensors' base pointers
 cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residual& r, const FastQuant& fast,
                          void* out, int out_dtype, int m_base, int* status_word, cudaStream_t s);
+
+// Widens packed 4-bit weights [rows_src][row_bytes / 2] into int8 [rows][row_bytes] in the row order a kernel expects.  Row n of the
+// destination is real channel perm_real_channel(n, ng_dst); ng_src says how the packed rows are ordered (0: naturally).
+// Destination rows of channels that do not exist are zero.
+cudaError_t launch_widen_int4(const uint8_t* packed, int rows_src, int ng_src, int8_t* dst, int rows, int ng_dst, size_t row_bytes, cudaStream_t s);
 
 // ---- first-layer convolution (<= 4 input channels) on the tensor cores ----
 struct StemPlan {

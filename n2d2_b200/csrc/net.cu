@@ -100,6 +100,13 @@ struct CellRec {
     void* d_colpad = nullptr;
     // stride-1 convolution from a shared-memory patch
     PatchPlan patch{};
+    // packed 4-bit weights at large batches: widened to int8 by a small kernel into the network's scratch, then the int8
+    // kernel of the layer (see plan_widened)
+    enum { W8_NONE, W8_IGEMM, W8_PATCH } w8 = W8_NONE;
+    IgemmPlan plan8{};
+    PatchPlan patch8{};
+    int w8_rows = 0, w8_ng_src = 0, w8_ng_dst = 0;
+    void* d_w8_out = nullptr;     // padded output matrix (see pad_O) of a widened cell
     // tensor-core plan
     IgemmPlan plan{};
     bool has_plan = false;
@@ -117,6 +124,7 @@ struct n2d2b_net {
     std::vector<void*> buffers;
     std::vector<size_t> buffer_bytes;
     int* d_status = nullptr;
+    void* d_w8 = nullptr;         // widened weights of the packed cell that is running
     int launches = 0;
     const void* last_input = nullptr;
     void* d_labels_scratch = nullptr;   // device labels / scores of the host-buffer top-N entry point
@@ -645,7 +653,9 @@ void n2d2b_net_destroy(n2d2b_net* net)
         cudaFree(c.d_fast);
         cudaFree(c.d_pad4);
         cudaFree(c.d_colpad);
+        cudaFree(c.d_w8_out);
     }
+    cudaFree(net->d_w8);
     cudaFree(net->d_status);
     cudaFree(net->d_small);
     cudaFree(net->d_labels_scratch);
@@ -975,6 +985,65 @@ static int final_tensor_of(const n2d2b_net* net)
     return -1;
 }
 
+// Whether a packed cell takes the widened form: its in-kernel expansion repeats for every tile, the widening once per call for
+// 2 to 3 us.  The line lies where a CTA has more than two tiles.
+static bool use_widened(const n2d2b_net* net, const CellRec& c, int batch)
+{
+    if (c.w8 == CellRec::W8_NONE) return false;
+    const long long m_tiles = ((long long)batch * c.geom.oH * c.geom.oW + 127) / 128;
+    return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) > 2ll * net->num_sms;
+}
+
+// Plans the widened form of every packed cell.  The weights stay packed in HBM; one scratch block, as large as the largest such cell,
+// holds the int8 weights of the cell that is running.  3x3 256 -> 256 at 14 x 14, 2048 images: 0.51 ms with the expansion
+// in the kernel (its warps' shared-memory stores bound it).
+static int plan_widened(n2d2b_net* net)
+{
+    size_t most = 0;
+    for (CellRec& c : net->cells) {
+        if (c.skipped || c.engine != ENG_TCGEN05 || !c.plan.w4 || !c.fast.enabled || !c.plan_input) continue;
+        const int rows = (c.geom.O + 31) & ~31;
+        most = std::max(most, (size_t)rows * c.geom.kH * c.geom.kW * c.geom.C);
+    }
+    if (!most) return 0;
+    CUDA_TRY(cudaMalloc(&net->d_w8, most + 256));
+    for (CellRec& c : net->cells) {
+        if (c.skipped || c.engine != ENG_TCGEN05 || !c.plan.w4 || !c.fast.enabled || !c.plan_input) continue;
+        ConvGeom g = c.geom;
+        g.B = net->max_batch;
+        const TensorRec& tout = net->tensors[c.output];
+        if (tout.dtype != DT_I8) continue;
+        const int in_u = net->tensors[c.inputs[0]].is_unsigned;
+        const void* res = c.residual >= 0 ? tensor_ptr(net, c.residual, nullptr) : nullptr;
+        const char* why = "";
+        c.w8_ng_src = c.plan.perm / 8;
+        c.w8_rows = g.O;
+        if (!res && patch_eligible(g) && patch_make_plan(&c.patch8, c.plan_input, (const int8_t*)net->d_w8, g, in_u, net->num_sms, &why) == 0) {
+            c.patch8.late_weights = 1;
+            c.w8_ng_dst = 4;
+            c.w8 = CellRec::W8_PATCH;
+            continue;
+        }
+        void* out = tensor_ptr(net, c.output, nullptr);
+        if (g.O % 32 != 0) {
+            if (res) continue;
+            g.O = c.w8_rows = (g.O + 31) & ~31;
+            CUDA_TRY(cudaMalloc(&c.d_w8_out, (size_t)net->max_batch * g.oH * g.oW * g.O + 256));
+            out = c.d_w8_out;
+        }
+        if (igemm_make_plan(&c.plan8, c.plan_input, (const int8_t*)net->d_w8, out, res, g, in_u, 0, 0, net->num_sms, &why)
+            || !igemm_uses_fast_epilogue(c.plan8, c.fast, res != nullptr, DT_I8))
+            continue;
+        c.plan8.late_weights = 1;
+        c.plan8.perm = igemm_perm_block(c.plan8);
+        c.w8_ng_dst = c.plan8.perm / 8;
+        c.w8 = CellRec::W8_IGEMM;
+    }
+    for (const CellRec& c : net->cells)
+        if (!c.skipped && use_widened(net, c, net->max_batch)) net->launches += c.d_w8_out ? 2 : 1;
+    return 0;
+}
+
 // A chain of convolutions, poolings and fully-connected cells whose weights fit one SM's shared memory runs as one kernel
 // (small_net.cu).  The bound on the arithmetic keeps out what the tensor cores do better: 2^20 multiply-accumulates
 // take an SM about 8 us there, and a batch of b images b / 148 times that.
@@ -1252,6 +1321,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
             }
         }
     }
+    if (int rc = plan_widened(net)) return rc;
     if (int rc = plan_small_net(net)) return rc;
     if (net->d_small) net->launches = 1;
     CUDA_TRY(cudaMalloc(&net->d_stage_in, net->tensors[0].bytes_per_image() * (size_t)max_batch + 256));
@@ -1347,6 +1417,23 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         r.ptr = tensor_ptr(net, c.residual, d_input);
         r.is_unsigned = net->tensors[c.residual].is_unsigned;
         r.q2 = c.q2.dev;
+    }
+    if (use_widened(net, c, batch)) {
+        const size_t row_bytes = (size_t)c.geom.kH * c.geom.kW * c.geom.C;
+        CUDA_TRY(launch_widen_int4((const uint8_t*)c.d_weights, c.geom.O, c.w8_ng_src, (int8_t*)net->d_w8, c.w8_rows, c.w8_ng_dst, row_bytes, s));
+        ConvGeom g = c.geom;
+        g.B = batch;
+        if (c.w8 == CellRec::W8_PATCH) {
+            CUDA_TRY(launch_patch(c.patch8, g, img0, c.fast, out, net->d_status, s));
+            return 0;
+        }
+        IgemmPlan p = c.plan8;
+        p.M = batch * g.oH * g.oW;
+        const size_t row0 = (size_t)img0 * g.oH * g.oW;
+        CUDA_TRY(launch_igemm(p, c.q.dev, r, c.fast, c.d_w8_out ? c.d_w8_out : out, DT_I8, (int)row0, net->d_status, s));
+        if (c.d_w8_out)
+            CUDA_TRY(launch_drop_padded_columns((const uint8_t*)c.d_w8_out + row0 * c.w8_rows, c.w8_rows, (uint8_t*)out + row0 * g.O, g.O, (size_t)p.M, s));
+        return 0;
     }
     switch (c.engine) {
     case ENG_TCGEN05: {

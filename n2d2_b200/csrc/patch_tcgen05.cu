@@ -47,6 +47,7 @@ struct PatchArgs {
     int n_base;             // first image of this call within the tensors (batch slices)
     int patch_bytes;        // bytes one patch load delivers (the full TMA box)
     int patch_alloc;        // bytes reserved per patch buffer (box + the rows a last tile may read past it)
+    int late_weights;       // weights only after the dependency wait
     int b_stream;           // weights too large to stay resident: their tap blocks stream through a ring
     int bring;              // slots of that ring
     int stage_cols;         // columns an epilogue warp stages per pass (BN, or 32 to leave room for the ring)
@@ -168,6 +169,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
             prefetch_tensor_map(&tmA);
             prefetch_tensor_map(&tmB);
             unsigned pre = 0, wt = 0;   // ring fills issued before the wait, ring fills so far
+            if (a.late_weights) pdl_wait();
             if (a.b_stream) {
                 pre = (unsigned)(taps < a.bring ? taps : a.bring);
                 for (unsigned t = 0; t < pre; ++t) {
@@ -552,6 +554,7 @@ cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, 
     a.n_base = n_base;
     a.patch_bytes = plan.patch_bytes; a.patch_alloc = plan.patch_alloc;
     a.b_stream = plan.b_stream;
+    a.late_weights = plan.late_weights;
     a.bring = plan.bring;
     a.stage_cols = plan.stage_cols;
     a.rcp_Wp = (unsigned)(((1ull << 32) + (unsigned)plan.Wp - 1) / (unsigned)plan.Wp);

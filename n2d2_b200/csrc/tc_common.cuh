@@ -144,7 +144,9 @@ __device__ __forceinline__ bool mbar_wait_issuer(unsigned bar, unsigned parity, 
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-        if (++rounds > 8) __nanosleep(128);
+        // the first rounds (about 0.5 us) catch what is nearly there; four or five warps that polled on through a wait for the
+        // epilogue took 8 % from layers the epilogue bounds
+        if (++rounds > 2) __nanosleep(200);
         if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
         if (__any_sync(0xffffffffu, globaltimer_ns() - t0 > WAIT_LIMIT_NS)) {
             *abort_flag = 1;

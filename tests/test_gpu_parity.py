@@ -790,3 +790,31 @@ def test_small_networks_as_one_kernel(kind, mode, batch):
     finally:
         qn.close()
         other.close()
+
+
+# enough tiles for the widened form: patch kernel, implicit GEMM with 64- and 256-column tiles, a residual sum, padded outputs
+@pytest.mark.parametrize('case', [(64, 56, 64, 3, 1, 1, 13), (128, 28, 128, 3, 1, 1, 50), (64, 40, 128, 3, 2, 1, 97), (128, 30, 512, 1, 1, 0, 44),
+                                  (32, 44, 32, 5, 1, 2, 21), (256, 21, 100, 1, 1, 0, 91)], ids=lambda c: 'C%d_H%d_O%d_k%d_s%d' % c[:5])
+@pytest.mark.parametrize('mode', ['double', 'fixed'])
+def test_packed_int4_weights_widened_for_large_batches(case, mode):
+    C, H, O, k, s, p, batch = case
+    b = netdesc.NetBuilder('w4', 16, H, H, 43, mode, weight_bits=4)
+    x = b.conv(-1, C, 1)                    # the layer under test reads a tensor of the network's own
+    y = b.conv(x, O, k, stride=s, pad=p, act='linear')
+    if C == O and s == 1:
+        b.sum([b.conv(y, O, 1, act='linear'), x])
+    net = b.net
+    x = netdesc.make_input(net, batch, seed=6)
+    picks = [0, batch // 2, batch - 1]
+    ref = oracle.run_net(net, x[picks], 'i64')[-1].reshape(len(picks), -1)
+    qn = runtime.QuantizedNet(net, batch)
+    few = runtime.QuantizedNet(net, 3)      # the in-kernel expansion
+    try:
+        assert 'tcgen05-w4' in qn.engines()
+        assert qn.launches_per_forward() > few.launches_per_forward()
+        out = qn.forward_host(x)
+        assert np.array_equal(out[picks].astype(np.int64), ref)
+        assert np.array_equal(few.forward_host(x[picks]), out[picks])
+    finally:
+        qn.close()
+        few.close()
