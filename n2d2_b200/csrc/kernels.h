@@ -225,14 +225,15 @@ struct SmallCell {
     int O, Opad, oH, oW, kH, kW;
     int words;                      // 32-bit words of a filter row's run of kW * C bytes
     int step_x, step_y, step_ky;    // bytes from one output pixel / output row / filter row to the next in the padded input
-    int aligned;                    // every run starts on a word
-    int two;                        // a thread takes two neighbouring outputs
+    int copy_stride;                // bytes between the moved copies of the input of a cell whose windows start on any byte
+    int log_split;                  // a window's words are dealt out to 2^log_split threads
     int in_off, out_off, out_row;   // activation area: this cell's input, where its output goes, bytes per output row there
+    int out_copies, out_copy_stride;    // copies of the output that the next cell wants
     int w_off, cst_off;             // weights and constants in the blob
     int form;                       // rescale: 0, EF_WIDE, EF_FLOAT, or -1 for the exact 64-bit one (q)
     int in_unsigned, out_unsigned;
     int inH, inW, sY, sX, padY, padX;   // pooling
-    unsigned rcp_O, rcp_O2, rcp_oW;     // reciprocals of Opad (channels for a pooling), Opad / 2 and oW
+    unsigned rcp_O, rcp_oW;             // reciprocals of Opad / 2 (channels for a pooling) and oW
     QuantDev q;
 };
 struct SmallNetArgs {
@@ -240,21 +241,21 @@ struct SmallNetArgs {
     int nb_cells;
     const uint8_t* blob;
     int blob_bytes, act_stride;
-    int in_bytes, in_place, in_pitch, in_row, in_words;
+    int in_bytes, in_place, in_pitch, in_row, in_words, in_copies, in_copy_stride;
     int out_bytes;
 };
 struct SmallNetPlan {
     std::vector<SmallCell> cells;
     std::vector<uint8_t> blob;      // weights and constants of every cell, as the kernel keeps them in shared memory
     int act_bytes = 0;              // activations of one image
-    int in_bytes = 0, in_place = 0, in_pitch = 0, in_row = 0, in_words = 0;
+    int in_bytes = 0, in_place = 0, in_pitch = 0, in_row = 0, in_words = 0, in_copies = 1, in_copy_stride = 0;
     int out_bytes = 0;
     int group = 1;                  // images per pass the shared memory holds: 4 or 1
 };
 void small_net_add_conv(SmallNetPlan* p, const ConvGeom& g, int in_unsigned, int out_unsigned, const int8_t* w, int form, const int32_t* consts,
                         int cpad, const QuantDev& q);
 void small_net_add_pool(SmallNetPlan* p, const PoolGeom& g, int in_unsigned);
-void small_net_link(SmallNetPlan* p, int pT, int pL, int pitch, int row_bytes, int pixel, int H, int W, int C);
+void small_net_link(SmallNetPlan* p, int in_off, int copies, int copy_stride, int pT, int pL, int pitch, int row_bytes, int pixel, int H, int W, int C);
 bool small_net_finish(SmallNetPlan* p, int out_bytes);
 // out: the network's final tensor, out2: the caller's copy of it (or nullptr)
 cudaError_t launch_small_net(const SmallNetPlan& p, const void* d_blob, const void* in, int batch, void* out, void* out2, int num_sms,
