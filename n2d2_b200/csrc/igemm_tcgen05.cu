@@ -7,10 +7,10 @@
 // multi-stage shared-memory ring (A tile through a 2-D tiled map for a plain GEMM, or through an
 // im2col map that applies stride / padding / dilation and zero-fills the halo; B tile through a 2-D
 // map, or once into a resident block when the layer's weights are small), warp 1 issues
-// tcgen05.mma kind::i8 into one of two TMEM accumulators, warps 2-17 drain the other accumulator with
+// tcgen05.mma kind::i8 into a ring of TMEM accumulators, warps 2-17 drain the finished ones with
 // tcgen05.ld and run the fused epilogue (bias, per-channel rescale, rounding, saturation, ReLU,
-// optional residual add + second rescale) straight to int8 NHWC: every warp owns the 32 rows of its
-// TMEM lane quadrant and a quarter of the tile's columns.  Cells on the 32-bit epilogue store their weight
+// optional residual add + second rescale) straight to int8 NHWC: a warp takes the 32 rows of its
+// TMEM lane quadrant and 64 of the tile's columns, so narrow tiles go to the warps in groups of one tile each.  Cells on the 32-bit epilogue store their weight
 // rows permuted inside blocks of 32 (16) output channels, so that the column pairs a TMEM load hands a
 // thread are 8 (4) consecutive channels: constants, residual and output move as 128- and 64-bit accesses.  This replaces the reference's
 // cudnnConvolutionForward + cudnnAddTensor + Scaling kernel + cudnnActivationForward sequence
@@ -33,7 +33,8 @@ namespace n2d2b {
 
 static constexpr int BM = 128;
 static constexpr int EPI_WARP0 = 2;
-static constexpr int NUM_EPI_WARPS = 16;      // four per TMEM lane quadrant, a quarter of the columns each
+static constexpr int NUM_EPI_WARPS = 16;      // four per TMEM lane quadrant
+static constexpr int MAX_ACC = 8;             // TMEM accumulators: 512 columns of 64
 static constexpr int REGION_BYTES = 2048;     // staging per epilogue warp: 32 rows x up to 64 bytes
 static constexpr int NUM_PRODUCERS = 3;       // warps that issue TMA loads: warp 0 and the last two of the CTA
 static constexpr int NUM_THREADS = 32 * (EPI_WARP0 + NUM_EPI_WARPS + NUM_PRODUCERS - 1);
@@ -48,6 +49,8 @@ struct IgemmArgs {
     int res_slots;          // staging regions per epilogue warp of a residual cell (2 or 4)
     int m_base;         // first output row of this call within the tensors (a batch slice starts at image img0)
     int late_weights;   // weights only after the dependency wait
+    int parts, groups;  // warps per quadrant that share a tile, and tiles in the hands of the epilogue at once (parts * groups = 4)
+    int acc_shift;      // log2 of the number of TMEM accumulators
     int b_resident;     // the CTA's whole weight block stays in shared memory (its column block never changes)
     int oW, oH, kW, sX, sY, pL, pT, dX, dY;
     int num_m_tiles, num_n_tiles;
@@ -134,17 +137,17 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     // cells with a fused residual keep two or four regions per warp so that the residual of the next tiles arrives early
     const int regions_per_warp = RES ? a.res_slots : 1;
     unsigned long long* bars = (unsigned long long*)(stage_out + NUM_EPI_WARPS * REGION_BYTES * regions_per_warp);
-    // bars: full[stages], empty[stages], tmem_full[2], tmem_empty[2], params_ready[2], residual[4 * NUM_EPI_WARPS],
-    //       resident weights
+    // bars: full[stages], empty[stages], tmem_full[8], tmem_empty[8], params_ready[2], residual[4 * NUM_EPI_WARPS],
+    //       resident weights, dry run
     const unsigned full0 = smem_u32(bars);
     const unsigned empty0 = full0 + 8u * a.stages;
     const unsigned tfull0 = empty0 + 8u * a.stages;
-    const unsigned tempty0 = tfull0 + 16u;
-    const unsigned pready0 = tempty0 + 16u;
+    const unsigned tempty0 = tfull0 + 8u * MAX_ACC;
+    const unsigned pready0 = tempty0 + 8u * MAX_ACC;
     const unsigned rbar0 = pready0 + 16u;
     const unsigned bfull = rbar0 + 8u * (4 * NUM_EPI_WARPS);
     const unsigned bready0 = bfull + 16u;                                       // W4: expanded weights of a stage are in place
-    unsigned* tmem_slot = (unsigned*)(bars + 2 * a.stages + 6 + 4 * NUM_EPI_WARPS + 2 + (W4 ? a.stages : 0));
+    unsigned* tmem_slot = (unsigned*)(bars + 2 * a.stages + 2 * MAX_ACC + 2 + 4 * NUM_EPI_WARPS + 2 + (W4 ? a.stages : 0));
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     // [2 buffers][2 quant sets][FAST_NP][256], 16-byte aligned for vector loads
     int* epi_params = (int*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);
@@ -158,10 +161,14 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 
     if (warp == 0) {
         // one barrier per lane and pass: 80 of them in turn on one thread delayed the whole CTA
-        const int nb = 2 * a.stages + 6 + 4 * NUM_EPI_WARPS + 1;
+        const int nb = 2 * a.stages + 2 * MAX_ACC + 2 + 4 * NUM_EPI_WARPS + 2;
         for (int i = lane; i < nb; i += 32) {
-            const int j = i - (2 * a.stages + 2);   // tmem_empty[2] and params_ready[2] collect the epilogue warps
-            mbar_init(full0 + 8u * i, j >= 0 && j < 4 ? NUM_EPI_WARPS : (i == nb - 1 ? NUM_PRODUCERS : 1));   // the last one: resident weights
+            const int j = i - (2 * a.stages + MAX_ACC);   // tmem_empty collects the warps of a tile, params_ready[2] all epilogue warps
+            unsigned n = 1;
+            if (j >= 0 && j < MAX_ACC) n = FAST ? 4u * a.parts : NUM_EPI_WARPS;
+            else if (j >= MAX_ACC && j < MAX_ACC + 2) n = NUM_EPI_WARPS;
+            else if (i == nb - 2) n = NUM_PRODUCERS;      // resident weights
+            mbar_init(full0 + 8u * i, n);
         }
         if (W4 && lane < a.stages) mbar_init(bready0 + 8u * lane, W4_UNPACK_WARPS);
         if (lane == 0) {
@@ -185,6 +192,9 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     const unsigned tiles_s = smem_u32(tiles), res_b_s = smem_u32(res_b);
 
     const int num_tiles = a.num_m_tiles * a.num_n_tiles;
+    // A short launch (up to two tiles per CTA) spends a microsecond per role on instruction-cache misses once its data is there: its
+    // issuer and epilogue warps run through their loop bodies once, without effect, while the previous kernel still works.
+    const bool dry_run = FAST && num_tiles <= 2 * (int)gridDim.x;
 
     if (producer >= 0) {
         // ------------------------------------------------------------------ TMA producers
@@ -241,7 +251,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             }
             __syncwarp();
         }
-        pdl_wait();   // weights are constants; the activations are the previous kernel's output
+        bool waited = false;
         const bool im2col = a.a_im2col != 0, load_b = !a.b_resident;
         const unsigned ring_end = full0 + 8u * a.stages, to_empty = 8u * a.stages;
         unsigned bar = full0, dst = tiles_s, ph = 1u, it = 0;
@@ -253,6 +263,10 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                 if (turn == 0) {
                     turn = takers;
                     if (!mbar_wait_issuer(bar + to_empty, ph, abort_flag, a.status, 1)) { ok = false; break; }
+                    if (!waited) {   // weights are constants; the activations are the previous kernel's output
+                        pdl_wait();
+                        waited = true;
+                    }
                     if (elect_one()) {
                         const bool weights = it >= pre;   // else they are on their way
                         if (weights) mbar_expect_tx(bar, (unsigned)tx_bytes);
@@ -300,21 +314,27 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         const unsigned stage16 = (unsigned)(stage_bytes >> 4), a16 = (unsigned)(a_stage_bytes >> 4);
         const unsigned b16 = (unsigned)(b_stage_bytes >> 4);
         unsigned a_lo = a_lo0;
+        MBAR_PEEK_DECLARE();
+        bool dry = dry_run;
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++acc_it) {
-            const unsigned as = acc_it & 1u;
-            const unsigned aph = (acc_it >> 1) & 1u;
+            const unsigned as = acc_it & ((1u << a.acc_shift) - 1u);
+            const unsigned aph = (acc_it >> a.acc_shift) & 1u;
             if (!mbar_wait_issuer(tempty0 + 8u * as, aph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
             const unsigned d_tmem = tmem_base + as * (unsigned)a.BN;
             unsigned b_res = b_res0;
-            for (int kb = 0; kb < num_kb; ++kb) {
-                if (!mbar_wait_issuer(full0 + 8u * s, ph, abort_flag, a.status, 3)) { ok = false; break; }
-                if (W4 && !mbar_wait_issuer(bready0 + 8u * s, ph, abort_flag, a.status, 11)) { ok = false; break; }
+            for (int kb = dry ? -1 : 0; kb < num_kb; ++kb) {   // -1: operands and accumulator of the first K block as they are
+                if (!dry && !mbar_peeked() && !mbar_wait_issuer(full0 + 8u * s, ph, abort_flag, a.status, 3)) { ok = false; break; }
+                if (W4 && !dry && !mbar_wait_issuer(bready0 + 8u * s, ph, abort_flag, a.status, 11)) { ok = false; break; }
                 tc_fence_after();
                 const unsigned al = a_lo, b_lo = a.b_resident ? b_res : a_lo + a16;
-                const unsigned acc = kb ? 1u : 0u, ebar = empty0 + 8u * s;
-                a_lo += stage16;
-                b_res += b16;
-                if (++s == a.stages) { s = 0; ph ^= 1u; a_lo = a_lo0; }
+                const unsigned acc = kb > 0 ? 1u : 0u, ebar = dry ? bfull + 8u : empty0 + 8u * s;
+                if (!dry) {
+                    a_lo += stage16;
+                    b_res += b16;
+                    if (++s == a.stages) { s = 0; ph ^= 1u; a_lo = a_lo0; }
+                }
+                dry = false;
+                mbar_peek(full0 + 8u * s, ph);
                 if (elect_one()) {
                     // advancing K by 32 bytes inside the swizzle span = +2 in the 16-byte address field
                     tc_mma_i8_lohi(d_tmem, al, b_lo, desc_hi, a.idesc, acc);
@@ -363,15 +383,20 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     } else {
         // ------------------------------------------------------------------ epilogue warps
         const int quad = warp & 3;                       // TMEM lane quadrant this warp may read
-        const int part = (warp - EPI_WARP0) >> 2;        // 0..3 within the quadrant: a quarter of the columns (32-bit epilogue)
+        // Warps w, w + 4, w + 8, w + 12 share a quadrant.  A tile of 256 columns goes to all four, 64 columns each; of narrower
+        // tiles every warp still takes 64 columns and 128 / 64-column tiles are dealt out to two / four groups: the fixed
+        // work of a warp per tile (waits, fences, the store) equals that of 16 to 32 columns of arithmetic.
+        const int part4 = (warp - EPI_WARP0) >> 2;       // 0..3 within the quadrant
+        const int part = FAST ? part4 & (a.parts - 1) : part4, group = FAST ? part4 / a.parts : 0;
+        const int wp = a.BN / a.parts;
         const int row = quad * 32 + lane;
         const int epi_tid = (warp - EPI_WARP0) * 32 + lane;
         // the exact 64-bit epilogue works in 32-column chunks on the first two warps of each quadrant
         const int cols_per_warp = a.BN / 2;
-        unsigned acc_it = 0;
+        unsigned acc_it = (unsigned)group, mine = 0;   // the CTA's tiles so far, and this group's
         unsigned stage_it = 0;
         EpiState est;
-        perm_rowbase(est.rb, a.BN >> 2, lane, (a.BN >> 2) >= 32 ? 4 : 2);
+        perm_rowbase(est.rb, wp, lane, wp >= 32 ? 4 : 2);
         int staged_n_tile = -1;
         int* par = epi_params;
         bool ok = true;
@@ -396,23 +421,31 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             return true;
         };
         if (FAST && (int)blockIdx.x < num_tiles) ok = stage_constants((int)blockIdx.x % a.num_n_tiles);   // constants: before the wait
-        pdl_wait();   // residual loads and output stores touch tensors the previous kernel reads or writes
-        int m_next = (int)blockIdx.x / a.num_n_tiles, n_next = (int)blockIdx.x % a.num_n_tiles;
+        bool dry = dry_run;
+        if (!dry) pdl_wait();   // residual loads and output stores touch tensors the previous kernel reads or writes
+        // several groups only where the CTA's column block never changes (step_n is 0 or the CTA has one tile)
+        const int groups = FAST ? a.groups : 1;
+        const int tile_step = groups * (int)gridDim.x, step_m = groups * a.step_m, step_n = groups > 1 ? 0 : a.step_n;
+        const int m_first = (int)blockIdx.x / a.num_n_tiles;
+        int m_next = m_first + group * a.step_m, n_next = (int)blockIdx.x - m_first * a.num_n_tiles;
+        const int first_tile = (int)blockIdx.x + group * (int)gridDim.x;
         // residual loads run ahead of the tiles: pf_* walk the same tile sequence, res_slots - 1 tiles in front
-        int pf_tile = blockIdx.x, pf_m = m_next, pf_n = n_next;
+        int pf_tile = first_tile, pf_m = m_next, pf_n = n_next;
         unsigned pf_it = 0;
         const unsigned slot_shift = a.res_slots == 4 ? 2u : 1u;
         const unsigned lookahead = a.res_slots == 4 ? 3u : 2u;
         const unsigned my_regions = (unsigned)(stage_out - smem_raw) + (unsigned)((warp - EPI_WARP0) * REGION_BYTES * regions_per_warp);
         const unsigned my_rbar = rbar0 + 32u * (unsigned)(warp - EPI_WARP0);
-        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++acc_it) {
+        for (int tile = first_tile; tile < num_tiles && ok;) {
             const int n_tile = n_next, m_tile = m_next;
-            m_next += a.step_m;
-            n_next += a.step_n;
-            if (n_next >= a.num_n_tiles) { n_next -= a.num_n_tiles; ++m_next; }
+            if (!dry) {
+                m_next += step_m;
+                n_next += step_n;
+                if (n_next >= a.num_n_tiles) { n_next -= a.num_n_tiles; ++m_next; }
+            }
             const int m0 = a.m_base + m_tile * BM, n0 = n_tile * a.BN;
-            const unsigned as = acc_it & 1u;
-            const unsigned aph = (acc_it >> 1) & 1u;
+            const unsigned as = acc_it & ((1u << a.acc_shift) - 1u);
+            const unsigned aph = (acc_it >> a.acc_shift) & 1u;
             if (FAST && n_tile != staged_n_tile)
                 if (!stage_constants(n_tile)) { ok = false; break; }
             const int m = m0 + row;
@@ -423,35 +456,43 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                 EpiTile e;
                 e.tmem_acc = tmem_base + as * (unsigned)a.BN;
                 e.BN = a.BN; e.N = a.N; e.M = a.m_base + a.M; e.m0 = m0; e.n0 = n0;
-                e.wp = a.BN >> 2;
+                e.wp = wp;
                 e.par_off = (unsigned)((unsigned char*)par - smem_raw);
                 e.region_off = my_regions;
                 e.region_stride = RES ? REGION_BYTES : 0;
                 e.slot_shift = slot_shift;
                 e.rbar = my_rbar;
-                if (RES) {
+                if (RES && !dry) {
                     if (lane == 0) {
                         // two regions: the previous tile's store has finished reading, its region takes the next
                         // tile.  Four regions: the store before that one has, its region takes the tile two ahead,
                         // and nobody waits on a store that has only just been issued.
                         if (a.res_slots == 4) bulk_wait_read_1(); else bulk_wait_read_all();
-                        while (pf_it < acc_it + lookahead && pf_tile < num_tiles) {
+                        while (pf_it < mine + lookahead && pf_tile < num_tiles) {
                             epi_issue_residual(&tmR, my_regions, REGION_BYTES, my_rbar, pf_it & ((1u << slot_shift) - 1u),
                                                pf_n * a.BN + part * e.wp, a.m_base + pf_m * BM + quad * 32, a.N, e.M, e.wp);
                             ++pf_it;
-                            pf_tile += (int)gridDim.x;
-                            pf_m += a.step_m;
-                            pf_n += a.step_n;
+                            pf_tile += tile_step;
+                            pf_m += step_m;
+                            pf_n += step_n;
                             if (pf_n >= a.num_n_tiles) { pf_n -= a.num_n_tiles; ++pf_m; }
                         }
                     }
                     __syncwarp();
                 }
                 e.tfull = tfull0 + 8u * as; e.tfull_parity = aph; e.tempty = tempty0 + 8u * as;
-                e.abort_flag = abort_flag; e.status = a.status;
+                e.abort_flag = abort_flag; e.status = a.status; e.dry = dry;
                 e.ef = a.ef;
                 e.t_lo = a.t_lo; e.t_hi = a.t_hi; e.dp_xor = a.dp_xor;
                 if (!fast_epilogue_tile<RES, CLAMP, DP, true, W4>(&tmO, &tmR, e, quad, part, lane, est)) { ok = false; break; }
+                if (dry) {
+                    dry = false;
+                    pdl_wait();
+                    continue;
+                }
+                tile += tile_step;
+                acc_it += (unsigned)groups;
+                ++mine;
                 continue;
             } else {
                 if (!mbar_wait_warp(tfull0 + 8u * as, aph, abort_flag, a.status, 4, lane)) { ok = false; break; }
@@ -504,6 +545,8 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty0 + 8u * as);
+            tile += (int)gridDim.x;
+            ++acc_it;
         }
         // no bulk store may still be reading this CTA's shared memory when it exits (its writes complete with the grid)
         if (FAST && lane == 0) bulk_wait_read_all();
@@ -840,7 +883,7 @@ static size_t igemm_smem_bytes(int stages, int BK, int BN, int regions, size_t r
 {
     return 1024 /*alignment slack*/ + resident_b + (size_t)stages * ((BM + (resident_b ? 0 : BN)) * BK + (w4 ? BN * BK / 2 : 0))
          + NUM_EPI_WARPS * REGION_BYTES * regions
-         + (2 * stages + 8 + 4 * NUM_EPI_WARPS + (w4 ? stages : 0)) * 8 + 32 + 2 * 2 * FAST_NP * 256 * 4 + 64;
+         + (2 * stages + 2 * MAX_ACC + 4 + 4 * NUM_EPI_WARPS + (w4 ? stages : 0)) * 8 + 32 + 2 * 2 * FAST_NP * 256 * 4 + 64;
 }
 
 // Channels per block-diagonal group of a depthwise layer this kernel takes (0: not such a layer): groups of 64
@@ -909,6 +952,8 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
     }
     plan->BN = bn;
     plan->grouped = grouped;
+    // groups of epilogue warps on different tiles need a CTA whose column block never changes
+    plan->parts = (g.O + bn - 1) / bn < num_sms ? (bn >= 256 ? 4 : (bn >= 128 ? 2 : 1)) : 4;
     plan->w4 = w4 ? 1 : 0;
     plan->a_unsigned = in_unsigned;
     plan->oW = g.oW; plan->oH = g.oH; plan->kW = g.kW;
@@ -999,10 +1044,10 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
             if (bytes < 131072) reinterpret_cast<unsigned long long*>(&plan->tmA)[1] &= ~(1ull << 21);
         }
     }
-    // output (and residual) as [M][N] bytes, one box = an epilogue warp's 32 rows x BN/4 columns
+    // output (and residual) as [M][N] bytes, one box = an epilogue warp's 32 rows and columns
     plan->has_out_maps = 0;
     if (out && g.O % 16 == 0 && !((uintptr_t)out & 15) && !((uintptr_t)res & 15)) {
-        const int wb = plan->BN / 4;   // an epilogue warp's columns: 64, 32 or 16
+        const int wb = plan->BN / plan->parts;   // an epilogue warp's columns: 64, or 32 or 16 with four warps on a narrow tile
         const cuuint64_t dims[2] = {(cuuint64_t)g.O, (cuuint64_t)plan->M};
         const cuuint64_t strides[1] = {(cuuint64_t)g.O};
         const cuuint32_t box[2] = {(cuuint32_t)wb, 32};
@@ -1082,7 +1127,7 @@ bool igemm_uses_fast_epilogue(const IgemmPlan& plan, const FastQuant& fast, bool
     return fast.enabled && out_dtype == DT_I8 && (plan.N % 32 == 0) && (!has_residual || fast.fq2) && plan.has_out_maps;
 }
 
-int igemm_perm_block(const IgemmPlan& plan) { return (plan.BN >> 2) >= 32 ? 32 : 16; }
+int igemm_perm_block(const IgemmPlan& plan) { return plan.BN / plan.parts >= 32 ? 32 : 16; }
 
 void igemm_permute_weights(const int8_t* w, int8_t* dst, int N, size_t row_bytes, int perm_block)
 {
@@ -1110,10 +1155,8 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     // instruction descriptor: D = s32, A = u8/s8, B = s8, both K-major, N and M extents
     a.idesc = (2u << 4) | ((plan.a_unsigned ? 0u : 1u) << 7) | (1u << 10) | ((unsigned)(plan.BN >> 3) << 17)
             | ((unsigned)(BM >> 4) << 24);
-    unsigned cols = 2u * plan.BN;
-    unsigned p2 = 32;
-    while (p2 < cols) p2 <<= 1;
-    a.tmem_cols = p2;
+    a.parts = plan.parts;
+    a.groups = 4 / plan.parts;
     a.out_dtype = out_dtype;
     a.out = out;
     a.status = status_word;
@@ -1129,6 +1172,9 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     const bool use_fast = igemm_uses_fast_epilogue(plan, fast, r.ptr != nullptr, out_dtype);
     // the weights of a cell on the 32-bit epilogue are stored permuted (and only those)
     if (use_fast != (plan.perm != 0)) return cudaErrorInvalidConfiguration;
+    // two accumulators per group of epilogue warps (two in all for the exact epilogue)
+    a.acc_shift = use_fast ? (plan.parts == 4 ? 1 : (plan.parts == 2 ? 2 : 3)) : 1;
+    a.tmem_cols = (unsigned)plan.BN << a.acc_shift;
     const int mode = !use_fast ? 0 : (r.ptr ? (fast.need_clamp ? 2 : (fast.dp4a ? 5 : 4)) : (fast.need_clamp ? 1 : 3));
     static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
     int dev = 0;

@@ -97,8 +97,14 @@ struct StemS2dPlan {
     int band_bytes, band_alloc, w_bytes;
     int in_unsigned;
     int num_sms;
+    int band_batch;       // images the band height was chosen for
+    const void* s2d;      // the re-laid image
+    int max_batch;
+    void* encode;         // cuTensorMapEncodeTiled
     size_t smem_bytes;
 };
+// Chooses the band height for a call of `batch` images (a no-op when it is the plan's already)
+int stem_s2d_set_batch(StemS2dPlan* plan, const ConvGeom& g, int batch);
 bool stem_s2d_eligible(const ConvGeom& g);
 bool stem_s2d_pool_eligible(const ConvGeom& g, const PoolGeom& p);
 void stem_s2d_dims(const ConvGeom& g, int* Hs, int* Ws);
@@ -127,8 +133,14 @@ struct PatchPlan {
     int num_sms;
     int late_weights;     // the weights are the previous kernel's output (see IgemmPlan)
     int G;                // channel groups: 1, or the block-diagonal groups of a depthwise layer
+    int band_batch;       // images the band height was chosen for
+    const void* in;       // the activations (max_batch images)
+    int max_batch;
+    void* encode;         // cuTensorMapEncodeTiled
     size_t smem_bytes;
 };
+// Chooses the band height for a call of `batch` images (a no-op when it is the plan's already)
+int patch_set_batch(PatchPlan* plan, const ConvGeom& g, int batch);
 // dense stride-1 layers with 32 / 64 / 128 input channels, and depthwise stride-1 layers whose channels are a
 // multiple of 32 (run as block-diagonal groups of 64 or 32 channels)
 bool patch_eligible(const ConvGeom& g);
@@ -155,6 +167,7 @@ struct IgemmPlan {
     int BK;               // bytes of K per pipeline stage: 32, 64 or 128 (also the swizzle width)
     int BN;               // tile N: 64, 128 or 256
     int stages;
+    int parts;            // epilogue warps that share a tile's columns per TMEM lane quadrant: 4, 2 or 1 (a warp then takes BN / parts columns)
     int grouped;          // depthwise layer as block-diagonal groups: column block n reads input channels [n * BN, (n + 1) * BN)
     int b_resident;       // weights of the CTA's column block stay in shared memory for the whole launch
     int res_slots;        // fused residual: staging regions per epilogue warp (2 or 4), 0 without a residual

@@ -1424,6 +1424,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         ConvGeom g = c.geom;
         g.B = batch;
         if (c.w8 == CellRec::W8_PATCH) {
+            if (patch_set_batch(&c.patch8, c.geom, batch)) return fail(N2D2B_ERR_INVALID, "patch plan failed for %d images", batch);
             CUDA_TRY(launch_patch(c.patch8, g, img0, c.fast, out, net->d_status, s));
             return 0;
         }
@@ -1470,6 +1471,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
                 return fail(N2D2B_ERR_INVALID, "patch plan failed: %s", why);
             c.plan_input = in0;
         }
+        if (patch_set_batch(&c.patch, c.geom, batch)) return fail(N2D2B_ERR_INVALID, "patch plan failed for %d images", batch);
         ConvGeom g = c.geom;
         g.B = batch;
         CUDA_TRY(launch_patch(c.patch, g, img0, c.fast, out, net->d_status, s));
@@ -1480,6 +1482,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         g.B = batch;
         int Hs = 0, Ws = 0;
         stem_s2d_dims(g, &Hs, &Ws);
+        if (stem_s2d_set_batch(&c.stem2, c.geom, batch)) return fail(N2D2B_ERR_INVALID, "first-layer plan failed for %d images", batch);
         CUDA_TRY(launch_s2d_image(in0, g, batch, (uint8_t*)c.d_pad4 + (size_t)img0 * Hs * Ws * 16, s));
         CUDA_TRY(launch_stem_s2d(c.stem2, g, img0, c.fast, out, net->d_status, s));
         break;

@@ -471,7 +471,6 @@ int patch_make_plan(PatchPlan* plan, const void* in, const int8_t* w, const Conv
     *why = kWhy;
     if (!patch_eligible(g0)) { *why = "geometry outside the patch kernel"; return -1; }
     const ConvGeom g = patch_group_geom(g0);   // one group (the layer itself when it is dense)
-    const int Ct = g0.C;                       // channels per pixel of the input tensor, rows of the weight matrix
     if (((uintptr_t)in & 15) || ((uintptr_t)w & 15)) { *why = "operands must be 16-byte aligned"; return -1; }
     cudaDriverEntryPointQueryResult qr;
     void* fn = nullptr;
@@ -486,34 +485,10 @@ int patch_make_plan(PatchPlan* plan, const void* in, const int8_t* w, const Conv
     plan->in_unsigned = in_unsigned;
     plan->num_sms = num_sms;
     plan->G = patch_groups(g0);
-    // rows per band: among the heights that fit shared memory (and the 256-row TMA box), the one that
-    // wastes the fewest 128-position tiles per image; ties go to the taller band (fewer halo rows re-read)
-    int best_R = 0;
-    long long best_tiles = 0;
     plan->b_stream = patch_streams(taps, g.C, plan->BN) ? 1 : 0;
-    for (int R = 1; R <= g.oH; ++R) {
-        if (R + (g.kH - 1) * g.dY > 256) break;
-        if (patch_smem_bytes(taps, g.C, plan->BN, patch_alloc_bytes(g, plan->Wp, R)) > 226 * 1024) break;
-        // streamed weights: every tile of a band accumulates while the taps pass, so a band has at most as many
-        // tiles as there are accumulators
-        if (plan->b_stream && (R * plan->Wp + PBM - 1) / PBM > P_SLOTS) break;
-        const int full = g.oH / R, rest = g.oH % R;
-        const long long tiles = (long long)full * ((R * plan->Wp + PBM - 1) / PBM)
-                              + (rest ? (rest * plan->Wp + PBM - 1) / PBM : 0);
-        if (best_R == 0 || tiles <= best_tiles) { best_R = R; best_tiles = tiles; }
-    }
-    if (best_R == 0) { *why = "no band height fits shared memory"; return -1; }
-    plan->R = best_R;
-    plan->bands = (g.oH + best_R - 1) / best_R;
-    const int box_rows = best_R + (g.kH - 1) * g.dY;
-    plan->patch_bytes = box_rows * plan->Wp * g.C;
-    plan->patch_alloc = patch_alloc_bytes(g, plan->Wp, best_R);
-    plan->stage_cols = patch_stage_cols(taps, g.C, plan->BN);
-    plan->bring = P_BRING_MIN;
-    while (plan->b_stream && plan->bring < P_BRING_MAX
-           && patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring + 1) <= 226 * 1024)
-        ++plan->bring;
-    plan->smem_bytes = patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring);
+    plan->in = in;
+    plan->max_batch = g.B;
+    plan->encode = fn;
     const CUtensorMapSwizzle swz = g.C == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                                               : (g.C == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
     CUresult rc;
@@ -527,17 +502,61 @@ int patch_make_plan(PatchPlan* plan, const void* in, const int8_t* w, const Conv
                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the weights"; return -1; }
     }
-    {   // NHWC activations as (C, W, H, B); one box = a whole patch, zero-filled outside the image
-        const cuuint64_t dims[4] = {(cuuint64_t)Ct, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.B};
-        const cuuint64_t strides[3] = {(cuuint64_t)Ct, (cuuint64_t)Ct * g.W, (cuuint64_t)Ct * g.W * g.H};
-        const cuuint32_t box[4] = {(cuuint32_t)g.C, (cuuint32_t)plan->Wp, (cuuint32_t)box_rows, 1};
-        const cuuint32_t estr[4] = {1, 1, 1, 1};
-        rc = ((EncodeTiledFn)fn)(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)in, dims, strides, box, estr,
-                                 CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the activation patch"; return -1; }
-    }
+    if (patch_set_batch(plan, g0, g.B)) { *why = "no band height fits shared memory"; return -1; }
     return 0;
+}
+
+// Rows per band.  A CTA takes every nth band, so the call lasts as long as the CTA with the most bands: the height with the
+// shortest such run wins, counted in 128-position tiles plus one tile per band (its load and hand-over); ties go to the
+// taller band (fewer halo rows re-read).  A tall band that wastes no tile leaves SMs idle at a small batch (one image of 55 x 55: 5 bands of 11 rows
+// 10.4 us) and rounds badly when an SM gets one band and a half.
+int patch_set_batch(PatchPlan* plan, const ConvGeom& g0, int batch)
+{
+    if (plan->band_batch == batch) return 0;
+    const ConvGeom g = patch_group_geom(g0);
+    const int taps = g.kH * g.kW, Wp = plan->Wp;
+    const long long ctas = plan->num_sms / plan->G > 0 ? plan->num_sms / plan->G : 1;
+    int best_R = 0;
+    double best = 0.0;
+    for (int R = 1; R <= g.oH; ++R) {
+        if (R + (g.kH - 1) * g.dY > 256) break;
+        if (patch_smem_bytes(taps, g.C, plan->BN, patch_alloc_bytes(g, Wp, R)) > 226 * 1024) break;
+        // streamed weights: every tile of a band accumulates while the taps pass, so a band has at most as many
+        // tiles as there are accumulators
+        if (plan->b_stream && (R * Wp + PBM - 1) / PBM > P_SLOTS) break;
+        const int bands = (g.oH + R - 1) / R, rest = g.oH - (bands - 1) * R;
+        const double per_image = (bands - 1) * ((R * Wp + PBM - 1) / PBM + 1.0) + (rest * Wp + PBM - 1) / PBM + 1.0;
+        const long long items = (long long)batch * bands, rounds = (items + ctas - 1) / ctas;
+        // the longest run: whole rounds of average bands, one tall band at least
+        double t = per_image / bands * (double)rounds;
+        if (items <= ctas) t = (R * Wp + PBM - 1) / PBM + 1.0;
+        if (best_R == 0 || t <= best * 1.0001) { best_R = R; best = t; }
+    }
+    if (best_R == 0) return -1;
+    plan->band_batch = batch;
+    if (best_R == plan->R) return 0;
+    plan->R = best_R;
+    plan->bands = (g.oH + best_R - 1) / best_R;
+    const int box_rows = best_R + (g.kH - 1) * g.dY;
+    plan->patch_bytes = box_rows * plan->Wp * g.C;
+    plan->patch_alloc = patch_alloc_bytes(g, plan->Wp, best_R);
+    plan->stage_cols = patch_stage_cols(taps, g.C, plan->BN);
+    plan->bring = P_BRING_MIN;
+    while (plan->b_stream && plan->bring < P_BRING_MAX
+           && patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring + 1) <= 226 * 1024)
+        ++plan->bring;
+    plan->smem_bytes = patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring);
+    // NHWC activations as (C, W, H, B); one box = a whole patch, zero-filled outside the image
+    const CUtensorMapSwizzle swz = g.C == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                              : (g.C == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+    const int Ct = g0.C;
+    const cuuint64_t dims[4] = {(cuuint64_t)Ct, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)plan->max_batch};
+    const cuuint64_t strides[3] = {(cuuint64_t)Ct, (cuuint64_t)Ct * g.W, (cuuint64_t)Ct * g.W * g.H};
+    const cuuint32_t box[4] = {(cuuint32_t)g.C, (cuuint32_t)plan->Wp, (cuuint32_t)box_rows, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return ((EncodeTiledFn)plan->encode)(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)plan->in, dims, strides, box, estr,
+                                         CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -1;
 }
 
 cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, const FastQuant& fast, void* out,

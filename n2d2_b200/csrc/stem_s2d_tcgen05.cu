@@ -515,6 +515,8 @@ bool stem_s2d_pool_eligible(const ConvGeom& g, const PoolGeom& p)
     return s2d_smem_bytes(KH * BN * KWp * 16, BN, s2d_band_alloc(Wp, KH, KWp, R), cbuf) <= 226 * 1024;
 }
 
+static int s2d_use_bands(StemS2dPlan* plan, const ConvGeom& g, int R);
+
 int stem_s2d_make_plan(StemS2dPlan* plan, const void* d_s2d, const int8_t* d_w_arranged, const ConvGeom& g, int max_batch,
                        int in_unsigned, int num_sms, const char** why, const PoolGeom* pool)
 {
@@ -536,11 +538,13 @@ int stem_s2d_make_plan(StemS2dPlan* plan, const void* d_s2d, const int8_t* d_w_a
     plan->w = d_w_arranged;
     plan->in_unsigned = in_unsigned;
     plan->num_sms = num_sms;
-    int best_R = 0;
-    long long best_tiles = 0;
+    plan->s2d = d_s2d;
+    plan->max_batch = max_batch;
+    plan->encode = fn;
     if (pool) {
         // the most pooled rows per band that fit: fewer bands recompute fewer overlapping convolution rows
         if (!stem_s2d_pool_eligible(g, *pool)) { *why = "pooling outside the fused first-layer kernel"; return -1; }
+        int best_R = 0;
         for (int P = 1; P <= pool->oH; ++P) {
             const int R = (P - 1) * pool->sY + pool->pH;
             if (R + plan->KH - 1 > 256) break;
@@ -552,39 +556,57 @@ int stem_s2d_make_plan(StemS2dPlan* plan, const void* d_s2d, const int8_t* d_w_a
         }
         if (best_R == 0) { *why = "no band of the fused pooling fits shared memory"; return -1; }
         plan->pool_k = pool->pH; plan->pool_s = pool->sY; plan->pool_oH = pool->oH; plan->pool_oW = pool->oW;
-        plan->R = best_R;
         plan->row_stride = plan->P * pool->sY;
         plan->bands = (pool->oH + plan->P - 1) / plan->P;
-    } else {
-    for (int R = 1; R <= g.oH; ++R) {
-        if (R + plan->KH - 1 > 256) break;
-        if (s2d_smem_bytes(plan->w_bytes, plan->BN, s2d_band_alloc(plan->Wp, plan->KH, plan->KWp, R)) > 226 * 1024) break;
-        const int full = g.oH / R, rest = g.oH % R;
-        const long long tiles = (long long)full * ((R * plan->Wp + ZBM - 1) / ZBM)
-                              + (rest ? (rest * plan->Wp + ZBM - 1) / ZBM : 0);
-        if (best_R == 0 || tiles <= best_tiles) { best_R = R; best_tiles = tiles; }
+        if (s2d_use_bands(plan, g, best_R)) { *why = "cuTensorMapEncodeTiled failed for the re-laid image"; return -1; }
+        return 0;
     }
-    if (best_R == 0) { *why = "no band height fits shared memory"; return -1; }
-    plan->R = best_R;
-    plan->row_stride = best_R;
-    plan->bands = (g.oH + best_R - 1) / best_R;
-    }
-    const int box_rows = best_R + plan->KH - 1;
+    if (stem_s2d_set_batch(plan, g, max_batch)) { *why = "no band height of the first layer fits"; return -1; }
+    return 0;
+}
+
+// Bands of R rows: sizes and the tensor map
+static int s2d_use_bands(StemS2dPlan* plan, const ConvGeom& g, int R)
+{
+    plan->R = R;
+    const int box_rows = R + plan->KH - 1;
     plan->band_bytes = box_rows * plan->Wp * 16;
-    plan->band_alloc = s2d_band_alloc(plan->Wp, plan->KH, plan->KWp, best_R);
+    plan->band_alloc = s2d_band_alloc(plan->Wp, plan->KH, plan->KWp, R);
     plan->smem_bytes = s2d_smem_bytes(plan->w_bytes, plan->BN, plan->band_alloc, plan->cbuf_alloc);
     int Hs, Ws;
     stem_s2d_dims(g, &Hs, &Ws);
     // the re-laid image as (8-byte words of a row, rows, images): one box = one band, rows below the image read as zero
-    const cuuint64_t dims[3] = {(cuuint64_t)Ws * 2, (cuuint64_t)Hs, (cuuint64_t)max_batch};
+    const cuuint64_t dims[3] = {(cuuint64_t)Ws * 2, (cuuint64_t)Hs, (cuuint64_t)plan->max_batch};
     const cuuint64_t strides[2] = {(cuuint64_t)Ws * 16, (cuuint64_t)Ws * 16 * Hs};
     const cuuint32_t box[3] = {(cuuint32_t)plan->Wp * 2, (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult rc = ((EncodeTiledFn)fn)(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, (void*)d_s2d, dims, strides, box, estr,
-                                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the re-laid image"; return -1; }
-    return 0;
+    return ((EncodeTiledFn)plan->encode)(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, (void*)plan->s2d, dims, strides, box, estr,
+                                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -1;
+}
+
+// The band height with the shortest longest run of a CTA (see patch_set_batch).  One 224 x 224 image in three bands of 38 rows: 20 us; 64 images in
+// 192 such bands: one CTA in four works twice as long as the others.
+int stem_s2d_set_batch(StemS2dPlan* plan, const ConvGeom& g, int batch)
+{
+    if (plan->P || plan->band_batch == batch) return 0;
+    int best_R = 0;
+    double best = 0.0;
+    for (int R = 1; R <= g.oH; ++R) {
+        if (R + plan->KH - 1 > 256) break;
+        if (s2d_smem_bytes(plan->w_bytes, plan->BN, s2d_band_alloc(plan->Wp, plan->KH, plan->KWp, R)) > 226 * 1024) break;
+        const int bands = (g.oH + R - 1) / R, rest = g.oH - (bands - 1) * R, tall = (R * plan->Wp + ZBM - 1) / ZBM;
+        const double per_image = (bands - 1) * (tall + 1.0) + (rest * plan->Wp + ZBM - 1) / ZBM + 1.0;
+        const long long items = (long long)batch * bands, rounds = (items + plan->num_sms - 1) / plan->num_sms;
+        const double t = items <= plan->num_sms ? tall + 1.0 : per_image / bands * (double)rounds;
+        if (best_R == 0 || t <= best * 1.0001) { best_R = R; best = t; }
+    }
+    if (best_R == 0) return -1;
+    plan->band_batch = batch;
+    if (best_R == plan->R) return 0;
+    plan->row_stride = best_R;
+    plan->bands = (g.oH + best_R - 1) / best_R;
+    return s2d_use_bands(plan, g, best_R);
 }
 
 cudaError_t launch_stem_s2d(const StemS2dPlan& plan, const ConvGeom& g, int n_base, const FastQuant& fast, void* out,

@@ -305,7 +305,7 @@ stem_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
             e.slot_shift = 0;
             e.rbar = 0;
             e.tfull = tfull0 + 8u * as; e.tfull_parity = aph; e.tempty = tempty0 + 8u * as;
-            e.abort_flag = abort_flag; e.status = a.status;
+            e.abort_flag = abort_flag; e.status = a.status; e.dry = false;
             e.ef = (a.out_unsigned ? EF_OUT_UNSIGNED : 0) | a.form;
             e.t_lo = 0; e.t_hi = 0; e.dp_xor = 0;
             if (!fast_epilogue_tile<false, CLAMP, false>(&tmO, &tmO, e, quad, cp, lane, est)) break;

@@ -156,6 +156,20 @@ __device__ __forceinline__ bool mbar_wait_issuer(unsigned bar, unsigned parity, 
     }
 }
 
+// A look at the next phase whose answer is fetched later: the instructions between the two run while the barrier is read (a
+// wait costs 70-100 cycles when its phase has long completed).  One pending look per kernel; MBAR_PEEK_DECLARE once at its start.
+#define MBAR_PEEK_DECLARE() asm volatile(".reg .pred n2d2_peek;\n\tsetp.ne.u32 n2d2_peek, 0, 0;" ::: "memory")
+__device__ __forceinline__ void mbar_peek(unsigned bar, unsigned parity)
+{
+    asm volatile("mbarrier.test_wait.parity.shared::cta.b64 n2d2_peek, [%0], %1;" ::"r"(bar), "r"(parity) : "memory");
+}
+__device__ __forceinline__ bool mbar_peeked()
+{
+    unsigned ok;
+    asm volatile("selp.u32 %0, 1, 0, n2d2_peek;" : "=r"(ok)::"memory");
+    return __all_sync(0xffffffffu, ok != 0);
+}
+
 // Warp-wide bounded wait: one lane polls (32 lanes polling one word, times many warps, crowd out the
 // arrivals and the shared-memory traffic of the working warps), then every lane observes the completed
 // phase itself, which costs one successful try_wait and gives each lane its own acquire.
@@ -729,6 +743,7 @@ struct EpiTile {
     unsigned slot_shift;    // residual cells: log2 of the number of regions (1 or 2)
     unsigned rbar;          // this warp's residual-arrival mbarriers (one per region, 8 bytes apart)
     unsigned tfull, tfull_parity, tempty;
+    bool dry;               // run through the arithmetic on whatever is there, for the instruction cache: no waits, no arrival, no store
     volatile int* abort_flag;
     int* status;
     int ef;                 // EF_* switches of this cell
@@ -801,9 +816,9 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
         if (lane == 0) bulk_wait_read_all();   // the earlier store has finished reading the region
         __syncwarp();
     }
-    if (!mbar_wait_warp(e.tfull, e.tfull_parity, e.abort_flag, e.status, 4, lane)) return false;
+    if (!e.dry && !mbar_wait_warp(e.tfull, e.tfull_parity, e.abort_flag, e.status, 4, lane)) return false;
     if (RES) {
-        if (!mbar_wait_warp(e.rbar + 8u * b, (st.t >> e.slot_shift) & 1u, e.abort_flag, e.status, 7, lane)) return false;
+        if (!e.dry && !mbar_wait_warp(e.rbar + 8u * b, (st.t >> e.slot_shift) & 1u, e.abort_flag, e.status, 7, lane)) return false;
     }
     tc_fence_after();
     if (active) {
@@ -849,14 +864,14 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
     // the accumulator is drained: hand it back before the store goes out
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(e.tempty);
+    if (lane == 0 && !e.dry) mbar_arrive(e.tempty);
     fence_async_smem();
     __syncwarp();
-    if (lane == 0 && active) {
+    if (lane == 0 && active && !e.dry) {
         tma_store_2d(tmO, region, gx, gy);
         bulk_commit();
     }
-    ++st.t;
+    if (!e.dry) ++st.t;
     return true;
 }
 
