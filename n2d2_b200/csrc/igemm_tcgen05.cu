@@ -25,6 +25,7 @@
 // *status_word and makes the whole CTA drain and exit, so a wrong descriptor cannot hang the GPU.
 #include <cstdio>
 #include <cstring>
+#include <algorithm>
 #include <atomic>
 #include "kernels.h"
 #include "tc_common.cuh"
@@ -48,6 +49,7 @@ struct IgemmArgs {
     int grouped;        // block-diagonal layer (depthwise as groups of BN channels): a column block reads its own input channels
     int res_slots;          // staging regions per epilogue warp of a residual cell (2 or 4)
     int m_base;         // first output row of this call within the tensors (a batch slice starts at image img0)
+    int takers;         // producers that work (at most as many as ring slots)
     int late_weights;   // weights only after the dependency wait
     int parts, groups;  // warps per quadrant that share a tile, and tiles in the hands of the epilogue at once (parts * groups = 4)
     int acc_shift;      // log2 of the number of TMEM accumulators
@@ -212,7 +214,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         PixelPos px;
         px.start(a, m0);
         int iw0 = px.ox * a.sX - a.pL, ih0 = px.oy * a.sY - a.pT, in0 = px.n;
-        const int takers = a.stages < NUM_PRODUCERS ? a.stages : NUM_PRODUCERS;
+        const int takers = a.takers;
         const int my_turn = producer < takers ? producer : 0x40000000;   // ring fills until this producer's first one (never, if idle)
         unsigned pre = 0;   // ring fills whose weights are issued before the wait
         if (a.late_weights) pdl_wait();
@@ -1145,6 +1147,10 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     a.M = plan.M; a.N = plan.N; a.Cin = plan.Cin; a.taps = plan.taps; a.BK = plan.BK; a.BN = plan.BN;
     a.b_resident = plan.b_resident;
     a.late_weights = plan.late_weights;
+    // As many producers as keep up (about 550 cycles a fill each) with a tile's epilogue, about 8 cycles per column: idle ones wait at the
+    // CTA's last barrier and poll nothing
+    a.takers = (plan.taps * ((plan.Cin + plan.BK - 1) / plan.BK) * 550 + plan.BN * 8 - 1) / (plan.BN * 8);
+    a.takers = std::min(a.takers, std::min(plan.stages, NUM_PRODUCERS));
     a.stages = plan.stages; a.a_im2col = plan.a_im2col;
     a.grouped = plan.grouped;
     a.res_slots = plan.res_slots ? plan.res_slots : 2;

@@ -128,7 +128,7 @@ struct PatchPlan {
     int patch_alloc;      // bytes reserved per patch buffer
     int b_stream;         // weights stream through a ring (too large to stay resident)
     int bring;            // slots of that ring (one filter tap each)
-    int stage_cols;       // columns an epilogue warp stages per pass
+    int nbuf;             // patch buffers
     int in_unsigned;
     int num_sms;
     int late_weights;     // the weights are the previous kernel's output (see IgemmPlan)

@@ -16,7 +16,7 @@
 // and the output rows are written into that slice.  The tensor core multiplies 64 times more than the layer needs,
 // and still outruns the CUDA cores, where a byte dot product issues at a quarter of the integer rate.
 //
-// Warp 0 loads (weights once, patches double-buffered), warps 1-2 issue tcgen05.mma kind::i8 for alternate
+// Warp 0 loads (weights once, patches into two to four buffers), warps 1-4 issue tcgen05.mma kind::i8 for alternate
 // tiles into a ring of four TMEM accumulators, and four groups of four epilogue warps (one warp per TMEM lane quadrant) each
 // drain every fourth tile: 32-bit requantisation in the fragment layout, the bytes going from the registers straight to
 // the NHWC output (eight consecutive channels per lane).  Every wait is bounded.
@@ -35,6 +35,7 @@ static constexpr int P_EPI_WARP0 = 1 + P_ISSUERS;
 static constexpr int P_THREADS = 32 * (P_EPI_WARP0 + P_EPI_WARPS);
 static constexpr int P_BRING_MIN = 4;         // weight ring slots (one filter tap each) when the weights stream:
 static constexpr int P_BRING_MAX = 8;         // as many as shared memory holds between these two
+static constexpr int P_BUFS_MAX = 4;          // patch buffers: small patches are consumed faster than two loads arrive
 
 struct PatchArgs {
     int B, oH, oW, N, BN, C;   // N, C: output and input channels of one group (= of the layer when G == 1)
@@ -47,10 +48,10 @@ struct PatchArgs {
     int n_base;             // first image of this call within the tensors (batch slices)
     int patch_bytes;        // bytes one patch load delivers (the full TMA box)
     int patch_alloc;        // bytes reserved per patch buffer (box + the rows a last tile may read past it)
+    int nbuf;               // patch buffers
     int late_weights;       // weights only after the dependency wait
     int b_stream;           // weights too large to stay resident: their tap blocks stream through a ring
     int bring;              // slots of that ring
-    int stage_cols;         // columns an epilogue warp stages per pass (BN, or 32 to leave room for the ring)
     unsigned rcp_Wp;        // ceil(2^32 / Wp)
     unsigned idesc, tmem_cols;
     void* out;
@@ -106,18 +107,16 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     const int b_tap_bytes = a.BN * a.C;
     unsigned char* res_b = smem;                                              // [taps][BN][C], or a ring of a.bring taps
     unsigned char* patch0 = smem + (((size_t)(a.b_stream ? a.bring : taps) * b_tap_bytes + 1023) & ~(size_t)1023);
-    unsigned char* stage_out = patch0 + 2 * (size_t)a.patch_alloc;             // [16 warps][32 rows][stage_cols]
-    const int region_bytes = 32 * a.stage_cols;
-    unsigned long long* bars = (unsigned long long*)(stage_out + (size_t)P_EPI_WARPS * region_bytes);
-    // bars: patch_full[2], patch_empty[2], tmem_full[4], tmem_empty[4], weights, (spare), ring_full[8], ring_empty[8]
+    unsigned long long* bars = (unsigned long long*)(patch0 + (size_t)a.nbuf * a.patch_alloc);
+    // bars: patch_full[4], patch_empty[4], tmem_full[4], tmem_empty[4], weights, (spare), ring_full[8], ring_empty[8]
     const unsigned pfull0 = smem_u32(bars);
-    const unsigned pempty0 = pfull0 + 16u;
-    const unsigned tfull0 = pempty0 + 16u;
+    const unsigned pempty0 = pfull0 + 8u * P_BUFS_MAX;
+    const unsigned tfull0 = pempty0 + 8u * P_BUFS_MAX;
     const unsigned tempty0 = tfull0 + 8u * P_SLOTS;
     const unsigned bfull = tempty0 + 8u * P_SLOTS;
     const unsigned rfull0 = bfull + 16u;
     const unsigned rempty0 = rfull0 + 8u * P_BRING_MAX;
-    unsigned* tmem_slot = (unsigned*)(bars + 4 + 2 * P_SLOTS + 2 + 2 * P_BRING_MAX);
+    unsigned* tmem_slot = (unsigned*)(bars + 2 * P_BUFS_MAX + 2 * P_SLOTS + 2 + 2 * P_BRING_MAX);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     int* par = (int*)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);   // [FAST_NP][256]
 
@@ -126,7 +125,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     pdl_launch_dependents();
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < P_BUFS_MAX; ++s) {
             mbar_init(pfull0 + 8u * s, 1);
             mbar_init(pempty0 + 8u * s, P_ISSUERS);
         }
@@ -182,14 +181,13 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                     tma_load_2d(smem_u32(res_b + (size_t)t * b_tap_bytes), &tmB, bfull, t * a.C, ch0);
             }
             pdl_wait();   // weights are constants; the activations are the previous kernel's output
-            unsigned it = 0;
+            unsigned pb = 0, ph = 0;   // patch buffer and its phase
             int rs = 0;              // weight ring slot and its phase
             unsigned rph = 0;
             bool ok = true;
             int n = cta / a.bands, band = cta % a.bands;
             const int step_n = nctas / a.bands, step_b = nctas % a.bands;
-            for (int item = cta; item < items; item += nctas, ++it) {
-                const unsigned pb = it & 1u, ph = (it >> 1) & 1u;
+            for (int item = cta; item < items; item += nctas) {
                 if (!mbar_wait(pempty0 + 8u * pb, ph ^ 1u, abort_flag, a.status, 1)) break;
                 mbar_expect_tx(pfull0 + 8u * pb, (unsigned)a.patch_bytes);
                 tma_load_4d(smem_u32(patch0 + (size_t)pb * a.patch_alloc), &tmA, pfull0 + 8u * pb, grp * a.C, -a.pL,
@@ -208,6 +206,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                     }
                     if (!ok) break;
                 }
+                if (++pb == (unsigned)a.nbuf) { pb = 0; ph ^= 1u; }
                 n += step_n;
                 band += step_b;
                 if (band >= a.bands) { band -= a.bands; ++n; }
@@ -226,14 +225,13 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
             const int ksteps = a.C / 32;
             const unsigned row_step = (unsigned)((a.dY * a.Wp * a.C) >> 4), col_step = (unsigned)((a.dX * a.C) >> 4);
             const unsigned btap = (unsigned)(b_tap_bytes >> 4);
-            unsigned it = 0, seq = 0;
+            unsigned pb = 0, ph = 0, seq = 0;
             int band = cta % a.bands;
             const int step_b = nctas % a.bands;
             const unsigned tile_step = (unsigned)((PBM * a.C) >> 4);
             int rs = 0;              // weight ring slot and its phase (streamed weights)
             unsigned rph = 0;
-            for (int item = cta; item < items && ok; item += nctas, ++it) {
-                const unsigned pb = it & 1u, ph = (it >> 1) & 1u;
+            for (int item = cta; item < items && ok; item += nctas) {
                 const int T = band_tiles(band);
                 if (!mbar_wait_uniform(pfull0 + 8u * pb, ph, abort_flag, a.status, 3)) { ok = false; break; }
                 tc_fence_after();
@@ -275,6 +273,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                     }
                     __syncwarp();
                     seq += (unsigned)T;
+                    if (++pb == (unsigned)a.nbuf) { pb = 0; ph ^= 1u; }
                     band += step_b;
                     if (band >= a.bands) band -= a.bands;
                     continue;
@@ -309,6 +308,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                 }
                 if (ok && elect_one()) tc_commit(pempty0 + 8u * pb);   // the patch is free once every issuer's MMAs have read it
                 __syncwarp();
+                if (++pb == (unsigned)a.nbuf) { pb = 0; ph ^= 1u; }
                 band += step_b;
                 if (band >= a.bands) band -= a.bands;
             }
@@ -384,17 +384,15 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 static constexpr size_t P_RESIDENT_MAX = 96 * 1024;
 static bool patch_streams(int taps, int C, int BN) { return (size_t)taps * BN * C > P_RESIDENT_MAX; }
 
-static int patch_stage_cols(int taps, int C, int BN) { return patch_streams(taps, C, BN) ? 32 : BN; }
-
-// (The term with patch_stage_cols is a staging area the epilogue no longer uses since it stores from its registers.  It
-// stays in the budget because it caps the band height: with that area given to the patches, the 64-channel 55 x 55
-// layers went from five bands of 11 rows to 22 + 22 + 11 and ran 18 % slower.)
-static size_t patch_smem_bytes(int taps, int C, int BN, int patch_alloc, int bring = P_BRING_MIN)
+// (`spare` caps the band height of two buffers: with that space given to the patches, the 64-channel 55 x 55 layers went from
+// five bands of 11 rows to 22 + 22 + 11 and ran 18 % slower.  More buffers may use it.)
+static size_t patch_smem_bytes(int taps, int C, int BN, int patch_alloc, int bring = P_BRING_MIN, int nbuf = 2)
 {
     const int blocks = patch_streams(taps, C, BN) ? bring : taps;
     const size_t b = (((size_t)blocks * BN * C) + 1023) & ~(size_t)1023;
-    return 1024 + b + 2 * (size_t)patch_alloc + (size_t)P_EPI_WARPS * 32 * patch_stage_cols(taps, C, BN)
-         + (4 + 2 * P_SLOTS + 2 + 2 * P_BRING_MAX) * 8 + 32 + FAST_NP * 256 * 4 + 64;
+    const size_t spare = nbuf == 2 ? (size_t)P_EPI_WARPS * 32 * (patch_streams(taps, C, BN) ? 32 : BN) : 0;
+    return 1024 + b + nbuf * (size_t)patch_alloc + spare + (2 * P_BUFS_MAX + 2 * P_SLOTS + 2 + 2 * P_BRING_MAX) * 8 + 32
+         + FAST_NP * 256 * 4 + 64;
 }
 
 // bytes a patch buffer must hold for bands of R rows: the tiles of a band read 128-row operands that start
@@ -506,10 +504,11 @@ int patch_make_plan(PatchPlan* plan, const void* in, const int8_t* w, const Conv
     return 0;
 }
 
-// Rows per band.  A CTA takes every nth band, so the call lasts as long as the CTA with the most bands: the height with the
-// shortest such run wins, counted in 128-position tiles plus one tile per band (its load and hand-over); ties go to the
-// taller band (fewer halo rows re-read).  A tall band that wastes no tile leaves SMs idle at a small batch (one image of 55 x 55: 5 bands of 11 rows
-// 10.4 us) and rounds badly when an SM gets one band and a half.
+// Rows per band: among the heights that fit shared memory (and the 256-row TMA box), the one that wastes the fewest
+// 128-position tiles per image; ties go to the taller band (fewer halo rows re-read).  When that leaves the SMs fewer than two bands
+// each, a CTA's longest run decides instead, counted in tiles plus one per band (one image of 55 x 55: 5 bands of 11 rows
+// 10.4 us, 28 bands of 2 rows 7.5 us).  At larger batches even runs do not pay for tall bands: 1024 such images take 124 us in bands of 11
+// rows (25 tiles per image), 159 us in bands of 17 (26).
 int patch_set_batch(PatchPlan* plan, const ConvGeom& g0, int batch)
 {
     if (plan->band_batch == batch) return 0;
@@ -517,20 +516,21 @@ int patch_set_batch(PatchPlan* plan, const ConvGeom& g0, int batch)
     const int taps = g.kH * g.kW, Wp = plan->Wp;
     const long long ctas = plan->num_sms / plan->G > 0 ? plan->num_sms / plan->G : 1;
     int best_R = 0;
-    double best = 0.0;
-    for (int R = 1; R <= g.oH; ++R) {
-        if (R + (g.kH - 1) * g.dY > 256) break;
-        if (patch_smem_bytes(taps, g.C, plan->BN, patch_alloc_bytes(g, Wp, R)) > 226 * 1024) break;
-        // streamed weights: every tile of a band accumulates while the taps pass, so a band has at most as many
-        // tiles as there are accumulators
-        if (plan->b_stream && (R * Wp + PBM - 1) / PBM > P_SLOTS) break;
-        const int bands = (g.oH + R - 1) / R, rest = g.oH - (bands - 1) * R;
-        const double per_image = (bands - 1) * ((R * Wp + PBM - 1) / PBM + 1.0) + (rest * Wp + PBM - 1) / PBM + 1.0;
-        const long long items = (long long)batch * bands, rounds = (items + ctas - 1) / ctas;
-        // the longest run: whole rounds of average bands, one tall band at least
-        double t = per_image / bands * (double)rounds;
-        if (items <= ctas) t = (R * Wp + PBM - 1) / PBM + 1.0;
-        if (best_R == 0 || t <= best * 1.0001) { best_R = R; best = t; }
+    for (int even = 0; even < 2; ++even) {
+        long long best = 0;
+        for (int R = 1; R <= g.oH; ++R) {
+            if (R + (g.kH - 1) * g.dY > 256) break;
+            if (patch_smem_bytes(taps, g.C, plan->BN, patch_alloc_bytes(g, Wp, R)) > 226 * 1024) break;
+            // streamed weights: every tile of a band accumulates while the taps pass, so a band has at most as many
+            // tiles as there are accumulators
+            const int tall = (R * Wp + PBM - 1) / PBM;
+            if (plan->b_stream && tall > P_SLOTS) break;
+            const int bands = (g.oH + R - 1) / R, rest = g.oH - (bands - 1) * R;
+            const long long cost = even ? ((long long)batch * bands + ctas - 1) / ctas * (tall + 1)
+                                        : (long long)(bands - 1) * tall + (rest * Wp + PBM - 1) / PBM;
+            if (best == 0 || cost <= best) { best_R = R; best = cost; }
+        }
+        if (best_R == 0 || (long long)batch * ((g.oH + best_R - 1) / best_R) >= 2 * ctas) break;
     }
     if (best_R == 0) return -1;
     plan->band_batch = batch;
@@ -540,12 +540,15 @@ int patch_set_batch(PatchPlan* plan, const ConvGeom& g0, int batch)
     const int box_rows = best_R + (g.kH - 1) * g.dY;
     plan->patch_bytes = box_rows * plan->Wp * g.C;
     plan->patch_alloc = patch_alloc_bytes(g, plan->Wp, best_R);
-    plan->stage_cols = patch_stage_cols(taps, g.C, plan->BN);
     plan->bring = P_BRING_MIN;
     while (plan->b_stream && plan->bring < P_BRING_MAX
            && patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring + 1) <= 226 * 1024)
         ++plan->bring;
-    plan->smem_bytes = patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring);
+    plan->nbuf = 2;
+    while (plan->nbuf < P_BUFS_MAX
+           && patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring, plan->nbuf + 1) <= 226 * 1024)
+        ++plan->nbuf;
+    plan->smem_bytes = patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring, plan->nbuf);
     // NHWC activations as (C, W, H, B); one box = a whole patch, zero-filled outside the image
     const CUtensorMapSwizzle swz = g.C == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                                               : (g.C == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
@@ -575,7 +578,7 @@ cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, 
     a.b_stream = plan.b_stream;
     a.late_weights = plan.late_weights;
     a.bring = plan.bring;
-    a.stage_cols = plan.stage_cols;
+    a.nbuf = plan.nbuf;
     a.rcp_Wp = (unsigned)(((1ull << 32) + (unsigned)plan.Wp - 1) / (unsigned)plan.Wp);
     a.idesc = (2u << 4) | ((plan.in_unsigned ? 0u : 1u) << 7) | (1u << 10) | ((unsigned)(plan.BN >> 3) << 17)
             | ((unsigned)(PBM >> 4) << 24);

@@ -585,21 +585,23 @@ static int s2d_use_bands(StemS2dPlan* plan, const ConvGeom& g, int R)
                                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -1;
 }
 
-// The band height with the shortest longest run of a CTA (see patch_set_batch).  One 224 x 224 image in three bands of 38 rows: 20 us; 64 images in
-// 192 such bands: one CTA in four works twice as long as the others.
+// The band height: fewest tiles per image, or a CTA's shortest run at small batches (see patch_set_batch).  One 224 x 224 image in three bands
+// of 38 rows: 20 us, in 112 bands of one row: 8 us.
 int stem_s2d_set_batch(StemS2dPlan* plan, const ConvGeom& g, int batch)
 {
     if (plan->P || plan->band_batch == batch) return 0;
     int best_R = 0;
-    double best = 0.0;
-    for (int R = 1; R <= g.oH; ++R) {
-        if (R + plan->KH - 1 > 256) break;
-        if (s2d_smem_bytes(plan->w_bytes, plan->BN, s2d_band_alloc(plan->Wp, plan->KH, plan->KWp, R)) > 226 * 1024) break;
-        const int bands = (g.oH + R - 1) / R, rest = g.oH - (bands - 1) * R, tall = (R * plan->Wp + ZBM - 1) / ZBM;
-        const double per_image = (bands - 1) * (tall + 1.0) + (rest * plan->Wp + ZBM - 1) / ZBM + 1.0;
-        const long long items = (long long)batch * bands, rounds = (items + plan->num_sms - 1) / plan->num_sms;
-        const double t = items <= plan->num_sms ? tall + 1.0 : per_image / bands * (double)rounds;
-        if (best_R == 0 || t <= best * 1.0001) { best_R = R; best = t; }
+    for (int even = 0; even < 2; ++even) {
+        long long best = 0;
+        for (int R = 1; R <= g.oH; ++R) {
+            if (R + plan->KH - 1 > 256) break;
+            if (s2d_smem_bytes(plan->w_bytes, plan->BN, s2d_band_alloc(plan->Wp, plan->KH, plan->KWp, R)) > 226 * 1024) break;
+            const int bands = (g.oH + R - 1) / R, rest = g.oH - (bands - 1) * R, tall = (R * plan->Wp + ZBM - 1) / ZBM;
+            const long long cost = even ? ((long long)batch * bands + plan->num_sms - 1) / plan->num_sms * (tall + 1)
+                                        : (long long)(bands - 1) * tall + (rest * plan->Wp + ZBM - 1) / ZBM;
+            if (best == 0 || cost <= best) { best_R = R; best = cost; }
+        }
+        if (best_R == 0 || (long long)batch * ((g.oH + best_R - 1) / best_R) >= 2 * plan->num_sms) break;
     }
     if (best_R == 0) return -1;
     plan->band_batch = batch;
