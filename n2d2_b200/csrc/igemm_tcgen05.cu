@@ -111,7 +111,11 @@ __device__ __forceinline__ void expand_int4_x16(unsigned x, unsigned& w0, unsign
 // W4: the weights sit in HBM as packed 4-bit values.  The producer's TMA load brings a BN x BK/2-byte packed block
 // into the stage beside the operand tiles; four extra warps expand it into the swizzled int8 B tile the MMA reads
 // (as 16 x the weight, see expand_int4_x16) and signal the issuing thread through one more barrier per stage.
-template <int MODE, bool W4>
+// DRY: a short launch (up to two tiles per CTA) spends a microsecond per role on instruction-cache misses once its data is
+// there, so its issuer and epilogue warps run through their loop bodies once, without effect, while the previous kernel
+// still works.  A variant of its own: the flag tests cost the epilogue of long launches 2-3 % (conv2.x of ResNet-50 at 1024 images
+// with the residual sum 418 us against 403).
+template <int MODE, bool W4, bool DRY>
 __global__ void __launch_bounds__(W4 ? NUM_THREADS + 32 * W4_UNPACK_WARPS : NUM_THREADS, 1)
 igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmR,
@@ -194,9 +198,6 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     const unsigned tiles_s = smem_u32(tiles), res_b_s = smem_u32(res_b);
 
     const int num_tiles = a.num_m_tiles * a.num_n_tiles;
-    // A short launch (up to two tiles per CTA) spends a microsecond per role on instruction-cache misses once its data is there: its
-    // issuer and epilogue warps run through their loop bodies once, without effect, while the previous kernel still works.
-    const bool dry_run = FAST && num_tiles <= 2 * (int)gridDim.x;
 
     if (producer >= 0) {
         // ------------------------------------------------------------------ TMA producers
@@ -317,7 +318,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         const unsigned b16 = (unsigned)(b_stage_bytes >> 4);
         unsigned a_lo = a_lo0;
         MBAR_PEEK_DECLARE();
-        bool dry = dry_run;
+        bool dry = DRY;
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++acc_it) {
             const unsigned as = acc_it & ((1u << a.acc_shift) - 1u);
             const unsigned aph = (acc_it >> a.acc_shift) & 1u;
@@ -423,7 +424,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             return true;
         };
         if (FAST && (int)blockIdx.x < num_tiles) ok = stage_constants((int)blockIdx.x % a.num_n_tiles);   // constants: before the wait
-        bool dry = dry_run;
+        bool dry = DRY;
         if (!dry) pdl_wait();   // residual loads and output stores touch tensors the previous kernel reads or writes
         // several groups only where the CTA's column block never changes (step_n is 0 or the CTA has one tile)
         const int groups = FAST ? a.groups : 1;
@@ -946,7 +947,9 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
     plan->BK = (g.C % 128 == 0) ? 128 : (g.C % 64 == 0 ? 64 : 32);
     int bn = force_bn;
     if (bn == 0) {
-        bn = (g.O >= 256) ? 256 : (g.O > 64 ? 128 : 64);
+        // 256 columns halve the activation traffic of a streamed layer.  With a residual sum 128 are better, two tiles in the
+        // epilogue at once: conv5.2 of ResNet-50 at 1024 images 74 us against 90, conv5.1 135 / 158, conv2.x and conv3.x even.
+        bn = (g.O >= 256 && !res) ? 256 : (g.O > 64 ? 128 : 64);
         // a layer with few output pixels (the classifier, late stages at small batch) would leave most
         // SMs without a tile: narrower column blocks give more tiles
         const long long m_tiles = ((long long)g.B * g.oH * g.oW + BM - 1) / BM;
@@ -1182,20 +1185,23 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     a.acc_shift = use_fast ? (plan.parts == 4 ? 1 : (plan.parts == 2 ? 2 : 3)) : 1;
     a.tmem_cols = (unsigned)plan.BN << a.acc_shift;
     const int mode = !use_fast ? 0 : (r.ptr ? (fast.need_clamp ? 2 : (fast.dp4a ? 5 : 4)) : (fast.need_clamp ? 1 : 3));
+    typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const IgemmArgs);
+    static const Kernel kernels[3][6] = {
+        {igemm_i8_tcgen05_kernel<0, false, false>, igemm_i8_tcgen05_kernel<1, false, false>, igemm_i8_tcgen05_kernel<2, false, false>,
+         igemm_i8_tcgen05_kernel<3, false, false>, igemm_i8_tcgen05_kernel<4, false, false>, igemm_i8_tcgen05_kernel<5, false, false>},
+        {igemm_i8_tcgen05_kernel<0, false, false>, igemm_i8_tcgen05_kernel<1, false, true>, igemm_i8_tcgen05_kernel<2, false, true>,
+         igemm_i8_tcgen05_kernel<3, false, true>, igemm_i8_tcgen05_kernel<4, false, true>, igemm_i8_tcgen05_kernel<5, false, true>},
+        {igemm_i8_tcgen05_kernel<0, true, false>, igemm_i8_tcgen05_kernel<1, true, false>, igemm_i8_tcgen05_kernel<2, true, false>,
+         igemm_i8_tcgen05_kernel<3, true, false>, igemm_i8_tcgen05_kernel<4, true, false>, igemm_i8_tcgen05_kernel<5, true, false>}};
     static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        const void* variants[12] = {(const void*)igemm_i8_tcgen05_kernel<0, false>, (const void*)igemm_i8_tcgen05_kernel<1, false>,
-                                    (const void*)igemm_i8_tcgen05_kernel<2, false>, (const void*)igemm_i8_tcgen05_kernel<3, false>,
-                                    (const void*)igemm_i8_tcgen05_kernel<4, false>, (const void*)igemm_i8_tcgen05_kernel<5, false>,
-                                    (const void*)igemm_i8_tcgen05_kernel<0, true>, (const void*)igemm_i8_tcgen05_kernel<1, true>,
-                                    (const void*)igemm_i8_tcgen05_kernel<2, true>, (const void*)igemm_i8_tcgen05_kernel<3, true>,
-                                    (const void*)igemm_i8_tcgen05_kernel<4, true>, (const void*)igemm_i8_tcgen05_kernel<5, true>};
-        for (const void* fn : variants) {
-            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (e != cudaSuccess) return e;
-        }
+        for (auto& set : kernels)
+            for (Kernel fn : set) {
+                cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+                if (e != cudaSuccess) return e;
+            }
         attr_set[dev] = true;
     }
     int tiles = a.num_m_tiles * a.num_n_tiles;
@@ -1238,13 +1244,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
                               plan.tmB, plan.tmO32, a);
         }
     }
-    typedef void (*Kernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const IgemmArgs);
-    static const Kernel kernels[2][6] = {
-        {igemm_i8_tcgen05_kernel<0, false>, igemm_i8_tcgen05_kernel<1, false>, igemm_i8_tcgen05_kernel<2, false>,
-         igemm_i8_tcgen05_kernel<3, false>, igemm_i8_tcgen05_kernel<4, false>, igemm_i8_tcgen05_kernel<5, false>},
-        {igemm_i8_tcgen05_kernel<0, true>, igemm_i8_tcgen05_kernel<1, true>, igemm_i8_tcgen05_kernel<2, true>,
-         igemm_i8_tcgen05_kernel<3, true>, igemm_i8_tcgen05_kernel<4, true>, igemm_i8_tcgen05_kernel<5, true>}};
-    return launch_pdl(kernels[plan.w4 ? 1 : 0][mode], grid, NUM_THREADS + (plan.w4 ? 32 * W4_UNPACK_WARPS : 0), plan.smem_bytes, s,
+    return launch_pdl(kernels[plan.w4 ? 2 : (tiles <= 2 * grid ? 1 : 0)][mode], grid, NUM_THREADS + (plan.w4 ? 32 * W4_UNPACK_WARPS : 0), plan.smem_bytes, s,
                       plan.tmA, plan.tmB, plan.tmO, plan.tmR, a);
 }
 
