@@ -244,7 +244,8 @@ int n2d2b_net_weight_bytes(const n2d2b_net* net, size_t* total_bytes, size_t* pa
 /* Number of kernel launches one forward of `batch` images issues. */
 int n2d2b_net_launches_per_forward(const n2d2b_net* net);
 /* Name of the kernel family cell `cell` runs on ("tcgen05", "tcgen05-pair", "tcgen05-w4", "patch-tcgen05",
- * "stem-tcgen05", "simt", "depthwise", "pool", "sum", "fused"). */
+ * "stem-tcgen05", "simt", "depthwise", "depthwise-tcgen05", "pool", "sum", "fused").  "depthwise-tcgen05" cells with 3x3 filters
+ * run on the CUDA-core kernel in calls where that one is faster. */
 const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell);
 /* Device time of every cell of one forward, in milliseconds (CUDA events on `stream`), like the
  * per-cell timings of DeepNet::propagate (src/DeepNet.cpp:2705-2717). ms has one entry per cell. */

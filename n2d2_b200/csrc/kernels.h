@@ -44,6 +44,10 @@ struct FastQuant;
 // `fast` (when enabled): the proved 32-bit rescale; 3x3 filters then take the dot-product kernel
 cudaError_t launch_conv_depthwise(const void* in, int in_unsigned, const int8_t* w_hwc, const ConvGeom& g,
                                   const QuantDev& q, const FastQuant& fast, void* out, cudaStream_t s);
+// 3x3 depthwise layers, stride 1 or 2, on the 32-bit or floating-point epilogue
+bool depthwise3x3_eligible(const ConvGeom& g);
+cudaError_t launch_depthwise3x3(const void* in, int in_unsigned, const int8_t* w_hwc, const ConvGeom& g, const FastQuant& fast, void* out,
+                                int num_sms, cudaStream_t s);
 cudaError_t launch_pool(const void* in, int in_unsigned, const PoolGeom& g, void* out, cudaStream_t s);
 cudaError_t launch_pool_i32(const void* in, const PoolGeom& g, void* out, cudaStream_t s);
 cudaError_t launch_elemwise_sum(const SumInputs& ins, size_t pixels, int C, const QuantDev& q,

@@ -107,6 +107,8 @@ struct CellRec {
     PatchPlan patch8{};
     int w8_rows = 0, w8_ng_src = 0, w8_ng_dst = 0;
     void* d_w8_out = nullptr;     // padded output matrix (see pad_O) of a widened cell
+    // 3x3 depthwise cells: weights as [kH][kW][C] for the dot-product kernel (see use_dw3x3)
+    int8_t* d_dw3x3 = nullptr;
     // tensor-core plan
     IgemmPlan plan{};
     bool has_plan = false;
@@ -653,6 +655,7 @@ void n2d2b_net_destroy(n2d2b_net* net)
         cudaFree(c.d_fast);
         cudaFree(c.d_pad4);
         cudaFree(c.d_colpad);
+        cudaFree(c.d_dw3x3);
         cudaFree(c.d_w8_out);
     }
     cudaFree(net->d_w8);
@@ -1172,6 +1175,14 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
             c.engine = ENG_DEPTHWISE;
             if (!(flags & N2D2B_EXACT64_EPILOGUE))
                 if (int rc = upload_fast(c, net->tensors[c.output])) return rc;
+            // [C][kH][kW] -> [kH][kW][C]: four or sixteen channels of a tap are one load
+            const int taps = g.kH * g.kW;
+            for (int ch = 0; ch < g.C; ++ch)
+                for (int t = 0; t < taps; ++t) laid[(size_t)t * g.C + ch] = c.weights[(size_t)ch * taps + t];
+            if (c.fast.enabled && !(flags & N2D2B_FORCE_SIMT) && depthwise3x3_eligible(g)) {
+                CUDA_TRY(cudaMalloc((void**)&c.d_dw3x3, laid.size()));
+                CUDA_TRY(cudaMemcpy(c.d_dw3x3, laid.data(), laid.size(), cudaMemcpyHostToDevice));
+            }
             // Stride-1 layers whose channels come in whole groups of 32 run on the tensor cores as block-diagonal
             // groups (patch kernel); it needs the 32-bit epilogue
             ConvGeom gb = g;
@@ -1221,10 +1232,6 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 cudaFree(c.d_weights);
                 c.d_weights = nullptr;
             }
-            // [C][kH][kW] -> [kH][kW][C] so that 16 channels of a tap are one 128-bit load
-            const int taps = g.kH * g.kW;
-            for (int ch = 0; ch < g.C; ++ch)
-                for (int t = 0; t < taps; ++t) laid[(size_t)t * g.C + ch] = c.weights[(size_t)ch * taps + t];
         } else {
             c.engine = ENG_SIMT;
         }
@@ -1395,6 +1402,15 @@ static int fuse_stem_pool(n2d2b_net* net)
 }
 
 // ---- forward --------------------------------------------------------------------------------
+// Whether a 3x3 depthwise cell runs on the dot-product kernel in a call of `batch` images.  The block-diagonal form on the tensor
+// cores moves whole bands of large maps at a time: it is even or ahead where there are many pixels of few channels (256 images:
+// 56 x 56 x 128 70 us against 74, 112 x 112 x 32 73 / 74), behind on deep maps (14 x 14 x 512 31 / 24, 7 x 7 x 1024 30 / 17) and in small
+// calls, whose bands leave SMs idle (33 images: 112 x 112 x 32 23 / 16, 14 x 14 x 512 12.4 / 10.3).
+static bool use_dw3x3(const CellRec& c, int batch)
+{
+    return c.d_dw3x3 && (c.geom.C >= 256 || (long long)batch * c.geom.oH * c.geom.oW * c.geom.C < (1ll << 24));
+}
+
 // Runs one cell on images [img0, img0 + batch) of the batch (img0 != 0 only for cells without tensor maps).
 static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, cudaStream_t s, int img0 = 0)
 {
@@ -1434,6 +1450,13 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         CUDA_TRY(launch_igemm(p, c.q.dev, r, c.fast, c.d_w8_out ? c.d_w8_out : out, DT_I8, (int)row0, net->d_status, s));
         if (c.d_w8_out)
             CUDA_TRY(launch_drop_padded_columns((const uint8_t*)c.d_w8_out + row0 * c.w8_rows, c.w8_rows, (uint8_t*)out + row0 * g.O, g.O, (size_t)p.M, s));
+        return 0;
+    }
+    if (use_dw3x3(c, batch)) {
+        ConvGeom g = c.geom;
+        g.B = batch;
+        const size_t in_off = mapped ? (size_t)img0 * tin.bytes_per_image() : 0, out_off = mapped ? (size_t)img0 * tout.bytes_per_image() : 0;
+        CUDA_TRY(launch_depthwise3x3((const uint8_t*)in0 + in_off, tin.is_unsigned, c.d_dw3x3, g, c.fast, (uint8_t*)out + out_off, net->num_sms, s));
         return 0;
     }
     switch (c.engine) {

@@ -23,10 +23,10 @@ __device__ __forceinline__ void prefetch_tensor_map(const CUtensorMap* tm) { asm
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... P, typename... A>
-static inline cudaError_t launch_pdl(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args)
+static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;

@@ -79,6 +79,21 @@ def test_depthwise_3x3(case, mode):
     compare_net(net, 3, flags=KEEP | R.EXACT64_EPILOGUE, want_engine='depthwise')
 
 
+# (C, H, W, stride, pad, input unsigned, activation, batch): the dot-product kernel - pairs of columns with an odd rest, one and
+# two columns, strips of rows, channel words that do not divide a block, and either side of where small calls take it
+DW_DOT_CASES = [(144, 15, 13, 1, 1, True, 'relu', 5), (528, 7, 9, 1, 0, False, 'linear', 3), (272, 9, 1, 1, 1, True, 'relu', 2),
+                (256, 2, 2, 2, 1, False, 'relu', 3), (1040, 11, 8, 2, 0, True, 'linear', 2), (256, 33, 31, 2, 2, True, 'relu', 4),
+                (2048, 5, 4, 1, 2, True, 'relu', 1), (64, 112, 112, 1, 1, True, 'relu', 20), (64, 112, 112, 1, 1, True, 'relu', 21),
+                (512, 14, 14, 1, 1, False, 'linear', 300)]
+
+
+@pytest.mark.parametrize('case', DW_DOT_CASES, ids=lambda c: 'C%d_%dx%d_s%d_p%d_%s_%s_b%d' % c)
+@pytest.mark.parametrize('mode', ['single', 'fixed', 'float'])
+def test_depthwise_3x3_dot_products(case, mode):
+    C, H, W, s, p, uns, act, batch = case
+    compare_net(single_conv_net(C, H, W, C, 3, s, p, in_unsigned=uns, act=act, mode=mode, groups=C), batch)
+
+
 # (C, H, W, k, pad, dilation, batch): depthwise layers as block-diagonal groups on the tensor cores - several bands
 # and images per CTA, more groups than fit the grid evenly, 5x5 and dilated filters, one group of 32
 # (C, H, W, k, stride, pad, dilation, batch): the strided ones through im2col loads of the group's channel slice
