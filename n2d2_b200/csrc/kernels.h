@@ -86,6 +86,7 @@ struct FastQuant {
     bool dp_t_unsigned = false; //   the cell's own output is packed as unsigned bytes (natively, or shifted by +128)
     unsigned dp_xor = 0;        //   bytes to flip from unsigned to signed (0x80 per byte)
     int dp_a_signed = 1;        //   signedness of the (t, r) byte vector
+    bool monotone = false;      // no multiplier of the cell's own rescale is negative: it never decreases
     bool enabled = false;
 };
 
@@ -112,6 +113,8 @@ int stem_s2d_set_batch(StemS2dPlan* plan, const ConvGeom& g, int batch);
 bool stem_s2d_eligible(const ConvGeom& g);
 bool stem_s2d_pool_eligible(const ConvGeom& g, const PoolGeom& p);
 void stem_s2d_dims(const ConvGeom& g, int* Hs, int* Ws);
+// Image shift, filter rows and (even) filter columns after space-to-depth
+void stem_s2d_filter(const ConvGeom& g, int* P, int* KH, int* KWp);
 size_t stem_s2d_weight_bytes(const ConvGeom& g);
 void stem_s2d_arrange_weights(const ConvGeom& g, const int8_t* w_ohwi, int8_t* dst);
 cudaError_t launch_s2d_image(const void* in, const ConvGeom& g, int batch, void* out, cudaStream_t s);
@@ -120,6 +123,20 @@ int stem_s2d_make_plan(StemS2dPlan* plan, const void* d_s2d, const int8_t* d_w_a
                        int in_unsigned, int num_sms, const char** why, const PoolGeom* pool = nullptr);
 cudaError_t launch_stem_s2d(const StemS2dPlan& plan, const ConvGeom& g, int n_base, const FastQuant& fast, void* out,
                             int* status_word, cudaStream_t s);
+
+// ---- stride-2 first layer of 64 channels with the 3x3 / 2 max pooling behind it (monotone rescales only) ----
+struct StemPoolPlan {
+    CUtensorMap tmX;      // re-laid image as (8-byte words, rows, images); box = two rows
+    const int8_t* w;
+    int KH, KWp, Wp, w_bytes, poH, poW, in_unsigned, num_sms;
+    size_t smem_bytes;
+};
+bool stem_pool_eligible(const ConvGeom& g, const PoolGeom& p);
+size_t stem_pool_weight_bytes(const ConvGeom& g);
+void stem_pool_arrange_weights(const ConvGeom& g, const int8_t* w_ohwi, int8_t* dst);
+int stem_pool_make_plan(StemPoolPlan* plan, const void* d_s2d, const int8_t* d_w_arranged, const ConvGeom& g, const PoolGeom& p, int max_batch,
+                        int in_unsigned, int num_sms, const char** why);
+cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_base, const FastQuant& fast, void* out, int* status_word, cudaStream_t s);
 
 // ---- stride-1 convolution from a shared-memory input patch (tcgen05 kind::i8) ----
 struct PatchPlan {

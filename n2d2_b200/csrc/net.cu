@@ -89,6 +89,8 @@ struct CellRec {
     // a max pooling folded into the first-layer kernel (the cell's output then is the pooled tensor)
     bool pool_fused = false;
     PoolGeom fused_pool{};
+    bool pool_first = false;  // by the kernel that pools the accumulators (stem_pool), else by the one that pools bytes
+    StemPoolPlan stem_pool{};
     // first-layer tensor-core kernels
     StemPlan stem{};
     StemS2dPlan stem2{};
@@ -540,6 +542,8 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
     c.fast.dp_t_unsigned = dp_t_unsigned;
     c.fast.dp_xor = dp_xor;
     c.fast.dp_a_signed = dp_a_signed;
+    c.fast.monotone = true;   // (row 2: a multiplier, or a factor as the bits of a float)
+    for (int ch = 0; ch < C; ++ch) c.fast.monotone = c.fast.monotone && f1[(size_t)2 * cpad + ch] >= 0;
     c.fast.enabled = true;
     return 0;
 }
@@ -1099,8 +1103,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
     net->max_batch = max_batch;
     net->flags = flags;
     if (!(flags & N2D2B_NO_FUSION)) fuse_residuals(net);
-    if ((flags & N2D2B_FUSE_FIRST_POOL)
-        && !(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE)))
+    if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE)))
         if (int rc = fuse_stem_pool(net)) return rc;
     net->head_limit = head_candidate_prefix(net);
     if (int rc = plan_buffers(net)) return rc;
@@ -1128,8 +1131,9 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 if (int rc = upload_fast(c, net->tensors[c.output])) return rc;
             if (c.fast.enabled && stem_s2d_eligible(g)) {
                 // stride 2: space-to-depth image, no gather
-                std::vector<int8_t> arranged(stem_s2d_weight_bytes(g));
-                stem_s2d_arrange_weights(g, c.weights.data(), arranged.data());
+                std::vector<int8_t> arranged(c.pool_first ? stem_pool_weight_bytes(g) : stem_s2d_weight_bytes(g));
+                if (c.pool_first) stem_pool_arrange_weights(g, c.weights.data(), arranged.data());
+                else stem_s2d_arrange_weights(g, c.weights.data(), arranged.data());
                 CUDA_TRY(cudaMalloc((void**)&c.d_weights, arranged.size() + 256));
                 CUDA_TRY(cudaMemcpy(c.d_weights, arranged.data(), arranged.size(), cudaMemcpyHostToDevice));
                 c.d_weight_bytes = arranged.size();
@@ -1137,8 +1141,10 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 stem_s2d_dims(g, &Hs, &Ws);
                 CUDA_TRY(cudaMalloc(&c.d_pad4, (size_t)max_batch * Hs * Ws * 16 + 256));
                 const char* why = "";
-                if (stem_s2d_make_plan(&c.stem2, c.d_pad4, c.d_weights, g, max_batch, net->tensors[c.inputs[0]].is_unsigned,
-                                       net->num_sms, &why, c.pool_fused ? &c.fused_pool : nullptr) == 0) {
+                const int uns = net->tensors[c.inputs[0]].is_unsigned;
+                if ((c.pool_first ? stem_pool_make_plan(&c.stem_pool, c.d_pad4, c.d_weights, g, c.fused_pool, max_batch, uns, net->num_sms, &why)
+                                  : stem_s2d_make_plan(&c.stem2, c.d_pad4, c.d_weights, g, max_batch, uns, net->num_sms, &why,
+                                                       c.pool_fused ? &c.fused_pool : nullptr)) == 0) {
                     net->launches++;
                     c.engine = ENG_STEM_S2D;
                     continue;
@@ -1385,10 +1391,12 @@ static int fuse_stem_pool(n2d2b_net* net)
             if (!net->cells[cj].skipped && net->cells[cj].inputs.size() == 1 && net->cells[cj].inputs[0] == t) { pj = (int)cj; break; }
         if (pj < 0 || net->cells[pj].type != CELL_POOL) continue;
         CellRec& p = net->cells[pj];
-        if (!stem_s2d_pool_eligible(c.geom, p.pgeom)) continue;
-        // the first-layer kernel needs the 32-bit epilogue
+        const bool first = stem_pool_eligible(c.geom, p.pgeom), bytes = (net->flags & N2D2B_FUSE_FIRST_POOL) && stem_s2d_pool_eligible(c.geom, p.pgeom);
+        if (!first && !bytes) continue;
+        // the first-layer kernels need the 32-bit epilogue
         if (int rc = upload_fast(c, net->tensors[t])) return rc;
-        if (!c.fast.enabled) continue;
+        c.pool_first = first && c.fast.enabled && c.fast.monotone;
+        if (!c.fast.enabled || !(c.pool_first || bytes)) continue;
         c.pool_fused = true;
         c.fused_pool = p.pgeom;
         net->tensors[t].readable = false;
@@ -1505,6 +1513,11 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         g.B = batch;
         int Hs = 0, Ws = 0;
         stem_s2d_dims(g, &Hs, &Ws);
+        if (c.pool_first) {
+            CUDA_TRY(launch_s2d_image(in0, g, batch, (uint8_t*)c.d_pad4 + (size_t)img0 * Hs * Ws * 16, s));
+            CUDA_TRY(launch_stem_pool(c.stem_pool, g, img0, c.fast, out, net->d_status, s));
+            break;
+        }
         if (stem_s2d_set_batch(&c.stem2, c.geom, batch)) return fail(N2D2B_ERR_INVALID, "first-layer plan failed for %d images", batch);
         CUDA_TRY(launch_s2d_image(in0, g, batch, (uint8_t*)c.d_pad4 + (size_t)img0 * Hs * Ws * 16, s));
         CUDA_TRY(launch_stem_s2d(c.stem2, g, img0, c.fast, out, net->d_status, s));

@@ -403,7 +403,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 
 // filter extents after space-to-depth; `off` = 1 when the padding is odd (the image is shifted by one more
 // pixel so that every output's window starts on an even pixel)
-static void s2d_filter(const ConvGeom& g, int* P, int* KH, int* KWp)
+void stem_s2d_filter(const ConvGeom& g, int* P, int* KH, int* KWp)
 {
     const int offy = g.pT & 1, offx = g.pL & 1;
     *P = g.pT + offy;
@@ -435,7 +435,7 @@ bool stem_s2d_eligible(const ConvGeom& g)
     if (g.pT != g.pL || g.kH > 16 || g.kW > 16) return false;
     if (g.O % 32 != 0 || g.O > 128 || g.oW < 2 || g.oH < 1) return false;
     int P, KH, KWp;
-    s2d_filter(g, &P, &KH, &KWp);
+    stem_s2d_filter(g, &P, &KH, &KWp);
     const int Wp = g.oW + KWp - 1;
     if (Wp * 2 > 256) return false;   // one row of the band is one row of the TMA box (8-byte elements)
     const int BN = g.O <= 64 ? 64 : 128;
@@ -447,7 +447,7 @@ bool stem_s2d_eligible(const ConvGeom& g)
 void stem_s2d_dims(const ConvGeom& g, int* Hs, int* Ws)
 {
     int P, KH, KWp;
-    s2d_filter(g, &P, &KH, &KWp);
+    stem_s2d_filter(g, &P, &KH, &KWp);
     *Hs = g.oH + KH - 1;
     *Ws = g.oW + KWp - 1;
 }
@@ -455,7 +455,7 @@ void stem_s2d_dims(const ConvGeom& g, int* Hs, int* Ws)
 size_t stem_s2d_weight_bytes(const ConvGeom& g)
 {
     int P, KH, KWp;
-    s2d_filter(g, &P, &KH, &KWp);
+    stem_s2d_filter(g, &P, &KH, &KWp);
     const int BN = g.O <= 64 ? 64 : 128;
     return (size_t)KH * BN * KWp * 16;
 }
@@ -466,7 +466,7 @@ size_t stem_s2d_weight_bytes(const ConvGeom& g)
 void stem_s2d_arrange_weights(const ConvGeom& g, const int8_t* w_ohwi, int8_t* dst)
 {
     int P, KH, KWp;
-    s2d_filter(g, &P, &KH, &KWp);
+    stem_s2d_filter(g, &P, &KH, &KWp);
     const int BN = g.O <= 64 ? 64 : 128;
     const int offy = P - g.pT, offx = P - g.pL;
     const size_t row_block = (size_t)BN * KWp * 16;
@@ -490,7 +490,7 @@ void stem_s2d_arrange_weights(const ConvGeom& g, const int8_t* w_ohwi, int8_t* d
 cudaError_t launch_s2d_image(const void* in, const ConvGeom& g, int batch, void* out, cudaStream_t s)
 {
     int P, KH, KWp, Hs, Ws;
-    s2d_filter(g, &P, &KH, &KWp);
+    stem_s2d_filter(g, &P, &KH, &KWp);
     stem_s2d_dims(g, &Hs, &Ws);
     const long long rows = (long long)batch * Hs;
     if (rows == 0) return cudaSuccess;
@@ -509,7 +509,7 @@ bool stem_s2d_pool_eligible(const ConvGeom& g, const PoolGeom& p)
         return false;
     // one pooled row per band must fit shared memory
     int P0, KH, KWp;
-    s2d_filter(g, &P0, &KH, &KWp);
+    stem_s2d_filter(g, &P0, &KH, &KWp);
     const int Wp = g.oW + KWp - 1, BN = g.O <= 64 ? 64 : 128, R = p.pH;
     const int cbuf = ((R * Wp + ZBM - 1) / ZBM) * ZBM * BN;
     return s2d_smem_bytes(KH * BN * KWp * 16, BN, s2d_band_alloc(Wp, KH, KWp, R), cbuf) <= 226 * 1024;
@@ -531,7 +531,7 @@ int stem_s2d_make_plan(StemS2dPlan* plan, const void* d_s2d, const int8_t* d_w_a
     }
     memset(plan, 0, sizeof(*plan));
     int P;
-    s2d_filter(g, &P, &plan->KH, &plan->KWp);
+    stem_s2d_filter(g, &P, &plan->KH, &plan->KWp);
     plan->BN = g.O <= 64 ? 64 : 128;
     plan->Wp = g.oW + plan->KWp - 1;
     plan->w_bytes = plan->KH * plan->BN * plan->KWp * 16;

@@ -499,6 +499,28 @@ def test_packed_int4_weights_stay_packed_in_hbm_and_fuse_residuals():
         assert 'fused' in eng and 'tcgen05-w4' in eng
 
 
+# (C, H, W, k, pad, activation, input unsigned, batch): first layers of 64 channels whose accumulators are pooled - every split of
+# the pooled columns over the epilogue lanes, odd sizes, one pooled row, filters of one to four image rows, one band per image and many
+STEM_FIRST_POOL_CASES = [(3, 224, 224, 7, 3, 'relu', True, 3), (3, 224, 224, 7, 3, 'relu', True, 160), (3, 97, 250, 7, 3, 'linear', True, 2),
+                         (3, 254, 254, 3, 1, 'relu', True, 1), (1, 161, 160, 5, 2, 'linear', False, 40), (4, 64, 65, 7, 0, 'relu', False, 5),
+                         (3, 6, 6, 2, 0, 'relu', True, 4), (3, 5, 191, 3, 1, 'linear', True, 150), (2, 40, 12, 6, 2, 'relu', True, 7)]
+
+
+@pytest.mark.parametrize('case', STEM_FIRST_POOL_CASES, ids=lambda c: 'C%d_%dx%d_k%d_p%d_%s_%s_b%d' % c)
+@pytest.mark.parametrize('mode', ['double', 'single', 'fixed', 'float'])
+def test_first_layer_with_its_accumulators_pooled(case, mode):
+    C, H, W, k, p, act, uns, batch = case
+    b = netdesc.NetBuilder('stempool', C, H, W, 13, mode, input_unsigned=uns, weight_dist=('normal', 30))
+    c = b.conv(-1, 64, k, stride=2, pad=p, act=act, name='conv1')
+    b.pool(c, 'max', 3, 2, name='pool1')
+    n, eng = compare_net(b.net, batch, flags=0)
+    assert eng == ['stem-pool-tcgen05', 'fused']
+    if mode == 'float':   # a scaling that decreases somewhere: the maximum cannot be taken first
+        b.net['layers'][0]['quant']['fscale'][5] *= -1
+        n, eng = compare_net(b.net, batch, flags=0)
+        assert eng[1] == 'pool'
+
+
 # (C, H, W, O, k, pad, activation, pooling window, pooling stride, input unsigned)
 STEM_POOL_CASES = [(3, 64, 64, 64, 7, 3, 'relu', 3, 2, True), (3, 224, 224, 64, 7, 3, 'relu', 3, 2, True),
                    (3, 33, 29, 32, 3, 1, 'relu', 2, 2, True), (1, 24, 24, 32, 4, 0, 'linear', 2, 2, True),
