@@ -19,7 +19,7 @@
 // half), and the third row of a window is the first row of the next pair, which the same warp drains.  No barrier joins
 // the epilogue warps, four of which (16 channels each) share a quarter of the columns.
 //
-// Warp 0 loads pairs of image rows through a ring, warp 1 issues the MMAs into four accumulators, warps 2-17 are the
+// Warp 0 loads pairs of image rows through a ring, warps 1 and 18 issue the MMAs into four accumulators, warps 2-17 are the
 // epilogue.  A work item is a band of pooled rows of one image; bands are as tall as the batch allows, each
 // computes one row pair more than it has pooled rows.  Every wait is bounded.
 #include <cstring>
@@ -34,7 +34,8 @@ static constexpr int SP_SLOTS = 4;            // TMEM accumulators of 128 column
 static constexpr int SP_EPI_WARP0 = 2;
 static constexpr int SP_GROUPS = 4;           // epilogue warps per TMEM lane quadrant, a quarter of the pooled columns each
 static constexpr int SP_EPI_WARPS = 4 * SP_GROUPS;
-static constexpr int SP_THREADS = 32 * (SP_EPI_WARP0 + SP_EPI_WARPS);
+static constexpr int SP_ISSUERS = 2;           // MMA-issuing warps (warp 1 and the last one): row pairs alternate between them
+static constexpr int SP_THREADS = 32 * (SP_EPI_WARP0 + SP_EPI_WARPS + SP_ISSUERS - 1);
 static constexpr int SP_RING = 16;            // pairs of re-laid image rows in flight (a power of two)
 static constexpr int SP_CHANNELS = 64;
 
@@ -103,7 +104,8 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
     pdl_launch_dependents();
     if (warp == 0) {
         for (int i = lane; i < 2 * SP_RING + 2 * SP_SLOTS + 1; i += 32)
-            mbar_init(full0 + 8u * i, i >= 2 * SP_RING + SP_SLOTS && i < 2 * SP_RING + 2 * SP_SLOTS ? SP_EPI_WARPS : 1);
+            mbar_init(full0 + 8u * i, i >= SP_RING && i < 2 * SP_RING ? SP_ISSUERS
+                                                                      : (i >= 2 * SP_RING + SP_SLOTS && i < 2 * SP_RING + 2 * SP_SLOTS ? SP_EPI_WARPS : 1));
         if (lane == 0) {
             *abort_flag = 0;
             prefetch_tensor_map(&tmX);
@@ -151,8 +153,10 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
             band += step_b;
             if (band >= a.bands) { band -= a.bands; ++n; }
         }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer
+    } else if (warp == 1 || warp >= SP_EPI_WARP0 + SP_EPI_WARPS) {
+        // ------------------------------------------------------------------ MMA issuers
+        // One alone took 1030 cycles per row pair, its waits and commits on top of the 620 the tensor pipe is busy
+        const unsigned me = warp == 1 ? 0u : 1u;
         bool ok = (int)blockIdx.x >= a.items || mbar_wait_issuer(wfull, 0, abort_flag, a.status, 8);
         // weights per filter row: [m / 8][k / 16][m % 8][16 bytes]; positions: 16-byte rows, the next 16 bytes of K one pixel on
         const unsigned w_hi = sp_desc_hi((unsigned)(a.KWp * 128)), x_hi = sp_desc_hi(128u);
@@ -163,6 +167,7 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
         for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
             const int pairs = band_rows(band) + 1;
             for (int q = 0; q < pairs; ++q, ++seq, ++acc) {
+                if ((acc & 1u) != me) continue;
                 const unsigned slot = acc & (SP_SLOTS - 1), sph = (acc / SP_SLOTS) & 1u;
                 if (!mbar_wait_issuer(tempty0 + 8u * slot, sph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
                 for (; ok && have <= seq + (unsigned)ahead; ++have)
@@ -182,10 +187,12 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
                             for (int j = 0; 2 * j < a.KWp; ++j)
                                 sp_mma(d, w_lo0 + (unsigned)ky * w_row + 16u * j, w_hi, xr + 2u * j, x_hi, a.idesc, (ky | j) ? 1u : 0u);
                         }
-                    tc_commit(empty0 + 8u * (seq & (SP_RING - 1)));
-                    if (q + 1 == pairs)
-                        for (int i = 1; i <= ahead; ++i) tc_commit(empty0 + 8u * ((seq + (unsigned)i) & (SP_RING - 1)));
                     tc_commit(tfull0 + 8u * slot);
+                    // This issuer is done with chunks q and q + 1 (its next pair is q + 2), after its last pair of the band with all of
+                    // them.  A chunk is free when both issuers are; chunk 0 only has this one.
+                    const int last = q >= pairs - 2 ? pairs - 1 + ahead : q + 1;
+                    if (q == 0) tc_commit(empty0 + 8u * (seq & (SP_RING - 1)));
+                    for (int i = q; i <= last; ++i) tc_commit(empty0 + 8u * ((seq + (unsigned)(i - q)) & (SP_RING - 1)));
                 }
                 __syncwarp();
             }
