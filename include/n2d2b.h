@@ -291,11 +291,12 @@ int n2d2b_probe_i8_mma_rate(int device, int n, int reps, double* tops, double* c
  *   - All calls on a device share the one array: calls whose GPU work overlaps (different streams,
  *     different threads) race on it.  Issue them on one stream, or order them yourself.
  *   - The first call on a device looks up the array's device address; make that call before any
- *     stream capture begins.  The call copies the small layer constants and waits for that copy
- *     (a stream synchronisation), then enqueues the kernels asynchronously.
+ *     stream capture begins; it also pins one page of the library's own host memory.  Every call waits for
+ *     the work before it (a stream synchronisation), then enqueues the kernels asynchronously; weights and constants
+ *     travel as kernel parameters (stride 2) or as two small copies ahead of that wait.
  *   - It calls no cudaMalloc, cudaFree or other allocating CUDA routine.
  *   - The kernels are enqueued asynchronously, so a device-side wait that gave up is not known when the call
- *     returns.  The status word sits in the same array; the NEXT call on that device reads it during the wait
+ *     returns.  The status word is kept per device; the NEXT call on that device reads it behind the wait
  *     it makes anyway and returns N2D2B_ERR_TIMEOUT ("the previous call's kernel gave up...") without
  *     launching; the call after that runs normally.  The caller's current device is restored on return.
  */

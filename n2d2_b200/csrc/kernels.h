@@ -103,6 +103,7 @@ struct StemS2dPlan {
     int in_unsigned;
     int num_sms;
     int band_batch;       // images the band height was chosen for
+    int late_layer;       // weights and constants are written by the kernel before
     const void* s2d;      // the re-laid image
     int max_batch;
     void* encode;         // cuTensorMapEncodeTiled
@@ -118,6 +119,16 @@ void stem_s2d_filter(const ConvGeom& g, int* P, int* KH, int* KWp);
 size_t stem_s2d_weight_bytes(const ConvGeom& g);
 void stem_s2d_arrange_weights(const ConvGeom& g, const int8_t* w_ohwi, int8_t* dst);
 cudaError_t launch_s2d_image(const void* in, const ConvGeom& g, int batch, void* out, cudaStream_t s);
+// The layer as parameters of the kernel that re-lays the image; weights OHWI, constants [5][O]
+struct S2dLayer {
+    int O, kH, kW, C, offy, offx, KH, KWp, BN, blocks;
+    int8_t* w_dst;
+    int* const_dst;       // [5][256]
+    int consts[5 * 128];
+    int8_t w[28 * 1024];
+};
+static_assert(sizeof(S2dLayer) <= 32000, "kernel parameters end at 32764 bytes");
+cudaError_t launch_s2d_layer_and_image(S2dLayer* l, const void* in, const ConvGeom& g, int batch, void* out, cudaStream_t s);
 // pool: a max pooling folded into the kernel (stem_s2d_pool_eligible); `out` of the launch is then the pooled tensor
 int stem_s2d_make_plan(StemS2dPlan* plan, const void* d_s2d, const int8_t* d_w_arranged, const ConvGeom& g, int max_batch,
                        int in_unsigned, int num_sms, const char** why, const PoolGeom* pool = nullptr);

@@ -58,6 +58,7 @@ struct S2dArgs {
     unsigned rcp_Wp;        // ceil(2^32 / Wp)
     unsigned idesc, tmem_cols;
     const int8_t* w;        // weights in the canonical unswizzled K-major layout
+    int late_layer;         // weights and constants come from the previous kernel too
     void* out;
     int* status;
     const int* fq;
@@ -67,12 +68,20 @@ struct S2dArgs {
 
 // [B][H][W][C] (C <= 4) -> [B][Hs][Ws][2][2][4]: block (dy, dx) of pixel (Y, X) = input pixel
 // (2Y + dy - P, 2X + dx - P), zero outside the image and in the unused channels.  One block per output row.
-__global__ void s2d_image_kernel(const uint8_t* __restrict__ in, int C, int H, int W, int Hs, int Ws, int P, int rows,
-                                 uint4* __restrict__ out)
+struct S2dImage {
+    const uint8_t* in;
+    uint4* out;
+    int C, H, W, Hs, Ws, P;
+    int rows;                          // output rows of all images
+    unsigned threads_per_row, total;   // word form: threads of a row and of all (0: not eligible)
+};
+
+__device__ __forceinline__ void s2d_image_bytes(const S2dImage& im, int block, int blocks)
 {
-    pdl_launch_dependents();
-    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
-    for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    const uint8_t* __restrict__ in = im.in;
+    uint4* __restrict__ out = im.out;
+    const int C = im.C, H = im.H, W = im.W, Hs = im.Hs, Ws = im.Ws, P = im.P;
+    for (int row = block; row < im.rows; row += blocks) {
         const int n = row / Hs, Y = row - n * Hs;
         const uint8_t* img = in + (size_t)n * H * W * C;
         uint4* orow = out + (size_t)row * Ws;
@@ -93,6 +102,78 @@ __global__ void s2d_image_kernel(const uint8_t* __restrict__ in, int C, int H, i
             }
             orow[X] = make_uint4(v[0], v[1], v[2], v[3]);
         }
+    }
+}
+
+// The same for three channels and rows of whole 32-bit words (width a multiple of four).  A thread owns the two output pixels whose
+// blocks are four adjacent input pixels, 12 bytes of each of two rows: six word loads and a handful of byte permutes where the
+// general kernel takes 24 byte loads with their conditions (1024 images of 224 x 224: 130 us, instruction-bound, against 65).
+__device__ __forceinline__ void s2d_image_words(const S2dImage& im, unsigned block, unsigned blocks)
+{
+    const uint8_t* __restrict__ in = im.in;
+    const int H = im.H, W = im.W, Hs = im.Hs, Ws = im.Ws, P = im.P;
+    const unsigned threads_per_row = im.threads_per_row;
+    const unsigned row_words = (unsigned)W * 3u / 4u;
+    for (unsigned i = block * blockDim.x + threadIdx.x; i < im.total; i += blocks * blockDim.x) {
+        const unsigned row = i / threads_per_row, n = row / (unsigned)Hs;
+        const int Y = (int)(row - n * (unsigned)Hs), x0 = 4 * (int)(i - row * threads_per_row) - (P + 3) / 4 * 4;
+        const int X = (x0 + P) / 2;   // first of the two output pixels; -1 where P is no multiple of four
+        unsigned px[2][4];
+#pragma unroll
+        for (int dy = 0; dy < 2; ++dy) {
+            const int y = 2 * Y + dy - P;
+            unsigned w0 = 0, w1 = 0, w2 = 0;
+            if ((unsigned)y < (unsigned)H && (unsigned)x0 < (unsigned)W) {
+                const unsigned* p = (const unsigned*)in + (size_t)(n * (unsigned)H + (unsigned)y) * row_words + (unsigned)x0 * 3u / 4u;
+                w0 = __ldg(p);
+                w1 = __ldg(p + 1);
+                w2 = __ldg(p + 2);
+            }
+            px[dy][0] = w0 & 0xffffffu;
+            px[dy][1] = __byte_perm(w0, w1, 0x0543) & 0xffffffu;
+            px[dy][2] = __byte_perm(w1, w2, 0x0432) & 0xffffffu;
+            px[dy][3] = w2 >> 8;
+        }
+        uint4* o = im.out + (size_t)row * Ws + X;
+        if (X >= 0 && X < Ws) o[0] = make_uint4(px[0][0], px[0][1], px[1][0], px[1][1]);
+        if (X + 1 < Ws) o[1] = make_uint4(px[0][2], px[0][3], px[1][2], px[1][3]);
+    }
+}
+
+template <bool WORDS>
+__global__ void __launch_bounds__(256) s2d_image_kernel(const S2dImage im)
+{
+    pdl_launch_dependents();
+    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
+    if (WORDS) s2d_image_words(im, blockIdx.x, gridDim.x);
+    else s2d_image_bytes(im, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// The same with the layer itself in the launch's parameters (callers that own no device memory): the first blocks write the weights
+// in the order of stem_s2d_arrange_weights and the constants, the others the image.  Neither host copies nor their
+// waits: a call with eight 224 x 224 images went from 48.4 us to 23.6.
+__global__ void __launch_bounds__(256) s2d_layer_and_image_kernel(const __grid_constant__ S2dLayer l, const S2dImage im)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    if ((int)blockIdx.x >= l.blocks) {
+        if (im.total) s2d_image_words(im, blockIdx.x - l.blocks, gridDim.x - l.blocks);
+        else s2d_image_bytes(im, (int)blockIdx.x - l.blocks, (int)gridDim.x - l.blocks);
+        return;
+    }
+    const int i0 = (int)(blockIdx.x * blockDim.x + threadIdx.x), step = l.blocks * (int)blockDim.x;
+    for (int i = i0; i < 5 * l.O; i += step) l.const_dst[i / l.O * 256 + i % l.O] = l.consts[i];
+    const int row_words = l.BN * l.KWp * 4, words = l.KH * row_words, group = l.KWp * 32;   // 32-bit words: one tap's channels each
+    for (int d = i0; d < words; d += step) {
+        const int Y = d / row_words, r = d - Y * row_words, n8 = r / group, q = r - n8 * group;
+        const int X = q >> 5, n = n8 * 8 + ((q >> 2) & 7), dy = (q >> 1) & 1, dx = q & 1;
+        const int o = perm_real_channel(n, 4), ky = 2 * Y + dy - l.offy, kx = 2 * X + dx - l.offx;
+        unsigned w = 0;
+        if (o < l.O && ky >= 0 && ky < l.kH && kx >= 0 && kx < l.kW) {
+            const int8_t* src = l.w + ((o * l.kH + ky) * l.kW + kx) * l.C;
+            for (int c = 0; c < l.C; ++c) w |= (unsigned)(uint8_t)src[c] << (8 * c);
+        }
+        ((unsigned*)l.w_dst)[d] = w;
     }
 }
 
@@ -175,6 +256,7 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     pdl_launch_dependents();
+    if (a.late_layer) pdl_wait();
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) {
@@ -488,60 +570,58 @@ void stem_s2d_arrange_weights(const ConvGeom& g, const int8_t* w_ohwi, int8_t* d
     }
 }
 
-// The same for three channels and rows of whole 32-bit words (width a multiple of four).  A thread owns the two output pixels whose
-// blocks are four adjacent input pixels, 12 bytes of each of two rows: six word loads and a handful of byte permutes where the
-// general kernel takes 24 byte loads with their conditions (1024 images of 224 x 224: 130 us, instruction-bound, against 65).
-__global__ void __launch_bounds__(256)
-s2d_image_rgb_kernel(const uint8_t* __restrict__ in, int H, int W, int Hs, int Ws, int P, unsigned threads_per_row, unsigned total, uint4* __restrict__ out)
+static S2dImage s2d_image_of(const void* in, const ConvGeom& g, int batch, void* out)
 {
-    pdl_launch_dependents();
-    pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
-    const unsigned row_words = (unsigned)W * 3u / 4u;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const unsigned row = i / threads_per_row, n = row / (unsigned)Hs;
-        const int Y = (int)(row - n * (unsigned)Hs), x0 = 4 * (int)(i - row * threads_per_row) - (P + 3) / 4 * 4;
-        const int X = (x0 + P) / 2;   // first of the two output pixels; -1 where P is no multiple of four
-        unsigned px[2][4];
-#pragma unroll
-        for (int dy = 0; dy < 2; ++dy) {
-            const int y = 2 * Y + dy - P;
-            unsigned w0 = 0, w1 = 0, w2 = 0;
-            if ((unsigned)y < (unsigned)H && (unsigned)x0 < (unsigned)W) {
-                const unsigned* p = (const unsigned*)in + (size_t)(n * (unsigned)H + (unsigned)y) * row_words + (unsigned)x0 * 3u / 4u;
-                w0 = __ldg(p);
-                w1 = __ldg(p + 1);
-                w2 = __ldg(p + 2);
-            }
-            px[dy][0] = w0 & 0xffffffu;
-            px[dy][1] = __byte_perm(w0, w1, 0x0543) & 0xffffffu;
-            px[dy][2] = __byte_perm(w1, w2, 0x0432) & 0xffffffu;
-            px[dy][3] = w2 >> 8;
-        }
-        uint4* o = out + (size_t)row * Ws + X;
-        if (X >= 0 && X < Ws) o[0] = make_uint4(px[0][0], px[0][1], px[1][0], px[1][1]);
-        if (X + 1 < Ws) o[1] = make_uint4(px[0][2], px[0][3], px[1][2], px[1][3]);
-    }
+    S2dImage im;
+    int KH, KWp;
+    stem_s2d_filter(g, &im.P, &KH, &KWp);
+    stem_s2d_dims(g, &im.Hs, &im.Ws);
+    im.in = (const uint8_t*)in;
+    im.out = (uint4*)out;
+    im.C = g.C; im.H = g.H; im.W = g.W;
+    im.rows = batch * im.Hs;
+    // three channels and whole words per row (the padding is even): groups of four input pixels, the first at -(P + 3) / 4 * 4
+    im.threads_per_row = (unsigned)(((im.P + 3) / 4 * 4 - im.P + 2 * im.Ws + 3) / 4);
+    const long long total = (long long)im.rows * im.threads_per_row;
+    const bool words = g.C == 3 && g.W % 4 == 0 && im.P % 2 == 0 && ((uintptr_t)in & 3) == 0 && total < (1ll << 31) && (long long)batch * g.H < (1ll << 31);
+    im.total = words ? (unsigned)total : 0u;
+    return im;
+}
+
+static int s2d_image_blocks(const S2dImage& im)
+{
+    return im.total ? (int)std::min((im.total + 255u) / 256u, 148u * 32u) : std::min(im.rows, 1 << 20);
 }
 
 cudaError_t launch_s2d_image(const void* in, const ConvGeom& g, int batch, void* out, cudaStream_t s)
 {
-    int P, KH, KWp, Hs, Ws;
-    stem_s2d_filter(g, &P, &KH, &KWp);
-    stem_s2d_dims(g, &Hs, &Ws);
-    const long long rows = (long long)batch * Hs;
-    if (rows == 0) return cudaSuccess;
-    const int start = (P + 3) / 4 * 4;   // the first group of four input pixels starts at -start
-    const unsigned per_row = (unsigned)((start - P + 2 * Ws + 3) / 4);
-    const long long total = rows * per_row;
-    if (g.C == 3 && g.W % 4 == 0 && P % 2 == 0 && ((uintptr_t)in & 3) == 0 && total < (1ll << 31) && (long long)batch * g.H < (1ll << 31)) {
-        const long long blocks = (total + 255) / 256;
-        return launch_pdl(s2d_image_rgb_kernel, (unsigned)std::min(blocks, 148ll * 32), 256, 0, s, (const uint8_t*)in, g.H, g.W, Hs, Ws, P, per_row,
-                          (unsigned)total, (uint4*)out);
-    }
-    const unsigned grid = (unsigned)(rows < (1ll << 20) ? rows : (1ll << 20));
-    const int threads = Ws >= 128 ? 128 : ((Ws + 31) / 32) * 32;
-    launch_pdl(s2d_image_kernel, grid, threads, 0, s, (const uint8_t*)in, g.C, g.H, g.W, Hs, Ws, P, (int)rows, (uint4*)out);
-    return cudaGetLastError();
+    const S2dImage im = s2d_image_of(in, g, batch, out);
+    if (im.rows == 0) return cudaSuccess;
+    if (im.total) return launch_pdl(s2d_image_kernel<true>, s2d_image_blocks(im), 256, 0, s, im);
+    return launch_pdl(s2d_image_kernel<false>, s2d_image_blocks(im), im.Ws >= 128 ? 128 : ((im.Ws + 31) / 32) * 32, 0, s, im);
+}
+
+// `l` comes with its weights, constants and destinations
+cudaError_t launch_s2d_layer_and_image(S2dLayer* l, const void* in, const ConvGeom& g, int batch, void* out, cudaStream_t s)
+{
+    const S2dImage im = s2d_image_of(in, g, batch, out);
+    int P;
+    stem_s2d_filter(g, &P, &l->KH, &l->KWp);
+    l->O = g.O; l->kH = g.kH; l->kW = g.kW; l->C = g.C;
+    l->offy = P - g.pT; l->offx = P - g.pL;
+    l->BN = g.O <= 64 ? 64 : 128;
+    l->blocks = (l->KH * l->BN * l->KWp * 4 + 255) / 256;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(l->blocks + s2d_image_blocks(im)));
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void* args[2] = {(void*)l, (void*)&im};   // (30 KB of parameters: not copied around)
+    return cudaLaunchKernelExC(&cfg, (const void*)s2d_layer_and_image_kernel, args);
 }
 
 // A max pooling this kernel can fold in: square window, same stride both ways, no padding, 8-bit channels in whole
@@ -673,6 +753,7 @@ cudaError_t launch_stem_s2d(const StemS2dPlan& plan, const ConvGeom& g, int n_ba
             | ((unsigned)(ZBM >> 4) << 24);
     a.tmem_cols = (unsigned)(Z_SLOTS * plan.BN);
     a.w = plan.w;
+    a.late_layer = plan.late_layer;
     a.out = out;
     a.status = status_word;
     a.fq = fast.fq;

@@ -478,6 +478,11 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_SCRATCH_BYTE
 // In host code the array's name is only a handle; its device address comes from the runtime, once per
 // device, with that device current.
 static unsigned char* g_noalloc_ptr[64] = {nullptr};
+// Status words of the bounded waits, 64 bytes apart: a page of the library's own host memory that kernels can write (they do only
+// when a wait gives up), so that looking at one takes no copy.  Where it cannot be mapped they live in the scratch.
+alignas(4096) static int g_noalloc_status[1024];
+static int* g_noalloc_status_dev = nullptr;
+static bool g_noalloc_status_tried = false;
 static bool g_noalloc_used[64] = {false};   // the status word of a device means something only after a first call
 static std::mutex g_noalloc_mutex;   // first calls from several host threads look the address up one at a time
 
@@ -491,6 +496,15 @@ static int noalloc_scratch_for(int device, unsigned char** ptr)
         if (e != cudaSuccess || !p)
             return n2d2b::set_error(N2D2B_ERR_CUDA, "cudaGetSymbolAddress(scratch) failed: %s", cudaGetErrorString(e));
         g_noalloc_ptr[device] = (unsigned char*)p;
+        if (!g_noalloc_status_tried) {
+            g_noalloc_status_tried = true;
+            void* d = nullptr;
+            if (cudaHostRegister(g_noalloc_status, sizeof(g_noalloc_status), cudaHostRegisterPortable | cudaHostRegisterMapped) == cudaSuccess
+                && cudaHostGetDevicePointer(&d, g_noalloc_status, 0) == cudaSuccess)
+                g_noalloc_status_dev = (int*)d;
+            else
+                cudaGetLastError();
+        }
     }
     *ptr = g_noalloc_ptr[device];
     return 0;
@@ -557,34 +571,69 @@ extern "C" int n2d2b_first_conv_noalloc(int device, const void* d_input, int bat
     if (prc > 0 || cpad != 256)
         return set_error(N2D2B_ERR_INVALID,
                          "this entry point takes shift or fixed-point scalings whose products fit 32 bits and 8-bit outputs");
-    std::vector<int8_t> arranged(stem_weight_bytes(g));
-    stem_arrange_weights(g, weights, arranged.data());
-
     cudaStream_t s = (cudaStream_t)stream;
-    // both copies are ordered on the caller's stream behind any earlier call that still reads the scratch;
-    // the host buffers are released when this function returns, hence the synchronisation
-    e = cudaMemcpyAsync(scratch, arranged.data(), arranged.size(), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(scratch + NA_CONST_OFFSET, consts.data(), consts.size() * 4, cudaMemcpyHostToDevice, s);
-    // The status word of the bounded waits lives in the scratch too (last 16 bytes of the constants area).  It
-    // still holds what the previous call's kernel left: read it behind that kernel, during the wait this call
-    // makes anyway, so a time-out of call k is reported by call k + 1.
-    int* status = (int*)(scratch + NA_PAD_OFFSET - 16);
+    // A stride-2 layer whose re-laid image fits takes the space-to-depth kernels, the layer itself as parameters of the re-layout:
+    // nothing to copy.  The others copy the arranged weights and the constants ahead, ordered on the caller's stream behind any
+    // earlier call that still reads the scratch; the host buffers are released when this function returns, hence the wait.
+    int Hs = 0, Ws = 0;
+    bool s2d = stem_s2d_eligible(g) && (size_t)g.O * g.kH * g.kW * g.C <= sizeof(S2dLayer::w) && stem_s2d_weight_bytes(g) <= NA_WEIGHT_BYTES;
+    if (s2d) {
+        stem_s2d_dims(g, &Hs, &Ws);
+        s2d = (size_t)batch * Hs * Ws * 4 <= (size_t)N2D2B_NOALLOC_MAX_PIXELS;
+    }
+    std::vector<int8_t> arranged;
+    if (!s2d) {
+        arranged.resize(stem_weight_bytes(g));
+        stem_arrange_weights(g, weights, arranged.data());
+        e = cudaMemcpyAsync(scratch, arranged.data(), arranged.size(), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(scratch + NA_CONST_OFFSET, consts.data(), consts.size() * 4, cudaMemcpyHostToDevice, s);
+    }
+    // The status word still holds what the previous call's kernel left: look at it behind that kernel, so a time-out of call k is
+    // reported by call k + 1.  (In the scratch: the last 16 bytes of the constants area.)
+    int* const mapped = g_noalloc_status_dev ? g_noalloc_status + 16 * device : nullptr;
+    int* const status = mapped ? g_noalloc_status_dev + 16 * device : (int*)(scratch + NA_PAD_OFFSET - 16);
     int prev_status = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&prev_status, status, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && !mapped) e = cudaMemcpyAsync(&prev_status, status, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "copy of the layer constants failed: %s", cudaGetErrorString(e));
+    if (mapped) prev_status = *(volatile int*)mapped;
     bool first_call_here;
     {
         std::lock_guard<std::mutex> lock(g_noalloc_mutex);
         first_call_here = !g_noalloc_used[device];
         g_noalloc_used[device] = true;
     }
-    if (!first_call_here && prev_status != 0) {
-        cudaMemsetAsync(status, 0, sizeof(int), s);
-        return set_error(N2D2B_ERR_TIMEOUT,
-                         "the previous call's kernel gave up waiting on a pipeline barrier (role %d); its output is incomplete",
-                         prev_status);
+    if (prev_status != 0 || !mapped) {
+        if (mapped) *(volatile int*)mapped = 0;
+        else e = cudaMemsetAsync(status, 0, sizeof(int), s);
+        if (!first_call_here && prev_status != 0)
+            return set_error(N2D2B_ERR_TIMEOUT,
+                             "the previous call's kernel gave up waiting on a pipeline barrier (role %d); its output is incomplete",
+                             prev_status);
+        if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "first-layer launch failed: %s", cudaGetErrorString(e));
+    }
+    FastQuant fq;
+    fq.fq = (const int*)(scratch + NA_CONST_OFFSET);
+    fq.cpad = cpad;
+    fq.out_unsigned = out_unsigned;
+    fq.need_clamp = need_clamp;
+    fq.enabled = true;
+    if (s2d) {
+        StemS2dPlan plan2;
+        const char* why = "";
+        if (stem_s2d_make_plan(&plan2, scratch + NA_PAD_OFFSET, (const int8_t*)scratch, g, batch, in_unsigned ? 1 : 0, sms, &why, nullptr))
+            return set_error(N2D2B_ERR_INVALID, "first-layer plan failed: %s", why);
+        plan2.late_layer = 1;
+        static thread_local S2dLayer layer;
+        layer.w_dst = (int8_t*)scratch;
+        layer.const_dst = (int*)(scratch + NA_CONST_OFFSET);
+        for (int p = 0; p < 5; ++p) memcpy(layer.consts + (size_t)p * g.O, consts.data() + (size_t)p * cpad, (size_t)g.O * 4);
+        memcpy(layer.w, weights, (size_t)g.O * g.kH * g.kW * g.C);
+        // every pixel of the re-laid image is rewritten in full, so nothing of an earlier call survives
+        e = launch_s2d_layer_and_image(&layer, d_input, g, batch, scratch + NA_PAD_OFFSET, s);
+        if (e == cudaSuccess) e = launch_stem_s2d(plan2, g, 0, fq, d_output, status, s);
+        if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "first-layer launch failed: %s", cudaGetErrorString(e));
+        return 0;
     }
 
     StemPlan plan;
@@ -595,14 +644,7 @@ extern "C" int n2d2b_first_conv_noalloc(int device, const void* d_input, int bat
     e = launch_pad_image(d_input, g, batch, scratch + NA_PAD_OFFSET, s);
     if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "re-layout launch failed: %s", cudaGetErrorString(e));
     const void* in4 = scratch + NA_PAD_OFFSET;
-    FastQuant fq;
-    fq.fq = (const int*)(scratch + NA_CONST_OFFSET);
-    fq.cpad = cpad;
-    fq.out_unsigned = out_unsigned;
-    fq.need_clamp = need_clamp;
-    fq.enabled = true;
-    e = cudaMemsetAsync(status, 0, sizeof(int), s);
-    if (e == cudaSuccess) e = launch_stem(plan, in4, g, fq, d_output, status, s);
+    e = launch_stem(plan, in4, g, fq, d_output, status, s);
     if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "first-layer launch failed: %s", cudaGetErrorString(e));
     return 0;
 }

@@ -118,38 +118,38 @@ def check(rc):
 
 
 def _ptr(a):
-    return None if a is None else a.ctypes.data_as(C.c_void_p)
+    if a is None:
+        return None
+    try:
+        return a.__array_interface__['data'][0]   # the address as an integer: half the time of a.ctypes.data_as
+    except AttributeError:
+        return a.ctypes.data_as(C.c_void_p)
+
+
+_QUANT_ARRAYS = (('fscale', 'fscale', np.float32), ('mult', 'mult', np.int32), ('frac_bits_per_ch', 'frac_bits_per_channel', np.uint8),
+                 ('shift0', 'shift0', np.uint8), ('shift1', 'shift1', np.uint8), ('clip', 'clip', np.float32))
 
 
 def make_quant(q, channels):
     """Builds the C struct for a quant dict; returns (struct, keepalive list)."""
     keep = []
-
-    def arr(key, dtype):
-        v = q.get(key)
-        if v is None:
-            return None
-        a = np.ascontiguousarray(v, dtype)
-        keep.append(a)
-        return _ptr(a)
-
-    s = Scaling()
+    get = q.get
+    qq = Quant()
+    s = qq.scaling
     s.mode = MODES[q['mode']]
     s.nb_channels = channels
-    s.fscale = arr('fscale', np.float32)
-    s.mult = arr('mult', np.int32)
-    s.frac_bits = int(q.get('frac_bits', 0))
-    s.frac_bits_per_channel = arr('frac_bits_per_ch', np.uint8)
-    s.shift0 = arr('shift0', np.uint8)
-    s.shift1 = arr('shift1', np.uint8)
-    s.is_clipped = 1 if q.get('is_clipped') else 0
-    s.clip = arr('clip', np.float32)
-    qq = Quant()
-    qq.scaling = s
-    qq.activation = ACTS[q.get('act', 'linear')]
-    qq.out_bits = int(q.get('out_bits', 8))
-    qq.out_unsigned = 1 if q.get('out_unsigned') else 0
-    qq.saturation_threshold = int(q.get('sat_thr', 0))
+    s.frac_bits = int(get('frac_bits', 0))
+    s.is_clipped = 1 if get('is_clipped') else 0
+    for key, field, dtype in _QUANT_ARRAYS:
+        v = get(key)
+        if v is not None:
+            a = np.ascontiguousarray(v, dtype)
+            keep.append(a)
+            setattr(s, field, _ptr(a))
+    qq.activation = ACTS[get('act', 'linear')]
+    qq.out_bits = int(get('out_bits', 8))
+    qq.out_unsigned = 1 if get('out_unsigned') else 0
+    qq.saturation_threshold = int(get('sat_thr', 0))
     return qq, keep
 
 

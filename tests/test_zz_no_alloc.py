@@ -71,3 +71,17 @@ def test_noalloc_first_conv_rejects_what_it_cannot_hold():
     wide = single_conv_net(16, 16, 16, 64, 3, 1, 1, mode='double')['layers'][0]
     with pytest.raises(runtime.N2D2BError, match='first-layer kernel'):
         runtime.first_conv_noalloc(d.data_ptr(), 1, 16, 16, 16, True, wide, d.data_ptr())
+
+
+# (C, H, W, O, k, stride, pad, batch): the space-to-depth form with its layer as kernel parameters (whole words per row and not, 32 to
+# 128 outputs, the widest filters) and, for what does not fit it (wide rows, weights beyond the parameters), the copied form
+NOALLOC_CASES = [(3, 224, 224, 64, 7, 2, 3, 3), (3, 97, 99, 32, 3, 2, 1, 5), (1, 40, 44, 96, 5, 2, 2, 2), (4, 64, 60, 128, 7, 2, 3, 2),
+                 (4, 33, 30, 128, 8, 2, 3, 1), (3, 254, 256, 64, 7, 2, 3, 2), (3, 30, 28, 64, 3, 1, 1, 2)]
+
+
+@pytest.mark.parametrize('case', NOALLOC_CASES, ids=lambda c: 'C%d_%dx%d_O%d_k%d_s%d_p%d_b%d' % c)
+@pytest.mark.parametrize('mode', ['double', 'single'])
+def test_noalloc_first_conv_forms(case, mode):
+    C, H, W, O, k, s, p, batch = case
+    got, want = _both_paths(single_conv_net(C, H, W, O, k, s, p, mode=mode, seed=23), batch, seed=8)
+    assert np.array_equal(got, want)
