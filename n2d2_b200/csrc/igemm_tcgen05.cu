@@ -911,6 +911,34 @@ void igemm_dw_arrange_weights(const ConvGeom& g, const int8_t* w_ct, int8_t* dst
         for (int t = 0; t < taps; ++t) dst[(size_t)o * row_bytes + (size_t)t * cg + (o % cg)] = w_ct[(size_t)o * taps + t];
 }
 
+// Columns of a tile: 256, 128 or 64, whichever finishes the busiest CTA first by an estimate in cycles.  A K block costs its MMAs
+// (128 x 256 x 32 128 cycles, x 128 64, x 64 48) or, where that is longer, its loads (71 bytes per clock and SM with
+// all of them loading, 40 through an im2col map; resident weights are loaded once), a tile its K blocks or its epilogue (a cycle count per column that is
+// smaller where two or four groups of warps drain a tile each), a CTA its tiles and one epilogue nothing covers.  Wide tiles
+// load the least per value; narrow ones fill the chip when there are few rows, or its second wave.  With a residual sum 256
+// columns never pay (conv5.2 of ResNet-50 at 1024 images 90 us against 74 with two tiles in the epilogue at once).
+// ResNet-50 at 33 images 481 -> 464 us against a rule that only filled the chip, ResNet-18 at 64 images 310 -> 291.
+static int igemm_tile_columns(const ConvGeom& g, int BK, bool im2col, bool res, int w4, int num_sms, int force_pair)
+{
+    const int widest = g.O >= 256 && !res ? 256 : (g.O > 64 ? 128 : 64);
+    if (force_pair) return widest;
+    const long long m_tiles = ((long long)g.B * g.oH * g.oW + BM - 1) / BM;
+    const int num_kb = g.kH * g.kW * ((g.C + BK - 1) / BK);
+    int best_bn = widest;
+    double best = 0;
+    for (int bn = widest; bn >= 64; bn >>= 1) {
+        const long long n_tiles = (g.O + bn - 1) / bn, tiles = m_tiles * n_tiles, per_cta = (tiles + num_sms - 1) / num_sms;
+        const bool resident = !w4 && (long long)num_kb * BK * bn <= 96 * 1024 && (n_tiles == 1 || num_sms > n_tiles);
+        const double mma = (bn == 256 ? 128.0 : (bn == 128 ? 64.0 : 48.0)) * BK / 32;
+        const double rate = tiles < num_sms ? 114.0 - 43.0 * tiles / num_sms : 71.0;
+        const double load = BK * (BM / (im2col ? std::min(rate, 40.0) : rate) + (resident && per_cta > 1 ? 0 : bn) / rate);
+        const double epi = bn * (bn == 256 ? 10.0 : (bn == 128 ? 11.0 : 15.0)) * (res ? 1.9 : 1.0);
+        const double cost = per_cta * std::max(num_kb * std::max(mma, load), per_cta > 1 ? epi : 0.0) + epi;
+        if (best == 0 || cost < 0.93 * best) { best = cost; best_bn = bn; }
+    }
+    return best_bn;
+}
+
 int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void* out, const void* res,
                     const ConvGeom& g0, int in_unsigned, int force_im2col, int force_bn, int num_sms, const char** why,
                     int force_pair, int w4)
@@ -947,13 +975,7 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
     plan->BK = (g.C % 128 == 0) ? 128 : (g.C % 64 == 0 ? 64 : 32);
     int bn = force_bn;
     if (bn == 0) {
-        // 256 columns halve the activation traffic of a streamed layer.  With a residual sum 128 are better, two tiles in the
-        // epilogue at once: conv5.2 of ResNet-50 at 1024 images 74 us against 90, conv5.1 135 / 158, conv2.x and conv3.x even.
-        bn = (g.O >= 256 && !res) ? 256 : (g.O > 64 ? 128 : 64);
-        // a layer with few output pixels (the classifier, late stages at small batch) would leave most
-        // SMs without a tile: narrower column blocks give more tiles
-        const long long m_tiles = ((long long)g.B * g.oH * g.oW + BM - 1) / BM;
-        while (!force_pair && bn > 64 && m_tiles * ((g.O + bn - 1) / bn) < num_sms) bn >>= 1;
+        bn = igemm_tile_columns(g, plan->BK, plan->a_im2col != 0, res != nullptr, w4, num_sms, force_pair);
     }
     plan->BN = bn;
     plan->grouped = grouped;
