@@ -982,6 +982,7 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
     // groups of epilogue warps on different tiles need a CTA whose column block never changes
     plan->parts = (g.O + bn - 1) / bn < num_sms ? (bn >= 256 ? 4 : (bn >= 128 ? 2 : 1)) : 4;
     plan->w4 = w4 ? 1 : 0;
+    plan->num_sms = num_sms;
     plan->a_unsigned = in_unsigned;
     plan->oW = g.oW; plan->oH = g.oH; plan->kW = g.kW;
     plan->sX = g.sX; plan->sY = g.sY; plan->pL = g.pL; plan->pT = g.pT; plan->dX = g.dX; plan->dY = g.dY;
@@ -1110,6 +1111,252 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
     return 0;
 }
 
+// ----------------------------------------------------------------------------- few tiles, long K: a cluster per tile
+// A late layer at a small batch has a handful of 128 x 64 tiles and up to 36 K blocks, each of which costs one CTA about 400
+// cycles of waits, loads and MMAs while most of the chip idles (ResNet-50's 3x3 layers of 7 x 7 maps, one image: 8 tiles).  Here the S = 8
+// CTAs of a cluster share a tile: CTA s multiplies its part of K (at most SPLIT_STAGES blocks, each with a stage of its own, so
+// nothing ever waits for a slot), sends the 64 / S columns that CTA t finishes to t's shared memory, and finishes its own
+// columns from the S partial sums.  Sums of 32-bit integers: the same bits in any order.  A 7 x 7 x 512 3x3
+// layer at one image: 16.4 us -> 12.3, ResNet-18 155 us -> 141.
+static constexpr int SPLIT = 8;               // CTAs of a cluster
+static constexpr int SPLIT_STAGES = 7;
+static constexpr int SPLIT_EPI_WARPS = 8;
+static constexpr int SPLIT_THREADS = 32 * (EPI_WARP0 + SPLIT_EPI_WARPS);
+static constexpr int SPLIT_BN = 64;
+
+struct SplitArgs {
+    IgemmArgs g;
+    int per;            // K blocks per CTA
+    int perm_ng;        // permutation of the stored weight rows (perm_block / 8)
+    int form, need_clamp, dp, ef;
+};
+
+static size_t split_smem_bytes(int per, int BK)
+{
+    return 1024 + (size_t)per * (BM + SPLIT_BN) * BK + (size_t)BM * SPLIT_BN * 4 + 2 * FAST_NP * SPLIT_BN * 4 + (SPLIT_STAGES + 1) * 8 + 32;
+}
+
+__device__ __forceinline__ int split_rescale(int x, int form, bool clamp, const int* c, int stride)
+{
+    if (form == EF_FLOAT) {
+        return clamp ? rescale<true, EF_FLOAT>(x, c[0], c[stride], c[2 * stride], c[3 * stride], c[4 * stride])
+                     : rescale<false, EF_FLOAT>(x, 0, 0, c[2 * stride], c[3 * stride], c[4 * stride]);
+    }
+    if (form == EF_WIDE) return rescale<false, EF_WIDE>(x, c[0], 0, c[2 * stride], c[3 * stride], c[4 * stride]);
+    return clamp ? rescale<true, 0>(x, c[0], c[stride], c[2 * stride], c[3 * stride], c[4 * stride])
+                 : rescale<false, 0>(x, 0, 0, c[2 * stride], c[3 * stride], c[4 * stride]);
+}
+
+__global__ void __launch_bounds__(SPLIT_THREADS, 1)
+igemm_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const SplitArgs sa)
+{
+    const IgemmArgs& a = sa.g;
+    constexpr int S = SPLIT, COLS = SPLIT_BN / S, PAIRS = COLS / 2, CHUNKS = COLS / 4;   // columns, column pairs and 16-byte chunks a CTA finishes
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int a_bytes = BM * a.BK, stage_bytes = a_bytes + SPLIT_BN * a.BK;
+    unsigned char* sums = smem + (size_t)sa.per * stage_bytes;       // [S][128][COLS] int32, chunks of a row swizzled
+    int* cst = (int*)(sums + BM * SPLIT_BN * 4);                     // [2][FAST_NP][COLS], stored column order
+    unsigned long long* bars = (unsigned long long*)(cst + 2 * FAST_NP * SPLIT_BN);
+    const unsigned full0 = smem_u32(bars), tfull = full0 + 8u * SPLIT_STAGES;
+    unsigned* tmem_slot = (unsigned*)(bars + SPLIT_STAGES + 1);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const int lane = threadIdx.x & 31;
+    pdl_launch_dependents();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // (waited for before the first remote store)
+
+    const int tile = (int)blockIdx.x / S, rank = (int)blockIdx.x % S;   // clusters are S consecutive CTAs
+    const int m_tile = tile / a.num_n_tiles, n_tile = tile - m_tile * a.num_n_tiles;
+    const int m0 = a.m_base + m_tile * BM, n0 = n_tile * SPLIT_BN, part0 = rank * COLS;
+    const int kchunks = (a.Cin + a.BK - 1) / a.BK, num_kb = a.taps * kchunks;
+    const int kb0 = rank * sa.per, nkb = max(0, min(sa.per, num_kb - kb0));
+    if (warp == 0) {
+        if (lane <= SPLIT_STAGES) mbar_init(full0 + 8u * lane, 1);
+        if (lane == 0) {
+            *abort_flag = 0;
+            prefetch_tensor_map(&tmA);
+            prefetch_tensor_map(&tmB);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(64u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    for (int i = threadIdx.x; i < (a.fq2 ? 2 : 1) * FAST_NP * COLS; i += SPLIT_THREADS) {
+        const int set = i / (FAST_NP * COLS), j = i - set * FAST_NP * COLS, prm = j / COLS, c = j - prm * COLS;
+        cst[(set * FAST_NP + prm) * COLS + c] = __ldg((set ? a.fq2 : a.fq) + (size_t)prm * a.cpad + n0 + perm_real_channel(part0 + c, sa.perm_ng));
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem_base = *tmem_slot, tiles_s = smem_u32(smem);
+
+    // epilogue threads: this thread's column pairs of the tile, u = pair index + PAIRS * row
+    constexpr int UNITS = BM * PAIRS / (32 * SPLIT_EPI_WARPS);
+    const int et = (int)threadIdx.x - 32 * EPI_WARP0;
+    unsigned short res[UNITS];
+    bool ok = true;
+    if (warp == 0) {
+        // ------------------------------------------------------------------ TMA producer
+        PixelPos px;
+        px.start(a, m0);
+        const int iw0 = px.ox * a.sX - a.pL, ih0 = px.oy * a.sY - a.pT;
+        const int tap0 = kb0 / kchunks, kc0 = kb0 - tap0 * kchunks;
+        const int ky0 = tap0 / a.kW, kx0 = tap0 - ky0 * a.kW;
+        if (a.late_weights) pdl_wait();
+        if (elect_one()) {
+            int kc = kc0, kcoord = tap0 * a.Cin + kc0 * a.BK;
+            for (int i = 0; i < nkb; ++i) {
+                mbar_expect_tx(full0 + 8u * i, (unsigned)stage_bytes);
+                tma_load_2d(tiles_s + (unsigned)(i * stage_bytes + a_bytes), &tmB, full0 + 8u * i, kcoord, n0);
+                if (++kc == kchunks) { kc = 0; kcoord += a.Cin - (kchunks - 1) * a.BK; }
+                else kcoord += a.BK;
+            }
+        }
+        __syncwarp();
+        pdl_wait();   // weights are constants; the activations are the previous kernel's output
+        if (elect_one()) {
+            int kc = kc0, kx = kx0, ky = ky0, kcoord = tap0 * a.Cin + kc0 * a.BK;
+            for (int i = 0; i < nkb; ++i) {
+                const unsigned dst = tiles_s + (unsigned)(i * stage_bytes);
+                if (a.a_im2col) tma_load_im2col_4d(dst, &tmA, full0 + 8u * i, kc * a.BK, iw0, ih0, px.n, (unsigned short)(kx * a.dX), (unsigned short)(ky * a.dY));
+                else tma_load_2d(dst, &tmA, full0 + 8u * i, kcoord, m0);
+                if (++kc == kchunks) {
+                    kc = 0;
+                    kcoord += a.Cin - (kchunks - 1) * a.BK;
+                    if (++kx == a.kW) { kx = 0; ++ky; }
+                } else {
+                    kcoord += a.BK;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------ MMA issuer
+        const unsigned desc_hi = (unsigned)(make_smem_desc(0u, a.BK) >> 32);
+        unsigned a_lo = (tiles_s & 0x3ffffu) >> 4;
+        const unsigned stage16 = (unsigned)(stage_bytes >> 4), a16 = (unsigned)(a_bytes >> 4);
+        for (int i = 0; i < nkb; ++i, a_lo += stage16) {
+            if (!mbar_wait_issuer(full0 + 8u * i, 0, abort_flag, a.status, 3)) { ok = false; break; }
+            tc_fence_after();
+            if (elect_one()) {
+                const unsigned b_lo = a_lo + a16;
+                tc_mma_i8_lohi(tmem_base, a_lo, b_lo, desc_hi, a.idesc, i > 0 ? 1u : 0u);
+                if (a.BK >= 64) tc_mma_i8_lohi(tmem_base, a_lo + 2u, b_lo + 2u, desc_hi, a.idesc, 1u);
+                if (a.BK == 128) {
+                    tc_mma_i8_lohi(tmem_base, a_lo + 4u, b_lo + 4u, desc_hi, a.idesc, 1u);
+                    tc_mma_i8_lohi(tmem_base, a_lo + 6u, b_lo + 6u, desc_hi, a.idesc, 1u);
+                }
+                if (i + 1 == nkb) tc_commit(tfull);
+            }
+            __syncwarp();
+        }
+    } else {
+        pdl_wait();   // the residual is an earlier kernel's output; the output may still be read by one
+        if (a.r.ptr) {
+#pragma unroll
+            for (int k = 0; k < UNITS; ++k) {
+                const int u = et + k * 32 * SPLIT_EPI_WARPS, row = u / PAIRS, p = u - row * PAIRS, m = m0 + row;
+                const int ch = n0 + perm_real_channel(part0 + 2 * p, sa.perm_ng);
+                res[k] = m < a.m_base + a.M && ch < a.N ? *(const unsigned short*)((const uint8_t*)a.r.ptr + (size_t)m * a.N + ch) : (unsigned short)0;
+            }
+        }
+    }
+    __syncwarp();
+    // every CTA of the cluster runs: its shared memory may be written
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp >= EPI_WARP0) {
+        const int quad = warp & 3, half = (warp - EPI_WARP0) >> 2, row = quad * 32 + lane;
+        unsigned v[32];
+        if (nkb > 0) {
+            ok = mbar_wait_warp(tfull, 0, abort_flag, a.status, 4, lane);
+            tc_fence_after();
+            if (ok) {
+                tc_ld32(tmem_base + ((unsigned)(quad * 32) << 16) + 32u * half, v);
+                tc_wait_ld_into(v);
+            }
+        }
+        if (nkb == 0 || !ok) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = 0u;
+        }
+        const unsigned swz = (unsigned)(row / (8 / CHUNKS)) & (CHUNKS - 1);
+        const unsigned mine = smem_u32(sums) + (unsigned)((rank * BM + row) * COLS * 4);
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            const unsigned col = 32u * half + (unsigned)j, target = col / COLS, chunk = (col % COLS) / 4;
+            unsigned addr;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(mine + ((chunk ^ swz) << 4)), "r"(target));
+            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[j]), "r"(v[j + 1]), "r"(v[j + 2]), "r"(v[j + 3]) : "memory");
+        }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp >= EPI_WARP0) {
+#pragma unroll
+        for (int k = 0; k < UNITS; ++k) {
+            const int u = et + k * 32 * SPLIT_EPI_WARPS, row = u / PAIRS, p = u - row * PAIRS, m = m0 + row;
+            const unsigned swz = (unsigned)(row / (8 / CHUNKS)) & (CHUNKS - 1);
+            const unsigned char* at = sums + (size_t)row * COLS * 4 + ((((unsigned)p >> 1) ^ swz) << 4) + (p & 1) * 8;
+            int x0 = 0, x1 = 0;
+#pragma unroll
+            for (int src = 0; src < S; ++src) {
+                const int2 w = *(const int2*)(at + (size_t)src * BM * COLS * 4);
+                x0 += w.x;
+                x1 += w.y;
+            }
+            const int* c = cst + 2 * p;
+            int y0 = split_rescale(x0, sa.form, sa.need_clamp != 0, c, COLS), y1 = split_rescale(x1, sa.form, sa.need_clamp != 0, c + 1, COLS);
+            if (a.r.ptr) {
+                const int* c2 = c + FAST_NP * COLS;
+                const unsigned rw = res[k];
+                if (sa.dp) {
+                    unsigned a4;
+                    if (sa.ef & EF_T_UNSIGNED) asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(a4) : "r"(y1), "r"(y0), "r"(rw));
+                    else asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(a4) : "r"(y1), "r"(y0), "r"(rw));
+                    a4 ^= a.dp_xor;
+                    // row 0 of the residual set holds the column-selecting multiplier words (see perm_block)
+                    if (sa.ef & EF_DP_A_SIGNED) {
+                        asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(y0) : "r"(a4), "r"(c2[0]), "r"(c2[3 * COLS]));
+                        asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(y1) : "r"(a4), "r"(c2[1]), "r"(c2[3 * COLS + 1]));
+                    } else {
+                        asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(y0) : "r"(a4), "r"(c2[0]), "r"(c2[3 * COLS]));
+                        asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(y1) : "r"(a4), "r"(c2[1]), "r"(c2[3 * COLS + 1]));
+                    }
+                    y0 >>= c2[4 * COLS];
+                    y1 >>= c2[4 * COLS + 1];
+                } else {
+                    const bool ru = (sa.ef & EF_RES_UNSIGNED) != 0;
+                    const int form2 = sa.form == EF_WIDE ? 0 : sa.form;   // the second stage of a wide cell is the 32-bit one
+                    y0 = split_rescale(min(max(y0, a.t_lo), a.t_hi) + byte_extend(rw, 0, ru), form2, sa.need_clamp != 0, c2, COLS);
+                    y1 = split_rescale(min(max(y1, a.t_lo), a.t_hi) + byte_extend(rw, 1, ru), form2, sa.need_clamp != 0, c2 + 1, COLS);
+                }
+            }
+            const unsigned w = pack4_sat(y0, y1, 0, 0, a.out_unsigned != 0);
+            const int ch = n0 + perm_real_channel(part0 + 2 * p, sa.perm_ng);
+            if (m < a.m_base + a.M && ch < a.N) *(unsigned short*)((uint8_t*)a.out + (size_t)m * a.N + ch) = (unsigned short)w;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(64u) : "memory");
+    }
+}
+
+// Whether the CTAs of a cluster share a tile: from 24 K blocks on and up to half the chip.  Measured with one image: at 36 blocks a
+// layer goes from 16.4 us to 12.3; at 16 and 18 it gains nothing and takes the idle SMs that the next kernel's prologue would run on
+// (ResNet-50 274 us with 36-block layers split, 286 with all from 12 on, 289 with none), as do 128 CTAs at four images.
+static bool igemm_split(long long tiles, int num_kb, int num_sms)
+{
+    return num_kb >= 24 && num_kb <= SPLIT * SPLIT_STAGES && tiles * SPLIT <= num_sms / 2;
+}
+
 // Eight weights per thread; at most a few megabytes that stay in L2
 __global__ void __launch_bounds__(256) widen_int4_kernel(const uint8_t* __restrict__ packed, int rows_src, int ng_src, int8_t* __restrict__ dst, int rows,
                                                          int ng_dst, unsigned words)
@@ -1227,6 +1474,38 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
         attr_set[dev] = true;
     }
     int tiles = a.num_m_tiles * a.num_n_tiles;
+    // Few tiles, long K: a cluster of CTAs per tile
+    const int num_kb = plan.taps * ((plan.Cin + plan.BK - 1) / plan.BK);
+    if (use_fast && !plan.w4 && !plan.grouped && plan.BN == SPLIT_BN && igemm_split(tiles, num_kb, plan.num_sms)) {
+        static std::atomic<bool> split_attr_set[64];
+        if (dev >= 0 && dev < 64 && !split_attr_set[dev]) {
+            cudaError_t e = cudaFuncSetAttribute(igemm_split_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            if (e != cudaSuccess) return e;
+            split_attr_set[dev] = true;
+        }
+        SplitArgs sa;
+        sa.g = a;
+        sa.per = (num_kb + SPLIT - 1) / SPLIT;
+        sa.perm_ng = plan.perm / 8;
+        sa.form = fast.form;
+        sa.need_clamp = fast.need_clamp ? 1 : 0;
+        sa.dp = r.ptr && fast.dp4a && !fast.need_clamp ? 1 : 0;
+        sa.ef = a.ef;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(tiles * SPLIT));
+        cfg.blockDim = dim3(SPLIT_THREADS);
+        cfg.dynamicSmemBytes = split_smem_bytes(sa.per, plan.BK);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = SPLIT;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        return cudaLaunchKernelEx(&cfg, igemm_split_tcgen05_kernel, plan.tmA, plan.tmB, sa);
+    }
     int grid = plan.grid < tiles ? plan.grid : tiles;
     // a grid that is a multiple of the number of column blocks keeps every CTA on one column block,
     // so its per-channel constants are staged once

@@ -212,6 +212,7 @@ struct IgemmPlan {
     // im2col geometry
     int oW, oH, kW, sX, sY, pL, pT, dX, dY;
     int grid;             // CTAs to launch
+    int num_sms;
     int late_weights;     // the weights are the previous kernel's output: not before griddepcontrol.wait
     size_t smem_bytes;
 };

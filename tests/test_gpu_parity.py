@@ -123,6 +123,28 @@ def test_depthwise_as_block_diagonal_groups_on_the_tensor_cores(case, mode):
     compare_net(net, batch, want_engine='depthwise-tcgen05')
 
 
+# (C, H, W, O, k, stride, pad, batch): few tiles and a long K, so the eight CTAs of a cluster share a tile - parts of K of unequal
+# length, the shortest and the longest K, rows and columns beyond the layer, narrow K slabs, im2col and plain loads
+SPLIT_K_CASES = [(512, 7, 7, 512, 3, 1, 1, 1), (3072, 3, 5, 320, 1, 1, 0, 2), (256, 9, 11, 96, 4, 1, 1, 2), (64, 6, 6, 64, 5, 2, 2, 3),
+                 (48, 10, 10, 160, 5, 1, 2, 1), (4096, 1, 1, 512, 1, 1, 0, 5), (96, 8, 8, 64, 3, 1, 1, 9), (768, 12, 12, 128, 3, 2, 1, 2)]
+
+
+@pytest.mark.parametrize('case', SPLIT_K_CASES, ids=lambda c: 'C%d_%dx%d_O%d_k%d_s%d_p%d_b%d' % c)
+@pytest.mark.parametrize('mode', ['double', 'fixed', 'float'])
+def test_clusters_share_a_tile(case, mode):
+    C, H, W, O, k, s, p, batch = case
+    for act, uns in (('relu', True), ('linear', False)):
+        compare_net(single_conv_net(C, H, W, O, k, s, p, in_unsigned=uns, act=act, mode=mode), batch)
+    if s == 1 and C == O:   # with a residual sum, in both signedness combinations
+        for act in ('relu', 'linear'):
+            b = netdesc.NetBuilder('split', C, H, W, 9, mode, weight_dist=('normal', 30))
+            c0 = b.conv(-1, C, 1, act=act, name='c0')
+            c1 = b.conv(c0, C, k, pad=p, act='linear', name='c1')
+            b.sum([c1, c0], act='relu', name='sum')
+            n, eng = compare_net(b.net, batch, flags=0)
+            assert 'fused' in eng
+
+
 # (C, H, W, O, k, stride, pad, input unsigned, builder keywords): layers the 256-row variant can take
 # (weight blocks beyond the resident limit, 128-byte K slabs, 256-column tiles, no residual)
 PAIR_CASES = [(512, 9, 9, 256, 1, 1, 0, True, {}), (256, 14, 14, 256, 3, 1, 1, True, {}),
