@@ -147,7 +147,9 @@ size_t stem_pool_weight_bytes(const ConvGeom& g);
 void stem_pool_arrange_weights(const ConvGeom& g, const int8_t* w_ohwi, int8_t* dst);
 int stem_pool_make_plan(StemPoolPlan* plan, const void* d_s2d, const int8_t* d_w_arranged, const ConvGeom& g, const PoolGeom& p, int max_batch,
                         int in_unsigned, int num_sms, const char** why);
-cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_base, const FastQuant& fast, void* out, int* status_word, cudaStream_t s);
+bool stem_pool_takes_image(const StemPoolPlan& plan, const ConvGeom& g, const void* in);
+cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_base, const void* raw, const FastQuant& fast, void* out, int* status_word,
+                             cudaStream_t s);
 
 // ---- stride-1 convolution from a shared-memory input patch (tcgen05 kind::i8) ----
 struct PatchPlan {

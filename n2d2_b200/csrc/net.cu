@@ -1145,7 +1145,9 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 if ((c.pool_first ? stem_pool_make_plan(&c.stem_pool, c.d_pad4, c.d_weights, g, c.fused_pool, max_batch, uns, net->num_sms, &why)
                                   : stem_s2d_make_plan(&c.stem2, c.d_pad4, c.d_weights, g, max_batch, uns, net->num_sms, &why,
                                                        c.pool_fused ? &c.fused_pool : nullptr)) == 0) {
-                    net->launches++;
+                    ConvGeom gb = g;
+                    gb.B = max_batch;
+                    if (!c.pool_first || !stem_pool_takes_image(c.stem_pool, gb, nullptr)) net->launches++;   // (of an aligned image)
                     c.engine = ENG_STEM_S2D;
                     continue;
                 }
@@ -1514,8 +1516,9 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         int Hs = 0, Ws = 0;
         stem_s2d_dims(g, &Hs, &Ws);
         if (c.pool_first) {
-            CUDA_TRY(launch_s2d_image(in0, g, batch, (uint8_t*)c.d_pad4 + (size_t)img0 * Hs * Ws * 16, s));
-            CUDA_TRY(launch_stem_pool(c.stem_pool, g, img0, c.fast, out, net->d_status, s));
+            const bool raw = stem_pool_takes_image(c.stem_pool, g, in0);
+            if (!raw) CUDA_TRY(launch_s2d_image(in0, g, batch, (uint8_t*)c.d_pad4 + (size_t)img0 * Hs * Ws * 16, s));
+            CUDA_TRY(launch_stem_pool(c.stem_pool, g, img0, raw ? in0 : nullptr, c.fast, out, net->d_status, s));
             break;
         }
         if (stem_s2d_set_batch(&c.stem2, c.geom, batch)) return fail(N2D2B_ERR_INVALID, "first-layer plan failed for %d images", batch);

@@ -35,7 +35,9 @@ static constexpr int SP_EPI_WARP0 = 2;
 static constexpr int SP_GROUPS = 4;           // epilogue warps per TMEM lane quadrant, a quarter of the pooled columns each
 static constexpr int SP_EPI_WARPS = 4 * SP_GROUPS;
 static constexpr int SP_ISSUERS = 2;           // MMA-issuing warps (warp 1 and the last one): row pairs alternate between them
+static constexpr int SP_WRITERS = 4;           // warps that re-lay the image where it does not come re-laid (warp 0 and the last three)
 static constexpr int SP_THREADS = 32 * (SP_EPI_WARP0 + SP_EPI_WARPS + SP_ISSUERS - 1);
+static constexpr int SP_THREADS_RAW = SP_THREADS + 32 * (SP_WRITERS - 1);
 static constexpr int SP_RING = 16;            // pairs of re-laid image rows in flight (a power of two)
 static constexpr int SP_CHANNELS = 64;
 
@@ -45,6 +47,9 @@ struct StemPoolArgs {
     int KH, KWp;            // filter rows and (even) filter columns after space-to-depth
     int Wp;                 // pixels per row of the re-laid image
     int n_base;             // first image of this call within the re-laid buffer
+    const uint8_t* raw;     // RAW: the image itself, three channels, rows of whole words
+    int H, W, shift;        // RAW: its size; what the re-laid image is moved by (even)
+    int groups_per_row;     // RAW: groups of four input pixels behind a row of the re-laid image
     int chunk_alloc;        // bytes between ring slots
     int w_bytes;
     unsigned idesc;
@@ -83,10 +88,21 @@ __device__ __forceinline__ void sp_issue_pair(unsigned d, const unsigned (&x)[5]
             sp_mma(d, w_lo + (unsigned)(ky * 128 * 2 * KP + 16 * j), w_hi, x[ky >> 1] + ((ky & 1) ? Wp : 0u) + 2u * j, x_hi, idesc, (ky | j) ? 1u : 0u);
 }
 
+__device__ __forceinline__ unsigned sp_pack2(int y0, int y1, bool out_unsigned)
+{
+    unsigned w;
+    if (out_unsigned) asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(y1), "r"(y0), "r"(0));
+    else asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(y1), "r"(y0), "r"(0));
+    return w;
+}
+
 // HP: pooled columns per lane and row (eight times as many per row and CTA)
 // SHAPE: 1 = 4 x 4 filter after space-to-depth (a 7x7/2 or 8x8/2 filter), 2 = 2 x 2 (a 3x3/2 filter), 0 = any
-template <int HP, int SHAPE, bool CLAMP, int FORM>
-__global__ void __launch_bounds__(SP_THREADS, 1)
+// RAW: the image comes as it is, [H][W][3] bytes; four warps write the re-laid rows into the ring.  A lane takes four adjacent pixels of
+// two image rows, 12 bytes of each as words, and writes the two 16-byte pixels they make (the separate re-layout wrote and read
+// 216 KB per 224 x 224 image; conv1 + pool1 of ResNet-50 at 1024 images went from 300 us to 270)
+template <int HP, int SHAPE, bool CLAMP, int FORM, bool RAW>
+__global__ void __launch_bounds__(RAW ? SP_THREADS_RAW : SP_THREADS, 1)
 stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPoolArgs a)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -125,9 +141,10 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
     const int step_n = (int)gridDim.x / a.bands, step_b = (int)gridDim.x - step_n * a.bands;
     const int n_first = (int)blockIdx.x / a.bands, band_first = (int)blockIdx.x - n_first * a.bands;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer: pairs of image rows
-        if (elect_one()) {
+    constexpr int WRITER1 = SP_EPI_WARP0 + SP_EPI_WARPS + SP_ISSUERS - 1;   // the second of the RAW form's writers
+    if (warp == 0 || (RAW && warp >= WRITER1)) {
+        // ------------------------------------------------------------------ TMA producer, or writers: pairs of image rows
+        if (warp == 0 && elect_one()) {
             mbar_expect_tx(wfull, (unsigned)a.w_bytes);
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                          ::"r"(smem_u32(smem)), "l"(a.w), "r"((unsigned)a.w_bytes), "r"(wfull) : "memory");
@@ -138,9 +155,53 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
         unsigned seq = 0;
         bool ok = true;
         int n = n_first, band = band_first;
+        const unsigned me = warp == 0 ? 0u : (unsigned)(warp - WRITER1 + 1);
+        constexpr int GROUPS = 5;   // per lane: two rows of at most 65 groups
         for (int item = blockIdx.x; item < a.items && ok; item += gridDim.x) {
             const int chunks = band_rows(band) + 1 + ahead, row0 = 2 * band * a.P;
             for (int c = 0; c < chunks; ++c, ++seq) {
+                if (RAW) {
+                    if (seq % SP_WRITERS != me) continue;
+                    // all loads of the chunk are on their way before the slot is waited for
+                    unsigned w[GROUPS][2][3];
+                    const unsigned row_words = (unsigned)a.W * 3u / 4u;
+#pragma unroll
+                    for (int k = 0; k < GROUPS; ++k) {
+                        const int t = lane + 32 * k, r = t >= a.groups_per_row ? 1 : 0, x0 = 4 * (t - r * a.groups_per_row) - (a.shift + 3) / 4 * 4;
+#pragma unroll
+                        for (int dy = 0; dy < 2; ++dy) {
+                            const int y = 2 * (row0 + 2 * c + r) + dy - a.shift;
+                            const bool in = t < 2 * a.groups_per_row && (unsigned)y < (unsigned)a.H && (unsigned)x0 < (unsigned)a.W;
+                            const unsigned* p = (const unsigned*)a.raw + (size_t)(unsigned)(n * a.H + y) * row_words + (unsigned)x0 * 3u / 4u;
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) w[k][dy][j] = in ? __ldg(p + j) : 0u;
+                        }
+                    }
+                    const unsigned slot = seq & (SP_RING - 1), ph = (seq / SP_RING) & 1u;
+                    if (!mbar_wait_issuer(empty0 + 8u * slot, ph ^ 1u, abort_flag, a.status, 1)) { ok = false; break; }
+#pragma unroll
+                    for (int k = 0; k < GROUPS; ++k) {
+                        const int t = lane + 32 * k, r = t >= a.groups_per_row ? 1 : 0, x0 = 4 * (t - r * a.groups_per_row) - (a.shift + 3) / 4 * 4;
+                        const int X = (x0 + a.shift) / 2;   // first of the two pixels; -1 where the shift is no multiple of four
+                        if (t >= 2 * a.groups_per_row) continue;
+                        unsigned px[2][4];
+#pragma unroll
+                        for (int dy = 0; dy < 2; ++dy) {
+                            const unsigned* v = w[k][dy];
+                            px[dy][0] = v[0] & 0xffffffu;
+                            px[dy][1] = __byte_perm(v[0], v[1], 0x0543) & 0xffffffu;
+                            px[dy][2] = __byte_perm(v[1], v[2], 0x0432) & 0xffffffu;
+                            px[dy][3] = v[2] >> 8;
+                        }
+                        uint4* o = (uint4*)(ring + (size_t)slot * a.chunk_alloc) + r * a.Wp + X;
+                        if (X >= 0 && X < a.Wp) o[0] = make_uint4(px[0][0], px[0][1], px[1][0], px[1][1]);
+                        if (X + 1 < a.Wp) o[1] = make_uint4(px[0][2], px[0][3], px[1][2], px[1][3]);
+                    }
+                    fence_async_smem();   // generic stores, read by the tensor core through the async proxy
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full0 + 8u * slot);
+                    continue;
+                }
                 const unsigned slot = seq & (SP_RING - 1), ph = (seq / SP_RING) & 1u;
                 if (!mbar_wait_issuer(empty0 + 8u * slot, ph ^ 1u, abort_flag, a.status, 1)) { ok = false; break; }
                 if (elect_one()) {
@@ -153,7 +214,7 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
             band += step_b;
             if (band >= a.bands) { band -= a.bands; ++n; }
         }
-    } else if (warp == 1 || warp >= SP_EPI_WARP0 + SP_EPI_WARPS) {
+    } else if (warp == 1 || warp == SP_EPI_WARP0 + SP_EPI_WARPS) {
         // ------------------------------------------------------------------ MMA issuers
         // One alone took 1030 cycles per row pair, its waits and commits on top of the 620 the tensor pipe is busy
         const unsigned me = warp == 1 ? 0u : 1u;
@@ -208,6 +269,7 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
         const int lo = __ldg(a.fq + 0 * a.cpad + ch), hi = __ldg(a.fq + 1 * a.cpad + ch), mu = __ldg(a.fq + 2 * a.cpad + ch);
         const int ad = __ldg(a.fq + 3 * a.cpad + ch), sh = __ldg(a.fq + 4 * a.cpad + ch);
         const int pos0 = group * 2 * HP + (second ? HP : 0);   // this lane's first pooled column
+        const int valid = min(HP, a.poW - pos0);               // and how many of its columns exist
         const unsigned lane_base = tmem_base + ((unsigned)(quad * 32) << 16);
         const unsigned col0 = (unsigned)(group * 4 * HP);      // first convolution column of the warp, 4 HP + 1 in all
         const unsigned col_last = min(col0 + 32u, 127u);       // HP = 8: the 33rd (rows of 64 pooled columns do not occur)
@@ -234,6 +296,7 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(tempty0 + 8u * slot);
+                int y[HP + 1];
 #pragma unroll
                 for (int i = 0; i < HP; ++i) {
                     // maxima of three columns: pooled columns i (left half) and i + HP (right half) of this lane's row
@@ -243,14 +306,19 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
                     const int own = second ? r : l;
                     const int other = __shfl_xor_sync(0xffffffffu, second ? l : r, 16);
                     const int first_row = second ? other : own;
-                    if (q > 0 && pos0 + i < a.poW) {
-                        int y = rescale<CLAMP, FORM>(max(best[i], first_row), lo, hi, mu, ad, sh);
-                        y = min(max(y, a.out_lo), a.out_hi);
-                        o[(size_t)i * SP_CHANNELS] = (uint8_t)y;
-                    }
+                    y[i] = rescale<CLAMP, FORM>(max(best[i], first_row), lo, hi, mu, ad, sh);
                     best[i] = max(own, other);
                 }
-                if (q > 0) o += (size_t)a.poW * SP_CHANNELS;
+                if (q > 0) {
+                    y[HP] = 0;
+#pragma unroll
+                    for (int i = 0; i < HP; i += 2) {
+                        const unsigned w = sp_pack2(y[i], y[i + 1], a.out_hi > 127);
+                        if (i < valid) o[(size_t)i * SP_CHANNELS] = (uint8_t)w;
+                        if (i + 1 < valid) o[(size_t)(i + 1) * SP_CHANNELS] = (uint8_t)(w >> 8);
+                    }
+                    o += (size_t)a.poW * SP_CHANNELS;
+                }
             }
             n += step_n;
             band += step_b;
@@ -319,6 +387,17 @@ void stem_pool_arrange_weights(const ConvGeom& g, const int8_t* w_ohwi, int8_t* 
     }
 }
 
+// The kernel re-lays the images of this call itself (see RAW): three channels, whole words per row, and bands of four pooled rows and
+// more - in short ones the latency of the first loads and the rows that bands share cost more than the other kernel (ResNet-50 at one
+// image 276 us against 280)
+bool stem_pool_takes_image(const StemPoolPlan& plan, const ConvGeom& g, const void* in)
+{
+    int P, KH, KWp;
+    stem_s2d_filter(g, &P, &KH, &KWp);
+    return (long long)g.B * plan.poH >= 4ll * plan.num_sms && g.C == 3 && g.W % 4 == 0 && P % 2 == 0 && ((uintptr_t)in & 3) == 0 && (long long)g.B * g.H < (1ll << 31)
+        && (P + 3) / 4 * 4 - P + 2 * plan.Wp + 3 <= 4 * 80;
+}
+
 int stem_pool_make_plan(StemPoolPlan* plan, const void* d_s2d, const int8_t* d_w_arranged, const ConvGeom& g, const PoolGeom& p, int max_batch,
                         int in_unsigned, int num_sms, const char** why)
 {
@@ -357,7 +436,9 @@ int stem_pool_make_plan(StemPoolPlan* plan, const void* d_s2d, const int8_t* d_w
     return 0;
 }
 
-cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_base, const FastQuant& fast, void* out, int* status_word, cudaStream_t s)
+// raw: the call's images as they are (stem_pool_takes_image), or nullptr: re-laid in the plan's buffer
+cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_base, const void* raw, const FastQuant& fast, void* out, int* status_word,
+                             cudaStream_t s)
 {
     if (g.B == 0) return cudaSuccess;
     StemPoolArgs a;
@@ -374,6 +455,12 @@ cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_
     if ((long long)g.B * a.bands >= (1ll << 31)) return cudaErrorInvalidValue;
     a.items = g.B * a.bands;
     a.n_base = n_base;
+    a.raw = (const uint8_t*)raw;
+    a.H = g.H;
+    a.W = g.W;
+    int KH, KWp;
+    stem_s2d_filter(g, &a.shift, &KH, &KWp);
+    a.groups_per_row = ((a.shift + 3) / 4 * 4 - a.shift + 2 * plan.Wp + 3) / 4;
     a.chunk_alloc = (2 * plan.Wp * 16 + 127) & ~127;
     a.w_bytes = plan.w_bytes;
     const int N = (g.oW + 15) & ~15;
@@ -387,30 +474,33 @@ cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_
     a.out_lo = fast.out_unsigned ? 0 : -128;
     a.out_hi = fast.out_unsigned ? 255 : 127;
     typedef void (*Kernel)(const CUtensorMap, const StemPoolArgs);
-#define N2D2B_SP1(S, C, F) {stem_pool_tcgen05_kernel<4, S, C, F>, stem_pool_tcgen05_kernel<6, S, C, F>, stem_pool_tcgen05_kernel<7, S, C, F>, \
-                            stem_pool_tcgen05_kernel<8, S, C, F>}
-#define N2D2B_SP(C, F) {N2D2B_SP1(0, C, F), N2D2B_SP1(1, C, F), N2D2B_SP1(2, C, F)}
-    static const Kernel variants[5][3][4] = {N2D2B_SP(false, 0), N2D2B_SP(true, 0), N2D2B_SP(false, EF_FLOAT), N2D2B_SP(true, EF_FLOAT),
-                                             N2D2B_SP(false, EF_WIDE)};   // the wide form has no clamps
+#define N2D2B_SP0(S, C, F, R) {stem_pool_tcgen05_kernel<4, S, C, F, R>, stem_pool_tcgen05_kernel<6, S, C, F, R>, \
+                               stem_pool_tcgen05_kernel<7, S, C, F, R>, stem_pool_tcgen05_kernel<8, S, C, F, R>}
+#define N2D2B_SP1(C, F, R) {N2D2B_SP0(0, C, F, R), N2D2B_SP0(1, C, F, R), N2D2B_SP0(2, C, F, R)}
+#define N2D2B_SP(R) {N2D2B_SP1(false, 0, R), N2D2B_SP1(true, 0, R), N2D2B_SP1(false, EF_FLOAT, R), N2D2B_SP1(true, EF_FLOAT, R), \
+                     N2D2B_SP1(false, EF_WIDE, R)}   // the wide form has no clamps
+    static const Kernel variants[2][5][3][4] = {N2D2B_SP(false), N2D2B_SP(true)};
 #undef N2D2B_SP
 #undef N2D2B_SP1
+#undef N2D2B_SP0
     static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        for (auto& set : variants)
-            for (auto& shapes : set)
-                for (Kernel k : shapes) {
-                    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-                    if (e != cudaSuccess) return e;
-                }
+        for (auto& layouts : variants)
+            for (auto& set : layouts)
+                for (auto& shapes : set)
+                    for (Kernel k : shapes) {
+                        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+                        if (e != cudaSuccess) return e;
+                    }
         attr_set[dev] = true;
     }
     const int shape = plan.KH == 4 && plan.KWp == 4 ? 1 : (plan.KH == 2 && plan.KWp == 2 ? 2 : 0);
     const int form = fast.form == EF_WIDE ? 4 : (fast.form == EF_FLOAT ? 2 : 0) + (fast.need_clamp ? 1 : 0);
     const int per_lane = (plan.poW + 7) / 8, hp = per_lane <= 4 ? 0 : (per_lane <= 6 ? 1 : (per_lane <= 7 ? 2 : 3));
     const int grid = a.items < plan.num_sms ? a.items : plan.num_sms;
-    return launch_pdl(variants[form][shape][hp], grid, SP_THREADS, plan.smem_bytes, s, plan.tmX, a);
+    return launch_pdl(variants[raw ? 1 : 0][form][shape][hp], grid, raw ? SP_THREADS_RAW : SP_THREADS, plan.smem_bytes, s, plan.tmX, a);
 }
 
 }  // namespace n2d2b
