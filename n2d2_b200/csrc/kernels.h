@@ -185,7 +185,8 @@ void patch_permute_weights(const int8_t* w, int8_t* dst, int O, size_t row_bytes
 int patch_make_plan(PatchPlan* plan, const void* in, const int8_t* w, const ConvGeom& g, int in_unsigned, int num_sms,
                     const char** why);
 // n_base: first image of this call within the tensors the plan was encoded for (`out` = the tensor's base)
-cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g, int n_base, const FastQuant& fast, void* out,
+bool patch_takes_residual(const ConvGeom& g);
+cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g, int n_base, const Residual& r, const FastQuant& fast, void* out,
                          int* status_word, cudaStream_t s);
 
 // ---- tensor-core implicit GEMM (tcgen05 kind::i8) ----

@@ -1025,7 +1025,7 @@ static int plan_widened(n2d2b_net* net)
         const char* why = "";
         c.w8_ng_src = c.plan.perm / 8;
         c.w8_rows = g.O;
-        if (!res && patch_eligible(g) && patch_make_plan(&c.patch8, c.plan_input, (const int8_t*)net->d_w8, g, in_u, net->num_sms, &why) == 0) {
+        if ((!res || (patch_takes_residual(g) && !c.fast.dp4a)) && patch_eligible(g) && patch_make_plan(&c.patch8, c.plan_input, (const int8_t*)net->d_w8, g, in_u, net->num_sms, &why) == 0) {
             c.patch8.late_weights = 1;
             c.w8_ng_dst = 4;
             c.w8 = CellRec::W8_PATCH;
@@ -1302,13 +1302,15 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 c.has_plan = true;
                 c.plan_input = in_ptr;  // nullptr = must be re-encoded with the real input
                 if (!(flags & N2D2B_EXACT64_EPILOGUE) && !c.pad_O) {
-                    const bool res_i8 = c.residual >= 0 && net->tensors[c.residual].dtype == DT_I8;
+                    // (the patch kernel's residual stage is not the dot-product form)
+                    const bool res_i8 = c.residual >= 0 && net->tensors[c.residual].dtype == DT_I8 && (w4 || !patch_takes_residual(gb));
                     if (int rc = upload_fast(c, net->tensors[c.output], res_i8,
                                              c.residual >= 0 ? net->tensors[c.residual].is_unsigned : 0, w4))
                         return rc;
                 }
                 // small-channel stride-1 layers read their input once, from a shared-memory patch
-                if (!w4 && !c.pad_O && c.fast.enabled && c.residual < 0 && net->tensors[c.output].dtype == DT_I8
+                if (!w4 && !c.pad_O && c.fast.enabled && (c.residual < 0 || (patch_takes_residual(gb) && net->tensors[c.residual].dtype == DT_I8))
+                    && net->tensors[c.output].dtype == DT_I8
                     && !(flags & (N2D2B_FORCE_IM2COL | N2D2B_EXACT64_EPILOGUE)) && patch_eligible(gb)
                     && patch_make_plan(&c.patch, enc_ptr, c.d_weights, gb, net->tensors[c.inputs[0]].is_unsigned,
                                        net->num_sms, &why) == 0)
@@ -1451,7 +1453,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         g.B = batch;
         if (c.w8 == CellRec::W8_PATCH) {
             if (patch_set_batch(&c.patch8, c.geom, batch)) return fail(N2D2B_ERR_INVALID, "patch plan failed for %d images", batch);
-            CUDA_TRY(launch_patch(c.patch8, g, img0, c.fast, out, net->d_status, s));
+            CUDA_TRY(launch_patch(c.patch8, g, img0, r, c.fast, out, net->d_status, s));
             return 0;
         }
         IgemmPlan p = c.plan8;
@@ -1507,7 +1509,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         if (patch_set_batch(&c.patch, c.geom, batch)) return fail(N2D2B_ERR_INVALID, "patch plan failed for %d images", batch);
         ConvGeom g = c.geom;
         g.B = batch;
-        CUDA_TRY(launch_patch(c.patch, g, img0, c.fast, out, net->d_status, s));
+        CUDA_TRY(launch_patch(c.patch, g, img0, r, c.fast, out, net->d_status, s));
         break;
     }
     case ENG_STEM_S2D: {

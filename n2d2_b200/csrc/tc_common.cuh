@@ -685,14 +685,16 @@ __device__ __forceinline__ void perm_block(const unsigned* vA, const unsigned* v
     }
 }
 
-// The same block (no residual) written straight to global memory: with the permuted layout a thread holds eight
+// The same block written straight to global memory: with the permuted layout a thread holds eight
 // consecutive channels of a row, four neighbouring lanes a whole 32-byte sector of it, so the bytes need no detour
 // through a staging region when the rows' addresses have no regular pattern a TMA store could follow (the band
 // kernels, whose rows are pixels of a padded raster).  out + rowoff[k] = address of channel pcol0's byte of row tr + 8k
-// in the output, rowok bit k = that row exists.
-template <bool CLAMP, int EF>
+// in the output, rowok bit k = that row exists.  RES: res[k] = the eight residual bytes of the thread's channels in row tr + 8k; the
+// constants of the sum stand 128 columns behind the cell's own.
+template <bool CLAMP, int EF, bool RES = false>
 __device__ __forceinline__ void perm_block_global(const unsigned* vA, const unsigned* vB, unsigned par_off, int pcol0,
-                                                  uint8_t* out, const unsigned (&rowoff)[4], unsigned rowok, int lane)
+                                                  uint8_t* out, const unsigned (&rowoff)[4], unsigned rowok, int lane, const uint2* res = nullptr,
+                                                  int t_lo = 0, int t_hi = 0)
 {
     unsigned char* const sm = dyn_smem();
     constexpr int NK = 4, NH = 2;
@@ -713,15 +715,34 @@ __device__ __forceinline__ void perm_block_global(const unsigned* vA, const unsi
         }
         const int muv[4] = {mu.x, mu.y, mu.z, mu.w}, adv[4] = {ad.x, ad.y, ad.z, ad.w}, shv[4] = {sh.x, sh.y, sh.z, sh.w};
         const int lov[4] = {lo.x, lo.y, lo.z, lo.w}, hiv[4] = {hi.x, hi.y, hi.z, hi.w};
+        int y[NK][4];
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
             const unsigned* v = (k < 2) ? vA : vB;
-            int y[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                y[c] = rescale<CLAMP, EF>((int)v[4 * (2 * h + (c >> 1)) + 2 * (k & 1) + (c & 1)], lov[c], hiv[c], muv[c], adv[c], shv[c]);
+                y[k][c] = rescale<CLAMP, EF>((int)v[4 * (2 * h + (c >> 1)) + 2 * (k & 1) + (c & 1)], lov[c], hiv[c], muv[c], adv[c], shv[c]);
+                if (RES) y[k][c] = min(max(y[k][c], t_lo), t_hi) + byte_extend(h ? res[k].y : res[k].x, c, (EF & EF_RES_UNSIGNED) != 0);
             }
-            outw[k][h] = pack4_sat(y[0], y[1], y[2], y[3], (EF & EF_OUT_UNSIGNED) != 0);
+            if (!RES) outw[k][h] = pack4_sat(y[k][0], y[k][1], y[k][2], y[k][3], (EF & EF_OUT_UNSIGNED) != 0);
+        }
+        if (RES) {
+            // the sum's constants only now: both sets at once are 40 registers
+            asm volatile("" ::: "memory");
+            const int4 mu2 = *(const int4*)(sm + pp + 512 + 2 * 1024), ad2 = *(const int4*)(sm + pp + 512 + 3 * 1024), sh2 = *(const int4*)(sm + pp + 512 + 4 * 1024);
+            int4 lo2 = make_int4(0, 0, 0, 0), hi2 = lo2;
+            if (CLAMP) {
+                lo2 = *(const int4*)(sm + pp + 512 + 0 * 1024);
+                hi2 = *(const int4*)(sm + pp + 512 + 1 * 1024);
+            }
+            const int mu2v[4] = {mu2.x, mu2.y, mu2.z, mu2.w}, ad2v[4] = {ad2.x, ad2.y, ad2.z, ad2.w}, sh2v[4] = {sh2.x, sh2.y, sh2.z, sh2.w};
+            const int lo2v[4] = {lo2.x, lo2.y, lo2.z, lo2.w}, hi2v[4] = {hi2.x, hi2.y, hi2.z, hi2.w};
+#pragma unroll
+            for (int k = 0; k < NK; ++k) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) y[k][c] = rescale<CLAMP, EF & ~EF_WIDE>(y[k][c], lo2v[c], hi2v[c], mu2v[c], ad2v[c], sh2v[c]);
+                outw[k][h] = pack4_sat(y[k][0], y[k][1], y[k][2], y[k][3], (EF & EF_OUT_UNSIGNED) != 0);
+            }
         }
     }
 #pragma unroll

@@ -123,6 +123,23 @@ def test_depthwise_as_block_diagonal_groups_on_the_tensor_cores(case, mode):
     compare_net(net, batch, want_engine='depthwise-tcgen05')
 
 
+# (H, W, batch): 64 -> 64 3x3 layers with a residual sum in the patch kernel - one and several bands, odd edges
+PATCH_RES_CASES = [(55, 55, 3), (9, 7, 1), (20, 33, 5), (4, 130, 2)]
+
+
+@pytest.mark.parametrize('case', PATCH_RES_CASES, ids=lambda c: '%dx%d_b%d' % c)
+@pytest.mark.parametrize('mode', ['single', 'double', 'fixed', 'float'])
+def test_patch_kernel_with_a_residual_sum(case, mode):
+    H, W, batch = case
+    for acts in (('relu', 'linear', 'relu'), ('linear', 'relu', 'linear'), ('linear', 'linear', 'relu'), ('relu', 'relu', 'relu')):
+        b = netdesc.NetBuilder('patchres', 64, H, W, 9, mode, weight_dist=('normal', 30))
+        c0 = b.conv(-1, 64, 1, act=acts[0], name='c0')
+        c1 = b.conv(c0, 64, 3, pad=1, act=acts[1], name='c1')
+        b.sum([c1, c0], act=acts[2], name='sum')
+        n, eng = compare_net(b.net, batch, flags=0)
+        assert eng == ['tcgen05', 'patch-tcgen05', 'fused']
+
+
 # (C, H, W, O, k, stride, pad, batch): few tiles and a long K, so the eight CTAs of a cluster share a tile - parts of K of unequal
 # length, the shortest and the longest K, rows and columns beyond the layer, narrow K slabs, im2col and plain loads
 SPLIT_K_CASES = [(512, 7, 7, 512, 3, 1, 1, 1), (3072, 3, 5, 320, 1, 1, 0, 2), (256, 9, 11, 96, 4, 1, 1, 2), (64, 6, 6, 64, 5, 2, 2, 3),
