@@ -365,7 +365,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         bool ok = true;
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
             for (int kb = 0; kb < num_kb; ++kb) {
-                if (!mbar_wait_warp(full0 + 8u * s, ph, abort_flag, a.status, 12, lane)) { ok = false; break; }
+                if (!mbar_wait_warp(full0 + 8u * s, ph, abort_flag, a.status, 12)) { ok = false; break; }
                 unsigned char* bt = tiles + (size_t)s * stage_bytes + a_stage_bytes;
                 const unsigned char* pk = bt + b_stage_bytes;
 #pragma unroll 2
@@ -418,7 +418,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             const unsigned pb = pready0 + 8u * (stage_it & 1u);
             __syncwarp();
             if (lane == 0) mbar_arrive(pb);
-            if (!mbar_wait_warp(pb, (stage_it >> 1) & 1u, abort_flag, a.status, 5, lane)) return false;
+            if (!mbar_wait_warp(pb, (stage_it >> 1) & 1u, abort_flag, a.status, 5)) return false;
             staged_n_tile = n_tile;
             ++stage_it;
             return true;
@@ -498,7 +498,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                 ++mine;
                 continue;
             } else {
-                if (!mbar_wait_warp(tfull0 + 8u * as, aph, abort_flag, a.status, 4, lane)) { ok = false; break; }
+                if (!mbar_wait_warp(tfull0 + 8u * as, aph, abort_flag, a.status, 4)) { ok = false; break; }
                 tc_fence_after();
                 for (int cc = 0; cc < cols_per_warp && part < 2; cc += 32) {
                     const int c0 = cbase + cc;
@@ -773,7 +773,7 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(pready);
-        bool ok = mbar_wait_warp(pready, 0, abort_flag, a.status, 5, lane);
+        bool ok = mbar_wait_warp(pready, 0, abort_flag, a.status, 5);
         pdl_wait();
         unsigned pit = 0;
         int m_pair = (int)blockIdx.x / a.num_n_tiles;
@@ -789,7 +789,7 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
             for (int h = 0; h < 2 && ok; ++h) {
                 const int gy = a.m_base + (2 * pair_now + h) * BM + quad * 32;
                 const bool active = gx < a.N && gy < m_end;
-                if (!mbar_wait_warp(tfull0 + 8u * h, pit & 1u, abort_flag, a.status, 4, lane)) { ok = false; break; }
+                if (!mbar_wait_warp(tfull0 + 8u * h, pit & 1u, abort_flag, a.status, 4)) { ok = false; break; }
                 tc_fence_after();
                 const unsigned tbase = tmem_base + ((unsigned)(quad * 32) << 16) + (unsigned)(h * 256 + cbase);
 #pragma unroll 1
@@ -1271,7 +1271,7 @@ igemm_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
         const int quad = warp & 3, half = (warp - EPI_WARP0) >> 2, row = quad * 32 + lane;
         unsigned v[32];
         if (nkb > 0) {
-            ok = mbar_wait_warp(tfull, 0, abort_flag, a.status, 4, lane);
+            ok = mbar_wait_warp(tfull, 0, abort_flag, a.status, 4);
             tc_fence_after();
             if (ok) {
                 tc_ld32(tmem_base + ((unsigned)(quad * 32) << 16) + 32u * half, v);

@@ -359,7 +359,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
 #pragma unroll
                     for (int k = 0; k < 4; ++k) res[k] = (rowok >> k) & 1u ? __ldg((const uint2*)(rp + rowoff[k])) : make_uint2(0u, 0u);
                 }
-                if (!mbar_wait_warp(tfull0 + 8u * group, sph, abort_flag, a.status, 4, lane)) { ok = false; break; }
+                if (!mbar_wait_warp(tfull0 + 8u * group, sph, abort_flag, a.status, 4)) { ok = false; break; }
                 tc_fence_after();
                 const unsigned tbase = tmem_base + ((unsigned)(quad * 32) << 16) + (unsigned)(group * a.BN);
                 if (RES) {

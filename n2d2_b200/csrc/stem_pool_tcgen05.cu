@@ -285,7 +285,7 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
             for (int i = 0; i < HP; ++i) best[i] = 0;
             for (int q = 0; q <= rows; ++q, ++acc) {
                 const unsigned slot = acc & (SP_SLOTS - 1), sph = (acc / SP_SLOTS) & 1u;
-                if (!mbar_wait_warp(tfull0 + 8u * slot, sph, abort_flag, a.status, 4, lane)) { ok = false; break; }
+                if (!mbar_wait_warp(tfull0 + 8u * slot, sph, abort_flag, a.status, 4)) { ok = false; break; }
                 tc_fence_after();
                 unsigned v[33];
                 const unsigned t = lane_base + slot * 128u;

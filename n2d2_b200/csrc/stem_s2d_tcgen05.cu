@@ -383,7 +383,7 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
                 for (int t = 0; t < T; ++t, ++seq) {
                     if ((int)(seq & (Z_SLOTS - 1)) != group) continue;
                     const unsigned sph = (seq / Z_SLOTS) & 1u;
-                    if (!mbar_wait_warp(tfull0 + 8u * group, sph, abort_flag, a.status, 4, lane)) { ok = false; break; }
+                    if (!mbar_wait_warp(tfull0 + 8u * group, sph, abort_flag, a.status, 4)) { ok = false; break; }
                     tc_fence_after();
                     const unsigned tbase = tmem_base + ((unsigned)(quad * 32) << 16) + (unsigned)(group * a.BN);
                     // this warp's 32 positions of the tile, at their place in the band buffer (a multiple of 32 rows
@@ -399,7 +399,7 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
                 // every warp has written its tiles of the band: meet, then pool from the complete band
                 __syncwarp();
                 if (lane == 0) mbar_arrive(cdone0 + 8u * cb);
-                if (!mbar_wait_warp(cdone0 + 8u * cb, (bandit >> 1) & 1u, abort_flag, a.status, 13, lane)) { ok = false; break; }
+                if (!mbar_wait_warp(cdone0 + 8u * cb, (bandit >> 1) & 1u, abort_flag, a.status, 13)) { ok = false; break; }
                 const int prow0 = band * a.P;
                 const int np = a.pool_oH - prow0 < a.P ? a.pool_oH - prow0 : a.P;
                 const int units = np * a.pool_oW * nvec;
@@ -436,7 +436,7 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
             for (int t = 0; t < T; ++t, ++seq) {
                 if ((int)(seq & (Z_SLOTS - 1)) != group) continue;
                 const unsigned sph = (seq / Z_SLOTS) & 1u;
-                if (!mbar_wait_warp(tfull0 + 8u * group, sph, abort_flag, a.status, 4, lane)) { ok = false; break; }
+                if (!mbar_wait_warp(tfull0 + 8u * group, sph, abort_flag, a.status, 4)) { ok = false; break; }
                 tc_fence_after();
                 const unsigned tbase = tmem_base + ((unsigned)(quad * 32) << 16) + (unsigned)(group * a.BN);
                 // This lane's four rows of the fragment (positions of the band's raster) and where they go: the bytes leave

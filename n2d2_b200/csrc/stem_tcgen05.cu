@@ -249,7 +249,7 @@ stem_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
             if (rem >= oHW) { rem -= oHW; ++n; }
         };
         auto flush = [&](const uint32_t (&w)[2][2][8]) -> bool {
-            if (!mbar_wait_warp(empty0 + 8u * s, ph ^ 1u, abort_flag, a.status, 1, lane)) return false;
+            if (!mbar_wait_warp(empty0 + 8u * s, ph ^ 1u, abort_flag, a.status, 1)) return false;
             unsigned char* dst = my_row + (size_t)s * a_stage_bytes;
 #pragma unroll
             for (int kb = 0; kb < 2; ++kb) {

@@ -170,19 +170,25 @@ __device__ __forceinline__ bool mbar_peeked()
     return __all_sync(0xffffffffu, ok != 0);
 }
 
-// Warp-wide bounded wait: one lane polls (32 lanes polling one word, times many warps, crowd out the
-// arrivals and the shared-memory traffic of the working warps), then every lane observes the completed
-// phase itself, which costs one successful try_wait and gives each lane its own acquire.
-__device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity, volatile int* abort_flag,
-                                               int* status, int code, int lane)
+// Warp-wide bounded wait.  Every lane polls, so that each has its own acquire and the wait ends with the poll that sees the phase.  One lane
+// polling for the warp, a shuffle and a second wait after it was the longer way round: the 64 -> 256 expansion of
+// ResNet-50 at 512 images 121 us against 102, the whole pass 3323 / 3249, one image 277 / 263; sleeping between polls
+// (20 or 100 ns) measures the same as not.
+__device__ __forceinline__ bool mbar_wait_warp(unsigned bar, unsigned parity, volatile int* abort_flag, int* status, int code)
 {
-    // the common case, a phase that completed long ago, costs one poll of the whole warp
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    unsigned ok = 1;
-    if (lane == 0) ok = mbar_wait(bar, parity, abort_flag, status, code) ? 1u : 0u;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    if (!ok) return false;
-    return mbar_wait(bar, parity, abort_flag, status, code);
+    const unsigned long long t0 = globaltimer_ns();
+    while (true) {
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i)
+            if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+        if (__any_sync(0xffffffffu, globaltimer_ns() - t0 > WAIT_LIMIT_NS)) {
+            *abort_flag = 1;
+            atomicCAS(status, 0, code);
+            return false;
+        }
+    }
 }
 
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* tm, unsigned bar, int x, int y)
@@ -837,9 +843,9 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
         if (lane == 0) bulk_wait_read_all();   // the earlier store has finished reading the region
         __syncwarp();
     }
-    if (!e.dry && !mbar_wait_warp(e.tfull, e.tfull_parity, e.abort_flag, e.status, 4, lane)) return false;
+    if (!e.dry && !mbar_wait_warp(e.tfull, e.tfull_parity, e.abort_flag, e.status, 4)) return false;
     if (RES) {
-        if (!e.dry && !mbar_wait_warp(e.rbar + 8u * b, (st.t >> e.slot_shift) & 1u, e.abort_flag, e.status, 7, lane)) return false;
+        if (!e.dry && !mbar_wait_warp(e.rbar + 8u * b, (st.t >> e.slot_shift) & 1u, e.abort_flag, e.status, 7)) return false;
     }
     tc_fence_after();
     if (active) {
