@@ -763,6 +763,7 @@ __device__ __forceinline__ void perm_block_global(const unsigned* vA, const unsi
 struct EpiTile {
     unsigned tmem_acc;      // TMEM address of the accumulator stage (lane 0, first column)
     int BN, N, M, m0, n0;
+    uint8_t* out;           // the output matrix [M][N]
     int wp;                 // columns per warp: BN / (epilogue warps per TMEM quadrant); 64, 32 or 16
     unsigned par_off;       // staged per-channel constants of this column block (byte offset in dynamic shared memory)
     unsigned region_off;    // this warp's staging region(s) (1024-byte aligned; byte offset in dynamic shared memory)
@@ -824,7 +825,21 @@ __device__ __forceinline__ void epi_issue_residual(const CUtensorMap* tmR, unsig
     }
 }
 
-template <bool RES, bool CLAMP, bool DP, bool PERM = false, bool W4 = false>
+// The tile's columns of one warp straight to global memory (32-column blocks)
+template <bool CLAMP, int EF>
+__device__ __forceinline__ void epi_drain_direct(const EpiTile& e, unsigned tbase, int cbase, uint8_t* out, const unsigned (&rowoff)[4], unsigned rowok, int lane)
+{
+#pragma unroll 1
+    for (int cb = 0; cb < e.wp; cb += 32) {
+        unsigned va[16], vb[16];
+        tc_ld_2x16x256b_x4_wait(tbase + (unsigned)cb, va, vb);
+        perm_block_global<CLAMP, EF>(va, vb, e.par_off, cbase + cb, out + cb, rowoff, e.n0 + cbase + cb < e.N ? rowok : 0u, lane);
+    }
+}
+
+// DIRECT: a launch of a tile or two per CTA, whose end is the latency of its last stores, writes from the registers (warps of 32 columns
+// and more); long launches store through TMA, whose issue costs fewer slots
+template <bool RES, bool CLAMP, bool DP, bool PERM = false, bool W4 = false, bool DIRECT = false>
 __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const CUtensorMap* tmR, const EpiTile& e, int quad,
                                                    int cp, int lane, EpiState& st)
 {
@@ -834,6 +849,34 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
     const int cbase = cp * wp;
     const int gx = e.n0 + cbase, gy = e.m0 + quad * 32;
     const bool active = gx < e.N && gy < e.M;
+    if (DIRECT && !RES && PERM && !W4 && e.wp >= 32) {
+        unsigned rowoff[4], rowok = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int row = (lane >> 2) + 8 * k;
+            rowoff[k] = (unsigned)row * (unsigned)e.N;
+            if (gy + row < e.M && !e.dry) rowok |= 1u << k;
+        }
+        uint8_t* const out = e.out + (size_t)gy * e.N + gx;
+        if (!e.dry && !mbar_wait_warp(e.tfull, e.tfull_parity, e.abort_flag, e.status, 4)) return false;
+        tc_fence_after();
+        if (active) {
+            const unsigned tbase = e.tmem_acc + ((unsigned)(quad * 32) << 16) + (unsigned)cbase;
+            switch (e.ef & (EF_OUT_UNSIGNED | EF_WIDE | EF_FLOAT)) {
+            case 0: epi_drain_direct<CLAMP, 0>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_OUT_UNSIGNED: epi_drain_direct<CLAMP, EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_WIDE: epi_drain_direct<false, EF_WIDE>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_FLOAT: epi_drain_direct<CLAMP, EF_FLOAT>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_FLOAT | EF_OUT_UNSIGNED: epi_drain_direct<CLAMP, EF_FLOAT | EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            default: epi_drain_direct<false, EF_WIDE | EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0 && !e.dry) mbar_arrive(e.tempty);
+        if (!e.dry) ++st.t;
+        return true;
+    }
     // a residual cell cycles through its staging regions; the caller issued this tile's residual load
     // (epi_issue_residual) into region t mod slots, after the store that last used the region had drained
     const unsigned b = RES ? (st.t & ((1u << e.slot_shift) - 1u)) : 0u;
