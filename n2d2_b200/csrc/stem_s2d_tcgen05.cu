@@ -436,9 +436,6 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
             for (int t = 0; t < T; ++t, ++seq) {
                 if ((int)(seq & (Z_SLOTS - 1)) != group) continue;
                 const unsigned sph = (seq / Z_SLOTS) & 1u;
-                if (!mbar_wait_warp(tfull0 + 8u * group, sph, abort_flag, a.status, 4)) { ok = false; break; }
-                tc_fence_after();
-                const unsigned tbase = tmem_base + ((unsigned)(quad * 32) << 16) + (unsigned)(group * a.BN);
                 // This lane's four rows of the fragment (positions of the band's raster) and where they go: the bytes leave
                 // the registers for global memory directly, eight channels per lane, a 32-byte sector per four lanes
                 unsigned rowoff[4];   // byte offsets within the band: below 2^32
@@ -451,6 +448,9 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
                     if (x < (unsigned)a.oW && yy < (unsigned)rows) rowok |= 1u << k;
                     rowoff[k] = (yy * (unsigned)a.oW + x) * (unsigned)a.N;
                 }
+                if (!mbar_wait_warp(tfull0 + 8u * group, sph, abort_flag, a.status, 4)) { ok = false; break; }
+                tc_fence_after();
+                const unsigned tbase = tmem_base + ((unsigned)(quad * 32) << 16) + (unsigned)(group * a.BN);
 #pragma unroll 1
                 for (int cb = 0; cb < a.N; cb += 32) {
                     unsigned va[16], vb[16];
