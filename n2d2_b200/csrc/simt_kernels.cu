@@ -1102,7 +1102,8 @@ cudaError_t launch_argmax(const void* scores, int dtype, int is_unsigned, size_t
 // moves its head to its tail on a score > r (when it holds more than one element).  The groups are emitted from the
 // highest score down until topN entries are out.  One warp per pixel takes 32 classes at a time: pass 0 is a prefix
 // minimum over (score, class), a block of classes without a score > r appends in parallel, and only the at most topN
-// larger scores are walked one by one (33 images, 1000 classes, top 5: 94 us with both scans on one lane).
+// larger scores are walked one by one (33 images, 1000 classes, top 5: 94 us with both scans on one lane, 18 with a scan and two
+// votes for every block, 13 since blocks that change nothing are passed over).
 // Shared memory: three int arrays of C entries.  Output [image][k][pixel of the image], like the reference.
 template <typename T>
 __global__ void topn_kernel(const T* __restrict__ scores, size_t pixels, size_t hw, int C, int topN, int32_t* __restrict__ labels,
@@ -1122,25 +1123,41 @@ __global__ void topn_kernel(const T* __restrict__ scores, size_t pixels, size_t 
         // key = score (biased to unsigned) and class: the smallest key is the first of the smallest scores
         const unsigned long long none = ~0ull;
         unsigned long long run = none;   // minimum of the blocks before this one
-        for (int c0 = 0; c0 < C; c0 += 32) {
-            const int c = c0 + lane;
-            const int v = c < C ? (int)row[c] : 0;
-            const unsigned long long own = c < C ? ((unsigned long long)((unsigned)v ^ 0x80000000u) << 32 | (unsigned)c) : none;
-            unsigned long long inc = own;
+        // (eight blocks' loads at a time; a block whose smallest score is not below the running minimum drops nothing: most of them)
+        int run_v = INT32_MAX;
+        for (int s0 = 0; s0 < C; s0 += 256) {
+            int ahead[8];
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, off);
-                if (lane >= off && o < inc) inc = o;
+            for (int j = 0; j < 8; ++j) ahead[j] = s0 + 32 * j + lane < C ? (int)row[s0 + 32 * j + lane] : INT32_MAX;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int c0 = s0 + 32 * j, c = c0 + lane, v = ahead[j];
+                if (c0 >= C) break;
+                if (c0 > 0 && __reduce_min_sync(0xffffffffu, v) >= run_v) {
+                    if (c < C) {
+                        val[c] = v;
+                        ids[c] = c;
+                    }
+                    continue;
+                }
+                const unsigned long long own = c < C ? ((unsigned long long)((unsigned)v ^ 0x80000000u) << 32 | (unsigned)c) : none;
+                unsigned long long inc = own;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, off);
+                    if (lane >= off && o < inc) inc = o;
+                }
+                unsigned long long prev = __shfl_up_sync(0xffffffffu, inc, 1);
+                if (lane == 0 || run < prev) prev = run;
+                if (c < C) {
+                    const bool drop = c > 0 && own < prev;
+                    val[c] = drop ? (int)((unsigned)(prev >> 32) ^ 0x80000000u) : v;
+                    ids[c] = drop ? (int)(unsigned)prev : c;
+                }
+                const unsigned long long blk = __shfl_sync(0xffffffffu, inc, 31);
+                if (blk < run) run = blk;
+                run_v = (int)((unsigned)(run >> 32) ^ 0x80000000u);
             }
-            unsigned long long prev = __shfl_up_sync(0xffffffffu, inc, 1);
-            if (lane == 0 || run < prev) prev = run;
-            if (c < C) {
-                const bool drop = c > 0 && own < prev;
-                val[c] = drop ? (int)((unsigned)(prev >> 32) ^ 0x80000000u) : v;
-                ids[c] = drop ? (int)(unsigned)prev : c;
-            }
-            const unsigned long long blk = __shfl_sync(0xffffffffu, inc, 31);
-            if (blk < run) run = blk;
         }
         __syncwarp();
         if (lane == 0) {
@@ -1156,6 +1173,7 @@ __global__ void topn_kernel(const T* __restrict__ scores, size_t pixels, size_t 
         while (emitted < topN) {
             // next group: the highest score below the previous group's, and its size
             int r = INT32_MIN, cnt = 0;
+#pragma unroll 4
             for (int c = lane; c < C; c += 32) {
                 const int v = val[c];
                 if ((long long)v < prev) {
@@ -1173,43 +1191,51 @@ __global__ void topn_kernel(const T* __restrict__ scores, size_t pixels, size_t 
             }
             if (cnt == 0) break;   // fewer than topN classes
             int h = 0, L = 0;      // head and length of the queue in buf[0, cnt)
-            for (int c0 = 0; c0 < C; c0 += 32) {
-                const int c = c0 + lane;
-                const int v = c < C ? val[c] : INT32_MIN;
-                const unsigned in = __ballot_sync(0xffffffffu, c < C && v == r);
-                unsigned up = __ballot_sync(0xffffffffu, c < C && v > r);
-                if (!(in | up)) continue;
-                if (up == 0) {
-                    if (in & (1u << lane)) {
-                        int t = h + L + __popc(in & before);
-                        if (t >= cnt) t -= cnt;
-                        buf[t] = ids[c];
-                    }
-                    L += __popc(in);
-                } else {
-                    unsigned left = in | up;
-                    while (left) {
-                        // the elements up to the next larger score append, then that score turns the queue by one
-                        const int u = up ? __ffs(up) - 1 : 32;
-                        const unsigned run_in = in & left & (u < 32 ? (1u << u) - 1u : 0xffffffffu);
-                        if (run_in & (1u << lane)) {
-                            int t = h + L + __popc(run_in & before);
+            // blocks with a score of the group or above: their numbers first, without a vote per block
+            for (int seg = 0; seg < C; seg += 1024) {
+                unsigned mine = 0;
+#pragma unroll 8
+                for (int i = 0; i < 32; ++i) {
+                    const int c = seg + 32 * i + lane;
+                    if (c < C && val[c] >= r) mine |= 1u << i;
+                }
+                for (unsigned live = __reduce_or_sync(0xffffffffu, mine); live; live &= live - 1) {
+                    const int c = seg + 32 * (__ffs(live) - 1) + lane;
+                    const int v = c < C ? val[c] : INT32_MIN;
+                    const unsigned in = __ballot_sync(0xffffffffu, c < C && v == r);
+                    unsigned up = __ballot_sync(0xffffffffu, c < C && v > r);
+                    if (up == 0) {
+                        if (in & (1u << lane)) {
+                            int t = h + L + __popc(in & before);
                             if (t >= cnt) t -= cnt;
                             buf[t] = ids[c];
                         }
-                        L += __popc(run_in);
-                        __syncwarp();
-                        if (u < 32 && L > 1) {
-                            if (L < cnt && lane == 0) {   // a full queue turns in place
-                                int t = h + L;
+                        L += __popc(in);
+                    } else {
+                        unsigned left = in | up;
+                        while (left) {
+                            // the elements up to the next larger score append, then that score turns the queue by one
+                            const int u = up ? __ffs(up) - 1 : 32;
+                            const unsigned run_in = in & left & (u < 32 ? (1u << u) - 1u : 0xffffffffu);
+                            if (run_in & (1u << lane)) {
+                                int t = h + L + __popc(run_in & before);
                                 if (t >= cnt) t -= cnt;
-                                buf[t] = buf[h];
+                                buf[t] = ids[c];
                             }
-                            if (++h == cnt) h = 0;
+                            L += __popc(run_in);
+                            __syncwarp();
+                            if (u < 32 && L > 1) {
+                                if (L < cnt && lane == 0) {   // a full queue turns in place
+                                    int t = h + L;
+                                    if (t >= cnt) t -= cnt;
+                                    buf[t] = buf[h];
+                                }
+                                if (++h == cnt) h = 0;
+                            }
+                            __syncwarp();
+                            left = u < 31 ? left & ~((2u << u) - 1u) : 0u;
+                            up = u < 31 ? up & ~((2u << u) - 1u) : 0u;
                         }
-                        __syncwarp();
-                        left = u < 31 ? left & ~((2u << u) - 1u) : 0u;
-                        up = u < 31 ? up & ~((2u << u) - 1u) : 0u;
                     }
                 }
             }
