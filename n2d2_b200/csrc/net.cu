@@ -911,8 +911,8 @@ static int head_candidate_prefix(const n2d2b_net* net)
 // a head tensor may be written while slices < k of every other head tensor are complete and still needed: two
 // head tensors share a buffer only when they have the same bytes per image (slice k of one then lies exactly
 // over slice k of the other, which the per-slice order of the cells has already retired).
-// A stride-2 first layer whose only reader is a max pooling writes the pooled tensor directly (the POOL variant of
-// the space-to-depth kernel): the convolution's output, the largest tensor of such a network, is never stored.
+// A stride-2 first layer whose only reader is a max pooling writes the pooled tensor directly (stem_pool_tcgen05.cu, or on request
+// the POOL variant of the space-to-depth kernel): the convolution's output, the largest tensor of such a network, is never stored.
 static int fuse_stem_pool(n2d2b_net* net);
 
 static int plan_buffers(n2d2b_net* net)
