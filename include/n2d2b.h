@@ -139,6 +139,7 @@ typedef struct n2d2b_tensor_info {
 #define N2D2B_EXACT64_EPILOGUE 16u /* tensor-core cells always use the 64-bit requantisation (cross-check of the 32-bit form) */
 #define N2D2B_FORCE_PAIR 32u      /* 256-row tiles wherever their structure allows, whatever the layer's size (tests) */
 #define N2D2B_FUSE_FIRST_POOL 64u /* a stride-2 first layer whose only reader is an unpadded max pooling writes the pooled tensor itself (its own output never reaches HBM) for every shape that can; without the flag only where that is faster (64 channels, 3x3 / 2 pooling, no negative scaling) */
+#define N2D2B_FORCE_DEPTHWISE_TENSOR 128u /* depthwise cells run as block-diagonal groups on the tensor cores wherever that form exists, also where the CUDA-core kernel is faster (tests) */
 
 const char* n2d2b_last_error(void);
 int n2d2b_version(void);
@@ -243,9 +244,9 @@ int n2d2b_net_read_tensor(n2d2b_net* net, int tensor_id, int batch, void* host_d
 int n2d2b_net_weight_bytes(const n2d2b_net* net, size_t* total_bytes, size_t* packed4_bytes);
 /* Number of kernel launches one forward of `batch` images issues. */
 int n2d2b_net_launches_per_forward(const n2d2b_net* net);
-/* Name of the kernel family cell `cell` runs on ("tcgen05", "tcgen05-pair", "tcgen05-w4", "patch-tcgen05",
- * "stem-tcgen05", "simt", "depthwise", "depthwise-tcgen05", "pool", "sum", "fused").  "depthwise-tcgen05" cells with 3x3 filters
- * run on the CUDA-core kernel in calls where that one is faster. */
+/* Name of the kernel family that runs cell `cell` in an n2d2b_net_forward of the finalized max_batch images ("tcgen05",
+ * "tcgen05-pair", "tcgen05-w4", "patch-tcgen05", "stem-tcgen05", "simt", "depthwise", "depthwise-tcgen05", "pool", "sum",
+ * "fused").  In calls of fewer images a "depthwise-tcgen05" cell may run on the "depthwise" (CUDA-core) kernel. */
 const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell);
 /* Device time of every cell of one forward, in milliseconds (CUDA events on `stream`), like the
  * per-cell timings of DeepNet::propagate (src/DeepNet.cpp:2705-2717). ms has one entry per cell. */

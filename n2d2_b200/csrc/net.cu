@@ -1187,7 +1187,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
             const int taps = g.kH * g.kW;
             for (int ch = 0; ch < g.C; ++ch)
                 for (int t = 0; t < taps; ++t) laid[(size_t)t * g.C + ch] = c.weights[(size_t)ch * taps + t];
-            if (c.fast.enabled && !(flags & N2D2B_FORCE_SIMT) && depthwise3x3_eligible(g)) {
+            if (c.fast.enabled && !(flags & (N2D2B_FORCE_SIMT | N2D2B_FORCE_DEPTHWISE_TENSOR)) && depthwise3x3_eligible(g)) {
                 CUDA_TRY(cudaMalloc((void**)&c.d_dw3x3, laid.size()));
                 CUDA_TRY(cudaMemcpy(c.d_dw3x3, laid.data(), laid.size(), cudaMemcpyHostToDevice));
             }
@@ -1907,9 +1907,11 @@ int n2d2b_net_launches_per_forward(const n2d2b_net* net)
     return net->launches;
 }
 
+// (decided by the same rules as a forward pass of max_batch images)
 const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
 {
     if (!net || cell < 0 || cell >= (int)net->cells.size()) return "";
+    if (use_dw3x3(net->cells[cell], net->max_batch)) return "depthwise";
     switch (net->cells[cell].engine) {
     case ENG_TCGEN05: {
         const CellRec& c = net->cells[cell];

@@ -23,6 +23,7 @@ FORCE_IM2COL = 8
 FORCE_PAIR = 32
 EXACT64_EPILOGUE = 16
 FUSE_FIRST_POOL = 64
+FORCE_DEPTHWISE_TENSOR = 128
 
 
 class N2D2BError(RuntimeError):

@@ -16,8 +16,18 @@ def single_conv_net(C, H, W, O, k, stride=1, pad=0, in_unsigned=True, act='relu'
     return b.net
 
 
-def compare_net(net, batch, flags=KEEP, flavour='i64', x=None, want_engine=None, slices=0, ref=None):
-    """Returns (number of compared layers, engines). Asserts bit-exact equality with the oracle."""
+def kernels_of(call):
+    """Names of the kernels a call launches, as the CUDA profiling interface reports them."""
+    import torch
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return [e.key for e in prof.key_averages()]
+
+
+def compare_net(net, batch, flags=KEEP, flavour='i64', x=None, want_engine=None, slices=0, ref=None, kernels=False):
+    """Returns (number of compared layers, engines), or with `kernels` the kernels that ran. Asserts bit-exact equality with the
+    oracle."""
     if x is None:
         x = netdesc.make_input(net, batch)
     if ref is None:
@@ -41,6 +51,6 @@ def compare_net(net, batch, flags=KEEP, flavour='i64', x=None, want_engine=None,
             bad = int((got != ref[i]).sum())
             assert bad == 0, f"layer {i} {l['name']} ({eng[i]}): {bad} of {ref[i].size} values differ"
             n += 1
-        return n, eng
+        return kernels_of(lambda: qn.forward_host(x)) if kernels else (n, eng)
     finally:
         qn.close()

@@ -74,7 +74,8 @@ def test_depthwise_3x3(case, mode):
     on_tensor_cores = C % 64 == 0 or C == 32 or (s == 1 and C % 32 == 0)
     # (fixed-point scalings with wide shifts have no 32-bit epilogue and stay on the exact CUDA-core kernel)
     want = 'depthwise' if not on_tensor_cores else (('depthwise-tcgen05', 'depthwise') if mode == 'fixed' else 'depthwise-tcgen05')
-    compare_net(net, 3, want_engine=want)
+    compare_net(net, 3, want_engine='depthwise')          # so few outputs: the dot-product kernel
+    compare_net(net, 3, flags=KEEP | R.FORCE_DEPTHWISE_TENSOR, want_engine=want)
     compare_net(net, 3, flags=KEEP | R.FORCE_SIMT, want_engine='depthwise')
     compare_net(net, 3, flags=KEEP | R.EXACT64_EPILOGUE, want_engine='depthwise')
 
@@ -107,7 +108,10 @@ DW_TC_STRIDED_CASES = [(64, 112, 112, 3, 2, 1, 1, 3), (128, 56, 56, 3, 2, 1, 1, 
 def test_strided_depthwise_as_block_diagonal_groups(case, mode):
     C, H, W, k, st, p, d, batch = case
     net = single_conv_net(C, H, W, C, k, st, p, mode=mode, dil=d, groups=C)
-    compare_net(net, batch, want_engine='depthwise-tcgen05')
+    x = netdesc.make_input(net, batch)
+    ref = oracle.run_net(net, x, 'i64')
+    compare_net(net, batch, x=x, ref=ref)
+    compare_net(net, batch, flags=KEEP | R.FORCE_DEPTHWISE_TENSOR, x=x, ref=ref, want_engine='depthwise-tcgen05')
 
 
 DW_TC_CASES = [(128, 56, 56, 3, 1, 1, 5), (512, 14, 14, 3, 1, 1, 37), (1024, 7, 7, 3, 1, 1, 9), (32, 112, 112, 3, 1, 1, 3),
@@ -120,7 +124,23 @@ DW_TC_CASES = [(128, 56, 56, 3, 1, 1, 5), (512, 14, 14, 3, 1, 1, 37), (1024, 7, 
 def test_depthwise_as_block_diagonal_groups_on_the_tensor_cores(case, mode):
     C, H, W, k, p, d, batch = case
     net = single_conv_net(C, H, W, C, k, 1, p, mode=mode, dil=d, groups=C)
-    compare_net(net, batch, want_engine='depthwise-tcgen05')
+    x = netdesc.make_input(net, batch)
+    ref = oracle.run_net(net, x, 'i64')
+    compare_net(net, batch, x=x, ref=ref)
+    compare_net(net, batch, flags=KEEP | R.FORCE_DEPTHWISE_TENSOR, x=x, ref=ref, want_engine='depthwise-tcgen05')
+
+
+# (C, H, W, stride, smallest batch on the tensor cores): the two forms of MobileNet's early depthwise layers at the line between the
+# kernels (2^24 outputs per call), strided groups of 64 and groups of 32
+@pytest.mark.parametrize('case', [(64, 112, 112, 2, 84), (32, 112, 112, 1, 42)], ids=lambda c: 'C%d_%dx%d_s%d' % c[:4])
+def test_depthwise_engine_is_the_kernel_that_runs(case):
+    C, H, W, s, first = case
+    net = single_conv_net(C, H, W, C, 3, s, 1, mode='single', groups=C)
+    x = netdesc.make_input(net, first)
+    ref = oracle.run_net(net, x, 'i64')
+    for batch, engine in ((first, 'depthwise-tcgen05'), (first - 1, 'depthwise')):
+        kernels = compare_net(net, batch, x=x[:batch], ref=[r[:batch] for r in ref], want_engine=engine, kernels=True)
+        assert any('depthwise3x3' in k for k in kernels) == (engine == 'depthwise')
 
 
 # (H, W, batch): 64 -> 64 3x3 layers with a residual sum in the patch kernel - one and several bands, odd edges
@@ -400,7 +420,10 @@ def test_saturation_activation_on_every_kernel_family(case, mode):
         net = _saturating(build(mode), thr)
         # float scalings and wide fixed-point shifts take the exact 64-bit kernels, whatever the family
         exact_only = mode == 'float' or (mode == 'fixed' and engine in ('stem-tcgen05', 'patch-tcgen05', 'depthwise-tcgen05'))
-        compare_net(net, 3, want_engine=None if exact_only else engine)
+        forced = R.FORCE_DEPTHWISE_TENSOR if engine == 'depthwise-tcgen05' else 0
+        compare_net(net, 3, flags=KEEP | forced, want_engine=None if exact_only else engine)
+        if forced:
+            compare_net(net, 3, want_engine=None if exact_only else 'depthwise')
         compare_net(net, 3, flags=KEEP | R.FORCE_SIMT)
         ref = oracle.run_net(net, netdesc.make_input(net, 3), 'i64')[-1]
         assert int(np.abs(ref).max()) <= thr
