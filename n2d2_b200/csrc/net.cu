@@ -109,7 +109,8 @@ struct CellRec {
     PatchPlan patch8{};
     int w8_rows = 0, w8_ng_src = 0, w8_ng_dst = 0;
     void* d_w8_out = nullptr;     // padded output matrix (see pad_O) of a widened cell
-    // 3x3 depthwise cells: weights as [kH][kW][C] for the dot-product kernel (see use_dw3x3)
+    // 3x3 depthwise cells on the tensor cores: weights as [kH][kW][C] for the calls that the dot-product kernel takes (see
+    // dw3x3_faster), behind the block-diagonal ones in d_weights
     int8_t* d_dw3x3 = nullptr;
     // tensor-core plan
     IgemmPlan plan{};
@@ -659,7 +660,6 @@ void n2d2b_net_destroy(n2d2b_net* net)
         cudaFree(c.d_fast);
         cudaFree(c.d_pad4);
         cudaFree(c.d_colpad);
-        cudaFree(c.d_dw3x3);
         cudaFree(c.d_w8_out);
     }
     cudaFree(net->d_w8);
@@ -1093,6 +1093,19 @@ static int plan_small_net(n2d2b_net* net)
     return 0;
 }
 
+// Whether the dot-product kernel is the faster one for a 3x3 depthwise layer in a call of `batch` images.  The block-diagonal form on
+// the tensor cores moves whole bands of large maps at a time: it is even or ahead where there are many pixels of few channels (256
+// images: 56 x 56 x 128 70 us against 74, 112 x 112 x 32 73 / 74), behind on deep maps (14 x 14 x 512 31 / 24, 7 x 7 x 1024 30 / 17) and
+// in small calls, whose bands leave SMs idle (33 images: 112 x 112 x 32 23 / 16, 14 x 14 x 512 12.4 / 10.3).
+static bool dw3x3_faster(const ConvGeom& g, int batch)
+{
+    return g.C >= 256 || (long long)batch * g.oH * g.oW * g.C < (1ll << 24);
+}
+
+// Whether a cell that has both forms runs on the dot-product kernel in a call of `batch` images (a cell for which that holds up to
+// max_batch has no other form, see finalize)
+static bool use_dw3x3(const CellRec& c, int batch) { return c.d_dw3x3 && dw3x3_faster(c.geom, batch); }
+
 int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
 {
     if (!net) return fail(N2D2B_ERR_INVALID, "net must not be NULL");
@@ -1187,58 +1200,68 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
             const int taps = g.kH * g.kW;
             for (int ch = 0; ch < g.C; ++ch)
                 for (int t = 0; t < taps; ++t) laid[(size_t)t * g.C + ch] = c.weights[(size_t)ch * taps + t];
-            if (c.fast.enabled && !(flags & (N2D2B_FORCE_SIMT | N2D2B_FORCE_DEPTHWISE_TENSOR)) && depthwise3x3_eligible(g)) {
-                CUDA_TRY(cudaMalloc((void**)&c.d_dw3x3, laid.size()));
-                CUDA_TRY(cudaMemcpy(c.d_dw3x3, laid.data(), laid.size(), cudaMemcpyHostToDevice));
-            }
+            // The block-diagonal form is made only where a call within max_batch can take it (the dot-product kernel's rule holds for
+            // every smaller call where it holds for max_batch); the dot-product weights then follow it in the same block.
+            const bool dot = c.fast.enabled && !(flags & (N2D2B_FORCE_SIMT | N2D2B_FORCE_DEPTHWISE_TENSOR)) && depthwise3x3_eligible(g);
+            const bool tensor = c.fast.enabled && !(flags & N2D2B_FORCE_SIMT) && !(dot && dw3x3_faster(g, max_batch));
+            auto alloc_blocks = [&](size_t bytes) -> int {
+                c.d_weight_bytes = bytes + (dot ? laid.size() : 0);
+                CUDA_TRY(cudaMalloc((void**)&c.d_weights, c.d_weight_bytes + 256));
+                return 0;
+            };
+            auto upload_blocks = [&](std::vector<int8_t>& rows) -> int {
+                if (dot) {
+                    c.d_dw3x3 = c.d_weights + rows.size();
+                    rows.insert(rows.end(), laid.begin(), laid.end());
+                }
+                CUDA_TRY(cudaMemcpy(c.d_weights, rows.data(), rows.size(), cudaMemcpyHostToDevice));
+                return 0;
+            };
+            auto drop_blocks = [&] {
+                cudaFree(c.d_weights);
+                c.d_weights = nullptr;
+                c.d_weight_bytes = 0;
+            };
             // Stride-1 layers whose channels come in whole groups of 32 run on the tensor cores as block-diagonal
             // groups (patch kernel); it needs the 32-bit epilogue
             ConvGeom gb = g;
             gb.B = max_batch;
-            if (c.fast.enabled && !(flags & N2D2B_FORCE_SIMT) && patch_eligible(gb)) {
+            const char* why = "";
+            const void* in_ptr = tensor_ptr(net, c.inputs[0], nullptr);
+            static char dw_placeholder[16] __attribute__((aligned(16)));
+            const void* enc_ptr = in_ptr ? in_ptr : (const void*)dw_placeholder;
+            if (tensor && patch_eligible(gb)) {
                 std::vector<int8_t> arranged(patch_dw_weight_bytes(g));
-                patch_dw_arrange_weights(g, c.weights.data(), arranged.data());
-                CUDA_TRY(cudaMalloc((void**)&c.d_weights, arranged.size() + 256));
-                CUDA_TRY(cudaMemcpy(c.d_weights, arranged.data(), arranged.size(), cudaMemcpyHostToDevice));
-                c.d_weight_bytes = arranged.size();
-                const char* why = "";
-                const void* in_ptr = tensor_ptr(net, c.inputs[0], nullptr);
-                static char dw_placeholder[16] __attribute__((aligned(16)));
-                if (patch_make_plan(&c.patch, in_ptr ? in_ptr : (const void*)dw_placeholder, c.d_weights, gb,
-                                    net->tensors[c.inputs[0]].is_unsigned, net->num_sms, &why) == 0) {
+                if (int rc = alloc_blocks(arranged.size())) return rc;
+                if (patch_make_plan(&c.patch, enc_ptr, c.d_weights, gb, net->tensors[c.inputs[0]].is_unsigned, net->num_sms, &why) == 0) {
+                    patch_dw_arrange_weights(g, c.weights.data(), arranged.data());
+                    if (int rc = upload_blocks(arranged)) return rc;
                     c.engine = ENG_PATCH;
                     c.plan_input = in_ptr;   // nullptr = re-encoded with the real input at the first forward pass
                     continue;
                 }
-                cudaFree(c.d_weights);
-                c.d_weights = nullptr;
+                drop_blocks();
             }
             // Strided ones (and whatever else the patch kernel leaves) take the implicit-GEMM kernel the same way: one
             // 64-column tile per group of 64 channels, im2col loads of the group's channel slice
-            if (c.fast.enabled && !(flags & (N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE)) && igemm_dw_group(gb)) {
+            if (tensor && igemm_dw_group(gb)) {
                 std::vector<int8_t> arranged(igemm_dw_weight_bytes(g));
-                igemm_dw_arrange_weights(g, c.weights.data(), arranged.data());
-                CUDA_TRY(cudaMalloc((void**)&c.d_weights, arranged.size() + 256));
-                c.d_weight_bytes = arranged.size();
-                const char* why = "";
-                const void* in_ptr = tensor_ptr(net, c.inputs[0], nullptr);
-                static char dwg_placeholder[16] __attribute__((aligned(16)));
-                if (igemm_make_plan(&c.plan, in_ptr ? in_ptr : (const void*)dwg_placeholder, c.d_weights,
-                                    tensor_ptr(net, c.output, nullptr), nullptr, gb, net->tensors[c.inputs[0]].is_unsigned, 1, 0,
-                                    net->num_sms, &why, 0, 0) == 0
+                if (int rc = alloc_blocks(arranged.size())) return rc;
+                if (igemm_make_plan(&c.plan, enc_ptr, c.d_weights, tensor_ptr(net, c.output, nullptr), nullptr, gb,
+                                    net->tensors[c.inputs[0]].is_unsigned, 1, 0, net->num_sms, &why, 0, 0) == 0
                     && igemm_uses_fast_epilogue(c.plan, c.fast, false, DT_I8)) {
+                    igemm_dw_arrange_weights(g, c.weights.data(), arranged.data());
                     const int pb = igemm_perm_block(c.plan);
                     std::vector<int8_t> rows(arranged.size());
                     igemm_permute_weights(arranged.data(), rows.data(), g.C, arranged.size() / (size_t)g.C, pb);
                     c.plan.perm = pb;
-                    CUDA_TRY(cudaMemcpy(c.d_weights, rows.data(), rows.size(), cudaMemcpyHostToDevice));
+                    if (int rc = upload_blocks(rows)) return rc;
                     c.engine = ENG_TCGEN05;
                     c.has_plan = true;
                     c.plan_input = in_ptr;
                     continue;
                 }
-                cudaFree(c.d_weights);
-                c.d_weights = nullptr;
+                drop_blocks();
             }
         } else {
             c.engine = ENG_SIMT;
@@ -1414,15 +1437,6 @@ static int fuse_stem_pool(n2d2b_net* net)
 }
 
 // ---- forward --------------------------------------------------------------------------------
-// Whether a 3x3 depthwise cell runs on the dot-product kernel in a call of `batch` images.  The block-diagonal form on the tensor
-// cores moves whole bands of large maps at a time: it is even or ahead where there are many pixels of few channels (256 images:
-// 56 x 56 x 128 70 us against 74, 112 x 112 x 32 73 / 74), behind on deep maps (14 x 14 x 512 31 / 24, 7 x 7 x 1024 30 / 17) and in small
-// calls, whose bands leave SMs idle (33 images: 112 x 112 x 32 23 / 16, 14 x 14 x 512 12.4 / 10.3).
-static bool use_dw3x3(const CellRec& c, int batch)
-{
-    return c.d_dw3x3 && (c.geom.C >= 256 || (long long)batch * c.geom.oH * c.geom.oW * c.geom.C < (1ll << 24));
-}
-
 // Runs one cell on images [img0, img0 + batch) of the batch (img0 != 0 only for cells without tensor maps).
 static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, cudaStream_t s, int img0 = 0)
 {

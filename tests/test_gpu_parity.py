@@ -143,6 +143,19 @@ def test_depthwise_engine_is_the_kernel_that_runs(case):
         assert any('depthwise3x3' in k for k in kernels) == (engine == 'depthwise')
 
 
+# (C, H, W, stride, capacity, finalize flags, groups' width of the block-diagonal form or 0, dot-product form kept)
+@pytest.mark.parametrize('case', [(512, 14, 14, 1, 300, 0, 0, True), (64, 112, 112, 2, 83, 0, 0, True), (64, 112, 112, 2, 84, 0, 64, True),
+                                  (32, 112, 112, 1, 42, 0, 32, True), (512, 14, 14, 1, 3, runtime.FORCE_DEPTHWISE_TENSOR, 64, False)],
+                         ids=lambda c: 'C%d_%dx%d_s%d_b%d_f%d' % c[:6])
+def test_depthwise_cells_keep_the_weights_their_calls_can_reach(case):
+    C, H, W, s, capacity, flags, group, dot = case
+    qn = runtime.QuantizedNet(single_conv_net(C, H, W, C, 3, s, 1, mode='single', groups=C), capacity, flags=flags)
+    try:
+        assert qn.weight_bytes() == (9 * C * (group + (1 if dot else 0)), 0)
+    finally:
+        qn.close()
+
+
 # (H, W, batch): 64 -> 64 3x3 layers with a residual sum in the patch kernel - one and several bands, odd edges
 PATCH_RES_CASES = [(55, 55, 3), (9, 7, 1), (20, 33, 5), (4, 130, 2)]
 
