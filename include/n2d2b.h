@@ -240,16 +240,21 @@ int n2d2b_net_tensor_info(const n2d2b_net* net, int tensor_id, n2d2b_tensor_info
 int n2d2b_net_read_tensor(n2d2b_net* net, int tensor_id, int batch, void* host_dst, size_t bytes);
 /* Bytes of weights the network keeps in HBM (*total_bytes), and how many of them are packed 4-bit weights
  * (*packed4_bytes: cells given weight_bits = 4 that run on the implicit-GEMM kernel, which expands them tile by
- * tile in shared memory; other cells hold int8).  Either pointer may be NULL. */
+ * tile in shared memory; other cells hold int8).  A network that runs as one kernel holds its weights a second time, with its rescale
+ * constants, as that kernel reads them.  Either pointer may be NULL. */
 int n2d2b_net_weight_bytes(const n2d2b_net* net, size_t* total_bytes, size_t* packed4_bytes);
-/* Number of kernel launches one forward of `batch` images issues. */
+/* Number of kernel launches one n2d2b_net_forward of max_batch images issues. */
 int n2d2b_net_launches_per_forward(const n2d2b_net* net);
 /* Name of the kernel family that runs cell `cell` in an n2d2b_net_forward of the finalized max_batch images ("tcgen05",
  * "tcgen05-pair", "tcgen05-w4", "patch-tcgen05", "stem-tcgen05", "simt", "depthwise", "depthwise-tcgen05", "pool", "sum",
- * "fused").  In calls of fewer images a "depthwise-tcgen05" cell may run on the "depthwise" (CUDA-core) kernel. */
+ * "fused", "small-net").  In calls of fewer images a "depthwise-tcgen05" cell may run on the "depthwise" (CUDA-core) kernel.
+ * "small-net": every cell of the network, which runs as one kernel; the sliced upload of n2d2b_net_forward_host alone runs such a
+ * network cell by cell. */
 const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell);
 /* Device time of every cell of one forward, in milliseconds (CUDA events on `stream`), like the
- * per-cell timings of DeepNet::propagate (src/DeepNet.cpp:2705-2717). ms has one entry per cell. */
+ * per-cell timings of DeepNet::propagate (src/DeepNet.cpp:2705-2717). ms has one entry per cell; a cell folded into another
+ * one reads about zero, and a network that runs as one kernel has its time in the first entry (finalized with
+ * N2D2B_KEEP_ALL_OUTPUTS or N2D2B_NO_FUSION it runs, and is timed, cell by cell). */
 int n2d2b_net_profile(n2d2b_net* net, const void* d_input, int batch, void* d_output, float* ms, int nb_cells,
                       n2d2b_stream stream);
 

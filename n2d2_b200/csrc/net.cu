@@ -1601,19 +1601,26 @@ static int forward_impl(n2d2b_net* net, const void* d_input, int batch, void* d_
     if (batch == 0) return 0;
     if (!d_input) return fail(N2D2B_ERR_INVALID, "d_input must not be NULL");
     CUDA_TRY(cudaSetDevice(net->device));
-    if (net->d_small && !ms && first_cell == 0) {
-        CUDA_TRY(launch_small_net(net->small, net->d_small, d_input, batch, tensor_ptr(net, final_tensor_of(net), d_input), d_output,
-                                  net->num_sms, s));
-        net->last_input = d_input;
-        return 0;
-    }
+    const bool one_kernel = net->d_small && first_cell == 0;
     std::vector<cudaEvent_t> ev;
     if (ms) {
         if (nb_cells != (int)net->cells.size())
             return fail(N2D2B_ERR_INVALID, "ms must have one entry per cell (%d)", (int)net->cells.size());
-        ev.resize(net->cells.size() + 1);
+        ev.resize((one_kernel ? 1 : net->cells.size()) + 1);
         for (auto& e : ev) CUDA_TRY(cudaEventCreate(&e));
         CUDA_TRY(cudaEventRecord(ev[0], s));
+    }
+    if (one_kernel) {
+        CUDA_TRY(launch_small_net(net->small, net->d_small, d_input, batch, tensor_ptr(net, final_tensor_of(net), d_input), d_output,
+                                  net->num_sms, s));
+        net->last_input = d_input;
+        if (!ms) return 0;
+        CUDA_TRY(cudaEventRecord(ev[1], s));
+        CUDA_TRY(cudaStreamSynchronize(s));
+        std::fill(ms, ms + nb_cells, 0.0f);   // the whole network is the first entry
+        CUDA_TRY(cudaEventElapsedTime(&ms[0], ev[0], ev[1]));
+        for (auto& e : ev) cudaEventDestroy(e);
+        return 0;
     }
     for (size_t ci = (size_t)first_cell; ci < net->cells.size(); ++ci) {
         CellRec& c = net->cells[ci];
@@ -1910,6 +1917,7 @@ int n2d2b_net_weight_bytes(const n2d2b_net* net, size_t* total_bytes, size_t* pa
         total += c.d_weight_bytes;
         if (c.engine == ENG_TCGEN05 && c.plan.w4) packed += c.d_weight_bytes;
     }
+    if (net->d_small) total += net->small.blob.size();
     if (total_bytes) *total_bytes = total;
     if (packed4_bytes) *packed4_bytes = packed;
     return 0;
@@ -1925,6 +1933,7 @@ int n2d2b_net_launches_per_forward(const n2d2b_net* net)
 const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
 {
     if (!net || cell < 0 || cell >= (int)net->cells.size()) return "";
+    if (net->d_small) return "small-net";
     if (use_dw3x3(net->cells[cell], net->max_batch)) return "depthwise";
     switch (net->cells[cell].engine) {
     case ENG_TCGEN05: {

@@ -19,7 +19,7 @@ def single_conv_net(C, H, W, O, k, stride=1, pad=0, in_unsigned=True, act='relu'
 def kernels_of(call):
     """Names of the kernels a call launches, as the CUDA profiling interface reports them."""
     import torch
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
         call()
         torch.cuda.synchronize()
     return [e.key for e in prof.key_averages()]

@@ -7,7 +7,7 @@ import pytest
 from n2d2_b200 import netdesc, runtime
 from oracle import oracle
 
-from gpu_common import KEEP, compare_net, single_conv_net
+from gpu_common import KEEP, compare_net, kernels_of, single_conv_net
 
 # (C, H, W, O, k, pad, dilation, input unsigned): stride-1 layers small enough for resident weights
 PATCH_CASES = [(64, 56, 56, 64, 3, 1, 1, True), (64, 20, 17, 64, 3, 1, 1, True), (32, 9, 9, 32, 3, 1, 1, False),
@@ -902,6 +902,26 @@ def test_small_networks_as_one_kernel(kind, mode, batch):
     finally:
         qn.close()
         other.close()
+
+
+def test_a_small_network_reports_the_kernel_that_runs():
+    import torch
+    net = netdesc.mnist24()
+    x = torch.from_numpy(netdesc.make_input(net, 64)).cuda()
+    for flags in (0, R.NO_FUSION):
+        qn = runtime.QuantizedNet(net, 64, flags=flags)
+        try:
+            y = torch.empty((64, qn.out_elems), dtype=torch.uint8, device='cuda')
+            ms = []
+            kernels = [k for k in kernels_of(lambda: ms.extend(qn.profile(x.data_ptr(), 64, y.data_ptr()))) if 'kernel' in k]
+            assert ms[0] > 0
+            if flags:
+                assert 'small-net' not in qn.engines() and min(ms) > 0 and not any('small_net' in k for k in kernels)
+            else:
+                assert set(qn.engines()) == {'small-net'} and not any(ms[1:]) and len(kernels) == 1 and 'small_net' in kernels[0]
+                assert qn.weight_bytes()[0] > 2 * sum(l['weights'].size for l in net['layers'] if 'weights' in l)
+        finally:
+            qn.close()
 
 
 # enough tiles for the widened form: patch kernel, implicit GEMM with 64- and 256-column tiles, a residual sum, padded outputs
