@@ -246,8 +246,10 @@ int n2d2b_net_weight_bytes(const n2d2b_net* net, size_t* total_bytes, size_t* pa
 /* Number of kernel launches one n2d2b_net_forward of max_batch images issues. */
 int n2d2b_net_launches_per_forward(const n2d2b_net* net);
 /* Name of the kernel family that runs cell `cell` in an n2d2b_net_forward of the finalized max_batch images ("tcgen05",
- * "tcgen05-pair", "tcgen05-w4", "patch-tcgen05", "stem-tcgen05", "simt", "depthwise", "depthwise-tcgen05", "pool", "sum",
+ * "tcgen05-pair", "tcgen05-w4", "tcgen05-widened", "patch-tcgen05", "patch-tcgen05-widened", "stem-tcgen05", "simt", "depthwise", "depthwise-tcgen05", "pool", "sum",
  * "fused", "small-net").  In calls of fewer images a "depthwise-tcgen05" cell may run on the "depthwise" (CUDA-core) kernel.
+ * "tcgen05-w4": packed 4-bit weights expanded in the kernel; "tcgen05-widened", "patch-tcgen05-widened": widened to int8 by a small
+ * kernel ahead of the int8 kernel, in calls of so many images (smaller ones expand in the kernel).
  * "small-net": every cell of the network, which runs as one kernel; the sliced upload of n2d2b_net_forward_host alone runs such a
  * network cell by cell. */
 const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell);

@@ -1934,10 +1934,11 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
 {
     if (!net || cell < 0 || cell >= (int)net->cells.size()) return "";
     if (net->d_small) return "small-net";
-    if (use_dw3x3(net->cells[cell], net->max_batch)) return "depthwise";
-    switch (net->cells[cell].engine) {
+    const CellRec& c = net->cells[cell];
+    if (use_dw3x3(c, net->max_batch)) return "depthwise";
+    if (use_widened(net, c, net->max_batch)) return c.w8 == CellRec::W8_PATCH ? "patch-tcgen05-widened" : "tcgen05-widened";
+    switch (c.engine) {
     case ENG_TCGEN05: {
-        const CellRec& c = net->cells[cell];
         const bool pair = c.plan.pair && c.fast.enabled && c.residual < 0
                           && net->tensors[c.output].dtype == DT_I8 && c.geom.O % 32 == 0;
         if (c.geom.groups > 1) return "depthwise-tcgen05";
@@ -1949,8 +1950,8 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     case ENG_SUM: return "sum";
     case ENG_FUSED: return "fused";
     case ENG_STEM: return "stem-tcgen05";
-    case ENG_STEM_S2D: return net->cells[cell].pool_fused ? "stem-pool-tcgen05" : "stem-tcgen05";
-    case ENG_PATCH: return net->cells[cell].geom.groups > 1 ? "depthwise-tcgen05" : "patch-tcgen05";
+    case ENG_STEM_S2D: return c.pool_fused ? "stem-pool-tcgen05" : "stem-tcgen05";
+    case ENG_PATCH: return c.geom.groups > 1 ? "depthwise-tcgen05" : "patch-tcgen05";
     }
     return "";
 }

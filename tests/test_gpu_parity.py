@@ -942,11 +942,15 @@ def test_packed_int4_weights_widened_for_large_batches(case, mode):
     qn = runtime.QuantizedNet(net, batch)
     few = runtime.QuantizedNet(net, 3)      # the in-kernel expansion
     try:
-        assert 'tcgen05-w4' in qn.engines()
+        assert 'tcgen05-w4' in few.engines() and not any('widened' in e for e in few.engines())
+        assert any('widened' in e for e in qn.engines()) and 'tcgen05-w4' not in qn.engines()
         assert qn.launches_per_forward() > few.launches_per_forward()
         out = qn.forward_host(x)
         assert np.array_equal(out[picks].astype(np.int64), ref)
         assert np.array_equal(few.forward_host(x[picks]), out[picks])
+        kernels, few_kernels = kernels_of(lambda: qn.forward_host(x)), kernels_of(lambda: few.forward_host(x[picks]))
+        assert any('widen_int4' in n for n in kernels) and not any('widen_int4' in n for n in few_kernels)
+        assert any('patch_conv' in n for n in kernels) == ('patch-tcgen05-widened' in qn.engines())
     finally:
         qn.close()
         few.close()
