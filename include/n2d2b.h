@@ -245,13 +245,19 @@ int n2d2b_net_read_tensor(n2d2b_net* net, int tensor_id, int batch, void* host_d
 int n2d2b_net_weight_bytes(const n2d2b_net* net, size_t* total_bytes, size_t* packed4_bytes);
 /* Number of kernel launches one n2d2b_net_forward of max_batch images issues. */
 int n2d2b_net_launches_per_forward(const n2d2b_net* net);
-/* Name of the kernel family that runs cell `cell` in an n2d2b_net_forward of the finalized max_batch images ("tcgen05",
- * "tcgen05-pair", "tcgen05-w4", "tcgen05-widened", "patch-tcgen05", "patch-tcgen05-widened", "stem-tcgen05", "simt", "depthwise", "depthwise-tcgen05", "pool", "sum",
- * "fused", "small-net").  In calls of fewer images a "depthwise-tcgen05" cell may run on the "depthwise" (CUDA-core) kernel.
- * "tcgen05-w4": packed 4-bit weights expanded in the kernel; "tcgen05-widened", "patch-tcgen05-widened": widened to int8 by a small
- * kernel ahead of the int8 kernel, in calls of so many images (smaller ones expand in the kernel).
- * "small-net": every cell of the network, which runs as one kernel; the sliced upload of n2d2b_net_forward_host alone runs such a
- * network cell by cell. */
+/* Name of the kernel family that runs cell `cell` in an n2d2b_net_forward of the finalized max_batch images:
+ *   "tcgen05", "tcgen05-pair"      implicit GEMM (256-row tiles)
+ *   "tcgen05-w4"                   the same, packed 4-bit weights expanded in the kernel
+ *   "tcgen05-widened", "patch-tcgen05-widened"
+ *                                  packed weights widened to int8 ahead of the int8 kernel; smaller calls expand in the kernel
+ *   "patch-tcgen05"                stride-1 layers from a shared-memory patch
+ *   "stem-tcgen05"                 first layers of up to 4 channels
+ *   "stem-pool-tcgen05"            the same with the pooling behind it
+ *   "depthwise-tcgen05"            depthwise as block-diagonal groups; smaller calls may run on the next one
+ *   "depthwise", "simt", "pool", "sum"   CUDA-core kernels
+ *   "fused"                        folded into another cell's kernel
+ *   "small-net"                    every cell of a network that runs as one kernel; the sliced upload of n2d2b_net_forward_host
+ *                                  alone runs such a network cell by cell */
 const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell);
 /* Device time of every cell of one forward, in milliseconds (CUDA events on `stream`), like the
  * per-cell timings of DeepNet::propagate (src/DeepNet.cpp:2705-2717). ms has one entry per cell; a cell folded into another

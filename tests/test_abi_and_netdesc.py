@@ -29,6 +29,16 @@ def test_library_exports_every_declared_entry_point():
         assert hasattr(lib, s), f'{s} is declared in include/ but not exported'
 
 
+def test_header_lists_every_engine_name():
+    source = open(os.path.join(ROOT, 'n2d2_b200', 'csrc', 'net.cu')).read()
+    body = source[source.index('const char* n2d2b_net_cell_engine('):]
+    names = set(re.findall(r'"([a-z][a-z0-9-]+)"', body[:body.index('\n}')]))
+    header = open(os.path.join(ROOT, 'include', 'n2d2b.h')).read()
+    doc = header[:header.index('const char* n2d2b_net_cell_engine(')]
+    listed = set(re.findall(r'"([a-z0-9-]+)"', doc[doc.rindex('/*'):]))
+    assert names and names == listed
+
+
 def test_no_cpu_fallback_without_a_device():
     import torch
     if torch.cuda.is_available():
