@@ -290,7 +290,7 @@ int n2d2b_probe_i8_mma_rate(int device, int n, int reps, double* tops, double* c
  *
  *   d_input / d_output  device buffers: batch x height x width x channels 8-bit values in, batch x
  *                       oH x oW x nb_outputs 8-bit values out (same layout and arithmetic as a conv
- *                       cell added with n2d2b_net_add_conv)
+ *                       cell added with n2d2b_net_add_conv); d_output 16-byte aligned
  *   desc, weights, bias, quant   host data, as for n2d2b_net_add_conv (desc->input is ignored);
  *                       8-bit weights; <= 4 channels, kernel <= 8x8, no dilation or groups, nb_outputs
  *                       a multiple of 32 and <= 128, output at least 2 wide; a shift or fixed-point scaling whose products

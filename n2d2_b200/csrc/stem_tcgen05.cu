@@ -521,6 +521,8 @@ extern "C" int n2d2b_first_conv_noalloc(int device, const void* d_input, int bat
     if (batch < 0 || height < 1 || width < 1 || channels < 1)
         return set_error(N2D2B_ERR_INVALID, "invalid input dimensions");
     if (batch == 0) return 0;
+    // one form stores through a tensor map, the other eight bytes per lane from the registers: neither may start anywhere
+    if ((uintptr_t)d_output & 15) return set_error(N2D2B_ERR_INVALID, "d_output must be 16-byte aligned");
     if (desc->weight_bits != 8) return set_error(N2D2B_ERR_INVALID, "this entry point takes 8-bit weights");
     if (desc->nb_outputs < 1 || desc->kernel_h < 1 || desc->kernel_w < 1 || desc->stride_y < 1 || desc->stride_x < 1
         || desc->pad_top < 0 || desc->pad_left < 0 || desc->pad_bottom < 0 || desc->pad_right < 0)

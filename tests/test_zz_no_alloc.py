@@ -73,6 +73,20 @@ def test_noalloc_first_conv_rejects_what_it_cannot_hold():
         runtime.first_conv_noalloc(d.data_ptr(), 1, 16, 16, 16, True, wide, d.data_ptr())
 
 
+# stride 2 and stride 1: both forms of the layer refuse an output they cannot store to, and the next call runs
+@pytest.mark.parametrize('stride', [2, 1])
+def test_noalloc_first_conv_refuses_a_misaligned_output(stride):
+    import torch
+    net = single_conv_net(3, 30, 28, 64, 3, stride, 1, mode='double', seed=23)
+    out = torch.zeros(2 * 30 * 28 * 64 + 16, dtype=torch.uint8, device='cuda')
+    x = torch.zeros(2 * 30 * 28 * 3, dtype=torch.uint8, device='cuda')
+    for shift in (1, 4, 8):
+        with pytest.raises(runtime.N2D2BError, match='16-byte aligned'):
+            runtime.first_conv_noalloc(x.data_ptr(), 2, 30, 28, 3, True, net['layers'][0], out.data_ptr() + shift)
+    got, want = _both_paths(net, 2, seed=8)
+    assert np.array_equal(got, want)
+
+
 # (C, H, W, O, k, stride, pad, batch): the space-to-depth form with its layer as kernel parameters (whole words per row and not, 32 to
 # 128 outputs, the widest filters) and, for what does not fit it (wide rows, weights beyond the parameters), the copied form
 NOALLOC_CASES = [(3, 224, 224, 64, 7, 2, 3, 3), (3, 97, 99, 32, 3, 2, 1, 5), (1, 40, 44, 96, 5, 2, 2, 2), (4, 64, 60, 128, 7, 2, 3, 2),
