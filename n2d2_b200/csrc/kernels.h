@@ -45,6 +45,8 @@ struct FastQuant;
 cudaError_t launch_conv_depthwise(const void* in, int in_unsigned, const int8_t* w_hwc, const ConvGeom& g,
                                   const QuantDev& q, const FastQuant& fast, void* out, cudaStream_t s);
 // 3x3 depthwise layers, stride 1 or 2, on the 32-bit or floating-point epilogue
+// Bytes on which the input of launch_conv_depthwise has to start: the widest load of the kernel it takes
+int depthwise_alignment(const ConvGeom& g, const FastQuant& fast);
 bool depthwise3x3_eligible(const ConvGeom& g);
 cudaError_t launch_depthwise3x3(const void* in, int in_unsigned, const int8_t* w_hwc, const ConvGeom& g, const FastQuant& fast, void* out,
                                 int num_sms, cudaStream_t s);

@@ -1437,6 +1437,17 @@ static int fuse_stem_pool(n2d2b_net* net)
 }
 
 // ---- forward --------------------------------------------------------------------------------
+// Whether a depthwise cell can read from `in`, which only the caller's own buffer may fail.  A cell that has the block-diagonal form
+// takes what that form's tensor maps take, whichever kernel runs it; the others what the loads of their kernel do.
+static bool depthwise_takes(const n2d2b_net* net, const CellRec& c, int batch, const void* in)
+{
+    if (((uintptr_t)in & 15) == 0) return true;
+    ConvGeom g = c.geom;
+    g.B = batch;
+    const bool block_form = c.fast.enabled && !(net->flags & N2D2B_FORCE_SIMT) && (patch_eligible(g) || igemm_dw_group(g));
+    return !block_form && (uintptr_t)in % depthwise_alignment(g, c.fast) == 0;
+}
+
 // Runs one cell on images [img0, img0 + batch) of the batch (img0 != 0 only for cells without tensor maps).
 static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, cudaStream_t s, int img0 = 0)
 {
@@ -1478,6 +1489,8 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
             CUDA_TRY(launch_drop_padded_columns((const uint8_t*)c.d_w8_out + row0 * c.w8_rows, c.w8_rows, (uint8_t*)out + row0 * g.O, g.O, (size_t)p.M, s));
         return 0;
     }
+    if ((c.engine == ENG_DEPTHWISE || c.d_dw3x3) && !depthwise_takes(net, c, batch, in0))
+        return fail(N2D2B_ERR_INVALID, "a depthwise cell cannot read an input at %p: operands must be 16-byte aligned", in0);
     if (use_dw3x3(c, batch)) {
         ConvGeom g = c.geom;
         g.B = batch;

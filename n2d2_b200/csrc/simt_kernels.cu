@@ -494,14 +494,25 @@ cudaError_t launch_depthwise3x3(const void* in, int in_unsigned, const int8_t* w
     }
 }
 
+// Dilated filters and larger strides whose rescale has the proved 32-bit form: the masked dot-product kernel
+static bool depthwise3x3_masked(const ConvGeom& g, const FastQuant& fast)
+{
+    const int cw = g.C / 4;
+    const bool idx32 = (long long)g.B * g.H * g.W * cw < (1ll << 31) && (long long)g.B * g.oH * g.oW * cw < (1ll << 31);
+    return fast.enabled && fast.form == 0 && g.kH == 3 && g.kW == 3 && 256 % cw == 0 && idx32;
+}
+
+int depthwise_alignment(const ConvGeom& g, const FastQuant& fast)
+{
+    return (fast.enabled && depthwise3x3_eligible(g)) || depthwise3x3_masked(g, fast) ? 4 : 16;
+}
+
 cudaError_t launch_conv_depthwise(const void* in, int in_unsigned, const int8_t* w_hwc,
                                   const ConvGeom& g, const QuantDev& q, const FastQuant& fast, void* out, cudaStream_t s)
 {
     if (fast.enabled && depthwise3x3_eligible(g)) return launch_depthwise3x3(in, in_unsigned, w_hwc, g, fast, out, 148, s);
-    // other 3x3 filters (dilated, larger strides) whose rescale has the proved 32-bit form: the masked dot-product kernel
-    const int cw = g.C / 4;
-    const bool idx32 = (long long)g.B * g.H * g.W * cw < (1ll << 31) && (long long)g.B * g.oH * g.oW * cw < (1ll << 31);
-    if (fast.enabled && fast.form == 0 && g.kH == 3 && g.kW == 3 && 256 % cw == 0 && idx32) {
+    if (depthwise3x3_masked(g, fast)) {
+        const int cw = g.C / 4;
         const long long rows = (long long)g.B * g.oH;
         if (rows == 0 || g.oW == 0) return cudaSuccess;
         // few, long-lived blocks: a thread's weights and constants (29 loads) are fetched once and serve many rows

@@ -95,6 +95,34 @@ def test_depthwise_3x3_dot_products(case, mode):
     compare_net(single_conv_net(C, H, W, C, 3, s, p, in_unsigned=uns, act=act, mode=mode, groups=C), batch)
 
 
+# (C, stride, dilation, finalize flags, alignment the cell asks for): a depthwise cell on the caller's own buffer, by the dot-product kernel,
+# the masked one (dilated), the exact one and as block-diagonal groups
+@pytest.mark.parametrize('case', [(256, 1, 1, 0, 16), (64, 2, 1, 0, 16), (64, 1, 1, runtime.FORCE_SIMT, 4), (16, 1, 1, 0, 4), (16, 1, 2, 0, 4),
+                                  (48, 1, 2, 0, 16), (16, 1, 1, runtime.EXACT64_EPILOGUE, 16), (64, 1, 1, runtime.FORCE_DEPTHWISE_TENSOR, 16)],
+                         ids=lambda c: 'C%d_s%d_d%d_f%d' % c[:4])
+def test_depthwise_cells_refuse_an_input_they_cannot_read(case):
+    import torch
+    C, s, d, flags, need = case
+    net = single_conv_net(C, 9, 11, C, 3, s, d, mode='single', dil=d, groups=C)
+    x = netdesc.make_input(net, 2)
+    ref = oracle.run_net(net, x, 'i64')[-1].reshape(2, -1)
+    qn = runtime.QuantizedNet(net, 2, flags=flags)
+    try:
+        room = torch.zeros(x.size + 16, dtype=torch.uint8, device='cuda')
+        y = torch.empty((2, qn.out_elems), dtype=torch.uint8, device='cuda')
+        for shift in (1, 2, 4, 8, 0):
+            room[shift:shift + x.size] = torch.from_numpy(x.reshape(-1)).cuda()
+            if shift % need:
+                with pytest.raises(runtime.N2D2BError, match='aligned'):
+                    qn.forward_device(room.data_ptr() + shift, 2, y.data_ptr())
+            else:
+                qn.forward_device(room.data_ptr() + shift, 2, y.data_ptr())
+                qn.check()
+                assert np.array_equal(y.cpu().numpy().astype(np.int64), ref)
+    finally:
+        qn.close()
+
+
 # (C, H, W, k, pad, dilation, batch): depthwise layers as block-diagonal groups on the tensor cores - several bands
 # and images per CTA, more groups than fit the grid evenly, 5x5 and dilated filters, one group of 32
 # (C, H, W, k, stride, pad, dilation, batch): the strided ones through im2col loads of the group's channel slice
