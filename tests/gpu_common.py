@@ -1,5 +1,7 @@
 """Helpers shared by the GPU parity tests: run a network description through the C ABI and compare
 every readable tensor with the CPU oracle, bit for bit."""
+import ctypes
+
 import numpy as np
 
 from n2d2_b200 import netdesc, runtime
@@ -16,13 +18,42 @@ def single_conv_net(C, H, W, O, k, stride=1, pad=0, in_unsigned=True, act='relu'
     return b.net
 
 
-def kernels_of(call):
-    """Names of the kernels a call launches, as the CUDA profiling interface reports them."""
+class _KernelNode(ctypes.Structure):   # CUDA_KERNEL_NODE_PARAMS
+    _fields_ = [('func', ctypes.c_void_p), ('sizes', ctypes.c_uint * 7), ('params', ctypes.c_void_p), ('extra', ctypes.c_void_p),
+                ('kern', ctypes.c_void_p), ('ctx', ctypes.c_void_p)]
+
+
+def kernels_of(qn, batch):
+    """Names of the kernels that a forward pass of `batch` images launches: the nodes of its captured graph."""
     import torch
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
-        call()
-        torch.cuda.synchronize()
-    return [e.key for e in prof.key_averages()]
+    i = qn.desc['input']
+    x = torch.zeros((batch, i['H'], i['W'], i['C']), dtype=torch.uint8, device='cuda')
+    y = torch.zeros((batch, qn.out_elems * np.dtype(qn.out_dtype).itemsize), dtype=torch.uint8, device='cuda')
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    cuda = ctypes.CDLL('libcuda.so.1')
+
+    def call(name, *args):
+        rc = getattr(cuda, name)(*args)
+        assert rc == 0, f'{name}: {rc}'
+
+    graph, count = ctypes.c_void_p(), ctypes.c_size_t()
+    call('cuStreamBeginCapture_v2', ctypes.c_void_p(stream.cuda_stream), 1)   # thread-local
+    qn.forward_device(x.data_ptr(), batch, y.data_ptr(), stream.cuda_stream)
+    call('cuStreamEndCapture', ctypes.c_void_p(stream.cuda_stream), ctypes.byref(graph))
+    call('cuGraphGetNodes', graph, None, ctypes.byref(count))
+    nodes = (ctypes.c_void_p * count.value)()
+    call('cuGraphGetNodes', graph, nodes, ctypes.byref(count))
+    names = []
+    for node in nodes:
+        kind, params, name = ctypes.c_int(), _KernelNode(), ctypes.c_char_p()
+        call('cuGraphNodeGetType', ctypes.c_void_p(node), ctypes.byref(kind))
+        if kind.value == 0:   # a kernel
+            call('cuGraphKernelNodeGetParams_v2', ctypes.c_void_p(node), ctypes.byref(params))
+            call('cuFuncGetName', ctypes.byref(name), ctypes.c_void_p(params.func))
+            names.append(name.value.decode())
+    call('cuGraphDestroy', graph)
+    return names
 
 
 def compare_net(net, batch, flags=KEEP, flavour='i64', x=None, want_engine=None, slices=0, ref=None, kernels=False):
@@ -51,6 +82,6 @@ def compare_net(net, batch, flags=KEEP, flavour='i64', x=None, want_engine=None,
             bad = int((got != ref[i]).sum())
             assert bad == 0, f"layer {i} {l['name']} ({eng[i]}): {bad} of {ref[i].size} values differ"
             n += 1
-        return kernels_of(lambda: qn.forward_host(x)) if kernels else (n, eng)
+        return kernels_of(qn, batch) if kernels else (n, eng)
     finally:
         qn.close()

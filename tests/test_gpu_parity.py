@@ -620,7 +620,7 @@ def test_first_layer_with_its_accumulators_pooled(case, mode):
     assert eng == ['stem-pool-tcgen05', 'fused']
     if mode == 'float':   # a scaling that decreases somewhere: the maximum cannot be taken first
         b.net['layers'][0]['quant']['fscale'][5] *= -1
-        n, eng = compare_net(b.net, batch, flags=0)
+        n, eng = compare_net(b.net, batch, flags=R.FORCE_PAIR)   # (the flag: tiny networks cell by cell, too)
         assert eng[1] == 'pool'
 
 
@@ -940,8 +940,7 @@ def test_a_small_network_reports_the_kernel_that_runs():
         qn = runtime.QuantizedNet(net, 64, flags=flags)
         try:
             y = torch.empty((64, qn.out_elems), dtype=torch.uint8, device='cuda')
-            ms = []
-            kernels = [k for k in kernels_of(lambda: ms.extend(qn.profile(x.data_ptr(), 64, y.data_ptr()))) if 'kernel' in k]
+            kernels, ms = kernels_of(qn, 64), qn.profile(x.data_ptr(), 64, y.data_ptr())
             assert ms[0] > 0
             if flags:
                 assert 'small-net' not in qn.engines() and min(ms) > 0 and not any('small_net' in k for k in kernels)
@@ -976,7 +975,7 @@ def test_packed_int4_weights_widened_for_large_batches(case, mode):
         out = qn.forward_host(x)
         assert np.array_equal(out[picks].astype(np.int64), ref)
         assert np.array_equal(few.forward_host(x[picks]), out[picks])
-        kernels, few_kernels = kernels_of(lambda: qn.forward_host(x)), kernels_of(lambda: few.forward_host(x[picks]))
+        kernels, few_kernels = kernels_of(qn, batch), kernels_of(few, 3)
         assert any('widen_int4' in n for n in kernels) and not any('widen_int4' in n for n in few_kernels)
         assert any('patch_conv' in n for n in kernels) == ('patch-tcgen05-widened' in qn.engines())
     finally:
