@@ -26,7 +26,6 @@
 #include <cstdio>
 #include <cstring>
 #include <algorithm>
-#include <atomic>
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -1464,27 +1463,13 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
          igemm_i8_tcgen05_kernel<3, false, true>, igemm_i8_tcgen05_kernel<4, false, true>, igemm_i8_tcgen05_kernel<5, false, true>},
         {igemm_i8_tcgen05_kernel<0, true, false>, igemm_i8_tcgen05_kernel<1, true, false>, igemm_i8_tcgen05_kernel<2, true, false>,
          igemm_i8_tcgen05_kernel<3, true, false>, igemm_i8_tcgen05_kernel<4, true, false>, igemm_i8_tcgen05_kernel<5, true, false>}};
-    static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        for (auto& set : kernels)
-            for (Kernel fn : set) {
-                cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-                if (e != cudaSuccess) return e;
-            }
-        attr_set[dev] = true;
-    }
+    static SmemLimitSet limits[3][6];
     int tiles = a.num_m_tiles * a.num_n_tiles;
     // Few tiles, long K: a cluster of CTAs per tile
     const int num_kb = plan.taps * ((plan.Cin + plan.BK - 1) / plan.BK);
     if (use_fast && !plan.w4 && !plan.grouped && plan.BN == SPLIT_BN && igemm_split(tiles, num_kb, plan.num_sms)) {
-        static std::atomic<bool> split_attr_set[64];
-        if (dev >= 0 && dev < 64 && !split_attr_set[dev]) {
-            cudaError_t e = cudaFuncSetAttribute(igemm_split_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (e != cudaSuccess) return e;
-            split_attr_set[dev] = true;
-        }
+        static SmemLimitSet split_limit;
+        if (cudaError_t e = raise_smem_limit(igemm_split_tcgen05_kernel, split_limit)) return e;
         SplitArgs sa;
         sa.g = a;
         sa.per = (num_kb + SPLIT - 1) / SPLIT;
@@ -1528,14 +1513,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     if (plan.pair && use_fast && !r.ptr) {
         typedef void (*PairKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const IgemmArgs);
         static const PairKernel pair_kernels[2] = {igemm_pair_i8_tcgen05_kernel<false>, igemm_pair_i8_tcgen05_kernel<true>};
-        static std::atomic<bool> pair_attr_set[64];
-        if (dev >= 0 && dev < 64 && !pair_attr_set[dev]) {
-            for (PairKernel k : pair_kernels) {
-                cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-                if (e != cudaSuccess) return e;
-            }
-            pair_attr_set[dev] = true;
-        }
+        static SmemLimitSet pair_limits[2];
         const int pair_tiles = ((a.num_m_tiles + 1) / 2) * a.num_n_tiles;
         int pgrid = plan.grid < pair_tiles ? plan.grid : pair_tiles;
         if (pair_tiles > pgrid && a.num_n_tiles > 1 && pgrid > a.num_n_tiles) pgrid -= pgrid % a.num_n_tiles;
@@ -1543,11 +1521,15 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
             a.step_m = pgrid / a.num_n_tiles;
             a.step_n = pgrid % a.num_n_tiles;
             a.adv_tiles = pixels(2ll * a.step_m * BM);
-            return launch_pdl(pair_kernels[fast.need_clamp ? 1 : 0], pgrid, NUM_THREADS, plan.pair_smem_bytes, s, plan.tmA,
+            const int v = fast.need_clamp ? 1 : 0;
+            if (cudaError_t e = raise_smem_limit(pair_kernels[v], pair_limits[v])) return e;
+            return launch_pdl(pair_kernels[v], pgrid, NUM_THREADS, plan.pair_smem_bytes, s, plan.tmA,
                               plan.tmB, plan.tmO32, a);
         }
     }
-    return launch_pdl(kernels[plan.w4 ? 2 : (tiles <= 2 * grid ? 1 : 0)][mode], grid, NUM_THREADS + (plan.w4 ? 32 * W4_UNPACK_WARPS : 0), plan.smem_bytes, s,
+    const int table = plan.w4 ? 2 : (tiles <= 2 * grid ? 1 : 0);
+    if (cudaError_t e = raise_smem_limit(kernels[table][mode], limits[table][mode])) return e;
+    return launch_pdl(kernels[table][mode], grid, NUM_THREADS + (plan.w4 ? 32 * W4_UNPACK_WARPS : 0), plan.smem_bytes, s,
                       plan.tmA, plan.tmB, plan.tmO, plan.tmR, a);
 }
 

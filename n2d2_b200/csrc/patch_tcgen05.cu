@@ -21,7 +21,6 @@
 // drain every fourth tile: 32-bit requantisation in the fragment layout, the bytes going from the registers straight to
 // the NHWC output (eight consecutive channels per lane).  Every wait is bounded.
 #include <cstring>
-#include <atomic>
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -639,22 +638,15 @@ cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, 
     static const PatchKernel variants[25] = {N2D2B_PATCH(false, 0), N2D2B_PATCH(true, 0), N2D2B_PATCH(false, EF_FLOAT),
                                              N2D2B_PATCH(true, EF_FLOAT), N2D2B_PATCH(false, EF_WIDE)};   // the wide form has no clamps
 #undef N2D2B_PATCH
-    static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        for (PatchKernel k : variants) {
-            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (e != cudaSuccess) return e;
-        }
-        attr_set[dev] = true;
-    }
+    static SmemLimitSet limits[25];
     // a multiple of the group count: CTA b works on group b % G
     const long long items = (long long)a.B * a.bands;
     const long long per_group = plan.num_sms / plan.G > 0 ? plan.num_sms / plan.G : 1;
     const int grid = (int)((items < per_group ? items : per_group) * plan.G);
     const int shape = r.ptr ? 4 : (g.kH == 3 && g.kW == 3 && !plan.b_stream) ? (g.C == 32 ? 1 : (g.C == 64 ? 2 : 3)) : 0;
-    return launch_pdl(variants[(fast.form == EF_WIDE ? 20 : (fast.form == EF_FLOAT ? 10 : 0) + (fast.need_clamp ? 5 : 0)) + shape], grid, r.ptr ? P_THREADS_RES : P_THREADS, plan.smem_bytes, s, plan.tmA, plan.tmB, a);
+    const int v = (fast.form == EF_WIDE ? 20 : (fast.form == EF_FLOAT ? 10 : 0) + (fast.need_clamp ? 5 : 0)) + shape;
+    if (cudaError_t e = raise_smem_limit(variants[v], limits[v])) return e;
+    return launch_pdl(variants[v], grid, r.ptr ? P_THREADS_RES : P_THREADS, plan.smem_bytes, s, plan.tmA, plan.tmB, a);
 }
 
 }  // namespace n2d2b

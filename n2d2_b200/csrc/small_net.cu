@@ -15,7 +15,6 @@
 #include <cstring>
 #include <algorithm>
 #include <vector>
-#include <atomic>
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -365,15 +364,7 @@ cudaError_t launch_small_net(const SmallNetPlan& p, const void* d_blob, const vo
     a.in_copies = p.in_copies; a.in_copy_stride = p.in_copy_stride;
     a.in_bytes = p.in_bytes; a.in_place = p.in_place; a.in_pitch = p.in_pitch; a.in_row = p.in_row; a.in_words = p.in_words;
     a.out_bytes = p.out_bytes;
-    static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(small_net_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SN_SMEM_MAX);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(small_net_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SN_SMEM_MAX);
-        if (e != cudaSuccess) return e;
-        attr_set[dev] = true;
-    }
+    static SmemLimitSet limits[2];
     // One image per CTA while that gives every image a CTA at once, four per pass beyond.  Up to one image per SM the CTA asks
     // for more than half of the shared memory: with room for two, the CTAs of a call pack onto the SMs that the call before
     // (64 images: 14.5 instead of 9.6 us) has left.
@@ -382,9 +373,11 @@ cudaError_t launch_small_net(const SmallNetPlan& p, const void* d_blob, const vo
     const int per_sm1 = smem1 <= 110 * 1024 ? 2 : 1, per_sm4 = smem4 <= 110 * 1024 ? 2 : 1;
     if (batch <= num_sms * per_sm1 || p.group == 1) {
         const int grid = std::min(batch, num_sms * per_sm1);
+        if (cudaError_t e = raise_smem_limit(small_net_kernel<1>, limits[0], SN_SMEM_MAX)) return e;
         if (batch <= num_sms) smem1 = std::max<size_t>(smem1, 120 * 1024);
         return launch_pdl(small_net_kernel<1>, grid, SN_THREADS, smem1, s, a, (const uint8_t*)in, batch, (uint8_t*)out, (uint8_t*)out2);
     }
+    if (cudaError_t e = raise_smem_limit(small_net_kernel<4>, limits[1], SN_SMEM_MAX)) return e;
     const int grid = std::min((batch + 3) / 4, num_sms * per_sm4);
     return launch_pdl(small_net_kernel<4>, grid, SN_THREADS, smem4, s, a, (const uint8_t*)in, batch, (uint8_t*)out, (uint8_t*)out2);
 }

@@ -24,7 +24,6 @@
 // computes one row pair more than it has pooled rows.  Every wait is bounded.
 #include <cstring>
 #include <algorithm>
-#include <atomic>
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -483,24 +482,14 @@ cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_
 #undef N2D2B_SP
 #undef N2D2B_SP1
 #undef N2D2B_SP0
-    static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        for (auto& layouts : variants)
-            for (auto& set : layouts)
-                for (auto& shapes : set)
-                    for (Kernel k : shapes) {
-                        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-                        if (e != cudaSuccess) return e;
-                    }
-        attr_set[dev] = true;
-    }
+    static SmemLimitSet limits[2][5][3][4];
     const int shape = plan.KH == 4 && plan.KWp == 4 ? 1 : (plan.KH == 2 && plan.KWp == 2 ? 2 : 0);
     const int form = fast.form == EF_WIDE ? 4 : (fast.form == EF_FLOAT ? 2 : 0) + (fast.need_clamp ? 1 : 0);
     const int per_lane = (plan.poW + 7) / 8, hp = per_lane <= 4 ? 0 : (per_lane <= 6 ? 1 : (per_lane <= 7 ? 2 : 3));
     const int grid = a.items < plan.num_sms ? a.items : plan.num_sms;
-    return launch_pdl(variants[raw ? 1 : 0][form][shape][hp], grid, raw ? SP_THREADS_RAW : SP_THREADS, plan.smem_bytes, s, plan.tmX, a);
+    const Kernel kernel = variants[raw ? 1 : 0][form][shape][hp];
+    if (cudaError_t e = raise_smem_limit(kernel, limits[raw ? 1 : 0][form][shape][hp])) return e;
+    return launch_pdl(kernel, grid, raw ? SP_THREADS_RAW : SP_THREADS, plan.smem_bytes, s, plan.tmX, a);
 }
 
 }  // namespace n2d2b

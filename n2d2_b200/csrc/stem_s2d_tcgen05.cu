@@ -29,7 +29,6 @@
 #include <cstring>
 #include <vector>
 #include <algorithm>
-#include <atomic>
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -766,20 +765,13 @@ cudaError_t launch_stem_s2d(const StemS2dPlan& plan, const ConvGeom& g, int n_ba
     static const Kernel variants[30] = {N2D2B_S2D(false, 0), N2D2B_S2D(true, 0), N2D2B_S2D(false, EF_FLOAT), N2D2B_S2D(true, EF_FLOAT),
                                         N2D2B_S2D(false, EF_WIDE)};   // the wide form has no clamps
 #undef N2D2B_S2D
-    static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        for (Kernel k : variants) {
-            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (e != cudaSuccess) return e;
-        }
-        attr_set[dev] = true;
-    }
+    static SmemLimitSet limits[30];
     const long long items = (long long)a.B * a.bands;
     const int grid = (int)(items < plan.num_sms ? items : plan.num_sms);
     const int shape = (plan.KH == 4 && plan.KWp == 4) ? 1 : ((plan.KH == 2 && plan.KWp == 2) ? 2 : 0);
-    return launch_pdl(variants[(fast.form == EF_WIDE ? 24 : (fast.form == EF_FLOAT ? 12 : 0) + (fast.need_clamp ? 6 : 0)) + (plan.P ? 3 : 0) + shape], grid, Z_THREADS, plan.smem_bytes, s, plan.tmA, a);
+    const int v = (fast.form == EF_WIDE ? 24 : (fast.form == EF_FLOAT ? 12 : 0) + (fast.need_clamp ? 6 : 0)) + (plan.P ? 3 : 0) + shape;
+    if (cudaError_t e = raise_smem_limit(variants[v], limits[v])) return e;
+    return launch_pdl(variants[v], grid, Z_THREADS, plan.smem_bytes, s, plan.tmA, a);
 }
 
 }  // namespace n2d2b

@@ -15,7 +15,6 @@
 // count per tile, not memory, sets the pace: hence the padded image, 8-byte loads where the stride
 // allows, and multiplications by reciprocals instead of divisions.
 #include <cstring>
-#include <atomic>
 #include <mutex>
 #include "kernels.h"
 #include "tc_common.cuh"
@@ -432,23 +431,16 @@ cudaError_t launch_stem(const StemPlan& plan, const void* in4, const ConvGeom& g
     typedef void (*StemKernel)(const CUtensorMap, const CUtensorMap, const StemArgs);
     static const StemKernel variants[4] = {stem_conv_tcgen05_kernel<false, false>, stem_conv_tcgen05_kernel<false, true>,
                                            stem_conv_tcgen05_kernel<true, false>, stem_conv_tcgen05_kernel<true, true>};
-    static std::atomic<bool> attr_set[64];   // set twice by racing first calls at worst: harmless
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        for (StemKernel k : variants) {
-            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            if (e != cudaSuccess) return e;
-        }
-        attr_set[dev] = true;
-    }
+    static SmemLimitSet limits[4];
     const int tiles = (a.M + SBM - 1) / SBM;
     const int grid = tiles < plan.num_sms ? tiles : plan.num_sms;
     const unsigned step = (unsigned)grid * SBM, oHW = (unsigned)(g.oH * g.oW);
     a.step_n = step / oHW;
     a.step_rem = step % oHW;
     const bool vec8 = (g.sX % 2 == 0) && ((uintptr_t)in4 % 8 == 0);
-    variants[(fast.need_clamp ? 2 : 0) + (vec8 ? 1 : 0)]<<<grid, S_THREADS, plan.smem_bytes, s>>>(plan.tmB, tmO, a);
+    const int v = (fast.need_clamp ? 2 : 0) + (vec8 ? 1 : 0);
+    if (cudaError_t e = raise_smem_limit(variants[v], limits[v])) return e;
+    variants[v]<<<grid, S_THREADS, plan.smem_bytes, s>>>(plan.tmB, tmO, a);
     return cudaGetLastError();
 }
 

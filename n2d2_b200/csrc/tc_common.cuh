@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include "common.cuh"
 
 namespace n2d2b {
@@ -36,6 +37,22 @@ static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int thread
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// Raises a kernel's limit of dynamic shared memory ahead of its first launch on each device (a bit of `set` per device; racing first
+// launches do it twice: harmless).  Setting the limit loads the kernel, so only the one about to be launched is touched: with
+// the whole tables of variants at once the first call of a process spent 28 ms on 172 kernels, most of which it never ran.
+typedef std::atomic<unsigned long long> SmemLimitSet;
+template <typename... P>
+static inline cudaError_t raise_smem_limit(void (*kernel)(P...), SmemLimitSet& set, int bytes = 227 * 1024)
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;   // (0: every time)
+    if (set.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) set.fetch_or(bit, std::memory_order_relaxed);
+    return e;
 }
 
 // ----------------------------------------------------------------------------- PTX wrappers
