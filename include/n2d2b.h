@@ -319,6 +319,9 @@ int n2d2b_probe_i8_mma_rate(int device, int n, int reps, double* tops, double* c
 int n2d2b_first_conv_noalloc(int device, const void* d_input, int batch, int height, int width, int channels,
                              int in_unsigned, const n2d2b_conv_desc* desc, const int8_t* weights, const int32_t* bias,
                              const n2d2b_quant* quant, void* d_output, n2d2b_stream stream);
+/* Test hook, n2d2b_net_selftest_wait_timeout for this entry point: a bounded wait runs out as if in a kernel of a call to
+ * n2d2b_first_conv_noalloc on that device and stream; the next call returns N2D2B_ERR_TIMEOUT. */
+int n2d2b_first_conv_noalloc_selftest_wait_timeout(int device, unsigned limit_us, n2d2b_stream stream);
 
 #ifdef __cplusplus
 }

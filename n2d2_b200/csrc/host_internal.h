@@ -1,5 +1,6 @@
 // Host-side helpers shared between translation units of the library (internal).
 #pragma once
+#include <cuda_runtime.h>
 #include <stdint.h>
 #include <vector>
 #include "../../include/n2d2b.h"
@@ -15,5 +16,8 @@ int set_error(int code, const char* fmt, ...);
 // 32-bit form.
 int prepare_fast_constants(const n2d2b_quant* quant, int channels, const int32_t* bias, long long acc_bound,
                            std::vector<int32_t>& consts, int* cpad, int* out_unsigned, bool* need_clamp);
+
+// Enqueues a one-CTA kernel that waits limit_us (1..100000) on a barrier nobody arrives at, gives up and raises the status word.
+int wait_timeout_selftest(int* status, unsigned limit_us, cudaStream_t s);
 
 }  // namespace n2d2b

@@ -615,6 +615,16 @@ __global__ void wait_timeout_selftest_kernel(int* status, unsigned long long lim
     __syncthreads();
 }
 
+namespace n2d2b {
+int wait_timeout_selftest(int* status, unsigned limit_us, cudaStream_t s)
+{
+    if (limit_us < 1 || limit_us > 100000) return fail(N2D2B_ERR_INVALID, "limit_us must be in 1..100000");
+    wait_timeout_selftest_kernel<<<1, 32, 0, s>>>(status, (unsigned long long)limit_us * 1000ull);
+    CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+}  // namespace n2d2b
+
 // ------------------------------------------------------------------------------------ C ABI
 extern "C" {
 
@@ -1685,11 +1695,8 @@ int n2d2b_net_selftest_wait_timeout(n2d2b_net* net, unsigned limit_us, n2d2b_str
 {
     if (!net) return fail(N2D2B_ERR_INVALID, "net must not be NULL");
     if (!net->finalized) return fail(N2D2B_ERR_STATE, "selftest before finalize");
-    if (limit_us < 1 || limit_us > 100000) return fail(N2D2B_ERR_INVALID, "limit_us must be in 1..100000");
     CUDA_TRY(cudaSetDevice(net->device));
-    wait_timeout_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(net->d_status, (unsigned long long)limit_us * 1000ull);
-    CUDA_TRY(cudaGetLastError());
-    return 0;
+    return wait_timeout_selftest(net->d_status, limit_us, (cudaStream_t)stream);
 }
 
 int n2d2b_net_profile(n2d2b_net* net, const void* d_input, int batch, void* d_output, float* ms, int nb_cells,

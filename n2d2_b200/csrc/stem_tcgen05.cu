@@ -502,6 +502,48 @@ static int noalloc_scratch_for(int device, unsigned char** ptr)
     return 0;
 }
 
+// The device's status word: as the kernels see it, and as the host does (nullptr where it could not be mapped: it then is the last 16
+// bytes of the constants area in the scratch)
+static int* noalloc_status(int device, unsigned char* scratch, int** mapped)
+{
+    *mapped = g_noalloc_status_dev ? g_noalloc_status + 16 * device : nullptr;
+    return *mapped ? g_noalloc_status_dev + 16 * device : (int*)(scratch + NA_PAD_OFFSET - 16);
+}
+
+static bool noalloc_first_use(int device)
+{
+    std::lock_guard<std::mutex> lock(g_noalloc_mutex);
+    const bool first = !g_noalloc_used[device];
+    g_noalloc_used[device] = true;
+    return first;
+}
+
+// The caller's current device is put back on every way out
+namespace {
+struct DeviceGuard {
+    int prev = -1;
+    DeviceGuard() { if (cudaGetDevice(&prev) != cudaSuccess) prev = -1; }
+    ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
+};
+}
+
+extern "C" int n2d2b_first_conv_noalloc_selftest_wait_timeout(int device, unsigned limit_us, n2d2b_stream stream)
+{
+    using namespace n2d2b;
+    const DeviceGuard guard;
+    cudaError_t e = cudaSetDevice(device);
+    if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "cudaSetDevice(%d) failed: %s", device, cudaGetErrorString(e));
+    unsigned char* scratch = nullptr;
+    if (int rc = noalloc_scratch_for(device, &scratch)) return rc;
+    int* mapped;
+    int* const status = noalloc_status(device, scratch, &mapped);
+    if (noalloc_first_use(device) && !mapped) {
+        e = cudaMemsetAsync(status, 0, sizeof(int), (cudaStream_t)stream);
+        if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "clearing the status word failed: %s", cudaGetErrorString(e));
+    }
+    return wait_timeout_selftest(status, limit_us, (cudaStream_t)stream);
+}
+
 extern "C" int n2d2b_first_conv_noalloc(int device, const void* d_input, int batch, int height, int width, int channels,
                                         int in_unsigned, const n2d2b_conv_desc* desc, const int8_t* weights,
                                         const int32_t* bias, const n2d2b_quant* quant, void* d_output,
@@ -542,12 +584,7 @@ extern "C" int n2d2b_first_conv_noalloc(int device, const void* d_input, int bat
                          (unsigned)N2D2B_NOALLOC_MAX_PIXELS);
     if (stem_weight_bytes(g) > NA_WEIGHT_BYTES)
         return set_error(N2D2B_ERR_TOO_LARGE, "arranged weights exceed the fixed scratch");
-    // the caller's current device is put back on every way out
-    struct DeviceGuard {
-        int prev = -1;
-        ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
-    } guard;
-    if (cudaGetDevice(&guard.prev) != cudaSuccess) guard.prev = -1;
+    const DeviceGuard guard;
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "cudaSetDevice(%d) failed: %s", device, cudaGetErrorString(e));
     int sms = 148;
@@ -583,20 +620,15 @@ extern "C" int n2d2b_first_conv_noalloc(int device, const void* d_input, int bat
         if (e == cudaSuccess) e = cudaMemcpyAsync(scratch + NA_CONST_OFFSET, consts.data(), consts.size() * 4, cudaMemcpyHostToDevice, s);
     }
     // The status word still holds what the previous call's kernel left: look at it behind that kernel, so a time-out of call k is
-    // reported by call k + 1.  (In the scratch: the last 16 bytes of the constants area.)
-    int* const mapped = g_noalloc_status_dev ? g_noalloc_status + 16 * device : nullptr;
-    int* const status = mapped ? g_noalloc_status_dev + 16 * device : (int*)(scratch + NA_PAD_OFFSET - 16);
+    // reported by call k + 1.
+    int* mapped;
+    int* const status = noalloc_status(device, scratch, &mapped);
     int prev_status = 0;
     if (e == cudaSuccess && !mapped) e = cudaMemcpyAsync(&prev_status, status, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "copy of the layer constants failed: %s", cudaGetErrorString(e));
     if (mapped) prev_status = *(volatile int*)mapped;
-    bool first_call_here;
-    {
-        std::lock_guard<std::mutex> lock(g_noalloc_mutex);
-        first_call_here = !g_noalloc_used[device];
-        g_noalloc_used[device] = true;
-    }
+    const bool first_call_here = noalloc_first_use(device);
     if (prev_status != 0 || !mapped) {
         if (mapped) *(volatile int*)mapped = 0;
         else e = cudaMemsetAsync(status, 0, sizeof(int), s);

@@ -108,6 +108,7 @@ def load():
         lib.n2d2b_first_conv_noalloc.argtypes = [C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
                                                  C.POINTER(ConvDesc), C.c_void_p, C.c_void_p, C.POINTER(Quant),
                                                  C.c_void_p, C.c_void_p]
+        lib.n2d2b_first_conv_noalloc_selftest_wait_timeout.argtypes = [C.c_int, C.c_uint, C.c_void_p]
         _lib = lib
     return _lib
 
@@ -342,3 +343,7 @@ def first_conv_noalloc(d_in_ptr, batch, height, width, channels, in_unsigned, la
                  int(layer.get('weight_bits', 8)))
     check(load().n2d2b_first_conv_noalloc(device, d_in_ptr, batch, height, width, channels, 1 if in_unsigned else 0,
                                           C.byref(d), _ptr(w), _ptr(b), C.byref(q), d_out_ptr, stream))
+
+
+def first_conv_noalloc_selftest_wait_timeout(limit_us=1000, device=0, stream=0):
+    check(load().n2d2b_first_conv_noalloc_selftest_wait_timeout(device, limit_us, stream))

@@ -99,3 +99,26 @@ def test_noalloc_first_conv_forms(case, mode):
     C, H, W, O, k, s, p, batch = case
     got, want = _both_paths(single_conv_net(C, H, W, O, k, s, p, mode=mode, seed=23), batch, seed=8)
     assert np.array_equal(got, want)
+
+
+# A bounded wait that runs out in one call's kernels (here in a one-CTA kernel that raises the same status word) is reported by the next
+# call, which launches nothing; the call after it runs.
+@pytest.mark.parametrize('stride', [2, 1])
+def test_noalloc_first_conv_reports_a_wait_that_ran_out(stride):
+    import torch
+    net = single_conv_net(3, 30, 28, 64, 3, stride, 1, mode='double', seed=23)
+    _both_paths(net, 2, seed=8)
+    out = torch.full((2 * 30 * 28 * 64,), 0x5A, dtype=torch.uint8, device='cuda')
+    x = torch.zeros(2 * 30 * 28 * 3, dtype=torch.uint8, device='cuda')
+    for stream in (0, torch.cuda.Stream().cuda_stream):
+        torch.cuda.synchronize()
+        runtime.first_conv_noalloc_selftest_wait_timeout(1000, stream=stream)
+        with pytest.raises(runtime.N2D2BError, match='status -4.*gave up waiting'):
+            runtime.first_conv_noalloc(x.data_ptr(), 2, 30, 28, 3, True, net['layers'][0], out.data_ptr(), stream=stream)
+        torch.cuda.synchronize()
+        assert bool((out == 0x5A).all())
+        got, want = _both_paths(net, 2, seed=9)
+        assert np.array_equal(got, want)
+    for limit in (0, 100001):
+        with pytest.raises(runtime.N2D2BError, match='limit_us'):
+            runtime.first_conv_noalloc_selftest_wait_timeout(limit)
