@@ -836,8 +836,8 @@ cudaError_t launch_widen_int4(const uint8_t* packed, int rows_src, int ng_src, i
     const unsigned long long total = (unsigned long long)rows * words;
     if (total == 0) return cudaSuccess;
     if (total >= (1ull << 31)) return cudaErrorInvalidValue;
-    const unsigned long long blocks = (total + 255) / 256;
-    return launch_pdl(widen_int4_kernel, (int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, s, packed, rows_src, ng_src, dst, rows, ng_dst, words);
+    const unsigned long long blocks = (total + 255) / 256, most = 8ull * current_sms();
+    return launch_pdl(widen_int4_kernel, (int)(blocks < most ? blocks : most), 256, 0, s, packed, rows_src, ng_src, dst, rows, ng_dst, words);
 }
 
 bool igemm_uses_fast_epilogue(const IgemmPlan& plan, const FastQuant& fast, bool has_residual, int out_dtype)

@@ -120,7 +120,7 @@ struct CellRec {
 
 struct n2d2b_net {
     int device = 0;
-    int num_sms = 148;
+    int num_sms = 0;
     bool finalized = false;
     int max_batch = 0;
     unsigned flags = 0;

@@ -12,7 +12,7 @@ namespace n2d2b {
 static inline unsigned grid_for(size_t n, int block)
 {
     size_t g = (n + block - 1) / block;
-    const size_t cap = 148u * 32u * 64u;
+    const size_t cap = 303104;   // loops beyond: more blocks than any device holds at once
     return (unsigned)(g < cap ? (g ? g : 1) : cap);
 }
 
@@ -293,13 +293,13 @@ int depthwise_alignment(const ConvGeom& g, const FastQuant& fast)
 cudaError_t launch_conv_depthwise(const void* in, int in_unsigned, const int8_t* w_hwc,
                                   const ConvGeom& g, const QuantDev& q, const FastQuant& fast, void* out, cudaStream_t s)
 {
-    if (fast.enabled && depthwise3x3_eligible(g)) return launch_depthwise3x3(in, in_unsigned, w_hwc, g, fast, out, 148, s);
+    if (fast.enabled && depthwise3x3_eligible(g)) return launch_depthwise3x3(in, in_unsigned, w_hwc, g, fast, out, current_sms(), s);
     if (depthwise3x3_masked(g, fast)) {
         const int cw = g.C / 4;
         const long long rows = (long long)g.B * g.oH;
         if (rows == 0 || g.oW == 0) return cudaSuccess;
         // few, long-lived blocks: a thread's weights and constants (29 loads) are fetched once and serve many rows
-        const long long max_blocks = 148ll * 6;
+        const long long max_blocks = 6ll * current_sms();
         const unsigned grid = (unsigned)(rows < max_blocks ? rows : max_blocks);
         // a block's threads cover 4 * (threads / cw) pixels of a row per pass
         int threads = 256;
@@ -752,7 +752,7 @@ static cudaError_t launch_rescale(const int32_t* in, void* out, size_t pixels, i
         a.per_block = vq >= 256 ? 1 : 256 / vq;
         const long long blocks = (a.rows + a.per_block - 1) / a.per_block;
         const int threads = vq * a.per_block;
-        const long long most = 148ll * (2048 / threads > 16 ? 16 : 2048 / threads);   // resident blocks
+        const long long most = (long long)current_sms() * (2048 / threads > 16 ? 16 : 2048 / threads);   // resident blocks
         kernels[(vec == 4 ? 3 : 0) + form]<<<(unsigned)(blocks < most ? blocks : most), threads, 0, s>>>(a);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -836,7 +836,7 @@ cudaError_t launch_drop_padded_columns(const uint8_t* src, int ld, uint8_t* dst,
     const bool vec = (C % 8 == 0) && (ld % 8 == 0) && !((uintptr_t)src & 7) && !((uintptr_t)dst & 7);
     const size_t total = vec ? rows * (size_t)(C / 8) : rows * (size_t)C;
     const int threads = 256;
-    const int blocks = (int)std::min<size_t>((total + threads - 1) / threads, 148 * 8);
+    const int blocks = (int)std::min<size_t>((total + threads - 1) / threads, 8 * (size_t)current_sms());
     if (vec)
         launch_pdl(drop_padded_columns_kernel<uint2>, blocks, threads, 0, s, (const uint2*)src, ld / 8, (uint2*)dst, C / 8, rows);
     else
@@ -1054,7 +1054,7 @@ cudaError_t launch_topn(const void* scores, int dtype, int is_unsigned, size_t p
 {
     if (pixels == 0 || C == 0 || topN == 0) return cudaSuccess;
     const size_t smem = (size_t)3 * C * sizeof(int);
-    const unsigned grid = (unsigned)std::min<size_t>(pixels, 148 * 16);
+    const unsigned grid = (unsigned)std::min<size_t>(pixels, 16 * (size_t)current_sms());
 #define N2D2B_TOPN(T)                                                                                                   \
     do {                                                                                                                \
         cudaError_t e = cudaFuncSetAttribute(topn_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
@@ -1137,7 +1137,8 @@ cudaError_t launch_quantize_stimuli(const float* in, int B, int C, int H, int W,
     // up to four pixels per thread; fewer when the blocks would not cover the GPU twice
     int run = STIM_BYTES / C & ~(STIM_THREADS - 1);
     if (run > 4 * STIM_THREADS) run = 4 * STIM_THREADS;
-    while (run > STIM_THREADS && (pixels + run - 1) / run < 2 * 148 * 4) run -= STIM_THREADS;
+    const size_t twice = 8 * (size_t)current_sms();
+    while (run > STIM_THREADS && (pixels + run - 1) / run < twice) run -= STIM_THREADS;
     const size_t blocks = (pixels + run - 1) / run;
     const unsigned grid = (unsigned)std::min<size_t>(blocks, 1u << 20);
     if (C == 3) quantize_stimuli_kernel<3><<<grid, STIM_THREADS, 0, s>>>(in, C, (unsigned)hw, (unsigned)pixels, run, factor, lo, hi, (uint8_t*)out);

@@ -228,7 +228,7 @@ static S2dImage s2d_image_of(const void* in, const ConvGeom& g, int batch, void*
 
 static int s2d_image_blocks(const S2dImage& im)
 {
-    return im.total ? (int)std::min((im.total + 255u) / 256u, 148u * 32u) : std::min(im.rows, 1 << 20);
+    return im.total ? (int)std::min((im.total + 255u) / 256u, 32u * (unsigned)current_sms()) : std::min(im.rows, 1 << 20);
 }
 
 cudaError_t launch_s2d_image(const void* in, const ConvGeom& g, int batch, void* out, cudaStream_t s)

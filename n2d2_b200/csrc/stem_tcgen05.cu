@@ -587,8 +587,7 @@ extern "C" int n2d2b_first_conv_noalloc(int device, const void* d_input, int bat
     const DeviceGuard guard;
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return set_error(N2D2B_ERR_CUDA, "cudaSetDevice(%d) failed: %s", device, cudaGetErrorString(e));
-    int sms = 148;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 148;
+    const int sms = current_sms();
     unsigned char* scratch = nullptr;
     if (int rc = noalloc_scratch_for(device, &scratch)) return rc;
 

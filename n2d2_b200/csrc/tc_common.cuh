@@ -39,6 +39,14 @@ static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int thread
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
+// Multiprocessors of the current device, for launchers that have no plan to read them from
+static inline int current_sms()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+    return sms;
+}
+
 // Raises a kernel's limit of dynamic shared memory ahead of its first launch on each device (a bit of `set` per device; racing first
 // launches do it twice: harmless).  Setting the limit loads the kernel, so only the one about to be launched is touched: with
 // the whole tables of variants at once the first call of a process spent 28 ms on 172 kernels, most of which it never ran.

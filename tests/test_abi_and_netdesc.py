@@ -39,6 +39,13 @@ def test_header_lists_every_engine_name():
     assert names and names == listed
 
 
+def test_launch_shapes_ask_the_device_for_its_multiprocessors():
+    csrc = os.path.join(ROOT, 'n2d2_b200', 'csrc')
+    for f in sorted(os.listdir(csrc)):
+        code = re.sub(r'//[^\n]*|/\*.*?\*/', '', open(os.path.join(csrc, f)).read(), flags=re.S)
+        assert not re.search(r'\b148(u|l|ll|ull)?\b', code), f'{f} assumes 148 multiprocessors'
+
+
 def test_no_cpu_fallback_without_a_device():
     import torch
     if torch.cuda.is_available():
