@@ -116,6 +116,7 @@ struct CellRec {
     IgemmPlan plan{};
     bool has_plan = false;
     const void* plan_input = nullptr;
+    const void* plan_res = nullptr;   // a residual that is the network's input: the address the plan holds
 };
 
 struct n2d2b_net {
@@ -1016,16 +1017,20 @@ static bool use_widened(const n2d2b_net* net, const CellRec& c, int batch)
 // in the kernel (its warps' shared-memory stores bound it).
 static int plan_widened(n2d2b_net* net)
 {
+    // (not where the input or the residual is the caller's buffer, whose address only the forward pass knows)
+    auto eligible = [](const CellRec& c) {
+        return !c.skipped && c.engine == ENG_TCGEN05 && c.plan.w4 && c.fast.enabled && c.plan_input && c.residual != 0;
+    };
     size_t most = 0;
     for (CellRec& c : net->cells) {
-        if (c.skipped || c.engine != ENG_TCGEN05 || !c.plan.w4 || !c.fast.enabled || !c.plan_input) continue;
+        if (!eligible(c)) continue;
         const int rows = (c.geom.O + 31) & ~31;
         most = std::max(most, (size_t)rows * c.geom.kH * c.geom.kW * c.geom.C);
     }
     if (!most) return 0;
     CUDA_TRY(cudaMalloc(&net->d_w8, most + 256));
     for (CellRec& c : net->cells) {
-        if (c.skipped || c.engine != ENG_TCGEN05 || !c.plan.w4 || !c.fast.enabled || !c.plan_input) continue;
+        if (!eligible(c)) continue;
         ConvGeom g = c.geom;
         g.B = net->max_batch;
         const TensorRec& tout = net->tensors[c.output];
@@ -1313,7 +1318,8 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
             const void* enc_ptr = in_ptr ? in_ptr : (const void*)placeholder;
             const void* out_ptr = c.pad_O ? c.d_colpad
                                 : net->tensors[c.output].dtype == DT_I8 ? tensor_ptr(net, c.output, nullptr) : nullptr;
-            const void* res_ptr = c.residual >= 0 ? tensor_ptr(net, c.residual, nullptr) : nullptr;
+            const void* res_ptr = c.residual == 0 ? (const void*)placeholder
+                                : c.residual > 0 ? tensor_ptr(net, c.residual, nullptr) : nullptr;
             int planned = igemm_make_plan(&c.plan, enc_ptr, c.d_weights, out_ptr, res_ptr, gb, net->tensors[c.inputs[0]].is_unsigned,
                                           (flags & N2D2B_FORCE_IM2COL) ? 1 : 0, 0, net->num_sms, &why,
                                           (flags & N2D2B_FORCE_PAIR) ? 1 : 0, w4 ? 1 : 0);
@@ -1481,6 +1487,9 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         r.is_unsigned = net->tensors[c.residual].is_unsigned;
         r.q2 = c.q2.dev;
     }
+    // the maps and the loads of a residual start on 16 bytes; the network's input is the caller's buffer
+    if (c.residual == 0 && mapped && ((uintptr_t)r.ptr & 15))
+        return fail(N2D2B_ERR_INVALID, "a residual sum cannot read an input at %p: operands must be 16-byte aligned", r.ptr);
     if (use_widened(net, c, batch)) {
         const size_t row_bytes = (size_t)c.geom.kH * c.geom.kW * c.geom.C;
         CUDA_TRY(launch_widen_int4((const uint8_t*)c.d_weights, c.geom.O, c.w8_ng_src, (int8_t*)net->d_w8, c.w8_rows, c.w8_ng_dst, row_bytes, s));
@@ -1511,7 +1520,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
     switch (c.engine) {
     case ENG_TCGEN05: {
         void* const gemm_out = c.pad_O ? c.d_colpad : out;
-        if (c.plan_input != in0) {
+        if (c.plan_input != in0 || (c.residual == 0 && c.plan_res != r.ptr)) {
             ConvGeom gb = c.geom;
             gb.B = net->max_batch;
             if (c.pad_O) gb.O = c.pad_O;
@@ -1523,6 +1532,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
                 return fail(N2D2B_ERR_INVALID, "tensor-core plan failed: %s", why);
             c.plan.perm = perm;
             c.plan_input = in0;
+            c.plan_res = r.ptr;
         }
         IgemmPlan p = c.plan;
         p.M = batch * c.geom.oH * c.geom.oW;

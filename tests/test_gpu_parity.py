@@ -201,6 +201,45 @@ def test_patch_kernel_with_a_residual_sum(case, mode):
         assert eng == ['tcgen05', 'patch-tcgen05', 'fused']
 
 
+# (C, H, W, kernel of the last convolution, convolutions, weight bits, batch): a sum with the network's own input, whose address only the
+# forward pass knows - implicit GEMM (two and four staging regions, a cluster per tile), patch kernel, packed weights, one and two layers
+INPUT_RES_CASES = [(128, 9, 11, 1, 2, 8, 5), (256, 14, 14, 1, 1, 8, 3), (256, 8, 8, 3, 2, 8, 40), (512, 7, 7, 3, 2, 8, 1), (64, 21, 20, 3, 2, 8, 3),
+                   (64, 21, 20, 3, 1, 8, 3), (128, 28, 28, 1, 2, 4, 60), (48, 9, 9, 1, 2, 8, 2)]
+
+
+@pytest.mark.parametrize('case', INPUT_RES_CASES, ids=lambda c: 'C%d_%dx%d_k%d_n%d_w%d_b%d' % c)
+@pytest.mark.parametrize('mode', ['double', 'fixed', 'float'])
+def test_residual_sum_with_the_network_input(case, mode):
+    import torch
+    C, H, W, k, n, bits, batch = case
+    for unsigned, act in ((True, 'linear'), (False, 'relu')):
+        b = netdesc.NetBuilder('inres', C, H, W, 19, mode, input_unsigned=unsigned, weight_dist=('normal', 30), weight_bits=bits)
+        x = b.conv(-1, C, 1, act='relu') if n == 2 else -1
+        x = b.conv(x, C, k, pad=k // 2, act=act)
+        b.sum([x, -1], act='relu')
+        net = b.net
+        n_layers, eng = compare_net(net, batch, flags=0)
+        assert 'fused' in eng
+        # another buffer, then the first again, through the device entry point
+        data = netdesc.make_input(net, batch, seed=3)
+        want = oracle.run_net(net, data, 'i64')[-1].reshape(batch, -1)
+        qn = runtime.QuantizedNet(net, batch)
+        try:
+            buf = [torch.zeros(data.size + 16, dtype=torch.uint8, device='cuda') for _ in range(2)]
+            y = torch.empty((batch, qn.out_elems), dtype=torch.uint8, device='cuda')
+            for i in (0, 1, 0):
+                buf[i][:data.size] = torch.from_numpy(data.view(np.uint8).reshape(-1)).cuda()
+                buf[1 - i].zero_()
+                qn.forward_device(buf[i].data_ptr(), batch, y.data_ptr())
+                qn.check()
+                assert np.array_equal(y.cpu().numpy().view(qn.out_dtype).astype(np.int64), want)
+            if eng[-2] != 'simt':
+                with pytest.raises(runtime.N2D2BError, match='aligned'):
+                    qn.forward_device(buf[0].data_ptr() + 8, batch, y.data_ptr())
+        finally:
+            qn.close()
+
+
 # (C, H, W, O, k, stride, pad, batch): few tiles and a long K, so the eight CTAs of a cluster share a tile - parts of K of unequal
 # length, the shortest and the longest K, rows and columns beyond the layer, narrow K slabs, im2col and plain loads
 SPLIT_K_CASES = [(512, 7, 7, 512, 3, 1, 1, 1), (3072, 3, 5, 320, 1, 1, 0, 2), (256, 9, 11, 96, 4, 1, 1, 2), (64, 6, 6, 64, 5, 2, 2, 3),
