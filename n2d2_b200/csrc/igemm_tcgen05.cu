@@ -381,6 +381,69 @@ static int igemm_tile_columns(const ConvGeom& g, int BK, bool im2col, bool res, 
     return best_bn;
 }
 
+// The map of the activations: `g.B` images at `in`, Ct channels per pixel (g: one group of a layer of several)
+static int encode_activations(IgemmPlan* plan, const void* in, const ConvGeom& g, int Ct, const char** why)
+{
+    const CUtensorMapSwizzle swz = swizzle_for(plan->BK);
+    CUresult rc;
+    if (!plan->a_im2col) {
+        const cuuint64_t dims[2] = {(cuuint64_t)g.C, (cuuint64_t)g.B * g.oH * g.oW};
+        const cuuint64_t strides[1] = {(cuuint64_t)g.C};
+        const cuuint32_t box[2] = {(cuuint32_t)plan->BK, (cuuint32_t)BM};
+        const cuuint32_t estr[2] = {1, 1};
+        rc = g_encode_tiled(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)in, dims, strides, box, estr,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the activation matrix"; return -1; }
+    } else {
+        // NHWC activations as a (C, W, H, N) tensor; the base pixel of output (ox, oy) is
+        // (ox*sX - pL, oy*sY - pT) and the filter tap is passed as an offset per load.
+        const cuuint64_t dims[4] = {(cuuint64_t)Ct, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.B};
+        const cuuint64_t strides[3] = {(cuuint64_t)Ct, (cuuint64_t)Ct * g.W, (cuuint64_t)Ct * g.W * g.H};
+        const int lower[2] = {-g.pL, -g.pT};
+        // last base pixel = (oW-1)*sX - pL  ->  upper corner relative to the tensor edge
+        const int upper[2] = {(g.oW - 1) * g.sX - g.pL - (g.W - 1), (g.oH - 1) * g.sY - g.pT - (g.H - 1)};
+        const cuuint32_t estr[4] = {1, (cuuint32_t)g.sX, (cuuint32_t)g.sY, 1};
+        rc = g_encode_im2col(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)in, dims, strides, lower, upper,
+                             (cuuint32_t)plan->BK, (cuuint32_t)BM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeIm2col failed for the activation tensor"; return -1; }
+        // Drivers up to CUDA 13.1 encode im2col maps of tensors smaller than 128 KiB with a flag
+        // (bit 21 of the second 64-bit word) that makes the load misbehave; clearing it is the
+        // documented remedy used by NVIDIA's own open-source templates.
+        int drv = 0;
+        if (cudaDriverGetVersion(&drv) == cudaSuccess && drv <= 13010) {
+            const size_t bytes = (size_t)Ct * g.W * g.H * g.B;
+            if (bytes < 131072) reinterpret_cast<unsigned long long*>(&plan->tmA)[1] &= ~(1ull << 21);
+        }
+    }
+    return 0;
+}
+
+// The map of the residual operand: `rows` pixels at `res`
+static int encode_residual(IgemmPlan* plan, const void* res, long long rows, const char** why)
+{
+    const int wb = plan->BN / plan->parts;   // an epilogue warp's columns: 64, or 32 or 16 with four warps on a narrow tile
+    const cuuint64_t dims[2] = {(cuuint64_t)plan->N, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)plan->N};
+    const cuuint32_t box[2] = {(cuuint32_t)wb, 32};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult rc = g_encode_tiled(&plan->tmR, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)res, dims, strides, box, estr,
+                                       CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(wb), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the residual matrix"; return -1; }
+    return 0;
+}
+
+int igemm_bind_buffers(IgemmPlan* plan, const void* in, const void* res, const ConvGeom& g0, const char** why)
+{
+    if (((uintptr_t)in & 15) || ((uintptr_t)res & 15)) { *why = "operands must be 16-byte aligned"; return -1; }
+    ConvGeom g = g0;
+    if (const int cg = igemm_dw_group(g0)) g.C = cg;
+    if (in && encode_activations(plan, in, g, g0.C, why)) return -1;
+    return res && plan->has_out_maps ? encode_residual(plan, res, (long long)g.B * g.oH * g.oW, why) : 0;
+}
+
 int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void* out, const void* res,
                     const ConvGeom& g0, int in_unsigned, int force_im2col, int force_bn, int num_sms, const char** why,
                     int force_pair, int w4)
@@ -485,37 +548,7 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the weight matrix"; return -1; }
     }
-    if (!plan->a_im2col) {
-        const cuuint64_t dims[2] = {(cuuint64_t)g.C, (cuuint64_t)plan->M};
-        const cuuint64_t strides[1] = {(cuuint64_t)g.C};
-        const cuuint32_t box[2] = {(cuuint32_t)plan->BK, (cuuint32_t)BM};
-        const cuuint32_t estr[2] = {1, 1};
-        rc = g_encode_tiled(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)in, dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the activation matrix"; return -1; }
-    } else {
-        // NHWC activations as a (C, W, H, N) tensor; the base pixel of output (ox, oy) is
-        // (ox*sX - pL, oy*sY - pT) and the filter tap is passed as an offset per load.
-        const cuuint64_t dims[4] = {(cuuint64_t)Ct, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.B};
-        const cuuint64_t strides[3] = {(cuuint64_t)Ct, (cuuint64_t)Ct * g.W, (cuuint64_t)Ct * g.W * g.H};
-        const int lower[2] = {-g.pL, -g.pT};
-        // last base pixel = (oW-1)*sX - pL  ->  upper corner relative to the tensor edge
-        const int upper[2] = {(g.oW - 1) * g.sX - g.pL - (g.W - 1), (g.oH - 1) * g.sY - g.pT - (g.H - 1)};
-        const cuuint32_t estr[4] = {1, (cuuint32_t)g.sX, (cuuint32_t)g.sY, 1};
-        rc = g_encode_im2col(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)in, dims, strides, lower, upper,
-                             (cuuint32_t)plan->BK, (cuuint32_t)BM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeIm2col failed for the activation tensor"; return -1; }
-        // Drivers up to CUDA 13.1 encode im2col maps of tensors smaller than 128 KiB with a flag
-        // (bit 21 of the second 64-bit word) that makes the load misbehave; clearing it is the
-        // documented remedy used by NVIDIA's own open-source templates.
-        int drv = 0;
-        if (cudaDriverGetVersion(&drv) == cudaSuccess && drv <= 13010) {
-            const size_t bytes = (size_t)Ct * g.W * g.H * g.B;
-            if (bytes < 131072) reinterpret_cast<unsigned long long*>(&plan->tmA)[1] &= ~(1ull << 21);
-        }
-    }
+    if (encode_activations(plan, in, g, Ct, why)) return -1;
     // output (and residual) as [M][N] bytes, one box = an epilogue warp's 32 rows and columns
     plan->has_out_maps = 0;
     if (out && g.O % 16 == 0 && !((uintptr_t)out & 15) && !((uintptr_t)res & 15)) {
@@ -529,12 +562,7 @@ int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the output matrix"; return -1; }
         plan->tmR = plan->tmO;
-        if (res) {
-            rc = g_encode_tiled(&plan->tmR, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)res, dims, strides, box, estr,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(wb), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (rc != CUDA_SUCCESS) { *why = "cuTensorMapEncodeTiled failed for the residual matrix"; return -1; }
-        }
+        if (res && encode_residual(plan, res, plan->M, why)) return -1;
         plan->has_out_maps = 1;
         // 256-row variant: 256-column tiles, 128-byte K slabs, no residual, weights not resident, and enough
         // work per CTA that halving the weight traffic pays for the un-overlapped epilogue

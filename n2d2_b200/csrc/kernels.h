@@ -231,6 +231,9 @@ void igemm_dw_arrange_weights(const ConvGeom& g, const int8_t* w_ct, int8_t* dst
 int igemm_make_plan(IgemmPlan* plan, const void* in, const int8_t* w, const void* out, const void* res,
                     const ConvGeom& g, int in_unsigned, int force_im2col, int force_bn, int num_sms, const char** why,
                     int force_pair = 0, int w4 = 0);
+// Points a plan at buffers that only the forward pass knows (either may be nullptr: left as it is).  The maps cover g.B images and no
+// more: the last tile's rows beyond them read as zero, where a map over max_batch images would read past the caller's buffer.
+int igemm_bind_buffers(IgemmPlan* plan, const void* in, const void* res, const ConvGeom& g, const char** why);
 // Whether a launch of this plan takes the 32-bit epilogue; such a cell's weight rows must be stored in the
 // permuted order (igemm_permute_weights with igemm_perm_block(plan)) and plan.perm set to that block size.
 bool igemm_uses_fast_epilogue(const IgemmPlan& plan, const FastQuant& fast, bool has_residual, int out_dtype);

@@ -117,6 +117,7 @@ struct CellRec {
     bool has_plan = false;
     const void* plan_input = nullptr;
     const void* plan_res = nullptr;   // a residual that is the network's input: the address the plan holds
+    int plan_images = 0;              // images that the plan's maps over the network's input cover
 };
 
 struct n2d2b_net {
@@ -1520,19 +1521,19 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
     switch (c.engine) {
     case ENG_TCGEN05: {
         void* const gemm_out = c.pad_O ? c.d_colpad : out;
-        if (c.plan_input != in0 || (c.residual == 0 && c.plan_res != r.ptr)) {
+        // tensors of the caller: their address and the images of this call
+        const void* const caller_in = c.inputs[0] == 0 ? in0 : nullptr;
+        const void* const caller_res = c.residual == 0 ? r.ptr : nullptr;
+        if (c.plan_input != in0 || c.plan_res != caller_res || ((caller_in || caller_res) && c.plan_images != img0 + batch)) {
             ConvGeom gb = c.geom;
-            gb.B = net->max_batch;
+            gb.B = img0 + batch;
             if (c.pad_O) gb.O = c.pad_O;
             const char* why = "";
-            const int perm = c.plan.perm, w4 = c.plan.w4;   // properties of the stored weights, not of the tensor maps
-            if (igemm_make_plan(&c.plan, in0, c.d_weights, tout.dtype == DT_I8 ? gemm_out : nullptr, r.ptr, gb, tin.is_unsigned,
-                                (net->flags & N2D2B_FORCE_IM2COL) ? 1 : 0, 0, net->num_sms, &why,
-                                (net->flags & N2D2B_FORCE_PAIR) ? 1 : 0, w4))
-                return fail(N2D2B_ERR_INVALID, "tensor-core plan failed: %s", why);
-            c.plan.perm = perm;
+            c.plan_images = 0;
+            if (igemm_bind_buffers(&c.plan, caller_in, caller_res, gb, &why)) return fail(N2D2B_ERR_INVALID, "tensor-core plan failed: %s", why);
             c.plan_input = in0;
-            c.plan_res = r.ptr;
+            c.plan_res = caller_res;
+            c.plan_images = gb.B;
         }
         IgemmPlan p = c.plan;
         p.M = batch * c.geom.oH * c.geom.oW;

@@ -240,6 +240,40 @@ def test_residual_sum_with_the_network_input(case, mode):
             qn.close()
 
 
+# A first cell on the tensor cores reads the caller's buffer through a map that ends with the call's last image: calls of changing sizes
+# on buffers that hold no more than the call's images
+@pytest.mark.parametrize('kind', ['plain', 'im2col', 'fc', 'depthwise', 'patch', 'residual', 'pair', 'w4'])
+def test_calls_of_changing_sizes_on_the_callers_buffer(kind):
+    import torch
+    flags = {'depthwise': R.FORCE_DEPTHWISE_TENSOR, 'pair': R.FORCE_PAIR}.get(kind, 0)
+    C, H, W = {'fc': (2048, 1, 1), 'pair': (512, 9, 9), 'depthwise': (64, 15, 15)}.get(kind, (128, 7, 9))
+    b = netdesc.NetBuilder('caller', C, H, W, 29, 'double', weight_dist=('normal', 30), weight_bits=4 if kind == 'w4' else 8)
+    if kind == 'fc':
+        b.fc(-1, 96, act='relu')
+    elif kind == 'depthwise':
+        b.conv(-1, C, 3, stride=2, pad=1, groups=C)
+    elif kind == 'patch':
+        b.conv(-1, 64, 3, pad=1)
+    elif kind == 'residual':
+        b.sum([b.conv(b.conv(-1, C, 1), C, 1, act='linear'), -1])
+    else:
+        b.conv(-1, 256, 3 if kind == 'im2col' else 1, stride=2 if kind == 'im2col' else 1, pad=1 if kind == 'im2col' else 0)
+    net = b.net
+    data = netdesc.make_input(net, 40, seed=4)
+    want = oracle.run_net(net, data, 'i64')[-1].reshape(40, -1)
+    qn = runtime.QuantizedNet(net, 40, flags=flags)
+    try:
+        for batch in (1, 40, 7, 33, 1, 2):
+            x = torch.from_numpy(data[:batch].view(np.uint8)).cuda()
+            y = torch.empty((batch, qn.out_elems), dtype=torch.uint8, device='cuda')
+            qn.forward_device(x.data_ptr(), batch, y.data_ptr())
+            qn.check()
+            assert np.array_equal(y.cpu().numpy().view(qn.out_dtype).astype(np.int64), want[:batch]), f'{batch} images'
+            assert np.array_equal(qn.forward_host(data[:batch]).astype(np.int64), want[:batch])
+    finally:
+        qn.close()
+
+
 # (C, H, W, O, k, stride, pad, batch): few tiles and a long K, so the eight CTAs of a cluster share a tile - parts of K of unequal
 # length, the shortest and the longest K, rows and columns beyond the layer, narrow K slabs, im2col and plain loads
 SPLIT_K_CASES = [(512, 7, 7, 512, 3, 1, 1, 1), (3072, 3, 5, 320, 1, 1, 0, 2), (256, 9, 11, 96, 4, 1, 1, 2), (64, 6, 6, 64, 5, 2, 2, 3),
