@@ -524,7 +524,8 @@ cudaError_t launch_pool(const void* in, int in_unsigned, const PoolGeom& g, void
 {
     // int8 tensors; int32 tensors go through launch_pool_i32
     const int block = 256;
-    if (g.C % 16 == 0 && g.is_max) {
+    const bool vec = g.C % 16 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0;   // (the input may be the caller's buffer)
+    if (vec && g.is_max) {
         const long long rows = (long long)g.B * g.oH;
         if (rows == 0 || g.oW == 0) return cudaSuccess;
         const int items = g.oW * (g.C / 16);
@@ -540,7 +541,7 @@ cudaError_t launch_pool(const void* in, int in_unsigned, const PoolGeom& g, void
             launch_pdl(pool_global_avg_kernel<true>, grid_for(total, block), block, 0, s, (const uint8_t*)in, g.H * g.W, g.C, total, (uint8_t*)out);
         else
             launch_pdl(pool_global_avg_kernel<false>, grid_for(total, block), block, 0, s, (const uint8_t*)in, g.H * g.W, g.C, total, (uint8_t*)out);
-    } else if (g.C % 16 == 0) {
+    } else if (vec) {
         const size_t total = (size_t)g.B * g.oH * g.oW * (g.C / 16);
         if (total == 0) return cudaSuccess;
         launch_pdl(pool_vec_kernel, grid_for(total, block), block, 0, s, (const uint8_t*)in, in_unsigned, g, (uint8_t*)out, total);
@@ -610,7 +611,7 @@ cudaError_t launch_elemwise_sum(const SumInputs& ins, size_t pixels, int C, cons
     if (total == 0) return cudaSuccess;
     const int block = 256;
     if (ins.n == 2 && out_dtype == DT_I8 && ins.dtype[0] == DT_I8 && ins.dtype[1] == DT_I8 && C % 16 == 0
-        && !q.bias) {
+        && !q.bias && (((uintptr_t)ins.ptr[0] | (uintptr_t)ins.ptr[1] | (uintptr_t)out) & 15) == 0) {
         launch_pdl(elemwise_sum2_vec_kernel, grid_for(total / 16, block), block, 0, s, 
             (const uint8_t*)ins.ptr[0], ins.is_unsigned[0], (const uint8_t*)ins.ptr[1], ins.is_unsigned[1],
             total / 16, C, q, (uint8_t*)out);

@@ -21,6 +21,7 @@ __device__ __forceinline__ void s2d_image_bytes(const S2dImage& im, int block, i
     const uint8_t* __restrict__ in = im.in;
     uint4* __restrict__ out = im.out;
     const int C = im.C, H = im.H, W = im.W, Hs = im.Hs, Ws = im.Ws, P = im.P;
+    const bool words = C == 4 && ((uintptr_t)in & 3) == 0;   // (the image is the caller's buffer)
     for (int row = block; row < im.rows; row += blocks) {
         const int n = row / Hs, Y = row - n * Hs;
         const uint8_t* img = in + (size_t)n * H * W * C;
@@ -33,7 +34,8 @@ __device__ __forceinline__ void s2d_image_bytes(const S2dImage& im, int block, i
                 uint32_t px = 0;
                 if (y >= 0 && y < H && x >= 0 && x < W) {
                     const uint8_t* p = img + ((size_t)y * W + x) * C;
-                    if (C == 4) px = __ldg((const uint32_t*)p);
+                    if (words) px = __ldg((const uint32_t*)p);
+                    else if (C == 4) px = __ldg(p) | ((uint32_t)__ldg(p + 1) << 8) | ((uint32_t)__ldg(p + 2) << 16) | ((uint32_t)__ldg(p + 3) << 24);
                     else if (C == 3) px = __ldg(p) | ((uint32_t)__ldg(p + 1) << 8) | ((uint32_t)__ldg(p + 2) << 16);
                     else if (C == 2) px = __ldg(p) | ((uint32_t)__ldg(p + 1) << 8);
                     else px = __ldg(p);

@@ -52,6 +52,7 @@ __global__ void pad_image_kernel(const uint8_t* __restrict__ in, int C, int H, i
 {
     pdl_launch_dependents();
     pdl_wait();   // also before the stores: the previous kernel may still read the output buffer
+    const bool words = C == 4 && ((uintptr_t)in & 3) == 0;   // (the image is the caller's buffer)
     for (int row0 = blockIdx.x * PAD_ROWS; row0 < rows; row0 += gridDim.x * PAD_ROWS) {
         const uint8_t* irow[PAD_ROWS];
 #pragma unroll
@@ -69,7 +70,8 @@ __global__ void pad_image_kernel(const uint8_t* __restrict__ in, int C, int H, i
                 v[j] = 0u;
                 if (inside && irow[j]) {
                     const uint8_t* p = irow[j] + (size_t)x * C;
-                    if (C == 4) v[j] = __ldg((const uint32_t*)p);
+                    if (words) v[j] = __ldg((const uint32_t*)p);
+                    else if (C == 4) v[j] = __ldg(p) | ((uint32_t)__ldg(p + 1) << 8) | ((uint32_t)__ldg(p + 2) << 16) | ((uint32_t)__ldg(p + 3) << 24);
                     else if (C == 3) v[j] = __ldg(p) | ((uint32_t)__ldg(p + 1) << 8) | ((uint32_t)__ldg(p + 2) << 16);
                     else if (C == 2) v[j] = __ldg(p) | ((uint32_t)__ldg(p + 1) << 8);
                     else v[j] = __ldg(p);

@@ -240,6 +240,45 @@ def test_residual_sum_with_the_network_input(case, mode):
             qn.close()
 
 
+# First cells on the CUDA cores and first layers take the caller's buffer at any address: wide loads where it allows them
+@pytest.mark.parametrize('kind', ['max', 'avg', 'global', 'sum', 'scaling', 'stem_s2d', 'stem_gather', 'stem_pool', 'stem_rgb', 'direct', 'small'])
+def test_first_cells_take_an_input_at_any_address(kind):
+    import torch
+    C, H, W = {'stem_s2d': (4, 20, 22), 'stem_gather': (4, 19, 23), 'stem_pool': (4, 64, 65), 'stem_rgb': (3, 32, 32), 'direct': (24, 9, 9),
+               'small': (1, 24, 24)}.get(kind, (32, 10, 9))
+    b = netdesc.NetBuilder('any', C, H, W, 31, 'double', weight_dist=('normal', 30))
+    if kind in ('max', 'avg'):
+        b.pool(-1, kind, 3, 2, pad=1)
+    elif kind == 'global':
+        b.pool(-1, 'avg', (H, W), 1)
+    elif kind == 'sum':
+        b.sum([b.pool(-1, 'max', 3, 1, pad=1), -1])
+    elif kind == 'scaling':
+        b.scaling(-1, act='relu')
+    elif kind == 'direct':
+        b.conv(-1, 7, 3, pad=1, groups=1)
+    elif kind == 'small':
+        b.fc(b.conv(-1, 9, 3, stride=2), 10)
+    else:
+        x = b.conv(-1, 64 if kind == 'stem_pool' else 32, 3 if kind != 'stem_rgb' else 7, stride=1 if kind == 'stem_gather' else 2, pad=1)
+        if kind == 'stem_pool':
+            b.pool(x, 'max', 3, 2)
+    net = b.net
+    x = netdesc.make_input(net, 3)
+    want = oracle.run_net(net, x, 'i64')[-1].reshape(3, -1)
+    qn = runtime.QuantizedNet(net, 3)
+    try:
+        room = torch.zeros(x.size + 16, dtype=torch.uint8, device='cuda')
+        y = torch.empty((3, qn.out_elems), dtype=torch.uint8, device='cuda')
+        for shift in (1, 2, 4, 8, 0):
+            room[shift:shift + x.size] = torch.from_numpy(x.reshape(-1)).cuda()
+            qn.forward_device(room.data_ptr() + shift, 3, y.data_ptr())
+            qn.check()
+            assert np.array_equal(y.cpu().numpy().view(qn.out_dtype).astype(np.int64), want), f'{kind} at + {shift}'
+    finally:
+        qn.close()
+
+
 # A first cell on the tensor cores reads the caller's buffer through a map that ends with the call's last image: calls of changing sizes
 # on buffers that hold no more than the call's images
 @pytest.mark.parametrize('kind', ['plain', 'im2col', 'fc', 'depthwise', 'patch', 'residual', 'pair', 'w4'])

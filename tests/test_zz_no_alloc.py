@@ -101,6 +101,20 @@ def test_noalloc_first_conv_forms(case, mode):
     assert np.array_equal(got, want)
 
 
+def test_noalloc_first_conv_takes_an_input_at_any_address():
+    import torch
+    for C, stride in ((4, 2), (4, 1), (3, 2)):
+        net = single_conv_net(C, 32, 32, 64, 3, stride, 1, mode='double', seed=25)
+        x = netdesc.make_input(net, 2, seed=8)
+        want = oracle.run_net(net, x, 'i64')[-1]
+        room = torch.zeros(x.size + 16, dtype=torch.uint8, device='cuda')
+        out = torch.empty(want.size, dtype=torch.uint8, device='cuda')
+        for shift in (1, 2, 4, 0):
+            room[shift:shift + x.size] = torch.from_numpy(x.view(np.uint8).reshape(-1)).cuda()
+            runtime.first_conv_noalloc(room.data_ptr() + shift, 2, 32, 32, C, True, net['layers'][0], out.data_ptr())
+            assert np.array_equal(out.cpu().numpy().astype(np.int64), want.reshape(-1))
+
+
 # A bounded wait that runs out in one call's kernels (here in a one-CTA kernel that raises the same status word) is reported by the next
 # call, which launches nothing; the call after it runs.
 @pytest.mark.parametrize('stride', [2, 1])
