@@ -1993,6 +1993,7 @@ int n2d2b_scaling_propagate(int device, const int32_t* d_in, void* d_out, size_t
     if (!quant) return fail(N2D2B_ERR_INVALID, "quant must not be NULL");
     if (!d_in || !d_out) return fail(N2D2B_ERR_INVALID, "device buffers must not be NULL");
     if (quant->scaling.mode == SC_NONE) return fail(N2D2B_ERR_INVALID, "a NONE scaling has nothing to do");
+    if (quant->scaling.nb_channels < 0) return fail(N2D2B_ERR_INVALID, "nb_channels must not be negative (got %d)", quant->scaling.nb_channels);
     CUDA_TRY(cudaSetDevice(device));
     QuantHost q;
     if (int rc = validate_quant(quant, quant->scaling.nb_channels, false, q, nullptr)) return rc;

@@ -54,6 +54,15 @@ def test_no_cpu_fallback_without_a_device():
         runtime.QuantizedNet(netdesc.mnist24(), 4)
 
 
+def test_negative_channel_count_is_an_error_and_not_an_exception():
+    quant = runtime.Quant()
+    quant.scaling.mode = netdesc.MODES['single']
+    quant.scaling.nb_channels = -1
+    buffer = ctypes.create_string_buffer(16)   # refused before anything looks at it
+    rc = runtime.load().n2d2b_scaling_propagate(0, ctypes.addressof(buffer), ctypes.addressof(buffer), 1, ctypes.byref(quant), None)
+    assert rc == -1 and b'nb_channels' in runtime.load().n2d2b_last_error()
+
+
 def test_product_never_touches_the_oracle():
     for dirpath, _, files in os.walk(os.path.join(ROOT, 'n2d2_b200')):
         for f in files:
