@@ -179,7 +179,8 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags);
 /* DeepNet::propagate(inference = true) on device buffers: d_input is batch x H x W x C 8-bit values,
  * d_output receives the last cell's output (batch x its size).  Asynchronous on `stream`: the call only
  * enqueues the kernels, so a device-side wait that gave up (N2D2B_ERR_TIMEOUT) is not known when it returns;
- * n2d2b_net_check reports it. */
+ * n2d2b_net_check reports it.  d_input should start on 16 bytes: networks whose first cell has 16 or more input channels and
+ * runs on a tensor map (or is depthwise), or that add the input to a later tensor, refuse another address with N2D2B_ERR_INVALID. */
 int n2d2b_net_forward(n2d2b_net* net, const void* d_input, int batch, void* d_output, n2d2b_stream stream);
 /* Waits for the work queued on `stream` and returns N2D2B_ERR_TIMEOUT if a kernel of this network gave up on a
  * bounded wait since the last check (its outputs are then incomplete), N2D2B_ERR_CUDA if the stream failed,

@@ -10,11 +10,13 @@
 // no data moves, and the MMAs of a tile (taps x C/32 of them) are issued back to back.  Positions in the
 // halo columns (x >= oW) compute values nobody stores.  The weights of all taps stay resident.
 //
-// Depthwise 3x3 layers take the same route as block-diagonal groups: the channels are cut into groups of 64 (32), a
+// Depthwise layers of many pixels take the same route as block-diagonal groups: the channels are cut into groups of 64 (32), a
 // CTA works on one group for its whole life (CTA b on group b mod G, so the group's weight block - its own taps on
 // the diagonal, zeros elsewhere - stays resident), the patch load takes the group's channel slice of the NHWC tensor
-// and the output rows are written into that slice.  The tensor core multiplies 64 times more than the layer needs,
-// and still outruns the CUDA cores, where a byte dot product issues at a quarter of the integer rate.
+// and the output rows are written into that slice.  The tensor core multiplies 64 times more than the layer needs.
+// With 3x3 filters that is level with the dot-product kernel on the CUDA cores (conv_depthwise3x3_kernel) on large maps of few channels
+// and behind it elsewhere (see dw3x3_faster); wider filters run 2 to 4 times faster than on their CUDA-core kernel (5x5 on 64 x 56 x 56,
+// 64 images: 37 us against 137).
 //
 // Warp 0 loads (weights once, patches into two to four buffers), warps 1-4 issue tcgen05.mma kind::i8 for alternate
 // tiles into a ring of four TMEM accumulators, and four groups of four epilogue warps (one warp per TMEM lane quadrant) each
@@ -223,8 +225,8 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         }
     } else if (warp < EPI_WARP0) {
         // ------------------------------------------------------------------ MMA issuers
-        // Issuing a tile costs one thread about 100 cycles per MMA, the tensor pipe about 60: two threads take
-        // alternate tiles (each tile has its own accumulator, so their MMAs are independent).
+        // An MMA of 128 x 64 x 32 costs its issuing warp about 48 cycles and the tensor pipe 50, but waits, commits and address updates
+        // come on top: four warps (two beside a residual sum) take alternate tiles, whose accumulators are independent.
         // every lane of the warp runs the loop, an elected one issues (see elect_one)
         const unsigned me = (unsigned)__shfl_sync(0xffffffffu, warp - 1, 0);
         if (cta < items) {
