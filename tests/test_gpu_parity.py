@@ -204,7 +204,7 @@ def test_patch_kernel_with_a_residual_sum(case, mode):
 # (C, H, W, kernel of the last convolution, convolutions, weight bits, batch): a sum with the network's own input, whose address only the
 # forward pass knows - implicit GEMM (two and four staging regions, a cluster per tile), patch kernel, packed weights, one and two layers
 INPUT_RES_CASES = [(128, 9, 11, 1, 2, 8, 5), (256, 14, 14, 1, 1, 8, 3), (256, 8, 8, 3, 2, 8, 40), (512, 7, 7, 3, 2, 8, 1), (64, 21, 20, 3, 2, 8, 3),
-                   (64, 21, 20, 3, 1, 8, 3), (128, 28, 28, 1, 2, 4, 60), (48, 9, 9, 1, 2, 8, 2)]
+                   (64, 21, 20, 3, 1, 8, 3), (128, 28, 28, 1, 2, 4, 60), (48, 9, 9, 1, 2, 8, 2), (64, 46, 48, 3, 2, 8, 7), (128, 46, 48, 1, 2, 8, 7)]
 
 
 @pytest.mark.parametrize('case', INPUT_RES_CASES, ids=lambda c: 'C%d_%dx%d_k%d_n%d_w%d_b%d' % c)
@@ -220,6 +220,8 @@ def test_residual_sum_with_the_network_input(case, mode):
         net = b.net
         n_layers, eng = compare_net(net, batch, flags=0)
         assert 'fused' in eng
+        if H * W >= 2048:   # the host-buffer entry point slice by slice
+            compare_net(net, batch, flags=0, slices=3)
         # another buffer, then the first again, through the device entry point
         data = netdesc.make_input(net, batch, seed=3)
         want = oracle.run_net(net, data, 'i64')[-1].reshape(batch, -1)
