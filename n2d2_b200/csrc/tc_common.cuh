@@ -49,7 +49,7 @@ static inline int current_sms()
 
 // Raises a kernel's limit of dynamic shared memory ahead of its first launch on each device (a bit of `set` per device; racing first
 // launches do it twice: harmless).  Setting the limit loads the kernel, so only the one about to be launched is touched: with
-// the whole tables of variants at once the first call of a process spent 28 ms on 172 kernels, most of which it never ran.
+// the whole tables of variants at once the first ResNet-50 pass of a process took 36 ms instead of 31 and held 6 MiB of code instead of 2.
 typedef std::atomic<unsigned long long> SmemLimitSet;
 template <typename... P>
 static inline cudaError_t raise_smem_limit(void (*kernel)(P...), SmemLimitSet& set, int bytes = 227 * 1024)
