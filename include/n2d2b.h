@@ -255,6 +255,7 @@ int n2d2b_net_launches_per_forward(const n2d2b_net* net);
  *   "stem-tcgen05"                 first layers of up to 4 channels
  *   "stem-pool-tcgen05"            the same with the pooling behind it
  *   "depthwise-tcgen05"            depthwise as block-diagonal groups; smaller calls may run on the next one
+ *   "depthwise-1x1-tcgen05"        a 1x1 layer together with the 3x3 depthwise layer in front of it (which is "fused")
  *   "depthwise", "simt", "pool", "sum"   CUDA-core kernels
  *   "fused"                        folded into another cell's kernel
  *   "small-net"                    every cell of a network that runs as one kernel; the sliced upload of n2d2b_net_forward_host

@@ -88,6 +88,7 @@ struct FastQuant {
     bool dp_t_unsigned = false; //   the cell's own output is packed as unsigned bytes (natively, or shifted by +128)
     unsigned dp_xor = 0;        //   bytes to flip from unsigned to signed (0x80 per byte)
     int dp_a_signed = 1;        //   signedness of the (t, r) byte vector
+    bool unit_multiplier = false;   // every multiplier of the cell's own 32-bit rescale is 1
     bool monotone = false;      // no multiplier of the cell's own rescale is negative: it never decreases
     bool enabled = false;
 };
@@ -190,6 +191,27 @@ int patch_make_plan(PatchPlan* plan, const void* in, const int8_t* w, const Conv
 bool patch_takes_residual(const ConvGeom& g);
 cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g, int n_base, const Residual& r, const FastQuant& fast, void* out,
                          int* status_word, cudaStream_t s);
+
+// ---- 3x3 depthwise layer and the 1x1 layer behind it (dwpw_tcgen05.cu) ----
+struct DwPwPlan {
+    CUtensorMap tmA;      // NHWC input, box = one patch row of bk channels
+    CUtensorMap tmB;      // 1x1 weights [N][C], rows permuted in blocks of 32
+    ConvGeom d;           // the depthwise layer
+    int N, bk, num_sms;
+    const void* dw_words; // its weights (dwpw_arrange_depthwise), device
+    // the split of a call of `batch` images (dwpw_set_batch; fields as in DwPwArgs)
+    int batch, units, seg, segs_per_row, rt, groups, nsplit, bn, passes, item, parts, pitch, patch_bytes, np, subs, a_sub, na, dw_shared,
+        b_bytes, nb;
+    size_t smem_bytes;
+};
+bool dwpw_eligible(const ConvGeom& d, const ConvGeom& p);
+bool dwpw_takes_forms(const FastQuant& dw, const FastQuant& pw);
+size_t dwpw_depthwise_words(const ConvGeom& d);
+void dwpw_arrange_depthwise(const ConvGeom& d, const int8_t* w, uint32_t* dst);
+int dwpw_make_plan(DwPwPlan* plan, const void* in, const void* dw_words, const int8_t* w, const ConvGeom& d, int N, int max_batch, int num_sms, const char** why);
+// Splits a call of `batch` images (a no-op when the plan is for that many already)
+int dwpw_set_batch(DwPwPlan* plan, int batch);
+cudaError_t launch_dwpw(const DwPwPlan& plan, int n_base, const FastQuant& dw, const FastQuant& pw, void* out, int* status_word, cudaStream_t s);
 
 // ---- tensor-core implicit GEMM (tcgen05 kind::i8) ----
 struct IgemmPlan {

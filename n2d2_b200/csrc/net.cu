@@ -39,7 +39,7 @@ static int fail(int code, const char* fmt, ...)
 
 // ------------------------------------------------------------------------------------ model
 enum CellType { CELL_CONV, CELL_FC, CELL_POOL, CELL_SUM, CELL_SCALING };
-enum Engine { ENG_TCGEN05, ENG_SIMT, ENG_DEPTHWISE, ENG_POOL, ENG_SUM, ENG_FUSED, ENG_STEM, ENG_PATCH, ENG_STEM_S2D };
+enum Engine { ENG_TCGEN05, ENG_SIMT, ENG_DEPTHWISE, ENG_POOL, ENG_SUM, ENG_FUSED, ENG_STEM, ENG_PATCH, ENG_STEM_S2D, ENG_DWPW };
 
 struct TensorRec {
     int C = 0, H = 0, W = 0;
@@ -102,6 +102,9 @@ struct CellRec {
     void* d_colpad = nullptr;
     // stride-1 convolution from a shared-memory patch
     PatchPlan patch{};
+    // a 1x1 cell that computes the depthwise cell in front of it too (its input then is that cell's input)
+    int dw_cell = -1;
+    DwPwPlan dwpw{};
     // packed 4-bit weights at large batches: widened to int8 by a small kernel into the network's scratch, then the int8
     // kernel of the layer (see plan_widened)
     enum { W8_NONE, W8_IGEMM, W8_PATCH } w8 = W8_NONE;
@@ -547,6 +550,8 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
     c.fast.dp_a_signed = dp_a_signed;
     c.fast.monotone = true;   // (row 2: a multiplier, or a factor as the bits of a float)
     for (int ch = 0; ch < C; ++ch) c.fast.monotone = c.fast.monotone && f1[(size_t)2 * cpad + ch] >= 0;
+    c.fast.unit_multiplier = !wide && !flt;
+    for (int ch = 0; ch < C; ++ch) c.fast.unit_multiplier = c.fast.unit_multiplier && f1[(size_t)2 * cpad + ch] == 1;
     c.fast.enabled = true;
     return 0;
 }
@@ -927,6 +932,9 @@ static int head_candidate_prefix(const n2d2b_net* net)
 // the POOL variant of the space-to-depth kernel): the convolution's output, the largest tensor of such a network, is never stored.
 static int fuse_stem_pool(n2d2b_net* net);
 
+// A 3x3 depthwise cell whose only reader is a 1x1 cell becomes part of it (dwpw_tcgen05.cu): its output is never stored.
+static int fuse_depthwise(n2d2b_net* net);
+
 static int plan_buffers(n2d2b_net* net)
 {
     const bool keep_all = (net->flags & N2D2B_KEEP_ALL_OUTPUTS) != 0;
@@ -1122,6 +1130,8 @@ static bool dw3x3_faster(const ConvGeom& g, int batch)
 // max_batch has no other form, see finalize)
 static bool use_dw3x3(const CellRec& c, int batch) { return c.d_dw3x3 && dw3x3_faster(c.geom, batch); }
 
+static int plan_dwpw(n2d2b_net* net, CellRec& c);
+
 int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
 {
     if (!net) return fail(N2D2B_ERR_INVALID, "net must not be NULL");
@@ -1134,6 +1144,9 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
     if (!(flags & N2D2B_NO_FUSION)) fuse_residuals(net);
     if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE)))
         if (int rc = fuse_stem_pool(net)) return rc;
+    if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE | N2D2B_FORCE_DEPTHWISE_TENSOR | N2D2B_FORCE_IM2COL
+                   | N2D2B_FORCE_PAIR)))
+        if (int rc = fuse_depthwise(net)) return rc;
     net->head_limit = head_candidate_prefix(net);
     if (int rc = plan_buffers(net)) return rc;
     CUDA_TRY(cudaMalloc(&net->d_status, 64));
@@ -1149,6 +1162,10 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
         if (c.type == CELL_SUM || c.type == CELL_SCALING) { c.engine = ENG_SUM; continue; }
         // conv / fc: choose the kernel family and lay the weights out for it
         const ConvGeom& g = c.geom;
+        if (c.dw_cell >= 0) {
+            if (int rc = plan_dwpw(net, c)) return rc;
+            continue;
+        }
         const bool depthwise = (c.type == CELL_CONV && g.groups == g.C && g.Cg == 1 && g.Og == 1 && g.C % 16 == 0
                                 && g.groups > 1 && c.residual < 0
                                 && net->tensors[c.output].dtype == DT_I8);
@@ -1397,7 +1414,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
         const CellRec& c = net->cells[ci];
         bool sliceable = true;
         if (!c.skipped) {
-            const bool mapped = c.engine == ENG_TCGEN05 || c.engine == ENG_PATCH;
+            const bool mapped = c.engine == ENG_TCGEN05 || c.engine == ENG_PATCH || c.engine == ENG_DWPW;
             const bool pointer_based = (c.engine == ENG_STEM || c.engine == ENG_STEM_S2D || c.engine == ENG_POOL
                                         || c.engine == ENG_DEPTHWISE || c.engine == ENG_SIMT)
                                        && c.residual < 0 && c.inputs.size() == 1;
@@ -1453,6 +1470,73 @@ static int fuse_stem_pool(n2d2b_net* net)
     return 0;
 }
 
+static int fuse_depthwise(n2d2b_net* net)
+{
+    std::vector<int> consumers(net->tensors.size(), 0);
+    for (const CellRec& c : net->cells)
+        if (!c.skipped)
+            for (int i : c.inputs) consumers[i]++;
+    for (size_t ci = 0; ci < net->cells.size(); ++ci) {
+        CellRec& c = net->cells[ci];
+        // (the maps of the input want its address, which of the caller's buffer only the forward pass knows)
+        if (c.skipped || c.type != CELL_CONV || c.residual >= 0 || c.inputs.size() != 1 || c.inputs[0] == 0) continue;
+        const int t = c.output;
+        const TensorRec &tin = net->tensors[c.inputs[0]], &tmid = net->tensors[t];
+        if (consumers[t] != 1 || tin.dtype != DT_I8 || tmid.dtype != DT_I8 || !tin.is_unsigned || !tmid.is_unsigned || c.wbits != 8) continue;
+        int pj = -1;
+        for (size_t cj = ci + 1; cj < net->cells.size(); ++cj)
+            if (!net->cells[cj].skipped && net->cells[cj].inputs.size() == 1 && net->cells[cj].inputs[0] == t) { pj = (int)cj; break; }
+        if (pj < 0) continue;
+        CellRec& p = net->cells[pj];
+        if (p.type != CELL_CONV || p.residual >= 0 || p.wbits != 8 || net->tensors[p.output].dtype != DT_I8 || !dwpw_eligible(c.geom, p.geom)) continue;
+        ConvGeom g = c.geom;
+        g.B = net->max_batch;
+        DwPwPlan probe{};
+        probe.d = g;
+        probe.N = p.geom.O;
+        probe.num_sms = net->num_sms;
+        if (dwpw_set_batch(&probe, net->max_batch)) continue;
+        if (int rc = upload_fast(c, tmid)) return rc;
+        if (int rc = upload_fast(p, net->tensors[p.output])) return rc;
+        if (!dwpw_takes_forms(c.fast, p.fast)) {
+            for (CellRec* x : {&c, &p}) {
+                cudaFree(x->d_fast);
+                x->d_fast = nullptr;
+                x->fast = FastQuant{};
+            }
+            continue;
+        }
+        p.dw_cell = (int)ci;
+        p.inputs[0] = c.inputs[0];
+        net->tensors[t].readable = false;
+        net->tensors[t].buffer = -2;   // never materialised
+        c.skipped = true;
+        c.engine = ENG_FUSED;
+    }
+    return 0;
+}
+
+// Weights and plan of a 1x1 cell that computes the depthwise cell in front of it
+static int plan_dwpw(n2d2b_net* net, CellRec& c)
+{
+    CellRec& d = net->cells[c.dw_cell];
+    std::vector<uint32_t> words(dwpw_depthwise_words(d.geom));
+    dwpw_arrange_depthwise(d.geom, d.weights.data(), words.data());
+    d.d_weight_bytes = words.size() * 4;
+    CUDA_TRY(cudaMalloc((void**)&d.d_weights, d.d_weight_bytes));
+    CUDA_TRY(cudaMemcpy(d.d_weights, words.data(), d.d_weight_bytes, cudaMemcpyHostToDevice));
+    std::vector<int8_t> rows(c.weights.size());
+    igemm_permute_weights(c.weights.data(), rows.data(), c.geom.O, (size_t)c.geom.C, 32);
+    c.d_weight_bytes = rows.size();
+    CUDA_TRY(cudaMalloc((void**)&c.d_weights, rows.size() + 256));
+    CUDA_TRY(cudaMemcpy(c.d_weights, rows.data(), rows.size(), cudaMemcpyHostToDevice));
+    const char* why = "";
+    if (dwpw_make_plan(&c.dwpw, tensor_ptr(net, c.inputs[0], nullptr), d.d_weights, c.d_weights, d.geom, c.geom.O, net->max_batch, net->num_sms, &why))
+        return fail(N2D2B_ERR_STATE, "internal: a depthwise and 1x1 cell without a plan (%s)", why);
+    c.engine = ENG_DWPW;
+    return 0;
+}
+
 // ---- forward --------------------------------------------------------------------------------
 // Whether a depthwise cell can read from `in`, which only the caller's own buffer may fail.  A cell that has the block-diagonal form
 // takes what that form's tensor maps take, whichever kernel runs it; the others what the loads of their kernel do.
@@ -1475,7 +1559,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
     if (!in0 || !out) return fail(N2D2B_ERR_STATE, "internal: tensor without a buffer");
     // the tensor-core cells address their tensors through maps encoded over the whole buffers: a batch slice
     // is an offset in rows / images there; every other cell takes offset pointers
-    const bool mapped = c.engine == ENG_TCGEN05 || c.engine == ENG_PATCH;
+    const bool mapped = c.engine == ENG_TCGEN05 || c.engine == ENG_PATCH || c.engine == ENG_DWPW;
     if (img0 && !mapped) {
         if (c.engine == ENG_SUM || c.residual >= 0)
             return fail(N2D2B_ERR_STATE, "internal: this cell cannot run on a slice");
@@ -1560,6 +1644,10 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         CUDA_TRY(launch_patch(c.patch, g, img0, r, c.fast, out, net->d_status, s));
         break;
     }
+    case ENG_DWPW:
+        if (dwpw_set_batch(&c.dwpw, batch)) return fail(N2D2B_ERR_INVALID, "depthwise plan failed for %d images", batch);
+        CUDA_TRY(launch_dwpw(c.dwpw, img0, net->cells[c.dw_cell].fast, c.fast, out, net->d_status, s));
+        break;
     case ENG_STEM_S2D: {
         ConvGeom g = c.geom;
         g.B = batch;
@@ -1982,6 +2070,7 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     case ENG_FUSED: return "fused";
     case ENG_STEM: return "stem-tcgen05";
     case ENG_STEM_S2D: return c.pool_fused ? "stem-pool-tcgen05" : "stem-tcgen05";
+    case ENG_DWPW: return "depthwise-1x1-tcgen05";
     case ENG_PATCH: return c.geom.groups > 1 ? "depthwise-tcgen05" : "patch-tcgen05";
     }
     return "";

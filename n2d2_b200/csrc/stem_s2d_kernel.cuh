@@ -80,12 +80,6 @@ __device__ __forceinline__ void tc_mma_i8_words(unsigned d_tmem, unsigned a_lo, 
         ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-__device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
 // The MMAs of one tile with compile-time filter extents (KH rows, KP column pairs)
 template <int KH, int KP>
 __device__ __forceinline__ void s2d_issue_tile(unsigned d_tmem, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi,
