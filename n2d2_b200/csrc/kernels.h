@@ -266,6 +266,18 @@ void igemm_permute_weights(const int8_t* w, int8_t* dst, int N, size_t row_bytes
 cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residual& r, const FastQuant& fast,
                          void* out, int out_dtype, int m_base, int* status_word, cudaStream_t s);
 
+// ---- two convolutions and the sum of their outputs (igemm_dual.cu) ----
+struct DualPlan {
+    IgemmPlan a, b;       // maps, extents and tiling of the branch and of the projection
+    int stages, slot_bytes, resident;
+    size_t smem_bytes;
+};
+int dual_make_plan(DualPlan* plan, const void* in_a, const int8_t* w_a, const ConvGeom& ga, int a_unsigned, const void* in_b, const int8_t* w_b, const ConvGeom& gb,
+                   int b_unsigned, const void* out, int num_sms, const char** why);
+// fb: the projection's rescale with the sum's; m_base: first output row of the call's images; gb.B images
+cudaError_t launch_dual(const DualPlan& plan, const ConvGeom& gb, const FastQuant& fa, const FastQuant& fb, int branch_unsigned, int m_base, int late_weights,
+                        int* status_word, cudaStream_t s);
+
 // Widens packed 4-bit weights [rows_src][row_bytes / 2] into int8 [rows][row_bytes] in the row order a kernel expects.  Row n of the
 // destination is real channel perm_real_channel(n, ng_dst); ng_src says how the packed rows are ordered (0: naturally).
 // Destination rows of channels that do not exist are zero.

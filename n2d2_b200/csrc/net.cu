@@ -115,6 +115,11 @@ struct CellRec {
     // 3x3 depthwise cells on the tensor cores: weights as [kH][kW][C] for the calls that the dot-product kernel takes (see
     // dw3x3_faster), behind the block-diagonal ones in d_weights
     int8_t* d_dw3x3 = nullptr;
+    // the two convolutions in front of a sum as one kernel (igemm_dual.cu): on the later one, which carries the sum, the index of the other and the
+    // plan; on the other one the index of the later
+    int dual_branch = -1, dual_sum = -1;
+    bool dual_on = false;
+    DualPlan dual{};
     // tensor-core plan
     IgemmPlan plan{};
     bool has_plan = false;
@@ -906,6 +911,27 @@ static void fuse_residuals(n2d2b_net* net)
     }
 }
 
+// Pairs of convolutions whose outputs only meet in a sum (the branch and the projection of a residual block's first unit): the branch may be computed
+// by the kernel of the later one, so its input has to live until then.  Which pairs are is settled when the kernels are chosen (plan_duals).
+static void mark_duals(n2d2b_net* net)
+{
+    std::vector<int> consumers(net->tensors.size(), 0);
+    for (const CellRec& c : net->cells)
+        if (!c.skipped)
+            for (int i : c.inputs) consumers[i]++;
+    for (size_t bi = 0; bi < net->cells.size(); ++bi) {
+        CellRec& b = net->cells[bi];
+        if (b.skipped || b.type != CELL_CONV || b.residual <= 0 || b.inputs[0] == 0) continue;
+        const int ai = net->tensors[b.residual].producer;
+        if (ai < 0 || ai >= (int)bi || consumers[b.residual] != 1) continue;
+        CellRec& a = net->cells[ai];
+        if (a.skipped || a.type != CELL_CONV || a.residual >= 0 || a.output != b.residual || a.inputs[0] == 0 || a.geom.groups != 1) continue;
+        b.dual_branch = ai;
+        a.dual_sum = (int)bi;
+        b.inputs.push_back(a.inputs[0]);
+    }
+}
+
 // Cells [0, n) that the host-buffer entry point may run slice by slice (a structural rule, applied before the
 // kernels are chosen; the engine-based rule in finalize can only shorten it): image-wise cells with large
 // per-image tensors, up to the first fully-connected cell or stand-alone sum.
@@ -1021,6 +1047,13 @@ static bool use_widened(const n2d2b_net* net, const CellRec& c, int batch)
     return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) > 2ll * net->num_sms;
 }
 
+// Bytes of widened weights of a packed cell, rounded so that another one's may follow
+static size_t widened_bytes(const CellRec& c)
+{
+    const size_t n = (size_t)((c.geom.O + 31) & ~31) * c.geom.kH * c.geom.kW * c.geom.C;
+    return (n + 255) & ~(size_t)255;
+}
+
 // Plans the widened form of every packed cell.  The weights stay packed in HBM; one scratch block, as large as the largest such cell,
 // holds the int8 weights of the cell that is running.  3x3 256 -> 256 at 14 x 14, 2048 images: 0.51 ms with the expansion
 // in the kernel (its warps' shared-memory stores bound it).
@@ -1033,8 +1066,8 @@ static int plan_widened(n2d2b_net* net)
     size_t most = 0;
     for (CellRec& c : net->cells) {
         if (!eligible(c)) continue;
-        const int rows = (c.geom.O + 31) & ~31;
-        most = std::max(most, (size_t)rows * c.geom.kH * c.geom.kW * c.geom.C);
+        // (a pair that runs as one kernel needs both)
+        most = std::max(most, widened_bytes(c) + (c.dual_branch >= 0 ? widened_bytes(net->cells[c.dual_branch]) : 0));
     }
     if (!most) return 0;
     CUDA_TRY(cudaMalloc(&net->d_w8, most + 256));
@@ -1072,6 +1105,46 @@ static int plan_widened(n2d2b_net* net)
     }
     for (const CellRec& c : net->cells)
         if (!c.skipped && use_widened(net, c, net->max_batch)) net->launches += c.d_w8_out ? 2 : 1;
+    return 0;
+}
+
+// Whether the pair of convolutions that ends in cell `b` runs as one kernel in a call of `batch` images: packed weights only where both are widened
+static bool use_dual(const n2d2b_net* net, const CellRec& b, int batch)
+{
+    if (!b.dual_on) return false;
+    const CellRec& a = net->cells[b.dual_branch];
+    return !a.plan.w4 || (use_widened(net, a, batch) && use_widened(net, b, batch));
+}
+
+static int plan_duals(n2d2b_net* net)
+{
+    for (size_t bi = 0; bi < net->cells.size(); ++bi) {
+        CellRec& b = net->cells[bi];
+        if (b.dual_branch < 0) continue;
+        CellRec& a = net->cells[b.dual_branch];
+        const bool packed = a.plan.w4 && b.plan.w4;
+        if (b.engine != ENG_TCGEN05 || (a.engine != ENG_TCGEN05 && a.engine != ENG_PATCH) || a.plan.w4 != b.plan.w4 || a.pad_O || b.pad_O) continue;
+        if (!a.fast.enabled || !b.fast.enabled || !b.fast.fq2 || net->tensors[b.output].dtype != DT_I8 || net->tensors[a.output].dtype != DT_I8) continue;
+        // one order of weight rows for both: blocks of 32 channels
+        if (packed ? (a.w8 == CellRec::W8_NONE || b.w8 == CellRec::W8_NONE || a.d_w8_out || b.d_w8_out)
+                   : (b.plan.perm != 32 || (a.engine == ENG_TCGEN05 && a.plan.perm != 32)))
+            continue;
+        // The patch kernel reads a 64-channel branch's input once, an im2col map nine times: 64 -> 64 channels of 55 x 55 with its projection at 2048 images
+        // 596 us as two kernels, 718 as one; 128 channels of 28 x 28 400 / 290
+        if ((a.engine == ENG_PATCH || a.w8 == CellRec::W8_PATCH) && a.geom.C <= 64) continue;
+        // (slices of the upload: both or neither)
+        if ((b.dual_branch < net->head_cells) != ((int)bi < net->head_cells)) continue;
+        ConvGeom ga = a.geom, gb = b.geom;
+        ga.B = gb.B = net->max_batch;
+        const int8_t* wa = packed ? (const int8_t*)net->d_w8 : a.d_weights;
+        const int8_t* wb = packed ? (const int8_t*)net->d_w8 + widened_bytes(a) : b.d_weights;
+        const char* why = "";
+        if (dual_make_plan(&b.dual, tensor_ptr(net, a.inputs[0], nullptr), wa, ga, net->tensors[a.inputs[0]].is_unsigned, tensor_ptr(net, b.inputs[0], nullptr), wb,
+                           gb, net->tensors[b.inputs[0]].is_unsigned, tensor_ptr(net, b.output, nullptr), net->num_sms, &why))
+            continue;
+        b.dual_on = true;
+        if (use_dual(net, b, net->max_batch)) net->launches--;
+    }
     return 0;
 }
 
@@ -1131,6 +1204,7 @@ static bool dw3x3_faster(const ConvGeom& g, int batch)
 static bool use_dw3x3(const CellRec& c, int batch) { return c.d_dw3x3 && dw3x3_faster(c.geom, batch); }
 
 static int plan_dwpw(n2d2b_net* net, CellRec& c);
+static int plan_duals(n2d2b_net* net);
 
 int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
 {
@@ -1147,6 +1221,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
     if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE | N2D2B_FORCE_DEPTHWISE_TENSOR | N2D2B_FORCE_IM2COL
                    | N2D2B_FORCE_PAIR)))
         if (int rc = fuse_depthwise(net)) return rc;
+    if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE | N2D2B_FORCE_IM2COL | N2D2B_FORCE_PAIR))) mark_duals(net);
     net->head_limit = head_candidate_prefix(net);
     if (int rc = plan_buffers(net)) return rc;
     CUDA_TRY(cudaMalloc(&net->d_status, 64));
@@ -1425,6 +1500,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
         if (!sliceable || (int)ci >= net->head_limit) break;
         net->head_cells = (int)ci + 1;
     }
+    if (int rc = plan_duals(net)) return rc;
     for (int k = 0; k < 2; ++k) {
         CUDA_TRY(cudaEventCreateWithFlags(&net->pipe_uploaded[k], cudaEventDisableTiming));
         CUDA_TRY(cudaEventCreateWithFlags(&net->pipe_computed[k], cudaEventDisableTiming));
@@ -1552,6 +1628,7 @@ static bool depthwise_takes(const n2d2b_net* net, const CellRec& c, int batch, c
 // Runs one cell on images [img0, img0 + batch) of the batch (img0 != 0 only for cells without tensor maps).
 static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, cudaStream_t s, int img0 = 0)
 {
+    if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], batch)) return 0;   // computed by the cell that carries the sum
     const void* in0 = tensor_ptr(net, c.inputs[0], d_input);
     void* out = tensor_ptr(net, c.output, d_input);
     const TensorRec& tin = net->tensors[c.inputs[0]];
@@ -1575,6 +1652,21 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
     // the maps and the loads of a residual start on 16 bytes; the network's input is the caller's buffer
     if (c.residual == 0 && mapped && ((uintptr_t)r.ptr & 15))
         return fail(N2D2B_ERR_INVALID, "a residual sum cannot read an input at %p: operands must be 16-byte aligned", r.ptr);
+    if (c.dual_branch >= 0 && use_dual(net, c, batch)) {
+        const CellRec& a = net->cells[c.dual_branch];
+        if (a.plan.w4) {
+            size_t off = 0;
+            for (const CellRec* x : {&a, (const CellRec*)&c}) {
+                CUDA_TRY(launch_widen_int4((const uint8_t*)x->d_weights, x->geom.O, x->w8_ng_src, (int8_t*)net->d_w8 + off, x->w8_rows, 4,
+                                           (size_t)x->geom.kH * x->geom.kW * x->geom.C, s));
+                off += widened_bytes(*x);
+            }
+        }
+        ConvGeom g = c.geom;
+        g.B = batch;
+        CUDA_TRY(launch_dual(c.dual, g, a.fast, c.fast, net->tensors[a.output].is_unsigned, img0 * g.oH * g.oW, a.plan.w4, net->d_status, s));
+        return 0;
+    }
     if (use_widened(net, c, batch)) {
         const size_t row_bytes = (size_t)c.geom.kH * c.geom.kW * c.geom.C;
         CUDA_TRY(launch_widen_int4((const uint8_t*)c.d_weights, c.geom.O, c.w8_ng_src, (int8_t*)net->d_w8, c.w8_rows, c.w8_ng_dst, row_bytes, s));
@@ -2054,6 +2146,8 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     if (!net || cell < 0 || cell >= (int)net->cells.size()) return "";
     if (net->d_small) return "small-net";
     const CellRec& c = net->cells[cell];
+    if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], net->max_batch)) return "fused";
+    if (c.dual_branch >= 0 && use_dual(net, c, net->max_batch)) return "tcgen05-dual";
     if (use_dw3x3(c, net->max_batch)) return "depthwise";
     if (use_widened(net, c, net->max_batch)) return c.w8 == CellRec::W8_PATCH ? "patch-tcgen05-widened" : "tcgen05-widened";
     switch (c.engine) {

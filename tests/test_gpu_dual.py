@@ -1,0 +1,64 @@
+"""The two convolutions in front of a residual sum as one kernel, against the oracle (whole numbers: no tolerance)."""
+import numpy as np
+import pytest
+
+from gpu_common import compare_net, kernels_of
+from n2d2_b200 import netdesc, runtime
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+ENGINE = 'tcgen05-dual'
+
+
+def unit_net(C, mid, H, W, O, k, stride, mode, unsigned_relu=True, clipped=False, act='linear', weight_bits=8, seed=5):
+    """A residual block's first unit: conv -> branch (k x k) beside a 1x1 projection of its input, their sum, and a cell that reads it."""
+    dist = ('normal', 30) if weight_bits == 8 else ('uniform', 7)
+    b = netdesc.NetBuilder('unit', 16, H, W, seed, mode, unsigned_relu=unsigned_relu, weight_dist=dist, clipped=clipped, weight_bits=weight_bits)
+    x = b.conv(-1, C, 1, name='front')
+    y = b.conv(x, mid, 1, name='reduce')
+    y = b.conv(y, O, k, stride=stride, pad=k // 2, act=act, name='branch')
+    p = b.conv(x, O, 1, stride=stride, act=act, name='projection')
+    b.conv(b.sum([y, p], act='relu', name='sum'), 32, 1, name='reader')
+    return b.net
+
+
+# (channels of the projection, of the branch, H, W, outputs, filter, stride, batch): K blocks of 32, 64 and 128 bytes on either side, weights
+# resident and streamed, columns of 64 and 128 with a part of a tile, rows that end inside a tile, one tile and many per CTA
+CASES = [(64, 64, 13, 11, 256, 1, 1, 3), (64, 64, 28, 28, 256, 1, 1, 40), (256, 128, 14, 14, 512, 1, 2, 7), (512, 256, 9, 9, 1024, 1, 2, 20),
+         (1024, 512, 8, 7, 2048, 1, 2, 33), (128, 256, 14, 14, 256, 3, 2, 5), (256, 512, 7, 7, 512, 3, 1, 1), (256, 512, 7, 7, 512, 3, 1, 160),
+         (32, 64, 20, 20, 96, 3, 1, 9), (96, 48, 15, 15, 160, 3, 2, 6), (32, 32, 5, 3, 32, 1, 1, 2), (64, 128, 28, 28, 128, 3, 1, 30)]
+
+
+@pytest.mark.parametrize('case', CASES, ids=lambda c: 'C%d_%d_%dx%d_O%d_k%d_s%d_b%d' % c)
+@pytest.mark.parametrize('mode', ['double', 'fixed', 'float'])
+def test_branch_and_projection(case, mode):
+    C, mid, H, W, O, k, s, batch = case
+    n, eng = compare_net(unit_net(C, mid, H, W, O, k, s, mode), batch, flags=0)
+    if O % 64 == 0 and not (k == 3 and s == 1 and O <= 128):   # (narrow branches may keep the patch kernel)
+        assert ENGINE in eng
+
+
+@pytest.mark.parametrize('mode, unsigned_relu, clipped, act', [('double', False, False, 'linear'), ('fixed', True, True, 'linear'), ('float', True, True, 'relu'),
+                                                               ('single', True, False, 'relu'), ('fixed', False, False, 'linear')])
+def test_branch_and_projection_forms(mode, unsigned_relu, clipped, act):
+    compare_net(unit_net(128, 64, 12, 10, 256, 1, 1, mode, unsigned_relu, clipped, act), 9, flags=0, want_engine=ENGINE)
+
+
+def test_packed_weights_and_calls_of_any_size_on_one_network():
+    # widened weights of both cells stand in the scratch block at once; calls below the line of the widened form run the two cells one by one
+    net = unit_net(128, 128, 14, 14, 256, 3, 1, 'fixed', weight_bits=4, clipped=True)
+    x = netdesc.make_input(net, 400)
+    ref = oracle.run_net(net, x, 'i64')[-1].reshape(400, -1)
+    qn = runtime.QuantizedNet(net, 400)
+    try:
+        assert ENGINE in qn.engines()
+        assert any('igemm_dual' in k for k in kernels_of(qn, 400)) and not any('igemm_dual' in k for k in kernels_of(qn, 2))
+        for batch in (400, 3, 399, 60):
+            assert np.array_equal(qn.forward_host(x[:batch]).astype(np.int64), ref[:batch])
+    finally:
+        qn.close()
+
+
+def test_slices_of_the_upload():
+    net = unit_net(64, 64, 56, 56, 256, 1, 1, 'double')
+    compare_net(net, 11, flags=0, slices=4, want_engine=ENGINE)
