@@ -829,43 +829,65 @@ static bool igemm_split(long long tiles, int num_kb, int num_sms)
     return num_kb >= 24 && num_kb <= SPLIT * SPLIT_STAGES && tiles * SPLIT <= num_sms / 2;
 }
 
-// Eight weights per thread; at most a few megabytes that stay in L2
-__global__ void __launch_bounds__(256) widen_int4_kernel(const uint8_t* __restrict__ packed, int rows_src, int ng_src, int8_t* __restrict__ dst, int rows,
-                                                         int ng_dst, unsigned words)
+// Eight weights per thread; at most a few megabytes that stay in L2.  All cells of a pass in one launch: with one launch each a ResNet-18 of packed weights
+// spent twenty hand-overs on them.
+static constexpr int WIDEN_JOBS = 32;
+struct WidenTable {
+    WidenJob job[WIDEN_JOBS];
+    unsigned first[WIDEN_JOBS + 1];   // destination words before each job
+    int count;
+};
+
+__global__ void __launch_bounds__(256) widen_int4_kernel(const __grid_constant__ WidenTable t)
 {
     pdl_launch_dependents();
     pdl_wait();   // the destination may still be read by the previous kernel
-    const unsigned total = (unsigned)rows * words;   // 8-byte words of the destination
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const unsigned n = i / words, w = i - n * words;
-        const int real = perm_real_channel((int)n, ng_dst);
+    int j = 0;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < t.first[t.count]; i += gridDim.x * blockDim.x) {
+        while (i >= t.first[j + 1]) ++j;   // (i only grows)
+        const WidenJob& job = t.job[j];
+        const unsigned at = i - t.first[j], n = at / job.words, w = at - n * job.words;
+        const int real = perm_real_channel((int)n, job.ng_dst);
         uint2 o = make_uint2(0u, 0u);
-        if (real < rows_src) {
+        if (real < job.rows_src) {
             int src = real;
-            if (ng_src) {   // where the packed rows hold this channel (the inverse of perm_real_channel)
-                const int j = real % (8 * ng_src), q = j / (2 * ng_src), r = j - q * 2 * ng_src;
-                src = real - j + 8 * (r >> 1) + 2 * q + (r & 1);
+            if (job.ng_src) {   // where the packed rows hold this channel (the inverse of perm_real_channel)
+                const int k = real % (8 * job.ng_src), q = k / (2 * job.ng_src), r = k - q * 2 * job.ng_src;
+                src = real - k + 8 * (r >> 1) + 2 * q + (r & 1);
             }
             unsigned lo, hi;
-            expand_int4_x16(__ldg((const unsigned*)packed + (size_t)src * words + w), lo, hi);
+            expand_int4_x16(__ldg((const unsigned*)job.packed + (size_t)src * job.words + w), lo, hi);
             auto down = [](unsigned x) {   // 16 x the value in every byte -> the value
                 const unsigned t = (x >> 4) & 0x0f0f0f0fu;
                 return t | ((t & 0x08080808u) * 0x1eu);
             };
             o = make_uint2(down(lo), down(hi));
         }
-        ((uint2*)dst)[i] = o;
+        ((uint2*)job.dst)[at] = o;
     }
 }
 
-cudaError_t launch_widen_int4(const uint8_t* packed, int rows_src, int ng_src, int8_t* dst, int rows, int ng_dst, size_t row_bytes, cudaStream_t s)
+cudaError_t launch_widen_int4(const WidenJob* jobs, int count, cudaStream_t s)
 {
-    const unsigned words = (unsigned)(row_bytes / 8);
-    const unsigned long long total = (unsigned long long)rows * words;
-    if (total == 0) return cudaSuccess;
-    if (total >= (1ull << 31)) return cudaErrorInvalidValue;
-    const unsigned long long blocks = (total + 255) / 256, most = 8ull * current_sms();
-    return launch_pdl(widen_int4_kernel, (int)(blocks < most ? blocks : most), 256, 0, s, packed, rows_src, ng_src, dst, rows, ng_dst, words);
+    for (int done = 0; done < count;) {
+        WidenTable t;
+        memset(&t, 0, sizeof(t));
+        unsigned long long total = 0;
+        for (; done < count && t.count < WIDEN_JOBS; ++done) {
+            const unsigned long long words = (unsigned long long)jobs[done].rows * jobs[done].words;
+            if (words >= (1ull << 30)) return cudaErrorInvalidValue;
+            if (words == 0) continue;
+            if (total + words >= (1ull << 31)) break;
+            t.job[t.count] = jobs[done];
+            t.first[t.count++] = (unsigned)total;
+            total += words;
+            t.first[t.count] = (unsigned)total;
+        }
+        if (t.count == 0) break;
+        const unsigned long long blocks = (total + 255) / 256, most = 8ull * current_sms();
+        if (cudaError_t e = launch_pdl(widen_int4_kernel, (int)(blocks < most ? blocks : most), 256, 0, s, t)) return e;
+    }
+    return cudaSuccess;
 }
 
 bool igemm_uses_fast_epilogue(const IgemmPlan& plan, const FastQuant& fast, bool has_residual, int out_dtype)

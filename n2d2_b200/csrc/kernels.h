@@ -278,10 +278,16 @@ int dual_make_plan(DualPlan* plan, const void* in_a, const int8_t* w_a, const Co
 cudaError_t launch_dual(const DualPlan& plan, const ConvGeom& gb, const FastQuant& fa, const FastQuant& fb, int branch_unsigned, int m_base, int late_weights,
                         int* status_word, cudaStream_t s);
 
-// Widens packed 4-bit weights [rows_src][row_bytes / 2] into int8 [rows][row_bytes] in the row order a kernel expects.  Row n of the
-// destination is real channel perm_real_channel(n, ng_dst); ng_src says how the packed rows are ordered (0: naturally).
+// Widens packed 4-bit weights [rows_src][8 words / 2 bytes] into int8 [rows][8 words] in the row order a kernel expects, several cells' in one launch.  Row n
+// of the destination is real channel perm_real_channel(n, ng_dst); ng_src says how the packed rows are ordered (0: naturally).
 // Destination rows of channels that do not exist are zero.
-cudaError_t launch_widen_int4(const uint8_t* packed, int rows_src, int ng_src, int8_t* dst, int rows, int ng_dst, size_t row_bytes, cudaStream_t s);
+struct WidenJob {
+    const uint8_t* packed;
+    int8_t* dst;
+    int rows_src, ng_src, rows, ng_dst;
+    unsigned words;       // 8-byte words of a destination row
+};
+cudaError_t launch_widen_int4(const WidenJob* jobs, int count, cudaStream_t s);
 
 // ---- first-layer convolution (<= 4 input channels) on the tensor cores ----
 struct StemPlan {

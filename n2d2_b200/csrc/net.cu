@@ -111,6 +111,7 @@ struct CellRec {
     IgemmPlan plan8{};
     PatchPlan patch8{};
     int w8_rows = 0, w8_ng_src = 0, w8_ng_dst = 0;
+    size_t w8_offset = 0;         // in the network's scratch
     void* d_w8_out = nullptr;     // padded output matrix (see pad_O) of a widened cell
     // 3x3 depthwise cells on the tensor cores: weights as [kH][kW][C] for the calls that the dot-product kernel takes (see
     // dw3x3_faster), behind the block-diagonal ones in d_weights
@@ -139,7 +140,10 @@ struct n2d2b_net {
     std::vector<void*> buffers;
     std::vector<size_t> buffer_bytes;
     int* d_status = nullptr;
-    void* d_w8 = nullptr;         // widened weights of the packed cell that is running
+    void* d_w8 = nullptr;         // widened weights of the packed cells, of the call that is running
+    long long w8_macs = 0;        // multiply-accumulates per image of the cells that have a widened form
+    int call_batch = 0;           // images of the call that is running (its upload slices are smaller)
+    bool call_widened = false;    // the call's weights are in d_w8
     int launches = 0;
     const void* last_input = nullptr;
     void* d_labels_scratch = nullptr;   // device labels / scores of the host-buffer top-N entry point
@@ -1038,11 +1042,18 @@ static int final_tensor_of(const n2d2b_net* net)
     return -1;
 }
 
-// Whether a packed cell takes the widened form: its in-kernel expansion repeats for every tile, the widening once per call for
-// 2 to 3 us.  The line lies where a CTA has more than two tiles.
-static bool use_widened(const n2d2b_net* net, const CellRec& c, int batch)
+// Whether a call of `call` images widens the packed weights of all cells at its start, in one launch of 3 to 4 us.  The line is drawn where a call is large
+// enough to pay for it whatever its cells are (ResNet-18 at 224 x 224, 1.7 G multiply-accumulates an image: four images 217 us with the expansion in the
+// kernels, 182 widened cell by cell, 162 in one launch; 128 images 656 / 460 / 421: the expansion warps' shared-memory stores bound every layer of long
+// K, and the classifier, which has no 32-bit epilogue in that form, took 38 to 110 us).
+static bool widen_all(const n2d2b_net* net, int call) { return net->w8_macs * call >= (1ll << 29); }
+
+// Whether a packed cell takes the widened form in a call of `call` images, `batch` of them at once.  In a smaller call a cell is widened by itself where a
+// CTA has more than two tiles, whose in-kernel expansions would repeat.
+static bool use_widened(const n2d2b_net* net, const CellRec& c, int batch, int call)
 {
     if (c.w8 == CellRec::W8_NONE) return false;
+    if (widen_all(net, call)) return true;
     const long long m_tiles = ((long long)batch * c.geom.oH * c.geom.oW + 127) / 128;
     return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) > 2ll * net->num_sms;
 }
@@ -1054,23 +1065,21 @@ static size_t widened_bytes(const CellRec& c)
     return (n + 255) & ~(size_t)255;
 }
 
-// Plans the widened form of every packed cell.  The weights stay packed in HBM; one scratch block, as large as the largest such cell,
-// holds the int8 weights of the cell that is running.  3x3 256 -> 256 at 14 x 14, 2048 images: 0.51 ms with the expansion
-// in the kernel (its warps' shared-memory stores bound it).
+// Plans the widened form of every packed cell.  The weights stay packed in HBM; a scratch block holds the int8 weights of the call that is running.
 static int plan_widened(n2d2b_net* net)
 {
     // (not where the input or the residual is the caller's buffer, whose address only the forward pass knows)
     auto eligible = [](const CellRec& c) {
         return !c.skipped && c.engine == ENG_TCGEN05 && c.plan.w4 && c.fast.enabled && c.plan_input && c.residual != 0;
     };
-    size_t most = 0;
+    size_t total = 0;
     for (CellRec& c : net->cells) {
         if (!eligible(c)) continue;
-        // (a pair that runs as one kernel needs both)
-        most = std::max(most, widened_bytes(c) + (c.dual_branch >= 0 ? widened_bytes(net->cells[c.dual_branch]) : 0));
+        c.w8_offset = total;
+        total += widened_bytes(c);
     }
-    if (!most) return 0;
-    CUDA_TRY(cudaMalloc(&net->d_w8, most + 256));
+    if (!total) return 0;
+    CUDA_TRY(cudaMalloc(&net->d_w8, total + 256));
     for (CellRec& c : net->cells) {
         if (!eligible(c)) continue;
         ConvGeom g = c.geom;
@@ -1082,7 +1091,7 @@ static int plan_widened(n2d2b_net* net)
         const char* why = "";
         c.w8_ng_src = c.plan.perm / 8;
         c.w8_rows = g.O;
-        if ((!res || (patch_takes_residual(g) && !c.fast.dp4a)) && patch_eligible(g) && patch_make_plan(&c.patch8, c.plan_input, (const int8_t*)net->d_w8, g, in_u, net->num_sms, &why) == 0) {
+        if ((!res || (patch_takes_residual(g) && !c.fast.dp4a)) && patch_eligible(g) && patch_make_plan(&c.patch8, c.plan_input, (const int8_t*)net->d_w8 + c.w8_offset, g, in_u, net->num_sms, &why) == 0) {
             c.patch8.late_weights = 1;
             c.w8_ng_dst = 4;
             c.w8 = CellRec::W8_PATCH;
@@ -1095,7 +1104,7 @@ static int plan_widened(n2d2b_net* net)
             CUDA_TRY(cudaMalloc(&c.d_w8_out, (size_t)net->max_batch * g.oH * g.oW * g.O + 256));
             out = c.d_w8_out;
         }
-        if (igemm_make_plan(&c.plan8, c.plan_input, (const int8_t*)net->d_w8, out, res, g, in_u, 0, 0, net->num_sms, &why)
+        if (igemm_make_plan(&c.plan8, c.plan_input, (const int8_t*)net->d_w8 + c.w8_offset, out, res, g, in_u, 0, 0, net->num_sms, &why)
             || !igemm_uses_fast_epilogue(c.plan8, c.fast, res != nullptr, DT_I8))
             continue;
         c.plan8.late_weights = 1;
@@ -1104,16 +1113,20 @@ static int plan_widened(n2d2b_net* net)
         c.w8 = CellRec::W8_IGEMM;
     }
     for (const CellRec& c : net->cells)
-        if (!c.skipped && use_widened(net, c, net->max_batch)) net->launches += c.d_w8_out ? 2 : 1;
+        if (c.w8 != CellRec::W8_NONE) net->w8_macs += (long long)c.geom.oH * c.geom.oW * c.geom.O * c.geom.kH * c.geom.kW * c.geom.C;
+    const bool all = widen_all(net, net->max_batch);
+    if (all) net->launches++;
+    for (const CellRec& c : net->cells)
+        if (use_widened(net, c, net->max_batch, net->max_batch)) net->launches += (all ? 0 : 1) + (c.d_w8_out ? 1 : 0);
     return 0;
 }
 
 // Whether the pair of convolutions that ends in cell `b` runs as one kernel in a call of `batch` images: packed weights only where both are widened
-static bool use_dual(const n2d2b_net* net, const CellRec& b, int batch)
+static bool use_dual(const n2d2b_net* net, const CellRec& b, int batch, int call)
 {
     if (!b.dual_on) return false;
     const CellRec& a = net->cells[b.dual_branch];
-    return !a.plan.w4 || (use_widened(net, a, batch) && use_widened(net, b, batch));
+    return !a.plan.w4 || (use_widened(net, a, batch, call) && use_widened(net, b, batch, call));
 }
 
 static int plan_duals(n2d2b_net* net)
@@ -1126,7 +1139,7 @@ static int plan_duals(n2d2b_net* net)
         if (b.engine != ENG_TCGEN05 || (a.engine != ENG_TCGEN05 && a.engine != ENG_PATCH) || a.plan.w4 != b.plan.w4 || a.pad_O || b.pad_O) continue;
         if (!a.fast.enabled || !b.fast.enabled || !b.fast.fq2 || net->tensors[b.output].dtype != DT_I8 || net->tensors[a.output].dtype != DT_I8) continue;
         // one order of weight rows for both: blocks of 32 channels
-        if (packed ? (a.w8 == CellRec::W8_NONE || b.w8 == CellRec::W8_NONE || a.d_w8_out || b.d_w8_out)
+        if (packed ? (a.w8 == CellRec::W8_NONE || b.w8 == CellRec::W8_NONE || a.d_w8_out || b.d_w8_out || a.w8_ng_dst != 4 || b.w8_ng_dst != 4)
                    : (b.plan.perm != 32 || (a.engine == ENG_TCGEN05 && a.plan.perm != 32)))
             continue;
         // The patch kernel reads a 64-channel branch's input once, an im2col map nine times: 64 -> 64 channels of 55 x 55 with its projection at 2048 images
@@ -1136,14 +1149,14 @@ static int plan_duals(n2d2b_net* net)
         if ((b.dual_branch < net->head_cells) != ((int)bi < net->head_cells)) continue;
         ConvGeom ga = a.geom, gb = b.geom;
         ga.B = gb.B = net->max_batch;
-        const int8_t* wa = packed ? (const int8_t*)net->d_w8 : a.d_weights;
-        const int8_t* wb = packed ? (const int8_t*)net->d_w8 + widened_bytes(a) : b.d_weights;
+        const int8_t* wa = packed ? (const int8_t*)net->d_w8 + a.w8_offset : a.d_weights;
+        const int8_t* wb = packed ? (const int8_t*)net->d_w8 + b.w8_offset : b.d_weights;
         const char* why = "";
         if (dual_make_plan(&b.dual, tensor_ptr(net, a.inputs[0], nullptr), wa, ga, net->tensors[a.inputs[0]].is_unsigned, tensor_ptr(net, b.inputs[0], nullptr), wb,
                            gb, net->tensors[b.inputs[0]].is_unsigned, tensor_ptr(net, b.output, nullptr), net->num_sms, &why))
             continue;
         b.dual_on = true;
-        if (use_dual(net, b, net->max_batch)) net->launches--;
+        if (use_dual(net, b, net->max_batch, net->max_batch)) net->launches--;
     }
     return 0;
 }
@@ -1625,10 +1638,33 @@ static bool depthwise_takes(const n2d2b_net* net, const CellRec& c, int batch, c
     return !block_form && (uintptr_t)in % depthwise_alignment(g, c.fast) == 0;
 }
 
+// Widens the packed weights of cell `c` into the scratch block, or in a large call those of every cell, once
+static int widen_weights(n2d2b_net* net, const CellRec& c, cudaStream_t s)
+{
+    const bool all = widen_all(net, net->call_batch);
+    if (all && net->call_widened) return 0;
+    std::vector<WidenJob> jobs;
+    for (const CellRec& x : net->cells) {
+        if (x.w8 == CellRec::W8_NONE || (!all && &x != &c)) continue;
+        WidenJob j;
+        j.packed = (const uint8_t*)x.d_weights;
+        j.dst = (int8_t*)net->d_w8 + x.w8_offset;
+        j.rows_src = x.geom.O;
+        j.ng_src = x.w8_ng_src;
+        j.rows = x.w8_rows;
+        j.ng_dst = x.w8_ng_dst;
+        j.words = (unsigned)((size_t)x.geom.kH * x.geom.kW * x.geom.C / 8);
+        jobs.push_back(j);
+    }
+    CUDA_TRY(launch_widen_int4(jobs.data(), (int)jobs.size(), s));
+    net->call_widened = all;
+    return 0;
+}
+
 // Runs one cell on images [img0, img0 + batch) of the batch (img0 != 0 only for cells without tensor maps).
 static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, cudaStream_t s, int img0 = 0)
 {
-    if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], batch)) return 0;   // computed by the cell that carries the sum
+    if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], batch, net->call_batch)) return 0;   // computed by the cell that carries the sum
     const void* in0 = tensor_ptr(net, c.inputs[0], d_input);
     void* out = tensor_ptr(net, c.output, d_input);
     const TensorRec& tin = net->tensors[c.inputs[0]];
@@ -1652,24 +1688,20 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
     // the maps and the loads of a residual start on 16 bytes; the network's input is the caller's buffer
     if (c.residual == 0 && mapped && ((uintptr_t)r.ptr & 15))
         return fail(N2D2B_ERR_INVALID, "a residual sum cannot read an input at %p: operands must be 16-byte aligned", r.ptr);
-    if (c.dual_branch >= 0 && use_dual(net, c, batch)) {
+    const bool dual = c.dual_branch >= 0 && use_dual(net, c, batch, net->call_batch), widened = use_widened(net, c, batch, net->call_batch);
+    if (widened) {
+        if (dual)
+            if (int rc = widen_weights(net, net->cells[c.dual_branch], s)) return rc;
+        if (int rc = widen_weights(net, c, s)) return rc;
+    }
+    if (dual) {
         const CellRec& a = net->cells[c.dual_branch];
-        if (a.plan.w4) {
-            size_t off = 0;
-            for (const CellRec* x : {&a, (const CellRec*)&c}) {
-                CUDA_TRY(launch_widen_int4((const uint8_t*)x->d_weights, x->geom.O, x->w8_ng_src, (int8_t*)net->d_w8 + off, x->w8_rows, 4,
-                                           (size_t)x->geom.kH * x->geom.kW * x->geom.C, s));
-                off += widened_bytes(*x);
-            }
-        }
         ConvGeom g = c.geom;
         g.B = batch;
         CUDA_TRY(launch_dual(c.dual, g, a.fast, c.fast, net->tensors[a.output].is_unsigned, img0 * g.oH * g.oW, a.plan.w4, net->d_status, s));
         return 0;
     }
-    if (use_widened(net, c, batch)) {
-        const size_t row_bytes = (size_t)c.geom.kH * c.geom.kW * c.geom.C;
-        CUDA_TRY(launch_widen_int4((const uint8_t*)c.d_weights, c.geom.O, c.w8_ng_src, (int8_t*)net->d_w8, c.w8_rows, c.w8_ng_dst, row_bytes, s));
+    if (widened) {
         ConvGeom g = c.geom;
         g.B = batch;
         if (c.w8 == CellRec::W8_PATCH) {
@@ -1816,6 +1848,10 @@ static int forward_impl(n2d2b_net* net, const void* d_input, int batch, void* d_
     if (!d_input) return fail(N2D2B_ERR_INVALID, "d_input must not be NULL");
     CUDA_TRY(cudaSetDevice(net->device));
     const bool one_kernel = net->d_small && first_cell == 0;
+    if (first_cell == 0) {   // (else the leading cells of the same call have run)
+        net->call_batch = batch;
+        net->call_widened = false;
+    }
     std::vector<cudaEvent_t> ev;
     if (ms) {
         if (nb_cells != (int)net->cells.size())
@@ -1942,6 +1978,8 @@ int n2d2b_net_forward_host(n2d2b_net* net, const void* h_input, int batch, void*
         CUDA_TRY(cudaEventRecord(net->stage_free, s));
         CUDA_TRY(cudaStreamWaitEvent(net->copy_stream, net->stage_free, 0));
         const size_t img_bytes = net->tensors[0].bytes_per_image();
+        net->call_batch = batch;
+        net->call_widened = false;
         for (int k = 0; k < nslices; ++k) {
             const int b0 = (int)((long long)batch * (2 * k) / wsum);
             const int b1 = k + 1 == nslices ? batch : (int)((long long)batch * (2 * k + 2) / wsum);
@@ -2146,10 +2184,10 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     if (!net || cell < 0 || cell >= (int)net->cells.size()) return "";
     if (net->d_small) return "small-net";
     const CellRec& c = net->cells[cell];
-    if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], net->max_batch)) return "fused";
-    if (c.dual_branch >= 0 && use_dual(net, c, net->max_batch)) return "tcgen05-dual";
+    if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], net->max_batch, net->max_batch)) return "fused";
+    if (c.dual_branch >= 0 && use_dual(net, c, net->max_batch, net->max_batch)) return "tcgen05-dual";
     if (use_dw3x3(c, net->max_batch)) return "depthwise";
-    if (use_widened(net, c, net->max_batch)) return c.w8 == CellRec::W8_PATCH ? "patch-tcgen05-widened" : "tcgen05-widened";
+    if (use_widened(net, c, net->max_batch, net->max_batch)) return c.w8 == CellRec::W8_PATCH ? "patch-tcgen05-widened" : "tcgen05-widened";
     switch (c.engine) {
     case ENG_TCGEN05: {
         const bool pair = c.plan.pair && c.fast.enabled && c.residual < 0
