@@ -174,7 +174,8 @@ template <bool IN_UNSIGNED, bool OUT_UNSIGNED, int S>
 static cudaError_t launch_depthwise3x3(dim3 grid, int threads, cudaStream_t s, const uint8_t* in, const int8_t* w, const ConvGeom& g,
                                        const FastQuant& f, uint8_t* out, const DwSplit& d)
 {
-    if (f.form == EF_WIDE) return launch_pdl(conv_depthwise3x3_kernel<IN_UNSIGNED, OUT_UNSIGNED, S, false, EF_WIDE>, grid, threads, 0, s, in, w, g, f.fq, f.cpad, out, d);
+    if (f.form == EF_WIDE) return launch_pdl(f.need_clamp ? conv_depthwise3x3_kernel<IN_UNSIGNED, OUT_UNSIGNED, S, true, EF_WIDE>
+                                                          : conv_depthwise3x3_kernel<IN_UNSIGNED, OUT_UNSIGNED, S, false, EF_WIDE>, grid, threads, 0, s, in, w, g, f.fq, f.cpad, out, d);
     if (f.form == EF_FLOAT) return launch_pdl(f.need_clamp ? conv_depthwise3x3_kernel<IN_UNSIGNED, OUT_UNSIGNED, S, true, EF_FLOAT>
                                                            : conv_depthwise3x3_kernel<IN_UNSIGNED, OUT_UNSIGNED, S, false, EF_FLOAT>,
                                               grid, threads, 0, s, in, w, g, f.fq, f.cpad, out, d);

@@ -41,6 +41,7 @@ static const DwPwKernel* kernels_for(const FastQuant& dw, const FastQuant& pw)
     static const DwPwKernel unit[2] = {dwpw_i8_tcgen05_kernel<1, DPF_UNIT, DPF_INT>, dwpw_i8_tcgen05_kernel<2, DPF_UNIT, DPF_INT>};
     static const DwPwKernel clamped[2] = {dwpw_i8_tcgen05_kernel<1, DPF_CLAMP, DPF_CLAMP>, dwpw_i8_tcgen05_kernel<2, DPF_CLAMP, DPF_CLAMP>};
     const int a = form_of(dw), b = form_of(pw);
+    if ((a == DPF_WIDE && dw.need_clamp) || (b == DPF_WIDE && pw.need_clamp)) return nullptr;
     if ((a == DPF_FLOAT) != (b == DPF_FLOAT)) return nullptr;
     if (a == DPF_FLOAT) return dwpw_float;
     if (a == DPF_WIDE) return b == DPF_WIDE ? dwpw_wide : dwpw_wide_depthwise;

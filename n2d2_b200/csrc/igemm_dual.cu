@@ -45,8 +45,8 @@ __device__ __forceinline__ void dual_drain_branch(const EpiTile& e, unsigned tba
     case EF_OUT_UNSIGNED: epi_drain<false, CLAMP, false, EF_OUT_UNSIGNED | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
     case EF_FLOAT: epi_drain<false, CLAMP, false, EF_FLOAT | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
     case EF_FLOAT | EF_OUT_UNSIGNED: epi_drain<false, CLAMP, false, EF_FLOAT | EF_OUT_UNSIGNED | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
-    case EF_WIDE: epi_drain<false, false, false, EF_WIDE | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
-    default: epi_drain<false, false, false, EF_WIDE | EF_OUT_UNSIGNED | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
+    case EF_WIDE: epi_drain<false, CLAMP, false, EF_WIDE | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
+    default: epi_drain<false, CLAMP, false, EF_WIDE | EF_OUT_UNSIGNED | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
     }
 }
 
@@ -68,7 +68,7 @@ __device__ __forceinline__ void dual_drain_sum(const EpiTile& e, unsigned tbase,
         }
         return;
     }
-#define N2D2B_DUAL_CASE(F, U) case (F) | (U): epi_drain<true, CLAMP && (F) != EF_WIDE, false, (F) | (U) | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
+#define N2D2B_DUAL_CASE(F, U) case (F) | (U): epi_drain<true, CLAMP, false, (F) | (U) | EF_PERM>(e, tbase, cbase, region_off, rb, lane); break;
     switch (ef & (EF_OUT_UNSIGNED | EF_RES_UNSIGNED | EF_WIDE | EF_FLOAT)) {
     N2D2B_DUAL_CASE(0, 0) N2D2B_DUAL_CASE(0, 1) N2D2B_DUAL_CASE(0, 2) N2D2B_DUAL_CASE(0, 3)
     N2D2B_DUAL_CASE(EF_FLOAT, 0) N2D2B_DUAL_CASE(EF_FLOAT, 1) N2D2B_DUAL_CASE(EF_FLOAT, 2) N2D2B_DUAL_CASE(EF_FLOAT, 3)

@@ -247,9 +247,9 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
                         case EF_OUT_UNSIGNED:
                             perm_block<4, false, CLAMP, false, EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
                             break;
-                        case EF_WIDE: perm_block<4, false, false, false, EF_WIDE | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
+                        case EF_WIDE: perm_block<4, false, CLAMP, false, EF_WIDE | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
                         case EF_WIDE | EF_OUT_UNSIGNED:
-                            perm_block<4, false, false, false, EF_WIDE | EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
+                            perm_block<4, false, CLAMP, false, EF_WIDE | EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
                             break;
                         case EF_FLOAT: perm_block<4, false, CLAMP, false, EF_FLOAT | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
                         default:
@@ -614,7 +614,9 @@ __device__ __forceinline__ int split_rescale(int x, int form, bool clamp, const 
         return clamp ? rescale<true, EF_FLOAT>(x, c[0], c[stride], c[2 * stride], c[3 * stride], c[4 * stride])
                      : rescale<false, EF_FLOAT>(x, 0, 0, c[2 * stride], c[3 * stride], c[4 * stride]);
     }
-    if (form == EF_WIDE) return rescale<false, EF_WIDE>(x, c[0], 0, c[2 * stride], c[3 * stride], c[4 * stride]);
+    if (form == EF_WIDE)
+        return clamp ? rescale<true, EF_WIDE>(x, c[0], c[stride], c[2 * stride], c[3 * stride], c[4 * stride])
+                     : rescale<false, EF_WIDE>(x, c[0], 0, c[2 * stride], c[3 * stride], c[4 * stride]);
     return clamp ? rescale<true, 0>(x, c[0], c[stride], c[2 * stride], c[3 * stride], c[4 * stride])
                  : rescale<false, 0>(x, 0, 0, c[2 * stride], c[3 * stride], c[4 * stride]);
 }

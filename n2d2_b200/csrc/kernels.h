@@ -82,7 +82,8 @@ struct FastQuant {
     int t_lo = 0, t_hi = 0;     // range the cell's own output saturates to
     int out_unsigned = 0;       // final 8-bit range
     bool need_clamp = true;     // false: no product can leave 32 bits and saturation is the final pack's
-    int form = 0;               // EF_WIDE: first rescale in 64 bits, row 0 of fq holds the upper words of the addends (no clamps);
+    int form = 0;               // EF_WIDE: first rescale in 64 bits, row 0 of fq holds the upper words of the addends, row 1 the bound
+                                // of the rescaled value (with need_clamp: values are clamped to [0, bound]);
                                 // EF_FLOAT: floating-point scaling (both stages of a residual cell); 0: the 32-bit form
     bool dp4a = false;          // residual stage as a byte dot product (multipliers <= 255, native 8-bit ranges)
     bool dp_t_unsigned = false; //   the cell's own output is packed as unsigned bytes (natively, or shifted by +128)

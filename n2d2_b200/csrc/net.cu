@@ -329,11 +329,14 @@ static long long ceil_div(long long a, long long b)  // b > 0
     return (a >= 0) ? (a + b - 1) / b : -((-a) / b);
 }
 
-// 64-bit form of the same rescale, for fixed-point scalings whose products leave 32 bits: no clamps (the final
-// pack saturates), so it applies when none is needed for other reasons; the shifted result must fit 32 bits.
-static bool build_wide_quant(const QuantHost& q, int cpad, long long x_bound, std::vector<int32_t>& out)
+// 64-bit form of the same rescale, for fixed-point scalings whose products leave 32 bits; the shifted result must fit 32 bits.  The final pack
+// saturates.  A clipping to [0, clip] and the ReLU of a signed output become a clamp of the rescaled value to [0, row 1] (`need_clamp`; callers
+// without one pass nullptr and are refused such cells): the rescale never decreases and gives 0 at 0.
+static bool build_wide_quant(const QuantHost& q, int cpad, long long x_bound, std::vector<int32_t>& out, bool* need_clamp = nullptr)
 {
-    if (q.is_clipped || (q.act == ACT_RECTIFIER && !q.out_unsigned) || q.act == ACT_SATURATION) return false;
+    const bool floor0 = q.is_clipped || (q.act == ACT_RECTIFIER && !q.out_unsigned);
+    if ((floor0 && !need_clamp) || q.act == ACT_SATURATION) return false;
+    if (floor0) *need_clamp = true;
     const int C = q.nb_channels;
     out.assign((size_t)5 * cpad, 0);
     for (int c = 0; c < C; ++c) {
@@ -348,6 +351,12 @@ static bool build_wide_quant(const QuantHost& q, int cpad, long long x_bound, st
         const long long add = b * m + half;                                   // < 2^62
         const long long worst = x_bound * m + std::llabs(add);               // < 2^62 for x_bound < 2^30
         if ((worst >> s) > (1ll << 31) - 2) return false;
+        long long top = q.out_unsigned ? 255 : 127;
+        if (q.is_clipped) {
+            if (!(q.clip_f[c] > 0.0f)) return false;
+            top = std::min(top, ((long long)q.clip_val[c] * m + half) >> s);
+        }
+        out[(size_t)1 * cpad + c] = (int32_t)top;
         out[(size_t)0 * cpad + c] = (int32_t)(add >> 32);
         out[(size_t)2 * cpad + c] = (int32_t)m;
         out[(size_t)3 * cpad + c] = (int32_t)(uint32_t)(add & 0xffffffffll);
@@ -477,7 +486,7 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
     // epilogue divides the sum by 16 again before anything else); the residual stage adds two 8-bit values
     const long long acc_bound = (long long)c.geom.kH * c.geom.kW * c.geom.Cg * 255ll * (w4 ? 8ll : 128ll);
     if (acc_bound * (w4 ? 16 : 1) > (1ll << 30)) return 0;
-    bool need_clamp = false, wide = false;
+    bool need_clamp = false, wide = false, wide_clamps = false;
     const bool with_res = c.residual >= 0;
     const bool flt = c.q.mode == SC_FLOAT_MULT;
     if (flt) {
@@ -492,15 +501,16 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
         if (c.q.out_bits != 8 || c.q.act == ACT_SATURATION
             || (c.q.mode != SC_SINGLE_SHIFT && c.q.mode != SC_DOUBLE_SHIFT && c.q.mode != SC_FIXED_MULT16
                 && c.q.mode != SC_FIXED_MULT32)
-            || !build_wide_quant(c.q, cpad, acc_bound, f1))
+            || !build_wide_quant(c.q, cpad, acc_bound, f1, &wide_clamps))
             return 0;
         wide = true;
+        need_clamp = wide_clamps;
         lo1 = c.q.out_unsigned ? 0 : -128;
         hi1 = c.q.out_unsigned ? 255 : 127;
         if (c.q.act == ACT_RECTIFIER && lo1 < 0) lo1 = 0;
     }
     if (with_res && !flt && !build_fast_quant(c.q2, cpad, 512, f2, &lo2, &hi2, &need_clamp)) return 0;
-    if (wide && need_clamp) return 0;   // the 64-bit form has no clamps
+    if (wide && need_clamp && !wide_clamps) return 0;   // the 64-bit form has the clamp at 0 or none
     // Dot-product form of the residual stage (see perm_block): every multiplier of the sum's scaling fits a byte,
     // both operands have a native 8-bit range and no clamp is needed.  The four bytes [t, t', r, r'] of a dot
     // product share one signedness: when the cell's own output is signed and the residual unsigned, the first

@@ -637,16 +637,16 @@ cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, 
     typedef void (*PatchKernel)(const CUtensorMap, const CUtensorMap, const PatchArgs);
 #define N2D2B_PATCH(C, F) patch_conv_tcgen05_kernel<C, 0, F, false>, patch_conv_tcgen05_kernel<C, 1, F, false>, \
                           patch_conv_tcgen05_kernel<C, 2, F, false>, patch_conv_tcgen05_kernel<C, 3, F, false>, patch_conv_tcgen05_kernel<C, 2, F, true>
-    static const PatchKernel variants[25] = {N2D2B_PATCH(false, 0), N2D2B_PATCH(true, 0), N2D2B_PATCH(false, EF_FLOAT),
-                                             N2D2B_PATCH(true, EF_FLOAT), N2D2B_PATCH(false, EF_WIDE)};   // the wide form has no clamps
+    static const PatchKernel variants[30] = {N2D2B_PATCH(false, 0), N2D2B_PATCH(true, 0), N2D2B_PATCH(false, EF_FLOAT),
+                                             N2D2B_PATCH(true, EF_FLOAT), N2D2B_PATCH(false, EF_WIDE), N2D2B_PATCH(true, EF_WIDE)};
 #undef N2D2B_PATCH
-    static SmemLimitSet limits[25];
+    static SmemLimitSet limits[30];
     // a multiple of the group count: CTA b works on group b % G
     const long long items = (long long)a.B * a.bands;
     const long long per_group = plan.num_sms / plan.G > 0 ? plan.num_sms / plan.G : 1;
     const int grid = (int)((items < per_group ? items : per_group) * plan.G);
     const int shape = r.ptr ? 4 : (g.kH == 3 && g.kW == 3 && !plan.b_stream) ? (g.C == 32 ? 1 : (g.C == 64 ? 2 : 3)) : 0;
-    const int v = (fast.form == EF_WIDE ? 20 : (fast.form == EF_FLOAT ? 10 : 0) + (fast.need_clamp ? 5 : 0)) + shape;
+    const int v = (fast.form == EF_WIDE ? 20 : (fast.form == EF_FLOAT ? 10 : 0)) + (fast.need_clamp ? 5 : 0) + shape;
     if (cudaError_t e = raise_smem_limit(variants[v], limits[v])) return e;
     return launch_pdl(variants[v], grid, r.ptr ? P_THREADS_RES : P_THREADS, plan.smem_bytes, s, plan.tmA, plan.tmB, a);
 }

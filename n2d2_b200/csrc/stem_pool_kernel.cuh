@@ -337,7 +337,7 @@ stem_pool_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const StemPool
 // (stem_pool_int.cu, stem_pool_float.cu, stem_pool_wide.cu): loading one takes time by its size, and a process rarely uses two.
 typedef void (*StemPoolKernel)(const CUtensorMap, const StemPoolArgs);
 extern const StemPoolKernel stem_pool_int[2][3][4], stem_pool_int_clamped[2][3][4], stem_pool_float[2][3][4], stem_pool_float_clamped[2][3][4],
-    stem_pool_wide[2][3][4];
+    stem_pool_wide[2][3][4], stem_pool_wide_clamped[2][3][4];
 #define N2D2B_SP0(S, C, F, R) {stem_pool_tcgen05_kernel<4, S, C, F, R>, stem_pool_tcgen05_kernel<6, S, C, F, R>, \
                                stem_pool_tcgen05_kernel<7, S, C, F, R>, stem_pool_tcgen05_kernel<8, S, C, F, R>}
 #define N2D2B_SP1(C, F, R) {N2D2B_SP0(0, C, F, R), N2D2B_SP0(1, C, F, R), N2D2B_SP0(2, C, F, R)}

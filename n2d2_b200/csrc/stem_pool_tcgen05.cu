@@ -144,10 +144,11 @@ cudaError_t launch_stem_pool(const StemPoolPlan& plan, const ConvGeom& g, int n_
     a.out_lo = fast.out_unsigned ? 0 : -128;
     a.out_hi = fast.out_unsigned ? 255 : 127;
     typedef const StemPoolKernel (*Table)[3][4];
-    static const Table forms[5] = {stem_pool_int, stem_pool_int_clamped, stem_pool_float, stem_pool_float_clamped, stem_pool_wide};
-    static SmemLimitSet limits[5][2][3][4];
+    static const Table forms[6] = {stem_pool_int, stem_pool_int_clamped, stem_pool_float, stem_pool_float_clamped, stem_pool_wide,
+                                    stem_pool_wide_clamped};
+    static SmemLimitSet limits[6][2][3][4];
     const int shape = plan.KH == 4 && plan.KWp == 4 ? 1 : (plan.KH == 2 && plan.KWp == 2 ? 2 : 0);
-    const int form = fast.form == EF_WIDE ? 4 : (fast.form == EF_FLOAT ? 2 : 0) + (fast.need_clamp ? 1 : 0);
+    const int form = (fast.form == EF_WIDE ? 4 : (fast.form == EF_FLOAT ? 2 : 0)) + (fast.need_clamp ? 1 : 0);
     const int per_lane = (plan.poW + 7) / 8, hp = per_lane <= 4 ? 0 : (per_lane <= 6 ? 1 : (per_lane <= 7 ? 2 : 3));
     const int grid = a.items < plan.num_sms ? a.items : plan.num_sms;
     const StemPoolKernel kernel = forms[form][raw ? 1 : 0][shape][hp];

@@ -359,12 +359,12 @@ stem_s2d_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const S2dArgs a
     }
 }
 
-// The kernels by [rescale: 32-bit, 32-bit with clamps, floating-point, the same with clamps, 64-bit (it has no clamps)][filter shape].
+// The kernels by [rescale: 32-bit, 32-bit with clamps, floating-point, the same with clamps, 64-bit, the same with clamps][filter shape].
 // Those with the pooling of bytes, which run on request only, are an object of their own (stem_s2d_pool.cu).
 typedef void (*StemS2dKernel)(const CUtensorMap, const S2dArgs);
-extern const StemS2dKernel stem_s2d_pool_kernels[5][3];
+extern const StemS2dKernel stem_s2d_pool_kernels[6][3];
 #define N2D2B_S2D(C, P, F) {stem_s2d_tcgen05_kernel<C, 0, P, F>, stem_s2d_tcgen05_kernel<C, 1, P, F>, stem_s2d_tcgen05_kernel<C, 2, P, F>}
 #define N2D2B_STEM_S2D_KERNELS(P) {N2D2B_S2D(false, P, 0), N2D2B_S2D(true, P, 0), N2D2B_S2D(false, P, EF_FLOAT), \
-                                   N2D2B_S2D(true, P, EF_FLOAT), N2D2B_S2D(false, P, EF_WIDE)}
+                                   N2D2B_S2D(true, P, EF_FLOAT), N2D2B_S2D(false, P, EF_WIDE), N2D2B_S2D(true, P, EF_WIDE)}
 
 }  // namespace n2d2b

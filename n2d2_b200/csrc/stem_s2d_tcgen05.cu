@@ -399,12 +399,12 @@ cudaError_t launch_stem_s2d(const StemS2dPlan& plan, const ConvGeom& g, int n_ba
     a.fq = fast.fq;
     a.cpad = fast.cpad;
     a.out_unsigned = fast.out_unsigned;
-    static const StemS2dKernel kernels[5][3] = N2D2B_STEM_S2D_KERNELS(false);
+    static const StemS2dKernel kernels[6][3] = N2D2B_STEM_S2D_KERNELS(false);
     static SmemLimitSet limits[2][5][3];
     const long long items = (long long)a.B * a.bands;
     const int grid = (int)(items < plan.num_sms ? items : plan.num_sms);
     const int shape = (plan.KH == 4 && plan.KWp == 4) ? 1 : ((plan.KH == 2 && plan.KWp == 2) ? 2 : 0);
-    const int form = fast.form == EF_WIDE ? 4 : (fast.form == EF_FLOAT ? 2 : 0) + (fast.need_clamp ? 1 : 0), pool = plan.P ? 1 : 0;
+    const int form = (fast.form == EF_WIDE ? 4 : (fast.form == EF_FLOAT ? 2 : 0)) + (fast.need_clamp ? 1 : 0), pool = plan.P ? 1 : 0;
     const StemS2dKernel kernel = (pool ? stem_s2d_pool_kernels : kernels)[form][shape];
     if (cudaError_t e = raise_smem_limit(kernel, limits[pool][form][shape])) return e;
     return launch_pdl(kernel, grid, Z_THREADS, plan.smem_bytes, s, plan.tmA, a);

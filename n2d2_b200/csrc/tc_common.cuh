@@ -474,14 +474,15 @@ __device__ __forceinline__ int rescale(int x, int lo, int hi, int mult, int add,
         if (CLAMP) f = fminf(fmaxf(f, __int_as_float(lo)), __int_as_float(hi));
         return float_round_scaled(f, __int_as_float(mult));
     }
-    if (CLAMP) x = min(max(x, lo), hi);
     if (EF & EF_WIDE) {
         // fixed-point scalings with many fractional bits: the product needs more than 32 bits, the shifted result does not
-        // (proved on the host, as is shift <= 31: the low word of the shifted pair is one funnel shift); no clamps in this
-        // form, the pack saturates
+        // (proved on the host, as is shift <= 31: the low word of the shifted pair is one funnel shift).  A clipping to [0, clip] before
+        // the rescale is one to [0, its value at clip] behind it (it never decreases, and is 0 at 0): hi; else the pack saturates
         const long long p = (long long)x * mult + (long long)(((unsigned long long)(unsigned)lo << 32) | (unsigned)add);
-        return (int)__funnelshift_r((unsigned)p, (unsigned)((unsigned long long)p >> 32), (unsigned)shift);
+        const int y = (int)__funnelshift_r((unsigned)p, (unsigned)((unsigned long long)p >> 32), (unsigned)shift);
+        return CLAMP ? min(max(y, 0), hi) : y;
     }
+    if (CLAMP) x = min(max(x, lo), hi);
     return (x * mult + add) >> shift;
 }
 
@@ -897,10 +898,10 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
             switch (e.ef & (EF_OUT_UNSIGNED | EF_WIDE | EF_FLOAT)) {
             case 0: epi_drain_direct<CLAMP, 0>(e, tbase, cbase, out, rowoff, rowok, lane); break;
             case EF_OUT_UNSIGNED: epi_drain_direct<CLAMP, EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
-            case EF_WIDE: epi_drain_direct<false, EF_WIDE>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_WIDE: epi_drain_direct<CLAMP, EF_WIDE>(e, tbase, cbase, out, rowoff, rowok, lane); break;
             case EF_FLOAT: epi_drain_direct<CLAMP, EF_FLOAT>(e, tbase, cbase, out, rowoff, rowok, lane); break;
             case EF_FLOAT | EF_OUT_UNSIGNED: epi_drain_direct<CLAMP, EF_FLOAT | EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
-            default: epi_drain_direct<false, EF_WIDE | EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            default: epi_drain_direct<CLAMP, EF_WIDE | EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
             }
         }
         tc_fence_before();
@@ -930,10 +931,10 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
             switch (e.ef & (EF_OUT_UNSIGNED | EF_WIDE | EF_FLOAT)) {
             case 0: epi_drain<RES, CLAMP, DP, (0) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_OUT_UNSIGNED: epi_drain<RES, CLAMP, DP, (EF_OUT_UNSIGNED) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
-            case EF_WIDE: epi_drain<RES, false, DP, (EF_WIDE) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_WIDE: epi_drain<RES, CLAMP, DP, (EF_WIDE) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_FLOAT: epi_drain<RES, CLAMP, DP, (EF_FLOAT) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_FLOAT | EF_OUT_UNSIGNED: epi_drain<RES, CLAMP, DP, (EF_FLOAT | EF_OUT_UNSIGNED) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
-            default: epi_drain<RES, false, DP, (EF_WIDE | EF_OUT_UNSIGNED) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            default: epi_drain<RES, CLAMP, DP, (EF_WIDE | EF_OUT_UNSIGNED) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             }
         } else if (!DP) {
             switch (e.ef & (EF_OUT_UNSIGNED | EF_RES_UNSIGNED | EF_WIDE | EF_FLOAT)) {
@@ -945,10 +946,10 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
             case EF_FLOAT | 1: epi_drain<RES, CLAMP, DP, (EF_FLOAT | 1) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_FLOAT | 2: epi_drain<RES, CLAMP, DP, (EF_FLOAT | 2) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             case EF_FLOAT | 3: epi_drain<RES, CLAMP, DP, (EF_FLOAT | 3) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
-            case EF_WIDE | 0: epi_drain<RES, false, DP, (EF_WIDE | 0) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
-            case EF_WIDE | 1: epi_drain<RES, false, DP, (EF_WIDE | 1) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
-            case EF_WIDE | 2: epi_drain<RES, false, DP, (EF_WIDE | 2) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
-            default: epi_drain<RES, false, DP, (EF_WIDE | 3) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_WIDE | 0: epi_drain<RES, CLAMP, DP, (EF_WIDE | 0) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_WIDE | 1: epi_drain<RES, CLAMP, DP, (EF_WIDE | 1) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            case EF_WIDE | 2: epi_drain<RES, CLAMP, DP, (EF_WIDE | 2) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
+            default: epi_drain<RES, CLAMP, DP, (EF_WIDE | 3) | P>(e, tbase, cbase, region_off, st.rb, lane); break;
             }
         } else {
             switch (e.ef & (EF_OUT_UNSIGNED | EF_T_UNSIGNED | EF_DP_A_SIGNED)) {
