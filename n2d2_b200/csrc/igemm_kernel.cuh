@@ -60,6 +60,7 @@ struct IgemmArgs {
     unsigned tmem_cols;
     int out_dtype;
     void* out;
+    int ldo;             // stores from the registers: bytes of an output row (N of them wanted)
     int* status;
     QuantDev q;
     Residual r;
@@ -455,7 +456,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                 // fragment-layout epilogue with swizzled staging, TMA store and TMA residual load
                 EpiTile e;
                 e.tmem_acc = tmem_base + as * (unsigned)a.BN;
-                e.BN = a.BN; e.N = a.N; e.M = a.m_base + a.M; e.m0 = m0; e.n0 = n0; e.out = (uint8_t*)a.out;
+                e.BN = a.BN; e.N = a.N; e.M = a.m_base + a.M; e.m0 = m0; e.n0 = n0; e.out = (uint8_t*)a.out; e.ldo = a.ldo;
                 e.wp = wp;
                 e.par_off = (unsigned)((unsigned char*)par - smem_raw);
                 e.region_off = my_regions;

@@ -905,10 +905,32 @@ void igemm_permute_weights(const int8_t* w, int8_t* dst, int N, size_t row_bytes
     for (int n = 0; n < N; ++n) memcpy(dst + (size_t)n * row_bytes, w + (size_t)perm_real_channel(n, ng) * row_bytes, row_bytes);
 }
 
+// Tiles of a launch, and its CTAs: a multiple of the number of column blocks keeps every CTA on one, whose constants are staged once
+static void igemm_grid(const IgemmPlan& plan, int* tiles, int* grid)
+{
+    const int num_n_tiles = (plan.N + plan.BN - 1) / plan.BN;
+    *tiles = (plan.M + BM - 1) / BM * num_n_tiles;
+    *grid = std::min(plan.grid, *tiles);
+    if (*tiles > *grid && num_n_tiles > 1 && *grid > num_n_tiles) *grid -= *grid % num_n_tiles;
+}
+
+// A launch of up to two tiles per CTA has the variant that stores from the registers (see DRY)
+static bool igemm_short(int tiles, int grid) { return tiles <= 2 * grid; }
+
+bool igemm_writes_rows(const IgemmPlan& plan, int columns)
+{
+    int tiles, grid;
+    igemm_grid(plan, &tiles, &grid);
+    const int num_kb = plan.taps * ((plan.Cin + plan.BK - 1) / plan.BK);
+    return plan.perm && !plan.w4 && !plan.grouped && !plan.pair && plan.BN / plan.parts >= 32 && columns % 8 == 0 && igemm_short(tiles, grid)
+        && !(plan.BN == SPLIT_BN && igemm_split(tiles, num_kb, plan.num_sms));
+}
+
 cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residual& r, const FastQuant& fast, void* out,
-                         int out_dtype, int m_base, int* status_word, cudaStream_t s)
+                         int out_dtype, int m_base, int* status_word, cudaStream_t s, void* rows, int columns)
 {
     if (plan.M == 0 || plan.N == 0) return cudaSuccess;
+    if (rows && (r.ptr || !igemm_writes_rows(plan, columns))) return cudaErrorInvalidConfiguration;
     IgemmArgs a;
     memset(&a, 0, sizeof(a));
     a.m_base = m_base;
@@ -933,6 +955,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     a.groups = 4 / plan.parts;
     a.out_dtype = out_dtype;
     a.out = out;
+    a.ldo = plan.N;
     a.status = status_word;
     a.q = q;
     a.r = r;
@@ -956,7 +979,8 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
         {igemm_i8_tcgen05_kernel<0, false, false>, igemm_i8_tcgen05_kernel<1, false, true>, igemm_i8_tcgen05_kernel<2, false, true>,
          igemm_i8_tcgen05_kernel<3, false, true>, igemm_i8_tcgen05_kernel<4, false, true>, igemm_i8_tcgen05_kernel<5, false, true>}};
     static SmemLimitSet limits[3][6];
-    int tiles = a.num_m_tiles * a.num_n_tiles;
+    int tiles, grid;
+    igemm_grid(plan, &tiles, &grid);
     // Few tiles, long K: a cluster of CTAs per tile
     const int num_kb = plan.taps * ((plan.Cin + plan.BK - 1) / plan.BK);
     if (use_fast && !plan.w4 && !plan.grouped && plan.BN == SPLIT_BN && igemm_split(tiles, num_kb, plan.num_sms)) {
@@ -985,11 +1009,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
         cfg.numAttrs = 2;
         return cudaLaunchKernelEx(&cfg, igemm_split_tcgen05_kernel, plan.tmA, plan.tmB, sa);
     }
-    int grid = plan.grid < tiles ? plan.grid : tiles;
-    // a grid that is a multiple of the number of column blocks keeps every CTA on one column block,
-    // so its per-channel constants are staged once
-    if (tiles > grid && a.num_n_tiles > 1 && grid > a.num_n_tiles) grid -= grid % a.num_n_tiles;
-    // resident weights rely on exactly that (or on one tile per CTA)
+    // resident weights rely on a column block that does not change (or on one tile per CTA)
     if (a.b_resident && tiles > grid && a.num_n_tiles > 1 && grid % a.num_n_tiles != 0) return cudaErrorInvalidConfiguration;
     auto pixels = [&](long long m) {
         PixelStep d;
@@ -1019,7 +1039,11 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
                               plan.tmB, plan.tmO32, a);
         }
     }
-    const int table = plan.w4 ? 2 : (tiles <= 2 * grid ? 1 : 0);
+    const int table = plan.w4 ? 2 : (igemm_short(tiles, grid) ? 1 : 0);
+    if (rows) {
+        a.N = a.ldo = columns;
+        a.out = rows;
+    }
     const IgemmKernel kernel = plan.w4 ? igemm_w4_kernels[mode] : kernels[table][mode];
     if (cudaError_t e = raise_smem_limit(kernel, limits[table][mode])) return e;
     return launch_pdl(kernel, grid, NUM_THREADS + (plan.w4 ? 32 * W4_UNPACK_WARPS : 0), plan.smem_bytes, s,

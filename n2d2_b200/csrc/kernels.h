@@ -264,8 +264,11 @@ int igemm_perm_block(const IgemmPlan& plan);
 void igemm_permute_weights(const int8_t* w, int8_t* dst, int N, size_t row_bytes, int perm_block);
 // m_base: first output row (pixel) of this call within the tensors the plan was encoded for; `out` and the
 // residual stay the tensors' base pointers
+// rows: where the output's rows go instead, stored from the registers without the columns the plan was padded with (only where igemm_writes_rows)
 cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residual& r, const FastQuant& fast,
-                         void* out, int out_dtype, int m_base, int* status_word, cudaStream_t s);
+                         void* out, int out_dtype, int m_base, int* status_word, cudaStream_t s, void* rows = nullptr, int columns = 0);
+// Whether a launch of plan.M rows stores from the registers and so may write rows of `columns` bytes
+bool igemm_writes_rows(const IgemmPlan& plan, int columns);
 
 // ---- two convolutions and the sum of their outputs (igemm_dual.cu) ----
 struct DualPlan {

@@ -1127,7 +1127,7 @@ static int plan_widened(n2d2b_net* net)
     const bool all = widen_all(net, net->max_batch);
     if (all) net->launches++;
     for (const CellRec& c : net->cells)
-        if (use_widened(net, c, net->max_batch, net->max_batch)) net->launches += (all ? 0 : 1) + (c.d_w8_out ? 1 : 0);
+        if (use_widened(net, c, net->max_batch, net->max_batch)) net->launches += (all ? 0 : 1) + (c.d_w8_out && !igemm_writes_rows(c.plan8, c.geom.O) ? 1 : 0);
     return 0;
 }
 
@@ -1416,7 +1416,6 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 gplan.O = c.pad_O;
                 laid.resize((size_t)c.pad_O * g.kH * g.kW * g.Cg, 0);
                 CUDA_TRY(cudaMalloc(&c.d_colpad, (size_t)max_batch * g.oH * g.oW * c.pad_O + 256));
-                net->launches++;
             }
         }
         c.d_weight_bytes = w4 ? laid.size() / 2 : laid.size();
@@ -1485,6 +1484,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                         igemm_permute_weights(laid.data(), rows.data(), gplan.O, (size_t)g.kH * g.kW * g.Cg, pb);
                         c.plan.perm = pb;
                     }
+                    if (c.pad_O && !igemm_writes_rows(c.plan, g.O)) net->launches++;   // the copy that drops the padding
                     if (w4) rows = pack4(rows);
                     CUDA_TRY(cudaMemcpy(c.d_weights, rows.data(), rows.size(), cudaMemcpyHostToDevice));
                 }
@@ -1671,6 +1671,22 @@ static int widen_weights(n2d2b_net* net, const CellRec& c, cudaStream_t s)
     return 0;
 }
 
+// The implicit GEMM of a cell, and where its columns were padded (into `padded`) its output in place: short launches store the wanted columns from
+// the registers, others leave them to a copy kernel
+static int run_igemm(n2d2b_net* net, const CellRec& c, IgemmPlan p, const Residual& r, void* padded, void* out, int out_dtype, int batch, int img0, cudaStream_t s)
+{
+    const ConvGeom& g = c.geom;
+    p.M = batch * g.oH * g.oW;
+    const size_t row0 = (size_t)img0 * g.oH * g.oW;
+    if (padded && !img0 && igemm_writes_rows(p, g.O)) {
+        CUDA_TRY(launch_igemm(p, c.q.dev, r, c.fast, padded, out_dtype, 0, net->d_status, s, out, g.O));
+        return 0;
+    }
+    CUDA_TRY(launch_igemm(p, c.q.dev, r, c.fast, padded ? padded : out, out_dtype, (int)row0, net->d_status, s));
+    if (padded) CUDA_TRY(launch_drop_padded_columns((const uint8_t*)padded + row0 * p.N, p.N, (uint8_t*)out + row0 * g.O, g.O, (size_t)p.M, s));
+    return 0;
+}
+
 // Runs one cell on images [img0, img0 + batch) of the batch (img0 != 0 only for cells without tensor maps).
 static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, cudaStream_t s, int img0 = 0)
 {
@@ -1719,13 +1735,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
             CUDA_TRY(launch_patch(c.patch8, g, img0, r, c.fast, out, net->d_status, s));
             return 0;
         }
-        IgemmPlan p = c.plan8;
-        p.M = batch * g.oH * g.oW;
-        const size_t row0 = (size_t)img0 * g.oH * g.oW;
-        CUDA_TRY(launch_igemm(p, c.q.dev, r, c.fast, c.d_w8_out ? c.d_w8_out : out, DT_I8, (int)row0, net->d_status, s));
-        if (c.d_w8_out)
-            CUDA_TRY(launch_drop_padded_columns((const uint8_t*)c.d_w8_out + row0 * c.w8_rows, c.w8_rows, (uint8_t*)out + row0 * g.O, g.O, (size_t)p.M, s));
-        return 0;
+        return run_igemm(net, c, c.plan8, r, c.d_w8_out, out, DT_I8, batch, img0, s);
     }
     if ((c.engine == ENG_DEPTHWISE || c.d_dw3x3) && !depthwise_takes(net, c, batch, in0))
         return fail(N2D2B_ERR_INVALID, "a depthwise cell cannot read an input at %p: operands must be 16-byte aligned", in0);
@@ -1738,7 +1748,6 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
     }
     switch (c.engine) {
     case ENG_TCGEN05: {
-        void* const gemm_out = c.pad_O ? c.d_colpad : out;
         // tensors of the caller: their address and the images of this call
         const void* const caller_in = c.inputs[0] == 0 ? in0 : nullptr;
         const void* const caller_res = c.residual == 0 ? r.ptr : nullptr;
@@ -1753,15 +1762,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
             c.plan_res = caller_res;
             c.plan_images = gb.B;
         }
-        IgemmPlan p = c.plan;
-        p.M = batch * c.geom.oH * c.geom.oW;
-        CUDA_TRY(launch_igemm(p, c.q.dev, r, c.fast, gemm_out, tout.dtype, img0 * c.geom.oH * c.geom.oW, net->d_status, s));
-        if (c.pad_O) {
-            const size_t row0 = (size_t)img0 * c.geom.oH * c.geom.oW;
-            CUDA_TRY(launch_drop_padded_columns((const uint8_t*)c.d_colpad + row0 * c.pad_O, c.pad_O,
-                                                (uint8_t*)out + row0 * c.geom.O, c.geom.O, (size_t)p.M, s));
-        }
-        break;
+        return run_igemm(net, c, c.plan, r, c.d_colpad, out, tout.dtype, batch, img0, s);
     }
     case ENG_PATCH: {
         if (c.plan_input != in0) {

@@ -796,7 +796,8 @@ __device__ __forceinline__ void perm_block_global(const unsigned* vA, const unsi
 struct EpiTile {
     unsigned tmem_acc;      // TMEM address of the accumulator stage (lane 0, first column)
     int BN, N, M, m0, n0;
-    uint8_t* out;           // the output matrix [M][N]
+    uint8_t* out;           // the output matrix [M][N]; stores from the registers: rows of ldo bytes, N of them wanted (a multiple of 8)
+    int ldo;
     int wp;                 // columns per warp: BN / (epilogue warps per TMEM quadrant); 64, 32 or 16
     unsigned par_off;       // staged per-channel constants of this column block (byte offset in dynamic shared memory)
     unsigned region_off;    // this warp's staging region(s) (1024-byte aligned; byte offset in dynamic shared memory)
@@ -858,15 +859,15 @@ __device__ __forceinline__ void epi_issue_residual(const CUtensorMap* tmR, unsig
     }
 }
 
-// The tile's columns of one warp straight to global memory (32-column blocks)
-template <bool CLAMP, int EF>
+// The tile's columns of one warp straight to global memory (32-column blocks, eight columns per lane).  PART: the last block may be wanted in part
+template <bool CLAMP, int EF, bool PART = false>
 __device__ __forceinline__ void epi_drain_direct(const EpiTile& e, unsigned tbase, int cbase, uint8_t* out, const unsigned (&rowoff)[4], unsigned rowok, int lane)
 {
 #pragma unroll 1
     for (int cb = 0; cb < e.wp; cb += 32) {
         unsigned va[16], vb[16];
         tc_ld_2x16x256b_x4_wait(tbase + (unsigned)cb, va, vb);
-        perm_block_global<CLAMP, EF>(va, vb, e.par_off, cbase + cb, out + cb, rowoff, e.n0 + cbase + cb < e.N ? rowok : 0u, lane);
+        perm_block_global<CLAMP, EF>(va, vb, e.par_off, cbase + cb, out + cb, rowoff, e.n0 + cbase + cb + (PART ? 8 * (lane & 3) : 0) < e.N ? rowok : 0u, lane);
     }
 }
 
@@ -887,21 +888,21 @@ __device__ __forceinline__ bool fast_epilogue_tile(const CUtensorMap* tmO, const
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int row = (lane >> 2) + 8 * k;
-            rowoff[k] = (unsigned)row * (unsigned)e.N;
+            rowoff[k] = (unsigned)row * (unsigned)e.ldo;
             if (gy + row < e.M && !e.dry) rowok |= 1u << k;
         }
-        uint8_t* const out = e.out + (size_t)gy * e.N + gx;
+        uint8_t* const out = e.out + (size_t)gy * e.ldo + gx;
         if (!e.dry && !mbar_wait_warp(e.tfull, e.tfull_parity, e.abort_flag, e.status, 4)) return false;
         tc_fence_after();
         if (active) {
             const unsigned tbase = e.tmem_acc + ((unsigned)(quad * 32) << 16) + (unsigned)cbase;
             switch (e.ef & (EF_OUT_UNSIGNED | EF_WIDE | EF_FLOAT)) {
-            case 0: epi_drain_direct<CLAMP, 0>(e, tbase, cbase, out, rowoff, rowok, lane); break;
-            case EF_OUT_UNSIGNED: epi_drain_direct<CLAMP, EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
-            case EF_WIDE: epi_drain_direct<CLAMP, EF_WIDE>(e, tbase, cbase, out, rowoff, rowok, lane); break;
-            case EF_FLOAT: epi_drain_direct<CLAMP, EF_FLOAT>(e, tbase, cbase, out, rowoff, rowok, lane); break;
-            case EF_FLOAT | EF_OUT_UNSIGNED: epi_drain_direct<CLAMP, EF_FLOAT | EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
-            default: epi_drain_direct<CLAMP, EF_WIDE | EF_OUT_UNSIGNED>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case 0: epi_drain_direct<CLAMP, 0, true>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_OUT_UNSIGNED: epi_drain_direct<CLAMP, EF_OUT_UNSIGNED, true>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_WIDE: epi_drain_direct<CLAMP, EF_WIDE, true>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_FLOAT: epi_drain_direct<CLAMP, EF_FLOAT, true>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            case EF_FLOAT | EF_OUT_UNSIGNED: epi_drain_direct<CLAMP, EF_FLOAT | EF_OUT_UNSIGNED, true>(e, tbase, cbase, out, rowoff, rowok, lane); break;
+            default: epi_drain_direct<CLAMP, EF_WIDE | EF_OUT_UNSIGNED, true>(e, tbase, cbase, out, rowoff, rowok, lane); break;
             }
         }
         tc_fence_before();
