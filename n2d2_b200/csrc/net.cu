@@ -1052,6 +1052,16 @@ static int final_tensor_of(const n2d2b_net* net)
     return -1;
 }
 
+// Whether a patch cell whose weights stream (128 channels) runs as an implicit GEMM in a call of `batch` images: up to one tile per SM.  A band then has few
+// tiles to share the stream of all its weights, which the implicit GEMM loads ahead, tile by tile (3x3, 128 channels of 28 x 28 in ResNet-50, the
+// whole network: one image 240 us -> 233, 8 images 301 / 298, 16 images 344 / 340; 32 images, two tiles per SM, 424 / 427).
+static bool patch_as_gemm(const n2d2b_net* net, const CellRec& c, int batch)
+{
+    if (c.engine != ENG_PATCH || c.inputs[0] == 0 || c.residual >= 0 || c.geom.groups != 1 || !c.patch.b_stream || c.plan.perm != 32) return false;
+    const long long m_tiles = ((long long)batch * c.geom.oH * c.geom.oW + 127) / 128;
+    return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) <= net->num_sms;
+}
+
 // Whether a call of `call` images widens the packed weights of all cells at its start, in one launch of 3 to 4 us.  The line is drawn where a call is large
 // enough to pay for it whatever its cells are (ResNet-18 at 224 x 224, 1.7 G multiply-accumulates an image: four images 217 us with the expansion in the
 // kernels, 182 widened cell by cell, 162 in one launch; 128 images 656 / 460 / 421: the expansion warps' shared-memory stores bound every layer of long
@@ -1474,6 +1484,8 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 const bool permute = c.engine == ENG_TCGEN05
                                      && igemm_uses_fast_epilogue(c.plan, c.fast, c.residual >= 0, net->tensors[c.output].dtype);
                 if (c.engine == ENG_PATCH) {
+                    // (the same order of rows as the implicit GEMM's, which small calls may take: patch_as_gemm)
+                    if (igemm_uses_fast_epilogue(c.plan, c.fast, c.residual >= 0, DT_I8) && igemm_perm_block(c.plan) == 32) c.plan.perm = 32;
                     std::vector<int8_t> rows(laid.size());
                     patch_permute_weights(laid.data(), rows.data(), g.O, (size_t)g.kH * g.kW * g.Cg);
                     CUDA_TRY(cudaMemcpy(c.d_weights, rows.data(), rows.size(), cudaMemcpyHostToDevice));
@@ -1765,6 +1777,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         return run_igemm(net, c, c.plan, r, c.d_colpad, out, tout.dtype, batch, img0, s);
     }
     case ENG_PATCH: {
+        if (patch_as_gemm(net, c, batch)) return run_igemm(net, c, c.plan, r, nullptr, out, tout.dtype, batch, img0, s);
         if (c.plan_input != in0) {
             ConvGeom gb = c.geom;
             gb.B = net->max_batch;
@@ -2214,7 +2227,9 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     case ENG_STEM: return "stem-tcgen05";
     case ENG_STEM_S2D: return c.pool_fused ? "stem-pool-tcgen05" : "stem-tcgen05";
     case ENG_DWPW: return "depthwise-1x1-tcgen05";
-    case ENG_PATCH: return c.geom.groups > 1 ? "depthwise-tcgen05" : "patch-tcgen05";
+    case ENG_PATCH:
+        if (patch_as_gemm(net, c, net->max_batch)) return "tcgen05";
+        return c.geom.groups > 1 ? "depthwise-tcgen05" : "patch-tcgen05";
     }
     return "";
 }
