@@ -171,6 +171,9 @@ struct PatchPlan {
     int num_sms;
     int late_weights;     // the weights are the previous kernel's output (see IgemmPlan)
     int G;                // channel groups: 1, or the block-diagonal groups of a depthwise layer
+    const void* proj_in;  // a 1x1 projection of this tensor beside the layer, and their sum (patch_add_projection); nullptr: none
+    CUtensorMap tmA2, tmB2;
+    int proj_unsigned, proj_alloc, proj_bytes;
     int band_batch;       // images the band height was chosen for
     const void* in;       // the activations (max_batch images)
     int max_batch;
@@ -191,7 +194,10 @@ int patch_make_plan(PatchPlan* plan, const void* in, const int8_t* w, const Conv
 // n_base: first image of this call within the tensors the plan was encoded for (`out` = the tensor's base)
 bool patch_takes_residual(const ConvGeom& g);
 cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g, int n_base, const Residual& r, const FastQuant& fast, void* out,
-                         int* status_word, cudaStream_t s);
+                         int* status_word, cudaStream_t s, const FastQuant* branch = nullptr);
+// Whether the kernel computes the projection `p` beside the layer `g` and the sum of both; adds it to the layer's plan (max_batch images of `in`)
+bool patch_takes_projection(const ConvGeom& g, const ConvGeom& p);
+int patch_add_projection(PatchPlan* plan, const void* in, const int8_t* w, const ConvGeom& g, int in_unsigned, const char** why);
 
 // ---- 3x3 depthwise layer and the 1x1 layer behind it (dwpw_tcgen05.cu) ----
 struct DwPwPlan {

@@ -121,6 +121,7 @@ struct CellRec {
     int dual_branch = -1, dual_sum = -1;
     bool dual_on = false;
     DualPlan dual{};
+    PatchPlan dual_patch{};   // or by the patch kernel (proj_in set)
     // tensor-core plan
     IgemmPlan plan{};
     bool has_plan = false;
@@ -1162,9 +1163,6 @@ static int plan_duals(n2d2b_net* net)
         if (packed ? (a.w8 == CellRec::W8_NONE || b.w8 == CellRec::W8_NONE || a.d_w8_out || b.d_w8_out || a.w8_ng_dst != 4 || b.w8_ng_dst != 4)
                    : (b.plan.perm != 32 || (a.engine == ENG_TCGEN05 && a.plan.perm != 32)))
             continue;
-        // The patch kernel reads a 64-channel branch's input once, an im2col map nine times: 64 -> 64 channels of 55 x 55 with its projection at 2048 images
-        // 596 us as two kernels, 718 as one; 128 channels of 28 x 28 400 / 290
-        if ((a.engine == ENG_PATCH || a.w8 == CellRec::W8_PATCH) && a.geom.C <= 64) continue;
         // (slices of the upload: both or neither)
         if ((b.dual_branch < net->head_cells) != ((int)bi < net->head_cells)) continue;
         ConvGeom ga = a.geom, gb = b.geom;
@@ -1172,7 +1170,18 @@ static int plan_duals(n2d2b_net* net)
         const int8_t* wa = packed ? (const int8_t*)net->d_w8 + a.w8_offset : a.d_weights;
         const int8_t* wb = packed ? (const int8_t*)net->d_w8 + b.w8_offset : b.d_weights;
         const char* why = "";
-        if (dual_make_plan(&b.dual, tensor_ptr(net, a.inputs[0], nullptr), wa, ga, net->tensors[a.inputs[0]].is_unsigned, tensor_ptr(net, b.inputs[0], nullptr), wb,
+        // The patch kernel reads a 64-channel branch's input once, an im2col map nine times: 64 -> 64 channels of 55 x 55 with its projection at 2048 images
+        // 596 us as two kernels, 718 as one of im2col loads; 128 channels of 28 x 28 400 / 290
+        if ((a.engine == ENG_PATCH || a.w8 == CellRec::W8_PATCH) && ga.C <= 64) {
+            // (a wide form's clamp is one at 0: both rescales have it or neither)
+            if (!patch_takes_projection(ga, gb) || b.fast.dp4a || a.fast.form != b.fast.form || (a.fast.form == EF_WIDE && a.fast.need_clamp != b.fast.need_clamp)) continue;
+            if (patch_make_plan(&b.dual_patch, tensor_ptr(net, a.inputs[0], nullptr), wa, ga, net->tensors[a.inputs[0]].is_unsigned, net->num_sms, &why)
+                || patch_add_projection(&b.dual_patch, tensor_ptr(net, b.inputs[0], nullptr), wb, ga, net->tensors[b.inputs[0]].is_unsigned, &why)) {
+                b.dual_patch.proj_in = nullptr;
+                continue;
+            }
+            b.dual_patch.late_weights = packed ? 1 : 0;
+        } else if (dual_make_plan(&b.dual, tensor_ptr(net, a.inputs[0], nullptr), wa, ga, net->tensors[a.inputs[0]].is_unsigned, tensor_ptr(net, b.inputs[0], nullptr), wb,
                            gb, net->tensors[b.inputs[0]].is_unsigned, tensor_ptr(net, b.output, nullptr), net->num_sms, &why))
             continue;
         b.dual_on = true;
@@ -1736,6 +1745,15 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
         const CellRec& a = net->cells[c.dual_branch];
         ConvGeom g = c.geom;
         g.B = batch;
+        if (c.dual_patch.proj_in) {
+            Residual branch{};
+            branch.is_unsigned = net->tensors[a.output].is_unsigned;
+            ConvGeom ga = a.geom;
+            ga.B = batch;
+            if (patch_set_batch(&c.dual_patch, a.geom, batch)) return fail(N2D2B_ERR_INVALID, "patch plan failed for %d images", batch);
+            CUDA_TRY(launch_patch(c.dual_patch, ga, img0, branch, c.fast, out, net->d_status, s, &a.fast));
+            return 0;
+        }
         CUDA_TRY(launch_dual(c.dual, g, a.fast, c.fast, net->tensors[a.output].is_unsigned, img0 * g.oH * g.oW, a.plan.w4, net->d_status, s));
         return 0;
     }
@@ -2209,7 +2227,7 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     if (net->d_small) return "small-net";
     const CellRec& c = net->cells[cell];
     if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], net->max_batch, net->max_batch)) return "fused";
-    if (c.dual_branch >= 0 && use_dual(net, c, net->max_batch, net->max_batch)) return "tcgen05-dual";
+    if (c.dual_branch >= 0 && use_dual(net, c, net->max_batch, net->max_batch)) return c.dual_patch.proj_in ? "patch-tcgen05-dual" : "tcgen05-dual";
     if (use_dw3x3(c, net->max_batch)) return "depthwise";
     if (use_widened(net, c, net->max_batch, net->max_batch)) return c.w8 == CellRec::W8_PATCH ? "patch-tcgen05-widened" : "tcgen05-widened";
     switch (c.engine) {

@@ -56,7 +56,7 @@ struct PatchArgs {
     int b_stream;           // weights too large to stay resident: their tap blocks stream through a ring
     int bring;              // slots of that ring
     unsigned rcp_Wp;        // ceil(2^32 / Wp)
-    unsigned idesc, tmem_cols;
+    unsigned idesc, idesc_proj, tmem_cols;
     void* out;
     int* status;
     const int* fq;
@@ -67,7 +67,13 @@ struct PatchArgs {
     int res_unsigned;
     const int* fq2;
     int t_lo, t_hi;
+    // RES_DUAL: the layer is the branch of a sum whose other operand, a 1x1 projection of a second tensor, is computed beside it
+    const int* fq_branch;   // the branch's rescale (fq: the projection's)
+    int cpad_branch, proj_alloc, proj_bytes;
 };
+
+// What the epilogue adds: nothing, a residual tensor, or the branch (the patch) to a projection
+static constexpr int RES_NONE = 0, RES_TENSOR = 1, RES_DUAL = 2;
 
 // The MMAs of one tile with compile-time tap counts: a straight run of address adds and MMAs.  The issuing
 // thread pays the latency of every instruction it executes, so loop control and address arithmetic around a
@@ -106,9 +112,13 @@ __device__ __forceinline__ void issue_tap(int ksteps, unsigned d_tmem, unsigned 
 // EF_FLOAT, the form of the rescale (0: 32-bit); a template because a choice per 32-column block inside the epilogue
 // cost 2 % of a MobileNet.  RES: a residual sum in the epilogue (64 -> 64 channels); the bytes are loaded before the wait for the
 // accumulator.  2.2_3x3_2 of ResNet-18 at 2048 images, clamped: 596 us on the implicit-GEMM kernel, 412 here
-template <bool CLAMP, int SHAPE, int FORM, bool RES>
+// RES_DUAL: a residual block's first unit, 64 -> 64 channels 3x3 beside a 64 -> 64 channel projection of the block's input, whose band arrives as a patch of its
+// own without a border: one more tap into an accumulator of its own.  The branch's bytes stay in registers.  conv2.1 of ResNet-18 at 128 images 28.4 and 28.8 us
+// by themselves, 40.8 here; 2048 images 603 / 469
+template <bool CLAMP, int SHAPE, int FORM, int RES>
 __global__ void __launch_bounds__(RES ? P_THREADS_RES : P_THREADS, 1)
-patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PatchArgs a)
+patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA2,
+                          const __grid_constant__ CUtensorMap tmB2, const PatchArgs a)
 {
     constexpr int ISSUERS = RES ? P_ISSUERS_RES : P_ISSUERS, EPI_WARP0 = 1 + ISSUERS, THREADS = RES ? P_THREADS_RES : P_THREADS;
     extern __shared__ unsigned char smem_raw[];
@@ -116,8 +126,9 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     const int taps = a.taps_y * a.taps_x;
     const int b_tap_bytes = a.BN * a.C;
     unsigned char* res_b = smem;                                              // [taps][BN][C], or a ring of a.bring taps
-    unsigned char* patch0 = smem + (((size_t)(a.b_stream ? a.bring : taps) * b_tap_bytes + 1023) & ~(size_t)1023);
-    unsigned long long* bars = (unsigned long long*)(patch0 + (size_t)a.nbuf * a.patch_alloc);
+    unsigned char* patch0 = smem + (((size_t)(a.b_stream ? a.bring : taps + (RES == RES_DUAL ? 1 : 0)) * b_tap_bytes + 1023) & ~(size_t)1023);
+    unsigned char* proj0 = patch0 + (size_t)a.nbuf * a.patch_alloc;            // RES_DUAL: the projection's bands
+    unsigned long long* bars = (unsigned long long*)(proj0 + (RES == RES_DUAL ? (size_t)a.nbuf * a.proj_alloc : 0));
     // bars: patch_full[4], patch_empty[4], tmem_full[4], tmem_empty[4], weights, (spare), ring_full[8], ring_empty[8]
     const unsigned pfull0 = smem_u32(bars);
     const unsigned pempty0 = pfull0 + 8u * P_BUFS_MAX;
@@ -161,7 +172,8 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     const int ch0 = grp * a.N;                       // first output channel (= first input channel) of the group
     for (int i = threadIdx.x; i < FAST_NP * 256; i += THREADS) {
         const int prm = i >> 8, c = i & 255;
-        if (RES && c >= 128) par[i] = __ldg(a.fq2 + (size_t)prm * a.cpad + c - 128);
+        if (RES == RES_DUAL && c >= 64 && c < 128) par[i] = __ldg(a.fq_branch + (size_t)prm * a.cpad_branch + c - 64);
+        else if (RES && c >= 128) par[i] = __ldg(a.fq2 + (size_t)prm * a.cpad + c - 128);
         else par[i] = (ch0 + c < a.cpad) ? __ldg(a.fq + (size_t)prm * a.cpad + ch0 + c) : 0;
     }
     tc_fence_before();
@@ -187,7 +199,8 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                     tma_load_2d(smem_u32(res_b + (size_t)t * b_tap_bytes), &tmB, rfull0 + 8u * t, (int)t * a.C, ch0);
                 }
             } else {
-                mbar_expect_tx(bfull, (unsigned)(taps * b_tap_bytes));
+                mbar_expect_tx(bfull, (unsigned)((taps + (RES == RES_DUAL ? 1 : 0)) * b_tap_bytes));
+                if (RES == RES_DUAL) tma_load_2d(smem_u32(res_b + (size_t)taps * b_tap_bytes), &tmB2, bfull, 0, 0);
                 for (int t = 0; t < taps; ++t)
                     tma_load_2d(smem_u32(res_b + (size_t)t * b_tap_bytes), &tmB, bfull, t * a.C, ch0);
             }
@@ -200,7 +213,9 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
             const int step_n = nctas / a.bands, step_b = nctas % a.bands;
             for (int item = cta; item < items; item += nctas) {
                 if (!mbar_wait(pempty0 + 8u * pb, ph ^ 1u, abort_flag, a.status, 1)) break;
-                mbar_expect_tx(pfull0 + 8u * pb, (unsigned)a.patch_bytes);
+                mbar_expect_tx(pfull0 + 8u * pb, (unsigned)(a.patch_bytes + (RES == RES_DUAL ? a.proj_bytes : 0)));
+                if (RES == RES_DUAL)
+                    tma_load_4d(smem_u32(proj0 + (size_t)pb * a.proj_alloc), &tmA2, pfull0 + 8u * pb, 0, 0, band * a.R, a.n_base + n);
                 tma_load_4d(smem_u32(patch0 + (size_t)pb * a.patch_alloc), &tmA, pfull0 + 8u * pb, grp * a.C, -a.pL,
                             band * a.R - a.pT, a.n_base + n);
                 if (a.b_stream) {
@@ -247,6 +262,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                 if (!mbar_wait_uniform(pfull0 + 8u * pb, ph, abort_flag, a.status, 3)) { ok = false; break; }
                 tc_fence_after();
                 unsigned a_lo = patch_lo + pb * (unsigned)(a.patch_alloc >> 4);
+                unsigned proj_lo = ((smem_u32(proj0) & 0x3ffffu) >> 4) + pb * (unsigned)(a.proj_alloc >> 4);
                 if (a.b_stream) {
                     // At most P_SLOTS tiles per item, each with its own accumulator: this thread owns tiles `me` and
                     // `me + P_ISSUERS` and walks the taps as their weights arrive, so one pass of the weights serves
@@ -289,7 +305,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                     if (band >= a.bands) band -= a.bands;
                     continue;
                 }
-                for (int t = 0; t < T; ++t, ++seq, a_lo += tile_step) {
+                for (int t = 0; t < T; ++t, ++seq, a_lo += tile_step, proj_lo += tile_step) {
                     if ((seq & (ISSUERS - 1)) != me) continue;
                     const unsigned slot = seq & (P_SLOTS - 1), sph = (seq / P_SLOTS) & 1u;
                     if (!mbar_wait_uniform(tempty0 + 8u * slot, sph ^ 1u, abort_flag, a.status, 2)) { ok = false; break; }
@@ -313,6 +329,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                                     }
                             }
                         }
+                        if (RES == RES_DUAL) issue_tap_n<2>(d_tmem + P_SLOTS * 64u, proj_lo, res_b_lo + (unsigned)taps * btap, desc_hi, a.idesc_proj, 0u);
                         tc_commit(tfull0 + 8u * slot);
                     }
                     __syncwarp();
@@ -356,7 +373,7 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
                 }
                 uint2 res[4];
                 const uint8_t* const rp = a.res + (band_out - (uint8_t*)a.out) + 8 * (lane & 3);
-                if (RES) {
+                if (RES == RES_TENSOR) {
 #pragma unroll
                     for (int k = 0; k < 4; ++k) res[k] = (rowok >> k) & 1u ? __ldg((const uint2*)(rp + rowoff[k])) : make_uint2(0u, 0u);
                 }
@@ -367,14 +384,19 @@ patch_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
 #pragma unroll 1
                     for (int cb = 0; cb < 64; cb += 32) {
                         unsigned va[16], vb[16];
-                        tc_ld_2x16x256b_x4_wait(tbase + (unsigned)cb, va, vb);
-                        switch ((a.out_unsigned ? EF_OUT_UNSIGNED : 0) | (a.res_unsigned ? EF_RES_UNSIGNED : 0)) {
-                        case 0: perm_block_global<CLAMP, FORM, RES>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane, res, a.t_lo, a.t_hi); break;
-                        case EF_OUT_UNSIGNED: perm_block_global<CLAMP, FORM | EF_OUT_UNSIGNED, RES>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane, res, a.t_lo, a.t_hi); break;
-                        case EF_RES_UNSIGNED: perm_block_global<CLAMP, FORM | EF_RES_UNSIGNED, RES>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane, res, a.t_lo, a.t_hi); break;
-                        default: perm_block_global<CLAMP, FORM | EF_OUT_UNSIGNED | EF_RES_UNSIGNED, RES>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane, res, a.t_lo, a.t_hi); break;
+                        if (RES == RES_DUAL) {
+                            tc_ld_2x16x256b_x4_wait(tbase + (unsigned)cb, va, vb);
+                            if (a.res_unsigned) perm_block_words<CLAMP, FORM | EF_OUT_UNSIGNED>(va, vb, par_off, 64 + cb, res, lane);
+                            else perm_block_words<CLAMP, FORM>(va, vb, par_off, 64 + cb, res, lane);
                         }
-                        if (cb == 0) {
+                        tc_ld_2x16x256b_x4_wait(tbase + (RES == RES_DUAL ? P_SLOTS * 64u : 0u) + (unsigned)cb, va, vb);
+                        switch ((a.out_unsigned ? EF_OUT_UNSIGNED : 0) | (a.res_unsigned ? EF_RES_UNSIGNED : 0)) {
+                        case 0: perm_block_global<CLAMP, FORM, RES != RES_NONE>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane, res, a.t_lo, a.t_hi); break;
+                        case EF_OUT_UNSIGNED: perm_block_global<CLAMP, FORM | EF_OUT_UNSIGNED, RES != RES_NONE>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane, res, a.t_lo, a.t_hi); break;
+                        case EF_RES_UNSIGNED: perm_block_global<CLAMP, FORM | EF_RES_UNSIGNED, RES != RES_NONE>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane, res, a.t_lo, a.t_hi); break;
+                        default: perm_block_global<CLAMP, FORM | EF_OUT_UNSIGNED | EF_RES_UNSIGNED, RES != RES_NONE>(va, vb, par_off, cb, band_out + cb, rowoff, rowok, lane, res, a.t_lo, a.t_hi); break;
+                        }
+                        if (RES == RES_TENSOR && cb == 0) {
 #pragma unroll
                             for (int k = 0; k < 4; ++k) res[k] = (rowok >> k) & 1u ? __ldg((const uint2*)(rp + rowoff[k] + 32)) : make_uint2(0u, 0u);
                         }
@@ -421,12 +443,13 @@ static bool patch_streams(int taps, int C, int BN) { return (size_t)taps * BN * 
 
 // (`spare` caps the band height of two buffers: with that space given to the patches, the 64-channel 55 x 55 layers went from
 // five bands of 11 rows to 22 + 22 + 11 and ran 18 % slower.  More buffers may use it.)
-static size_t patch_smem_bytes(int taps, int C, int BN, int patch_alloc, int bring = P_BRING_MIN, int nbuf = 2)
+// proj_alloc: bytes of a projection's band beside every patch (0: none)
+static size_t patch_smem_bytes(int taps, int C, int BN, int patch_alloc, int bring = P_BRING_MIN, int nbuf = 2, int proj_alloc = 0)
 {
     const int blocks = patch_streams(taps, C, BN) ? bring : taps;
-    const size_t b = (((size_t)blocks * BN * C) + 1023) & ~(size_t)1023;
-    const size_t spare = nbuf == 2 ? (size_t)P_EPI_WARPS * 32 * (patch_streams(taps, C, BN) ? 32 : BN) : 0;
-    return 1024 + b + nbuf * (size_t)patch_alloc + spare + (2 * P_BUFS_MAX + 2 * P_SLOTS + 2 + 2 * P_BRING_MAX) * 8 + 32
+    const size_t b = (((size_t)(blocks + (proj_alloc ? 1 : 0)) * BN * C) + 1023) & ~(size_t)1023;
+    const size_t spare = nbuf == 2 && !proj_alloc ? (size_t)P_EPI_WARPS * 32 * (patch_streams(taps, C, BN) ? 32 : BN) : 0;
+    return 1024 + b + nbuf * (size_t)(patch_alloc + proj_alloc) + spare + (2 * P_BUFS_MAX + 2 * P_SLOTS + 2 + 2 * P_BRING_MAX) * 8 + 32
          + FAST_NP * 256 * 4 + 64;
 }
 
@@ -497,6 +520,36 @@ void patch_dw_arrange_weights(const ConvGeom& g, const int8_t* w_ct, int8_t* dst
     }
 }
 
+// bytes of a projection's band of R rows: whole tiles of positions
+static int patch_proj_alloc(const ConvGeom& g, int Wp, int R) { return (R * Wp + PBM - 1) / PBM * PBM * g.C; }
+
+bool patch_takes_projection(const ConvGeom& g, const ConvGeom& p)
+{
+    return patch_takes_residual(g) && p.groups == 1 && p.C == 64 && p.O == 64 && p.kH == 1 && p.kW == 1 && p.sX == 1 && p.sY == 1 && p.pT == 0 && p.pL == 0 && p.oH == g.oH
+        && p.oW == g.oW && p.H == g.oH && p.W == g.oW;
+}
+
+int patch_add_projection(PatchPlan* plan, const void* in, const int8_t* w, const ConvGeom& g0, int in_unsigned, const char** why)
+{
+    static const char* kWhy = "";
+    *why = kWhy;
+    if (((uintptr_t)in & 15) || ((uintptr_t)w & 15)) { *why = "operands must be 16-byte aligned"; return -1; }
+    const cuuint64_t dims[2] = {64, 64};
+    const cuuint64_t strides[1] = {64};
+    const cuuint32_t box[2] = {64, 64};
+    const cuuint32_t estr[2] = {1, 1};
+    if (((EncodeTiledFn)plan->encode)(&plan->tmB2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)w, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        *why = "cuTensorMapEncodeTiled failed for the projection's weights";
+        return -1;
+    }
+    plan->proj_in = in;
+    plan->proj_unsigned = in_unsigned;
+    plan->band_batch = plan->R = 0;   // the bands are chosen anew, with the projection's beside them
+    if (patch_set_batch(plan, g0, plan->max_batch)) { *why = "no band height fits shared memory"; return -1; }
+    return 0;
+}
+
 int patch_make_plan(PatchPlan* plan, const void* in, const int8_t* w, const ConvGeom& g0, int in_unsigned, int num_sms,
                     const char** why)
 {
@@ -555,7 +608,7 @@ int patch_set_batch(PatchPlan* plan, const ConvGeom& g0, int batch)
         long long best = 0;
         for (int R = 1; R <= g.oH; ++R) {
             if (R + (g.kH - 1) * g.dY > 256) break;
-            if (patch_smem_bytes(taps, g.C, plan->BN, patch_alloc_bytes(g, Wp, R)) > 226 * 1024) break;
+            if (patch_smem_bytes(taps, g.C, plan->BN, patch_alloc_bytes(g, Wp, R), P_BRING_MIN, 2, plan->proj_in ? patch_proj_alloc(g, Wp, R) : 0) > 226 * 1024) break;
             // streamed weights: every tile of a band accumulates while the taps pass, so a band has at most as many
             // tiles as there are accumulators
             const int tall = (R * Wp + PBM - 1) / PBM;
@@ -575,15 +628,17 @@ int patch_set_batch(PatchPlan* plan, const ConvGeom& g0, int batch)
     const int box_rows = best_R + (g.kH - 1) * g.dY;
     plan->patch_bytes = box_rows * plan->Wp * g.C;
     plan->patch_alloc = patch_alloc_bytes(g, plan->Wp, best_R);
+    plan->proj_alloc = plan->proj_in ? patch_proj_alloc(g, plan->Wp, best_R) : 0;
+    plan->proj_bytes = plan->proj_in ? best_R * plan->Wp * g.C : 0;
     plan->bring = P_BRING_MIN;
     while (plan->b_stream && plan->bring < P_BRING_MAX
            && patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring + 1) <= 226 * 1024)
         ++plan->bring;
     plan->nbuf = 2;
     while (plan->nbuf < P_BUFS_MAX
-           && patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring, plan->nbuf + 1) <= 226 * 1024)
+           && patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring, plan->nbuf + 1, plan->proj_alloc) <= 226 * 1024)
         ++plan->nbuf;
-    plan->smem_bytes = patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring, plan->nbuf);
+    plan->smem_bytes = patch_smem_bytes(taps, g.C, plan->BN, plan->patch_alloc, plan->bring, plan->nbuf, plan->proj_alloc);
     // NHWC activations as (C, W, H, B); one box = a whole patch, zero-filled outside the image
     const CUtensorMapSwizzle swz = g.C == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                                               : (g.C == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
@@ -592,6 +647,14 @@ int patch_set_batch(PatchPlan* plan, const ConvGeom& g0, int batch)
     const cuuint64_t strides[3] = {(cuuint64_t)Ct, (cuuint64_t)Ct * g.W, (cuuint64_t)Ct * g.W * g.H};
     const cuuint32_t box[4] = {(cuuint32_t)g.C, (cuuint32_t)plan->Wp, (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
+    if (plan->proj_in) {   // the projection's input: the output's extents, a box without border rows
+        const cuuint64_t dims2[4] = {(cuuint64_t)g.C, (cuuint64_t)g.oW, (cuuint64_t)g.oH, (cuuint64_t)plan->max_batch};
+        const cuuint64_t strides2[3] = {(cuuint64_t)g.C, (cuuint64_t)g.C * g.oW, (cuuint64_t)g.C * g.oW * g.oH};
+        const cuuint32_t box2[4] = {(cuuint32_t)g.C, (cuuint32_t)plan->Wp, (cuuint32_t)best_R, 1};
+        if (((EncodeTiledFn)plan->encode)(&plan->tmA2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)plan->proj_in, dims2, strides2, box2, estr,
+                                          CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return -1;
+    }
     return ((EncodeTiledFn)plan->encode)(&plan->tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, (void*)plan->in, dims, strides, box, estr,
                                          CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -1;
@@ -604,8 +667,10 @@ bool patch_takes_residual(const ConvGeom& g)
 }
 
 cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, const Residual& r, const FastQuant& fast, void* out,
-                         int* status_word, cudaStream_t s)
+                         int* status_word, cudaStream_t s, const FastQuant* branch)
 {
+    // branch: the layer's own rescale where `fast` is that of the projection beside it (with the sum's), and r says how the branch's bytes are signed
+    if ((branch != nullptr) != (plan.proj_in != nullptr)) return cudaErrorInvalidConfiguration;
     if (r.ptr && (!patch_takes_residual(g0) || !fast.fq2 || fast.dp4a)) return cudaErrorInvalidConfiguration;
     const ConvGeom g = patch_group_geom(g0);
     PatchArgs a;
@@ -634,21 +699,29 @@ cudaError_t launch_patch(const PatchPlan& plan, const ConvGeom& g0, int n_base, 
     a.res_unsigned = r.is_unsigned;
     a.fq2 = fast.fq2;
     a.t_lo = fast.t_lo; a.t_hi = fast.t_hi;
-    typedef void (*PatchKernel)(const CUtensorMap, const CUtensorMap, const PatchArgs);
-#define N2D2B_PATCH(C, F) patch_conv_tcgen05_kernel<C, 0, F, false>, patch_conv_tcgen05_kernel<C, 1, F, false>, \
-                          patch_conv_tcgen05_kernel<C, 2, F, false>, patch_conv_tcgen05_kernel<C, 3, F, false>, patch_conv_tcgen05_kernel<C, 2, F, true>
-    static const PatchKernel variants[30] = {N2D2B_PATCH(false, 0), N2D2B_PATCH(true, 0), N2D2B_PATCH(false, EF_FLOAT),
+    if (branch) {
+        a.fq_branch = branch->fq;
+        a.cpad_branch = branch->cpad;
+        a.proj_alloc = plan.proj_alloc;
+        a.proj_bytes = plan.proj_bytes;
+        a.idesc_proj = (a.idesc & ~(1u << 7)) | ((plan.proj_unsigned ? 0u : 1u) << 7);
+        a.tmem_cols = 512;
+    }
+    typedef void (*PatchKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const PatchArgs);
+#define N2D2B_PATCH(C, F) patch_conv_tcgen05_kernel<C, 0, F, RES_NONE>, patch_conv_tcgen05_kernel<C, 1, F, RES_NONE>, patch_conv_tcgen05_kernel<C, 2, F, RES_NONE>, \
+                          patch_conv_tcgen05_kernel<C, 3, F, RES_NONE>, patch_conv_tcgen05_kernel<C, 2, F, RES_TENSOR>, patch_conv_tcgen05_kernel<C, 2, F, RES_DUAL>
+    static const PatchKernel variants[36] = {N2D2B_PATCH(false, 0), N2D2B_PATCH(true, 0), N2D2B_PATCH(false, EF_FLOAT),
                                              N2D2B_PATCH(true, EF_FLOAT), N2D2B_PATCH(false, EF_WIDE), N2D2B_PATCH(true, EF_WIDE)};
 #undef N2D2B_PATCH
-    static SmemLimitSet limits[30];
+    static SmemLimitSet limits[36];
     // a multiple of the group count: CTA b works on group b % G
     const long long items = (long long)a.B * a.bands;
     const long long per_group = plan.num_sms / plan.G > 0 ? plan.num_sms / plan.G : 1;
     const int grid = (int)((items < per_group ? items : per_group) * plan.G);
-    const int shape = r.ptr ? 4 : (g.kH == 3 && g.kW == 3 && !plan.b_stream) ? (g.C == 32 ? 1 : (g.C == 64 ? 2 : 3)) : 0;
-    const int v = (fast.form == EF_WIDE ? 20 : (fast.form == EF_FLOAT ? 10 : 0)) + (fast.need_clamp ? 5 : 0) + shape;
+    const int shape = branch ? 5 : r.ptr ? 4 : (g.kH == 3 && g.kW == 3 && !plan.b_stream) ? (g.C == 32 ? 1 : (g.C == 64 ? 2 : 3)) : 0;
+    const int v = (fast.form == EF_WIDE ? 24 : (fast.form == EF_FLOAT ? 12 : 0)) + (fast.need_clamp || (branch && branch->need_clamp) ? 6 : 0) + shape;
     if (cudaError_t e = raise_smem_limit(variants[v], limits[v])) return e;
-    return launch_pdl(variants[v], grid, r.ptr ? P_THREADS_RES : P_THREADS, plan.smem_bytes, s, plan.tmA, plan.tmB, a);
+    return launch_pdl(variants[v], grid, r.ptr || branch ? P_THREADS_RES : P_THREADS, plan.smem_bytes, s, plan.tmA, plan.tmB, plan.tmA2, plan.tmB2, a);
 }
 
 }  // namespace n2d2b

@@ -724,6 +724,33 @@ __device__ __forceinline__ void perm_block(const unsigned* vA, const unsigned* v
     }
 }
 
+// The block's bytes, eight consecutive channels of the thread's four rows: words[k] of row tr + 8k
+template <bool CLAMP, int EF>
+__device__ __forceinline__ void perm_block_words(const unsigned* vA, const unsigned* vB, unsigned par_off, int pcol0, uint2 (&words)[4], int lane)
+{
+    unsigned char* const sm = dyn_smem();
+    const unsigned pbase = par_off + (unsigned)(pcol0 + 8 * (lane & 3)) * 4u;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const unsigned pp = pbase + 16u * h;
+        const int4 mu = *(const int4*)(sm + pp + 2 * 1024), ad = *(const int4*)(sm + pp + 3 * 1024), sh = *(const int4*)(sm + pp + 4 * 1024);
+        int4 lo = make_int4(0, 0, 0, 0), hi = lo;
+        if (CLAMP || (EF & EF_WIDE)) lo = *(const int4*)(sm + pp + 0 * 1024);
+        if (CLAMP) hi = *(const int4*)(sm + pp + 1 * 1024);
+        const int muv[4] = {mu.x, mu.y, mu.z, mu.w}, adv[4] = {ad.x, ad.y, ad.z, ad.w}, shv[4] = {sh.x, sh.y, sh.z, sh.w};
+        const int lov[4] = {lo.x, lo.y, lo.z, lo.w}, hiv[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned* v = (k < 2) ? vA : vB;
+            int y[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) y[c] = rescale<CLAMP, EF>((int)v[4 * (2 * h + (c >> 1)) + 2 * (k & 1) + (c & 1)], lov[c], hiv[c], muv[c], adv[c], shv[c]);
+            const unsigned w = pack4_sat(y[0], y[1], y[2], y[3], (EF & EF_OUT_UNSIGNED) != 0);
+            if (h) words[k].y = w; else words[k].x = w;
+        }
+    }
+}
+
 // The same block written straight to global memory: with the permuted layout a thread holds eight
 // consecutive channels of a row, four neighbouring lanes a whole 32-byte sector of it, so the bytes need no detour
 // through a staging region when the rows' addresses have no regular pattern a TMA store could follow (the band

@@ -62,3 +62,27 @@ def test_packed_weights_and_calls_of_any_size_on_one_network():
 def test_slices_of_the_upload():
     net = unit_net(64, 64, 56, 56, 256, 1, 1, 'double')
     compare_net(net, 11, flags=0, slices=4, want_engine=ENGINE)
+
+
+# bands of one to eleven rows, images of one band, many bands per CTA, maps wider than a tile's share of a row
+@pytest.mark.parametrize('case', [(55, 55, 3), (55, 55, 40), (13, 9, 5), (30, 28, 60), (3, 61, 2), (40, 5, 7)], ids=lambda c: '%dx%d_b%d' % c)
+@pytest.mark.parametrize('mode, clipped, unsigned_relu, act', [('fixed', False, True, 'linear'), ('fixed', True, True, 'linear'), ('float', False, True, 'linear'),
+                                                               ('float', True, False, 'relu'), ('fixed', False, False, 'relu')])
+def test_patch_branch_and_projection(case, mode, clipped, unsigned_relu, act):
+    H, W, batch = case
+    compare_net(unit_net(64, 64, H, W, 64, 3, 1, mode, unsigned_relu, clipped, act), batch, flags=0, want_engine='patch-tcgen05-dual')
+
+
+def test_patch_branch_and_projection_with_packed_weights_and_slices():
+    net = unit_net(64, 64, 56, 56, 64, 3, 1, 'fixed', weight_bits=4, clipped=True)
+    x = netdesc.make_input(net, 9)
+    ref = oracle.run_net(net, x, 'i64')[-1].reshape(9, -1)
+    qn = runtime.QuantizedNet(net, 9)
+    try:
+        assert 'patch-tcgen05-dual' in qn.engines()
+        for batch in (9, 1, 8):
+            assert np.array_equal(qn.forward_host(x[:batch]).astype(np.int64), ref[:batch])
+        qn.set_slices(3)
+        assert np.array_equal(qn.forward_host(x).astype(np.int64), ref)
+    finally:
+        qn.close()
