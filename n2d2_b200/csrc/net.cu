@@ -1475,8 +1475,9 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 c.has_plan = true;
                 c.plan_input = in_ptr;  // nullptr = must be re-encoded with the real input
                 if (!(flags & N2D2B_EXACT64_EPILOGUE) && !c.pad_O) {
-                    // (the patch kernel's residual stage is not the dot-product form)
-                    const bool res_i8 = c.residual >= 0 && net->tensors[c.residual].dtype == DT_I8 && (w4 || !patch_takes_residual(gb));
+                    // (the patch kernel's residual stage is not the dot-product form, nor is its sum with a projection)
+                    const bool res_i8 = c.residual >= 0 && net->tensors[c.residual].dtype == DT_I8 && (w4 || !patch_takes_residual(gb))
+                                        && !(c.dual_branch >= 0 && patch_takes_projection(net->cells[c.dual_branch].geom, g));
                     if (int rc = upload_fast(c, net->tensors[c.output], res_i8,
                                              c.residual >= 0 ? net->tensors[c.residual].is_unsigned : 0, w4))
                         return rc;

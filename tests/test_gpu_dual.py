@@ -67,7 +67,8 @@ def test_slices_of_the_upload():
 # bands of one to eleven rows, images of one band, many bands per CTA, maps wider than a tile's share of a row
 @pytest.mark.parametrize('case', [(55, 55, 3), (55, 55, 40), (13, 9, 5), (30, 28, 60), (3, 61, 2), (40, 5, 7)], ids=lambda c: '%dx%d_b%d' % c)
 @pytest.mark.parametrize('mode, clipped, unsigned_relu, act', [('fixed', False, True, 'linear'), ('fixed', True, True, 'linear'), ('float', False, True, 'linear'),
-                                                               ('float', True, False, 'relu'), ('fixed', False, False, 'relu')])
+                                                               ('float', True, False, 'relu'), ('fixed', False, False, 'relu'),
+                                                               ('double', False, True, 'linear'), ('single', False, False, 'relu')])
 def test_patch_branch_and_projection(case, mode, clipped, unsigned_relu, act):
     H, W, batch = case
     compare_net(unit_net(64, 64, H, W, 64, 3, 1, mode, unsigned_relu, clipped, act), batch, flags=0, want_engine='patch-tcgen05-dual')
