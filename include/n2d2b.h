@@ -248,6 +248,7 @@ int n2d2b_net_weight_bytes(const n2d2b_net* net, size_t* total_bytes, size_t* pa
 int n2d2b_net_launches_per_forward(const n2d2b_net* net);
 /* Name of the kernel family that runs cell `cell` in an n2d2b_net_forward of the finalized max_batch images:
  *   "tcgen05", "tcgen05-pair"      implicit GEMM (256-row tiles)
+ *   "tcgen05-chain"                a 1x1 layer with its residual sum and the 1x1 layer behind it (which is "fused")
  *   "tcgen05-dual", "patch-tcgen05-dual"
  *                                  two convolutions and the sum of their outputs (the first one is "fused")
  *   "tcgen05-w4"                   the same, packed 4-bit weights expanded in the kernel

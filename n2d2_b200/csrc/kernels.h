@@ -288,6 +288,20 @@ int dual_make_plan(DualPlan* plan, const void* in_a, const int8_t* w_a, const Co
 cudaError_t launch_dual(const DualPlan& plan, const ConvGeom& gb, const FastQuant& fa, const FastQuant& fb, int branch_unsigned, int m_base, int late_weights,
                         int* status_word, cudaStream_t s);
 
+// ---- a 1x1 expansion to 256 channels with its residual sum, and the 1x1 layer behind it (igemm_chain.cu) ----
+struct ChainPlan {
+    IgemmPlan a;          // maps of the expansion's operands, its output and its residual
+    CUtensorMap tmB2;     // weights of the layer behind, box = 64 of its inputs x all outputs
+    int C, N2, slots, y_unsigned;
+    size_t smem_bytes;
+};
+bool chain_eligible(const ConvGeom& g, const ConvGeom& p);
+int chain_make_plan(ChainPlan* plan, const void* in, const int8_t* w, const void* y, const void* res, const ConvGeom& g, int in_unsigned, const int8_t* w_next,
+                    const ConvGeom& p, int y_unsigned, int num_sms, const char** why);
+// M rows from row m_base on; out: the next layer's tensor
+cudaError_t launch_chain(const ChainPlan& plan, int M, const FastQuant& fast, int res_unsigned, const FastQuant& next, void* out, int m_base, int* status_word,
+                         cudaStream_t s);
+
 // Widens packed 4-bit weights [rows_src][8 words / 2 bytes] into int8 [rows][8 words] in the row order a kernel expects, several cells' in one launch.  Row n
 // of the destination is real channel perm_real_channel(n, ng_dst); ng_src says how the packed rows are ordered (0: naturally).
 // Destination rows of channels that do not exist are zero.

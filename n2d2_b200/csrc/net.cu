@@ -122,6 +122,10 @@ struct CellRec {
     bool dual_on = false;
     DualPlan dual{};
     PatchPlan dual_patch{};   // or by the patch kernel (proj_in set)
+    // an expansion with its residual sum and the 1x1 cell behind it as one kernel (igemm_chain.cu): each other's index
+    int chain_next = -1, chain_prev = -1;
+    bool chain_on = false;
+    ChainPlan chain{};
     // tensor-core plan
     IgemmPlan plan{};
     bool has_plan = false;
@@ -947,6 +951,24 @@ static void mark_duals(n2d2b_net* net)
     }
 }
 
+// Expansions with a residual sum whose reader is the next cell, a 1x1 one: the kernel of the first may write the output of both, so the second's buffer
+// is taken while the first's operands still have theirs.  Settled when the kernels are chosen (plan_chains).
+static void mark_chains(n2d2b_net* net)
+{
+    for (size_t i = 0; i < net->cells.size(); ++i) {
+        CellRec& c = net->cells[i];
+        if (c.skipped || c.type != CELL_CONV || c.residual <= 0 || c.inputs[0] == 0 || c.wbits != 8 || c.dual_branch >= 0) continue;
+        size_t j = i + 1;
+        while (j < net->cells.size() && net->cells[j].skipped) ++j;
+        if (j == net->cells.size()) continue;
+        CellRec& p = net->cells[j];
+        if (p.type != CELL_CONV || p.residual >= 0 || p.inputs.size() != 1 || p.inputs[0] != c.output || p.wbits != 8 || p.dual_sum >= 0) continue;
+        if (!chain_eligible(c.geom, p.geom) || net->tensors[p.output].dtype != DT_I8) continue;
+        c.chain_next = (int)j;
+        p.chain_prev = (int)i;
+    }
+}
+
 // Cells [0, n) that the host-buffer entry point may run slice by slice (a structural rule, applied before the
 // kernels are chosen; the engine-based rule in finalize can only shorten it): image-wise cells with large
 // per-image tensors, up to the first fully-connected cell or stand-alone sum.
@@ -995,25 +1017,28 @@ static int plan_buffers(n2d2b_net* net)
     for (int ci = 0; ci < (int)net->cells.size(); ++ci) {
         CellRec& c = net->cells[ci];
         if (c.skipped) continue;
-        TensorRec& t = net->tensors[c.output];
-        const size_t need = ((t.bytes_per_image() * (size_t)net->max_batch + 255) / 256) * 256 + 256;
-        const bool in_head = ci < net->head_limit;
-        int pick = -1;
-        if (!keep_all) {
-            for (size_t f = 0; f < free_list.size(); ++f) {
-                const int b = free_list[f];
-                if (in_head && head_bpi[b] != t.bytes_per_image()) continue;
-                if (sizes[b] >= need && (pick < 0 || sizes[b] < sizes[free_list[pick]])) pick = (int)f;
+        auto take = [&](TensorRec& t, bool in_head) {
+            const size_t need = ((t.bytes_per_image() * (size_t)net->max_batch + 255) / 256) * 256 + 256;
+            int pick = -1;
+            if (!keep_all) {
+                for (size_t f = 0; f < free_list.size(); ++f) {
+                    const int b = free_list[f];
+                    if (in_head && head_bpi[b] != t.bytes_per_image()) continue;
+                    if (sizes[b] >= need && (pick < 0 || sizes[b] < sizes[free_list[pick]])) pick = (int)f;
+                }
             }
-        }
-        if (pick >= 0) {
-            t.buffer = free_list[pick];
-            free_list.erase(free_list.begin() + pick);
-        } else {
-            t.buffer = (int)sizes.size();
-            sizes.push_back(need);
-            head_bpi.push_back(in_head ? t.bytes_per_image() : 0);
-        }
+            if (pick >= 0) {
+                t.buffer = free_list[pick];
+                free_list.erase(free_list.begin() + pick);
+            } else {
+                t.buffer = (int)sizes.size();
+                sizes.push_back(need);
+                head_bpi.push_back(in_head ? t.bytes_per_image() : 0);
+            }
+        };
+        TensorRec& t = net->tensors[c.output];
+        if (c.chain_prev < 0) take(t, ci < net->head_limit);   // (else it was taken with the cell in front)
+        if (c.chain_next >= 0) take(net->tensors[net->cells[c.chain_next].output], c.chain_next < net->head_limit);
         if (!keep_all) {
             // release the inputs that die with this cell (never the network input or the final output)
             for (int i : c.inputs) {
@@ -1190,6 +1215,29 @@ static int plan_duals(n2d2b_net* net)
     return 0;
 }
 
+static int plan_chains(n2d2b_net* net)
+{
+    for (size_t ci = 0; ci < net->cells.size(); ++ci) {
+        CellRec& c = net->cells[ci];
+        if (c.chain_next < 0) continue;
+        CellRec& p = net->cells[c.chain_next];
+        if (c.engine != ENG_TCGEN05 || p.engine != ENG_TCGEN05 || !c.fast.enabled || !c.fast.fq2 || !p.fast.enabled || c.plan.perm != 32 || p.plan.perm != 32
+            || net->tensors[c.output].dtype != DT_I8)
+            continue;
+        // (slices of the upload: both or neither)
+        if (((int)ci < net->head_cells) != (c.chain_next < net->head_cells)) continue;
+        ConvGeom g = c.geom;
+        g.B = net->max_batch;
+        const char* why = "";
+        if (chain_make_plan(&c.chain, tensor_ptr(net, c.inputs[0], nullptr), c.d_weights, tensor_ptr(net, c.output, nullptr), tensor_ptr(net, c.residual, nullptr), g,
+                            net->tensors[c.inputs[0]].is_unsigned, p.d_weights, p.geom, net->tensors[c.output].is_unsigned, net->num_sms, &why))
+            continue;
+        c.chain_on = true;
+        net->launches--;
+    }
+    return 0;
+}
+
 // A chain of convolutions, poolings and fully-connected cells whose weights fit one SM's shared memory runs as one kernel
 // (small_net.cu).  The bound on the arithmetic keeps out what the tensor cores do better: 2^20 multiply-accumulates
 // take an SM about 8 us there, and a batch of b images b / 148 times that.
@@ -1247,6 +1295,7 @@ static bool use_dw3x3(const CellRec& c, int batch) { return c.d_dw3x3 && dw3x3_f
 
 static int plan_dwpw(n2d2b_net* net, CellRec& c);
 static int plan_duals(n2d2b_net* net);
+static int plan_chains(n2d2b_net* net);
 
 int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
 {
@@ -1263,7 +1312,10 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
     if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE | N2D2B_FORCE_DEPTHWISE_TENSOR | N2D2B_FORCE_IM2COL
                    | N2D2B_FORCE_PAIR)))
         if (int rc = fuse_depthwise(net)) return rc;
-    if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE | N2D2B_FORCE_IM2COL | N2D2B_FORCE_PAIR))) mark_duals(net);
+    if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE | N2D2B_FORCE_IM2COL | N2D2B_FORCE_PAIR))) {
+        mark_duals(net);
+        mark_chains(net);
+    }
     net->head_limit = head_candidate_prefix(net);
     if (int rc = plan_buffers(net)) return rc;
     CUDA_TRY(cudaMalloc(&net->d_status, 64));
@@ -1546,6 +1598,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
         net->head_cells = (int)ci + 1;
     }
     if (int rc = plan_duals(net)) return rc;
+    if (int rc = plan_chains(net)) return rc;
     for (int k = 0; k < 2; ++k) {
         CUDA_TRY(cudaEventCreateWithFlags(&net->pipe_uploaded[k], cudaEventDisableTiming));
         CUDA_TRY(cudaEventCreateWithFlags(&net->pipe_computed[k], cudaEventDisableTiming));
@@ -1713,6 +1766,7 @@ static int run_igemm(n2d2b_net* net, const CellRec& c, IgemmPlan p, const Residu
 static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, cudaStream_t s, int img0 = 0)
 {
     if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], batch, net->call_batch)) return 0;   // computed by the cell that carries the sum
+    if (c.chain_prev >= 0 && net->cells[c.chain_prev].chain_on) return 0;   // written by the cell in front
     const void* in0 = tensor_ptr(net, c.inputs[0], d_input);
     void* out = tensor_ptr(net, c.output, d_input);
     const TensorRec& tin = net->tensors[c.inputs[0]];
@@ -1736,6 +1790,12 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
     // the maps and the loads of a residual start on 16 bytes; the network's input is the caller's buffer
     if (c.residual == 0 && mapped && ((uintptr_t)r.ptr & 15))
         return fail(N2D2B_ERR_INVALID, "a residual sum cannot read an input at %p: operands must be 16-byte aligned", r.ptr);
+    if (c.chain_on) {
+        const CellRec& p = net->cells[c.chain_next];
+        const int pixels = c.geom.oH * c.geom.oW;
+        CUDA_TRY(launch_chain(c.chain, batch * pixels, c.fast, r.is_unsigned, p.fast, tensor_ptr(net, p.output, d_input), img0 * pixels, net->d_status, s));
+        return 0;
+    }
     const bool dual = c.dual_branch >= 0 && use_dual(net, c, batch, net->call_batch), widened = use_widened(net, c, batch, net->call_batch);
     if (widened) {
         if (dual)
@@ -2229,6 +2289,8 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     const CellRec& c = net->cells[cell];
     if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], net->max_batch, net->max_batch)) return "fused";
     if (c.dual_branch >= 0 && use_dual(net, c, net->max_batch, net->max_batch)) return c.dual_patch.proj_in ? "patch-tcgen05-dual" : "tcgen05-dual";
+    if (c.chain_prev >= 0 && net->cells[c.chain_prev].chain_on) return "fused";
+    if (c.chain_on) return "tcgen05-chain";
     if (use_dw3x3(c, net->max_batch)) return "depthwise";
     if (use_widened(net, c, net->max_batch, net->max_batch)) return c.w8 == CellRec::W8_PATCH ? "patch-tcgen05-widened" : "tcgen05-widened";
     switch (c.engine) {
