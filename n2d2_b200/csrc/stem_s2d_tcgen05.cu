@@ -400,7 +400,7 @@ cudaError_t launch_stem_s2d(const StemS2dPlan& plan, const ConvGeom& g, int n_ba
     a.cpad = fast.cpad;
     a.out_unsigned = fast.out_unsigned;
     static const StemS2dKernel kernels[6][3] = N2D2B_STEM_S2D_KERNELS(false);
-    static SmemLimitSet limits[2][5][3];
+    static SmemLimitSet limits[2][6][3];
     const long long items = (long long)a.B * a.bands;
     const int grid = (int)(items < plan.num_sms ? items : plan.num_sms);
     const int shape = (plan.KH == 4 && plan.KWp == 4) ? 1 : ((plan.KH == 2 && plan.KWp == 2) ? 2 : 0);
