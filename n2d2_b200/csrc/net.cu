@@ -1078,6 +1078,9 @@ static int final_tensor_of(const n2d2b_net* net)
     return -1;
 }
 
+// Whether a cell whose columns are padded stores the wanted ones from the registers: classifiers (one pixel per image) of launches that store that way
+static bool stores_rows(const CellRec& c, const IgemmPlan& p) { return c.geom.oH * c.geom.oW == 1 && igemm_writes_rows(p, c.geom.O); }
+
 // Whether a patch cell whose weights stream (128 channels) runs as an implicit GEMM in a call of `batch` images: up to one tile per SM.  A band then has few
 // tiles to share the stream of all its weights, which the implicit GEMM loads ahead, tile by tile (3x3, 128 channels of 28 x 28 in ResNet-50, the
 // whole network: one image 240 us -> 233, 8 images 301 / 298, 16 images 344 / 340; 32 images, two tiles per SM, 424 / 427).
@@ -1163,7 +1166,7 @@ static int plan_widened(n2d2b_net* net)
     const bool all = widen_all(net, net->max_batch);
     if (all) net->launches++;
     for (const CellRec& c : net->cells)
-        if (use_widened(net, c, net->max_batch, net->max_batch)) net->launches += (all ? 0 : 1) + (c.d_w8_out && !igemm_writes_rows(c.plan8, c.geom.O) ? 1 : 0);
+        if (use_widened(net, c, net->max_batch, net->max_batch)) net->launches += (all ? 0 : 1) + (c.d_w8_out && !stores_rows(c, c.plan8) ? 1 : 0);
     return 0;
 }
 
@@ -1558,7 +1561,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                         igemm_permute_weights(laid.data(), rows.data(), gplan.O, (size_t)g.kH * g.kW * g.Cg, pb);
                         c.plan.perm = pb;
                     }
-                    if (c.pad_O && !igemm_writes_rows(c.plan, g.O)) net->launches++;   // the copy that drops the padding
+                    if (c.pad_O && !stores_rows(c, c.plan)) net->launches++;   // the copy that drops the padding
                     if (w4) rows = pack4(rows);
                     CUDA_TRY(cudaMemcpy(c.d_weights, rows.data(), rows.size(), cudaMemcpyHostToDevice));
                 }
@@ -1746,14 +1749,14 @@ static int widen_weights(n2d2b_net* net, const CellRec& c, cudaStream_t s)
     return 0;
 }
 
-// The implicit GEMM of a cell, and where its columns were padded (into `padded`) its output in place: short launches store the wanted columns from
-// the registers, others leave them to a copy kernel
+// The implicit GEMM of a cell, and where its columns were padded (into `padded`) its output in place: short launches of a classifier store the wanted
+// columns from the registers, others leave them to a copy kernel
 static int run_igemm(n2d2b_net* net, const CellRec& c, IgemmPlan p, const Residual& r, void* padded, void* out, int out_dtype, int batch, int img0, cudaStream_t s)
 {
     const ConvGeom& g = c.geom;
     p.M = batch * g.oH * g.oW;
     const size_t row0 = (size_t)img0 * g.oH * g.oW;
-    if (padded && !img0 && igemm_writes_rows(p, g.O)) {
+    if (padded && !img0 && stores_rows(c, p)) {
         CUDA_TRY(launch_igemm(p, c.q.dev, r, c.fast, padded, out_dtype, 0, net->d_status, s, out, g.O));
         return 0;
     }
