@@ -190,11 +190,13 @@ def cpu_baseline(net, seconds_budget=20.0):
 def launch_groups(net, engines):
     """One entry per kernel launch of a forward pass: (name, layer indices, ops per image, algorithmic bytes per
     image, weight bytes).  A sum folded into a convolution's epilogue belongs to that convolution's launch: the
-    convolution's own output is never written, the residual operand is read once."""
+    convolution's own output is never written, the residual operand is read once.  A convolution folded into another cell's
+    launch belongs to that one: the layer behind a sum (its input is at hand), the branch beside a projection or the depthwise layer
+    in front of a 1x1 one (its output is never written)."""
     from n2d2_b200 import netdesc
     macs, shapes = netdesc.layer_macs(net)
     elems = {k: v[0] * v[1] * v[2] for k, v in shapes.items()}
-    groups, owner = [], {}
+    groups, owner, held = [], {}, {}
     for i, l in enumerate(net['layers']):
         if engines[i] == 'fused' and l['type'] == 'pool':
             # a max pooling folded into the first-layer kernel: that launch writes the pooled tensor only
@@ -205,12 +207,27 @@ def launch_groups(net, engines):
             g['name'] += '+' + l['name']
             owner[i] = owner[conv]
             continue
+        if engines[i] == 'fused' and l['type'] == 'conv':
+            w = float(l['weights'].size * l.get('weight_bits', 8) // 8)
+            src = l['inputs'][0]
+            if src in owner and groups[owner[src]]['engine'] == 'tcgen05-chain':
+                g = groups[owner[src]]
+                for key, more in (('ops', 2.0 * macs[i]), ('bytes', float(elems[i])), ('wbytes', w)):
+                    g[key] += more
+                g['layers'].append(i)
+                g['name'] += '+' + l['name']
+                owner[i] = owner[src]
+                continue
+            reader = next(k for k, r in enumerate(net['layers']) if i in r['inputs'])
+            carrier = reader if net['layers'][reader]['type'] == 'conv' else max(net['layers'][reader]['inputs'])
+            held.setdefault(carrier, []).append((i, w, reader != carrier))
+            continue
         if engines[i] == 'fused':
             conv = max(j for j in l['inputs'] if j >= 0 and net['layers'][j]['type'] == 'conv' and j in owner)
             g = groups[owner[conv]]
             other = [j for j in l['inputs'] if j != conv][0]
             g['layers'].append(i)
-            g['bytes'] += elems[other] + elems[i] - elems[conv]
+            g['bytes'] += (0 if owner.get(other) == owner[conv] else elems[other]) + elems[i] - elems[conv]
             g['name'] += '+sum'
             owner[i] = owner[conv]
             continue
@@ -225,6 +242,14 @@ def launch_groups(net, engines):
         owner[i] = len(groups)
         groups.append({'name': l['name'], 'layers': [i], 'ops': 2.0 * macs[i], 'bytes': float(b), 'wbytes': float(w),
                        'engine': engines[i]})
+        for k, wk, beside in held.pop(i, ()):
+            g, src = groups[-1], net['layers'][k]['inputs'][0]
+            g['ops'] += 2.0 * macs[k]
+            g['wbytes'] += wk
+            g['bytes'] += elems[src] - (0 if beside else elems[k])
+            g['layers'].append(k)
+            g['name'] = net['layers'][k]['name'] + '+' + g['name']
+            owner[k] = owner[i]
     return groups
 
 
@@ -419,13 +444,14 @@ def main():
     probe_tops, probe_cyc = runtime.probe_i8_mma_rate(local_rank, 256, 40000)
     int8_peak = 2.0 * peaks['bf16_burst']
     hbm_peak = peaks['hbm']
-    # the implicit-GEMM kernel and its 256-row variant (same file, same structure) count as one kernel family
-    tc_ms = sum(m for m, e in zip(prof, engines) if e.startswith('tcgen05'))
-    tc_ops = sum(2.0 * mc * B for mc, e in zip(macs, engines) if e.startswith('tcgen05'))
-    tc_launches = sum(1 for e in engines if e.startswith('tcgen05'))
+    # the implicit-GEMM kernel and its variants (256 rows, two layers and a sum, a layer behind a sum) count as one kernel family
+    groups = launch_groups(net, engines)
+    tc = [g for g in groups if g['engine'].startswith('tcgen05')]
+    tc_ms = float(sum(prof[j] for g in tc for j in g['layers']))
+    tc_ops = sum(g['ops'] * B for g in tc)
+    tc_launches = len(tc)
     achieved = tc_ops / (tc_ms * 1e-3) / 1e12 if tc_ms > 0 else 0.0
     # every launch against the roofline that bounds it: max(ops / int8 peak, algorithmic bytes / HBM peak)
-    groups = launch_groups(net, engines)
     rows, bound_sum, meas_sum, tc_alg_bytes = [], 0.0, 0.0, 0.0
     by_kind = {}
     for g in groups:
@@ -444,7 +470,7 @@ def main():
         kind = g['engine'] + (' + fused residual sum' if '+sum' in g['name'] else '')
         k = by_kind.setdefault(kind, [0, 0.0, 0.0])
         k[0] += 1; k[1] += ms; k[2] += bound
-    roofline = {'bound': 'tensor', 'kernel': 'igemm_i8_tcgen05_kernel (with its 256-row variant igemm_pair_i8_tcgen05_kernel)',
+    roofline = {'bound': 'tensor', 'kernel': 'igemm_i8_tcgen05_kernel (with its variants igemm_pair_i8_, igemm_dual_ and igemm_chain_tcgen05_kernel)',
                 'achieved': achieved, 'peak': int8_peak, 'unit': 'TOP/s', 'frac': achieved / int8_peak,
                 'peak_note': f"2 x {peaks['source']} burst bf16 cuBLAS TFLOP/s ({peaks['bf16_burst']}): the kind::i8 pipe "
                              'issues twice the bf16 rate and the timed region is a fraction of a second',
