@@ -10,8 +10,7 @@
 // over between two kernels.
 //
 // Roles, waits and the launch are those of the implicit-GEMM kernel.  What bounds it: the epilogue's issue slots (both rescales and
-// the sum per output value) on layers of few channels, the operand loads (128-column tiles: the sum's region and constants leave no room for
-// 256) on deep ones.
+// the sum per output value) on layers of few channels, the operand loads on deep ones (three ring slots beside tiles of 256 columns).
 #include <algorithm>
 #include <string.h>
 #include "igemm_kernel.cuh"
@@ -337,27 +336,33 @@ static size_t dual_smem_bytes(int stages, int slot_bytes, size_t resident)
          + DUAL_SETS * FAST_NP * 256 * 4 + 64;
 }
 
-// Columns of a tile by the estimate of igemm_tile_columns, for two multiplications and both rescales
+// Columns of a tile by an estimate in cycles like igemm_tile_columns', for two multiplications and both rescales.  Tiles of 128 columns keep two
+// tiles' accumulators in TMEM: the longer of loads and epilogue, and 0.4 of the shorter.  Tiles of 256 keep one: each multiplication runs under the
+// epilogue of the other one, 0.4 of it the branch's.  An activation block then serves twice the columns, which pays where the operand loads bound
+// the tile: 256 + 512 channels into 1024 at 1024 images of 14 x 14 go from 220 us to 172, 512 + 1024 into 2048 at 7 x 7 from 183 to 136 (at 128 images
+// from 31.3 to 26.9), but 64 + 64 into 256 at 55 x 55 and 128 images from 65.7 to 67.9.  Over 33 calls (4 to 1024 images) the choice is within 0.4 % of the
+// best of the three columns for each.
 static int dual_tile_columns(const ConvGeom* g, const int* bk, const bool* im2col, int num_sms)
 {
     const long long m_tiles = ((long long)g[1].B * g[1].oH * g[1].oW + BM - 1) / BM;
-    int best_bn = 64;
-    double best = 0;
-    for (int bn = g[1].O > 64 ? 128 : 64; bn >= 64; bn >>= 1) {
+    auto cost = [&](int bn) {
         const long long n_tiles = (g[1].O + bn - 1) / bn, tiles = m_tiles * n_tiles, per_cta = (tiles + num_sms - 1) / num_sms;
         const double rate = tiles < num_sms ? 114.0 - 43.0 * tiles / num_sms : 71.0;
-        double k = 0, weights = 0;
+        double weights = 0, k[2];
         for (int s = 0; s < 2; ++s) weights += (double)g[s].kH * g[s].kW * g[s].C * bn;
+        const bool resident = bn < 256 && weights <= 96 * 1024 && per_cta > 1;
         for (int s = 0; s < 2; ++s) {
             const double blocks = (double)g[s].kH * g[s].kW * ((g[s].C + bk[s] - 1) / bk[s]);
-            const double load = bk[s] * (BM / (im2col[s] ? std::min(rate, 40.0) : rate) + (weights <= 96 * 1024 && per_cta > 1 ? 0 : bn) / rate);
-            k += blocks * std::max((bn == 128 ? 64.0 : 48.0) * bk[s] / 32, load);
+            const double load = bk[s] * (BM / (im2col[s] ? std::min(rate, 34.0) : rate) + (resident ? 0 : bn) / rate);
+            k[s] = blocks * std::max((bn == 64 ? 48.0 : 0.5 * bn) * bk[s] / 32, load);
         }
-        const double epi = bn * (bn == 128 ? 11.0 : 15.0) * 2.6;
-        const double cost = per_cta * std::max(k, per_cta > 1 ? epi : 0.0) + epi;
-        if (best == 0 || cost < 0.93 * best) { best = cost; best_bn = bn; }
-    }
-    return best_bn;
+        const double epi = bn * (bn == 256 ? 23.0 : (bn == 128 ? 24.0 : 26.0)), sum = k[0] + k[1];
+        const double tile = bn == 256 ? std::max(k[1], 0.4 * epi) + std::max(k[0], 0.6 * epi) : std::max(sum, epi) + 0.4 * std::min(sum, epi);
+        return per_cta * (per_cta > 1 ? tile : sum) + epi * (bn == 256 ? 1.25 : 1.0);
+    };
+    if (g[1].O <= 64) return 64;
+    const int bn = cost(64) < 0.93 * cost(128) ? 64 : 128;
+    return g[1].O > 128 && cost(256) < 0.97 * cost(bn) ? 256 : bn;
 }
 
 // a: the branch, b: the projection, both with the output's extents and weights permuted in blocks of 32 channels

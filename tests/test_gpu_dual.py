@@ -23,10 +23,11 @@ def unit_net(C, mid, H, W, O, k, stride, mode, unsigned_relu=True, clipped=False
 
 
 # (channels of the projection, of the branch, H, W, outputs, filter, stride, batch): K blocks of 32, 64 and 128 bytes on either side, weights
-# resident and streamed, columns of 64 and 128 with a part of a tile, rows that end inside a tile, one tile and many per CTA
+# resident and streamed, columns of 64, 128 and 256 with a part of a tile, rows that end inside a tile, one tile and many per CTA
 CASES = [(64, 64, 13, 11, 256, 1, 1, 3), (64, 64, 28, 28, 256, 1, 1, 40), (256, 128, 14, 14, 512, 1, 2, 7), (512, 256, 9, 9, 1024, 1, 2, 20),
          (1024, 512, 8, 7, 2048, 1, 2, 33), (128, 256, 14, 14, 256, 3, 2, 5), (256, 512, 7, 7, 512, 3, 1, 1), (256, 512, 7, 7, 512, 3, 1, 160),
-         (32, 64, 20, 20, 96, 3, 1, 9), (96, 48, 15, 15, 160, 3, 2, 6), (32, 32, 5, 3, 32, 1, 1, 2), (64, 128, 28, 28, 128, 3, 1, 30)]
+         (32, 64, 20, 20, 96, 3, 1, 9), (96, 48, 15, 15, 160, 3, 2, 6), (32, 32, 5, 3, 32, 1, 1, 2), (64, 128, 28, 28, 128, 3, 1, 30),
+         (512, 256, 14, 14, 1024, 1, 1, 110), (512, 512, 9, 7, 1120, 1, 2, 300), (256, 512, 7, 7, 288, 3, 1, 400), (64, 64, 30, 30, 480, 1, 1, 90)]
 
 
 @pytest.mark.parametrize('case', CASES, ids=lambda c: 'C%d_%d_%dx%d_O%d_k%d_s%d_b%d' % c)
