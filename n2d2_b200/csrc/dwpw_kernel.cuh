@@ -15,7 +15,7 @@
 // whatever is there: their sums are not stored.
 //
 // What bounds it: the latency of the warps' instructions, six to eight cycles each at five working warps a scheduler (65 % of the issue slots); a
-// depthwise output takes eight to nine instructions and a 1x1 output four.  Sixteen-warp groups that did both kinds of work in turn were slower
+// depthwise output takes eight to nine instructions and a 1x1 output four.  The same twenty warps doing both kinds of work in turn were slower
 // (MobileNet at 256 images 814 us against 685): every wait then stalls both.
 // As two kernels the depthwise output crosses L2 or HBM twice, and the pair costs two hand-overs between kernels of 1.3 to 2 us each:
 // 14 x 14 x 512 at 256 images 46 us as two launches by themselves, 33 as one.
