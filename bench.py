@@ -28,11 +28,11 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# DRAM bytes (dram__bytes_read + dram__bytes_write) of the 47 implicit-GEMM launches of one ResNet-50 forward
+# DRAM bytes (dram__bytes_read + dram__bytes_write) of the 41 implicit-GEMM launches of one ResNet-50 forward
 # pass at batch 256, from the ncu capture summarised under profiles/: reported as the batch-256 capture it is
 # (at larger batches less of a layer's output is still in L2 when the next layer reads it).
-IGEMM_DRAM_BYTES_B256_CAPTURE = 4676.53e6
-IGEMM_LAUNCHES_B256_CAPTURE = 47
+IGEMM_DRAM_BYTES_B256_CAPTURE = 3731.49e6
+IGEMM_LAUNCHES_B256_CAPTURE = 41
 
 METRIC = 'int8_resnet50_images_per_sec'
 UNIT = 'images/s'
@@ -479,7 +479,7 @@ def main():
                                'what': 'tcgen05.mma kind::i8 128x256x32 issued back to back on every SM of this GPU, '
                                        'CUDA events (n2d2b_probe_i8_mma_rate)'},
                 'traffic': IGEMM_DRAM_BYTES_B256_CAPTURE / IGEMM_LAUNCHES_B256_CAPTURE,
-                'traffic_note': 'dram__bytes_read+write per launch of an ncu capture at batch 256 (47 launches of one '
+                'traffic_note': 'dram__bytes_read+write per launch of an ncu capture at batch 256 (41 launches of one '
                                 'forward pass), reported at that batch; see profiles/',
                 'traffic_batch': 256,
                 'algorithmic_bytes_per_launch': tc_alg_bytes / max(tc_launches, 1),
