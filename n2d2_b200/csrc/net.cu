@@ -119,16 +119,15 @@ struct CellRec {
     // the two convolutions in front of a sum as one kernel (igemm_dual.cu): on the later one, which carries the sum, the index of the other and the
     // plan; on the other one the index of the later
     int dual_branch = -1, dual_sum = -1;
-    bool dual_on = false;
+    bool dual_on = false, dual_always = false;   // always: in every call (packed weights: only where each call widens them)
     DualPlan dual{};
     PatchPlan dual_patch{};   // or by the patch kernel (proj_in set)
     // an expansion with its residual sum and the 1x1 cell behind it as one kernel (igemm_chain.cu): each other's index
     int chain_next = -1, chain_prev = -1;
-    bool chain_on = false;
     ChainPlan chain{};
     // tensor-core plan
     IgemmPlan plan{};
-    bool has_plan = false;
+    bool probed = false;              // engine, plans and constants were found ahead of the buffers (probe_dense)
     const void* plan_input = nullptr;
     const void* plan_res = nullptr;   // a residual that is the network's input: the address the plan holds
     int plan_images = 0;              // images that the plan's maps over the network's input cover
@@ -930,44 +929,10 @@ static void fuse_residuals(n2d2b_net* net)
     }
 }
 
-// Pairs of convolutions whose outputs only meet in a sum (the branch and the projection of a residual block's first unit): the branch may be computed
-// by the kernel of the later one, so its input has to live until then.  Which pairs are is settled when the kernels are chosen (plan_duals).
-static void mark_duals(n2d2b_net* net)
-{
-    std::vector<int> consumers(net->tensors.size(), 0);
-    for (const CellRec& c : net->cells)
-        if (!c.skipped)
-            for (int i : c.inputs) consumers[i]++;
-    for (size_t bi = 0; bi < net->cells.size(); ++bi) {
-        CellRec& b = net->cells[bi];
-        if (b.skipped || b.type != CELL_CONV || b.residual <= 0 || b.inputs[0] == 0) continue;
-        const int ai = net->tensors[b.residual].producer;
-        if (ai < 0 || ai >= (int)bi || consumers[b.residual] != 1) continue;
-        CellRec& a = net->cells[ai];
-        if (a.skipped || a.type != CELL_CONV || a.residual >= 0 || a.output != b.residual || a.inputs[0] == 0 || a.geom.groups != 1) continue;
-        b.dual_branch = ai;
-        a.dual_sum = (int)bi;
-        b.inputs.push_back(a.inputs[0]);
-    }
-}
-
-// Expansions with a residual sum whose reader is the next cell, a 1x1 one: the kernel of the first may write the output of both, so the second's buffer
-// is taken while the first's operands still have theirs.  Settled when the kernels are chosen (plan_chains).
-static void mark_chains(n2d2b_net* net)
-{
-    for (size_t i = 0; i < net->cells.size(); ++i) {
-        CellRec& c = net->cells[i];
-        if (c.skipped || c.type != CELL_CONV || c.residual <= 0 || c.inputs[0] == 0 || c.wbits != 8 || c.dual_branch >= 0) continue;
-        size_t j = i + 1;
-        while (j < net->cells.size() && net->cells[j].skipped) ++j;
-        if (j == net->cells.size()) continue;
-        CellRec& p = net->cells[j];
-        if (p.type != CELL_CONV || p.residual >= 0 || p.inputs.size() != 1 || p.inputs[0] != c.output || p.wbits != 8 || p.dual_sum >= 0) continue;
-        if (!chain_eligible(c.geom, p.geom) || net->tensors[p.output].dtype != DT_I8) continue;
-        c.chain_next = (int)j;
-        p.chain_prev = (int)i;
-    }
-}
+// Which cells share a kernel is settled before the buffers are planned, because it decides which tensors are stored and how long others live; the same
+// functions then make the plans over the real addresses (plan_duals, plan_chains).
+static int settle_duals(n2d2b_net* net);
+static int settle_chains(n2d2b_net* net);
 
 // Cells [0, n) that the host-buffer entry point may run slice by slice (a structural rule, applied before the
 // kernels are chosen; the engine-based rule in finalize can only shorten it): image-wise cells with large
@@ -987,10 +952,6 @@ static int head_candidate_prefix(const n2d2b_net* net)
     return n;
 }
 
-// Buffers are shared by lifetime.  Cells of the head run once per batch slice at an image offset, so slice k of
-// a head tensor may be written while slices < k of every other head tensor are complete and still needed: two
-// head tensors share a buffer only when they have the same bytes per image (slice k of one then lies exactly
-// over slice k of the other, which the per-slice order of the cells has already retired).
 // A stride-2 first layer whose only reader is a max pooling writes the pooled tensor directly (stem_pool_tcgen05.cu, or on request
 // the POOL variant of the space-to-depth kernel): the convolution's output, the largest tensor of such a network, is never stored.
 static int fuse_stem_pool(n2d2b_net* net);
@@ -998,6 +959,10 @@ static int fuse_stem_pool(n2d2b_net* net);
 // A 3x3 depthwise cell whose only reader is a 1x1 cell becomes part of it (dwpw_tcgen05.cu): its output is never stored.
 static int fuse_depthwise(n2d2b_net* net);
 
+// Buffers are shared by lifetime.  Cells of the head run once per batch slice at an image offset, so slice k of
+// a head tensor may be written while slices < k of every other head tensor are complete and still needed: two
+// head tensors share a buffer only when they have the same bytes per image (slice k of one then lies exactly
+// over slice k of the other, which the per-slice order of the cells has already retired).
 static int plan_buffers(n2d2b_net* net)
 {
     const bool keep_all = (net->flags & N2D2B_KEEP_ALL_OUTPUTS) != 0;
@@ -1037,6 +1002,11 @@ static int plan_buffers(n2d2b_net* net)
             }
         };
         TensorRec& t = net->tensors[c.output];
+        if (c.dual_sum >= 0 && net->cells[c.dual_sum].dual_always) {   // its output stays on chip, its input lives until the sum
+            t.readable = false;
+            t.buffer = -2;
+            continue;
+        }
         if (c.chain_prev < 0) take(t, ci < net->head_limit);   // (else it was taken with the cell in front)
         if (c.chain_next >= 0) take(net->tensors[net->cells[c.chain_next].output], c.chain_next < net->head_limit);
         if (!keep_all) {
@@ -1071,6 +1041,20 @@ static void* tensor_ptr(const n2d2b_net* net, int id, const void* d_input)
     return t.buffer >= 0 ? net->buffers[t.buffer] : nullptr;
 }
 
+// What a plan is made over where a tensor has no address: the network's input before a forward pass (encoded anew then), an output that is never
+// stored, and every tensor while cells that share a kernel are settled
+static void* placeholder()
+{
+    static char bytes[16] __attribute__((aligned(16)));
+    return bytes;
+}
+
+static void* tensor_or_placeholder(const n2d2b_net* net, int id)
+{
+    void* p = tensor_ptr(net, id, nullptr);
+    return p ? p : placeholder();
+}
+
 static int final_tensor_of(const n2d2b_net* net)
 {
     for (int ci = (int)net->cells.size() - 1; ci >= 0; --ci)
@@ -1095,7 +1079,8 @@ static bool patch_as_gemm(const n2d2b_net* net, const CellRec& c, int batch)
 // enough to pay for it whatever its cells are (ResNet-18 at 224 x 224, 1.7 G multiply-accumulates an image: four images 217 us with the expansion in the
 // kernels, 182 widened cell by cell, 162 in one launch; 128 images 656 / 460 / 421: the expansion warps' shared-memory stores bound every layer of long
 // K, and the classifier, which has no 32-bit epilogue in that form, took 38 to 110 us).
-static bool widen_all(const n2d2b_net* net, int call) { return net->w8_macs * call >= (1ll << 29); }
+static bool widens_all(long long macs, int call) { return macs * call >= (1ll << 29); }
+static bool widen_all(const n2d2b_net* net, int call) { return widens_all(net->w8_macs, call); }
 
 // Whether a packed cell takes the widened form in a call of `call` images, `batch` of them at once.  In a smaller call a cell is widened by itself where a
 // CTA has more than two tiles, whose in-kernel expansions would repeat.
@@ -1107,6 +1092,42 @@ static bool use_widened(const n2d2b_net* net, const CellRec& c, int batch, int c
     return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) > 2ll * net->num_sms;
 }
 
+// The implicit-GEMM plan of a dense cell
+static int plan_dense(n2d2b_net* net, CellRec& c, const ConvGeom& g, bool w4, const void* in, const int8_t* w, const void* out, const void* res, const char** why)
+{
+    ConvGeom gb = g;
+    gb.B = net->max_batch;
+    return igemm_make_plan(&c.plan, in, w, out, res, gb, net->tensors[c.inputs[0]].is_unsigned, (net->flags & N2D2B_FORCE_IM2COL) ? 1 : 0, 0, net->num_sms, why,
+                           (net->flags & N2D2B_FORCE_PAIR) ? 1 : 0, w4 ? 1 : 0);
+}
+
+// The kernel of a dense cell whose implicit-GEMM plan is made: its 32-bit constants, the patch kernel where that is the faster one, and the order of its
+// weight rows (plan.perm)
+static int choose_dense(n2d2b_net* net, CellRec& c, bool w4, const void* in, const int8_t* w)
+{
+    ConvGeom g = c.geom;
+    g.B = net->max_batch;
+    const TensorRec& tout = net->tensors[c.output];
+    const bool exact = (net->flags & N2D2B_EXACT64_EPILOGUE) != 0, with_res = c.residual >= 0;
+    const char* why = "";
+    c.engine = ENG_TCGEN05;
+    if (!exact && !c.pad_O && !c.d_fast) {
+        // (the patch kernel's residual stage is not the dot-product form, nor is its sum with a projection)
+        const bool res_i8 = with_res && net->tensors[c.residual].dtype == DT_I8 && (w4 || !patch_takes_residual(g))
+                            && !(c.dual_branch >= 0 && patch_takes_projection(net->cells[c.dual_branch].geom, g));
+        if (int rc = upload_fast(c, tout, res_i8, with_res ? net->tensors[c.residual].is_unsigned : 0, w4)) return rc;
+    }
+    // small-channel stride-1 layers read their input once, from a shared-memory patch
+    if (!w4 && !c.pad_O && c.fast.enabled && (!with_res || (patch_takes_residual(g) && net->tensors[c.residual].dtype == DT_I8)) && tout.dtype == DT_I8
+        && !exact && !(net->flags & N2D2B_FORCE_IM2COL) && patch_eligible(g)
+        && patch_make_plan(&c.patch, in, w, g, net->tensors[c.inputs[0]].is_unsigned, net->num_sms, &why) == 0)
+        c.engine = ENG_PATCH;
+    // (a patch cell's rows are in the order of the implicit GEMM, which small calls may take: patch_as_gemm)
+    if (igemm_uses_fast_epilogue(c.plan, c.fast, with_res, tout.dtype) && (c.engine == ENG_TCGEN05 || igemm_perm_block(c.plan) == 32))
+        c.plan.perm = igemm_perm_block(c.plan);
+    return 0;
+}
+
 // Bytes of widened weights of a packed cell, rounded so that another one's may follow
 static size_t widened_bytes(const CellRec& c)
 {
@@ -1114,15 +1135,46 @@ static size_t widened_bytes(const CellRec& c)
     return (n + 255) & ~(size_t)255;
 }
 
+// Whether a packed cell has a widened form, whose plans are made over the given addresses (out == nullptr: a padded matrix of the cell's own)
+static int plan_widened_cell(n2d2b_net* net, CellRec& c, const void* in, const int8_t* w, void* out, const void* res)
+{
+    ConvGeom g = c.geom;
+    g.B = net->max_batch;
+    const int in_u = net->tensors[c.inputs[0]].is_unsigned;
+    const char* why = "";
+    c.w8_ng_src = c.plan.perm / 8;
+    c.w8_rows = g.O;
+    if ((!res || (patch_takes_residual(g) && !c.fast.dp4a)) && patch_eligible(g) && patch_make_plan(&c.patch8, in, w, g, in_u, net->num_sms, &why) == 0) {
+        c.patch8.late_weights = 1;
+        c.w8_ng_dst = 4;
+        c.w8 = CellRec::W8_PATCH;
+        return 0;
+    }
+    if (!out) {
+        g.O = c.w8_rows = (g.O + 31) & ~31;
+        CUDA_TRY(cudaMalloc(&c.d_w8_out, (size_t)net->max_batch * g.oH * g.oW * g.O + 256));
+        out = c.d_w8_out;
+    }
+    if (igemm_make_plan(&c.plan8, in, w, out, res, g, in_u, 0, 0, net->num_sms, &why) || !igemm_uses_fast_epilogue(c.plan8, c.fast, res != nullptr, DT_I8)) return 0;
+    c.plan8.late_weights = 1;
+    c.plan8.perm = igemm_perm_block(c.plan8);
+    c.w8_ng_dst = c.plan8.perm / 8;
+    c.w8 = CellRec::W8_IGEMM;
+    return 0;
+}
+
+static long long cell_macs(const CellRec& c) { return (long long)c.geom.oH * c.geom.oW * c.geom.O * c.geom.kH * c.geom.kW * c.geom.C; }
+
 // Plans the widened form of every packed cell.  The weights stay packed in HBM; a scratch block holds the int8 weights of the call that is running.
 static int plan_widened(n2d2b_net* net)
 {
     // (not where the input or the residual is the caller's buffer, whose address only the forward pass knows)
-    auto eligible = [](const CellRec& c) {
-        return !c.skipped && c.engine == ENG_TCGEN05 && c.plan.w4 && c.fast.enabled && c.plan_input && c.residual != 0;
+    auto eligible = [&](const CellRec& c) {
+        return !c.skipped && c.engine == ENG_TCGEN05 && c.plan.w4 && c.fast.enabled && c.inputs[0] != 0 && c.residual != 0;
     };
     size_t total = 0;
     for (CellRec& c : net->cells) {
+        c.w8 = CellRec::W8_NONE;
         if (!eligible(c)) continue;
         c.w8_offset = total;
         total += widened_bytes(c);
@@ -1130,39 +1182,15 @@ static int plan_widened(n2d2b_net* net)
     if (!total) return 0;
     CUDA_TRY(cudaMalloc(&net->d_w8, total + 256));
     for (CellRec& c : net->cells) {
-        if (!eligible(c)) continue;
-        ConvGeom g = c.geom;
-        g.B = net->max_batch;
-        const TensorRec& tout = net->tensors[c.output];
-        if (tout.dtype != DT_I8) continue;
-        const int in_u = net->tensors[c.inputs[0]].is_unsigned;
+        if (!eligible(c) || net->tensors[c.output].dtype != DT_I8) continue;
         const void* res = c.residual >= 0 ? tensor_ptr(net, c.residual, nullptr) : nullptr;
-        const char* why = "";
-        c.w8_ng_src = c.plan.perm / 8;
-        c.w8_rows = g.O;
-        if ((!res || (patch_takes_residual(g) && !c.fast.dp4a)) && patch_eligible(g) && patch_make_plan(&c.patch8, c.plan_input, (const int8_t*)net->d_w8 + c.w8_offset, g, in_u, net->num_sms, &why) == 0) {
-            c.patch8.late_weights = 1;
-            c.w8_ng_dst = 4;
-            c.w8 = CellRec::W8_PATCH;
-            continue;
-        }
-        void* out = tensor_ptr(net, c.output, nullptr);
-        if (g.O % 32 != 0) {
-            if (res) continue;
-            g.O = c.w8_rows = (g.O + 31) & ~31;
-            CUDA_TRY(cudaMalloc(&c.d_w8_out, (size_t)net->max_batch * g.oH * g.oW * g.O + 256));
-            out = c.d_w8_out;
-        }
-        if (igemm_make_plan(&c.plan8, c.plan_input, (const int8_t*)net->d_w8 + c.w8_offset, out, res, g, in_u, 0, 0, net->num_sms, &why)
-            || !igemm_uses_fast_epilogue(c.plan8, c.fast, res != nullptr, DT_I8))
-            continue;
-        c.plan8.late_weights = 1;
-        c.plan8.perm = igemm_perm_block(c.plan8);
-        c.w8_ng_dst = c.plan8.perm / 8;
-        c.w8 = CellRec::W8_IGEMM;
+        if (c.residual >= 0 && !res) res = placeholder();
+        if (c.geom.O % 32 != 0 && res) continue;
+        if (int rc = plan_widened_cell(net, c, c.plan_input, (const int8_t*)net->d_w8 + c.w8_offset, c.geom.O % 32 ? nullptr : tensor_or_placeholder(net, c.output), res))
+            return rc;
     }
     for (const CellRec& c : net->cells)
-        if (c.w8 != CellRec::W8_NONE) net->w8_macs += (long long)c.geom.oH * c.geom.oW * c.geom.O * c.geom.kH * c.geom.kW * c.geom.C;
+        if (c.w8 != CellRec::W8_NONE) net->w8_macs += cell_macs(c);
     const bool all = widen_all(net, net->max_batch);
     if (all) net->launches++;
     for (const CellRec& c : net->cells)
@@ -1178,64 +1206,184 @@ static bool use_dual(const n2d2b_net* net, const CellRec& b, int batch, int call
     return !a.plan.w4 || (use_widened(net, a, batch, call) && use_widened(net, b, batch, call));
 }
 
-static int plan_duals(n2d2b_net* net)
+// The pair of cell `b`, which carries the sum, and its branch as one kernel, planned over the given addresses; false where they stay two
+static bool make_dual(n2d2b_net* net, CellRec& b, const void* in_a, const int8_t* w_a, const void* in_b, const int8_t* w_b, const void* out)
 {
+    CellRec& a = net->cells[b.dual_branch];
+    const bool packed = a.plan.w4 && b.plan.w4;
+    if (b.engine != ENG_TCGEN05 || (a.engine != ENG_TCGEN05 && a.engine != ENG_PATCH) || a.plan.w4 != b.plan.w4) return false;
+    if (!a.fast.enabled || !b.fast.enabled || !b.fast.fq2 || net->tensors[b.output].dtype != DT_I8 || net->tensors[a.output].dtype != DT_I8) return false;
+    // one order of weight rows for both: blocks of 32 channels
+    if (packed ? (a.w8 == CellRec::W8_NONE || b.w8 == CellRec::W8_NONE || a.w8_ng_dst != 4 || b.w8_ng_dst != 4)
+               : (b.plan.perm != 32 || (a.engine == ENG_TCGEN05 && a.plan.perm != 32)))
+        return false;
+    ConvGeom ga = a.geom, gb = b.geom;
+    ga.B = gb.B = net->max_batch;
+    const char* why = "";
+    // The patch kernel reads a 64-channel branch's input once, an im2col map nine times: 64 -> 64 channels of 55 x 55 with its projection at 2048 images
+    // 596 us as two kernels, 718 as one of im2col loads; 128 channels of 28 x 28 400 / 290
+    if ((a.engine == ENG_PATCH || a.w8 == CellRec::W8_PATCH) && ga.C <= 64) {
+        // (a wide form's clamp is one at 0: both rescales have it or neither)
+        if (!patch_takes_projection(ga, gb) || b.fast.dp4a || a.fast.form != b.fast.form || (a.fast.form == EF_WIDE && a.fast.need_clamp != b.fast.need_clamp)) return false;
+        if (patch_make_plan(&b.dual_patch, in_a, w_a, ga, net->tensors[a.inputs[0]].is_unsigned, net->num_sms, &why)
+            || patch_add_projection(&b.dual_patch, in_b, w_b, ga, net->tensors[b.inputs[0]].is_unsigned, &why)) {
+            b.dual_patch.proj_in = nullptr;
+            return false;
+        }
+        b.dual_patch.late_weights = packed ? 1 : 0;
+        return true;
+    }
+    return dual_make_plan(&b.dual, in_a, w_a, ga, net->tensors[a.inputs[0]].is_unsigned, in_b, w_b, gb, net->tensors[b.inputs[0]].is_unsigned, out, net->num_sms, &why) == 0;
+}
+
+// The same for cell `c`, an expansion with its residual sum, and the 1x1 cell behind it
+static bool make_chain(n2d2b_net* net, CellRec& c, const void* in, const int8_t* w, const void* out, const void* res, const int8_t* w_next)
+{
+    const CellRec& p = net->cells[c.chain_next];
+    if (c.engine != ENG_TCGEN05 || p.engine != ENG_TCGEN05 || !c.fast.enabled || !c.fast.fq2 || !p.fast.enabled || c.plan.perm != 32 || p.plan.perm != 32
+        || net->tensors[c.output].dtype != DT_I8)
+        return false;
+    ConvGeom g = c.geom;
+    g.B = net->max_batch;
+    const char* why = "";
+    return chain_make_plan(&c.chain, in, w, out, res, g, net->tensors[c.inputs[0]].is_unsigned, w_next, p.geom, net->tensors[c.output].is_unsigned, net->num_sms, &why) == 0;
+}
+
+// Kernel and constants of a cell that may share a kernel with another one, ahead of its buffers; false where it is not a dense cell of whole blocks of columns.
+// (The constants are kept, the plans are made again over the real addresses.)
+static int probe_dense(n2d2b_net* net, CellRec& c, bool* dense)
+{
+    *dense = c.probed;
+    if (c.probed) return 0;
+    const ConvGeom& g = c.geom;
+    if (c.dw_cell >= 0 || g.groups != 1 || g.C % 16 != 0 || g.O % 32 != 0) return 0;
+    const char* why = "";
+    void* const at = placeholder();
+    const void* const out = net->tensors[c.output].dtype == DT_I8 ? at : nullptr;
+    const void* const res = c.residual >= 0 ? at : nullptr;
+    bool w4 = c.wbits == 4;
+    int planned = plan_dense(net, c, g, w4, at, (const int8_t*)at, out, res, &why);
+    if (planned != 0 && w4) {
+        w4 = false;
+        planned = plan_dense(net, c, g, w4, at, (const int8_t*)at, out, res, &why);
+    }
+    if (planned != 0) return 0;
+    if (int rc = choose_dense(net, c, w4, at, (const int8_t*)at)) return rc;
+    if (w4 && c.engine == ENG_TCGEN05 && c.fast.enabled && c.inputs[0] != 0 && c.residual != 0 && out)
+        if (int rc = plan_widened_cell(net, c, at, (const int8_t*)at, at, res)) return rc;
+    *dense = c.probed = true;
+    return 0;
+}
+
+// What probe_dense found for a cell does not hold any more
+static void forget_probe(CellRec& c)
+{
+    cudaFree(c.d_fast);
+    c.d_fast = nullptr;
+    c.fast = FastQuant{};
+    c.probed = false;
+    c.w8 = CellRec::W8_NONE;
+}
+
+// Pairs of convolutions whose outputs only meet in a sum, the branch and the projection of a residual block's first unit: the branch is computed by the
+// kernel of the later one, so its input lives until then and its output is not stored
+static int settle_duals(n2d2b_net* net)
+{
+    std::vector<int> consumers(net->tensors.size(), 0);
+    for (const CellRec& c : net->cells)
+        if (!c.skipped)
+            for (int i : c.inputs) consumers[i]++;
+    const void* const at = placeholder();
+    const int8_t* const w = (const int8_t*)at;
+    bool packed = false;
     for (size_t bi = 0; bi < net->cells.size(); ++bi) {
         CellRec& b = net->cells[bi];
+        if (b.skipped || b.type != CELL_CONV || b.residual <= 0 || b.inputs[0] == 0) continue;
+        const int ai = net->tensors[b.residual].producer;
+        if (ai < 0 || ai >= (int)bi || consumers[b.residual] != 1) continue;
+        CellRec& a = net->cells[ai];
+        if (a.skipped || a.type != CELL_CONV || a.residual >= 0 || a.output != b.residual || a.inputs[0] == 0 || a.geom.groups != 1) continue;
+        b.dual_branch = ai;
+        bool both = false;
+        if (int rc = probe_dense(net, a, &both)) return rc;
+        if (both)
+            if (int rc = probe_dense(net, b, &both)) return rc;
+        if (!both || !make_dual(net, b, at, w, at, w, at)) {
+            b.dual_branch = -1;
+            forget_probe(b);   // (its constants may be those of the shared kernel)
+            continue;
+        }
+        a.dual_sum = (int)bi;
+        b.inputs.push_back(a.inputs[0]);
+        b.dual_always = !b.plan.w4;
+        packed = packed || b.plan.w4;
+    }
+    if (!packed) return 0;
+    // packed weights share a kernel where they are widened: in every call, if a single image is enough for that
+    long long macs = 0;
+    for (CellRec& c : net->cells) {
+        bool dense = false;
+        if (c.skipped || (c.type != CELL_CONV && c.type != CELL_FC) || c.wbits != 4) continue;
+        if (int rc = probe_dense(net, c, &dense)) return rc;
+        if (c.w8 != CellRec::W8_NONE) macs += cell_macs(c);
+    }
+    for (CellRec& b : net->cells)
+        if (b.dual_branch >= 0 && widens_all(macs, 1)) b.dual_always = true;
+    return 0;
+}
+
+// Expansions with a residual sum whose reader is the next cell, a 1x1 one: the kernel of the first writes the output of both, so the second's buffer
+// is taken while the first's operands still have theirs
+static int settle_chains(n2d2b_net* net)
+{
+    const void* const at = placeholder();
+    const int8_t* const w = (const int8_t*)at;
+    for (size_t i = 0; i < net->cells.size(); ++i) {
+        CellRec& c = net->cells[i];
+        if (c.skipped || c.type != CELL_CONV || c.residual <= 0 || c.inputs[0] == 0 || c.wbits != 8 || c.dual_branch >= 0) continue;
+        size_t j = i + 1;
+        while (j < net->cells.size() && net->cells[j].skipped) ++j;
+        if (j == net->cells.size()) continue;
+        CellRec& p = net->cells[j];
+        if (p.type != CELL_CONV || p.residual >= 0 || p.inputs.size() != 1 || p.inputs[0] != c.output || p.wbits != 8 || p.dual_sum >= 0) continue;
+        if (!chain_eligible(c.geom, p.geom) || net->tensors[p.output].dtype != DT_I8) continue;
+        c.chain_next = (int)j;
+        bool both = false;
+        if (int rc = probe_dense(net, c, &both)) return rc;
+        if (both)
+            if (int rc = probe_dense(net, p, &both)) return rc;
+        if (!both || !make_chain(net, c, at, w, at, at, w)) {
+            c.chain_next = -1;
+            continue;
+        }
+        p.chain_prev = (int)i;
+    }
+    return 0;
+}
+
+static int plan_duals(n2d2b_net* net)
+{
+    for (CellRec& b : net->cells) {
         if (b.dual_branch < 0) continue;
         CellRec& a = net->cells[b.dual_branch];
-        const bool packed = a.plan.w4 && b.plan.w4;
-        if (b.engine != ENG_TCGEN05 || (a.engine != ENG_TCGEN05 && a.engine != ENG_PATCH) || a.plan.w4 != b.plan.w4 || a.pad_O || b.pad_O) continue;
-        if (!a.fast.enabled || !b.fast.enabled || !b.fast.fq2 || net->tensors[b.output].dtype != DT_I8 || net->tensors[a.output].dtype != DT_I8) continue;
-        // one order of weight rows for both: blocks of 32 channels
-        if (packed ? (a.w8 == CellRec::W8_NONE || b.w8 == CellRec::W8_NONE || a.d_w8_out || b.d_w8_out || a.w8_ng_dst != 4 || b.w8_ng_dst != 4)
-                   : (b.plan.perm != 32 || (a.engine == ENG_TCGEN05 && a.plan.perm != 32)))
-            continue;
-        // (slices of the upload: both or neither)
-        if ((b.dual_branch < net->head_cells) != ((int)bi < net->head_cells)) continue;
-        ConvGeom ga = a.geom, gb = b.geom;
-        ga.B = gb.B = net->max_batch;
-        const int8_t* wa = packed ? (const int8_t*)net->d_w8 + a.w8_offset : a.d_weights;
-        const int8_t* wb = packed ? (const int8_t*)net->d_w8 + b.w8_offset : b.d_weights;
-        const char* why = "";
-        // The patch kernel reads a 64-channel branch's input once, an im2col map nine times: 64 -> 64 channels of 55 x 55 with its projection at 2048 images
-        // 596 us as two kernels, 718 as one of im2col loads; 128 channels of 28 x 28 400 / 290
-        if ((a.engine == ENG_PATCH || a.w8 == CellRec::W8_PATCH) && ga.C <= 64) {
-            // (a wide form's clamp is one at 0: both rescales have it or neither)
-            if (!patch_takes_projection(ga, gb) || b.fast.dp4a || a.fast.form != b.fast.form || (a.fast.form == EF_WIDE && a.fast.need_clamp != b.fast.need_clamp)) continue;
-            if (patch_make_plan(&b.dual_patch, tensor_ptr(net, a.inputs[0], nullptr), wa, ga, net->tensors[a.inputs[0]].is_unsigned, net->num_sms, &why)
-                || patch_add_projection(&b.dual_patch, tensor_ptr(net, b.inputs[0], nullptr), wb, ga, net->tensors[b.inputs[0]].is_unsigned, &why)) {
-                b.dual_patch.proj_in = nullptr;
-                continue;
-            }
-            b.dual_patch.late_weights = packed ? 1 : 0;
-        } else if (dual_make_plan(&b.dual, tensor_ptr(net, a.inputs[0], nullptr), wa, ga, net->tensors[a.inputs[0]].is_unsigned, tensor_ptr(net, b.inputs[0], nullptr), wb,
-                           gb, net->tensors[b.inputs[0]].is_unsigned, tensor_ptr(net, b.output, nullptr), net->num_sms, &why))
-            continue;
+        const bool packed = a.plan.w4;
+        if (!make_dual(net, b, tensor_ptr(net, a.inputs[0], nullptr), packed ? (const int8_t*)net->d_w8 + a.w8_offset : a.d_weights, tensor_ptr(net, b.inputs[0], nullptr),
+                       packed ? (const int8_t*)net->d_w8 + b.w8_offset : b.d_weights, tensor_ptr(net, b.output, nullptr)))
+            return fail(N2D2B_ERR_STATE, "internal: a branch and its projection without a plan");
         b.dual_on = true;
         if (use_dual(net, b, net->max_batch, net->max_batch)) net->launches--;
+        else if (b.dual_always) return fail(N2D2B_ERR_STATE, "internal: a branch without a buffer");
     }
     return 0;
 }
 
 static int plan_chains(n2d2b_net* net)
 {
-    for (size_t ci = 0; ci < net->cells.size(); ++ci) {
-        CellRec& c = net->cells[ci];
+    for (CellRec& c : net->cells) {
         if (c.chain_next < 0) continue;
-        CellRec& p = net->cells[c.chain_next];
-        if (c.engine != ENG_TCGEN05 || p.engine != ENG_TCGEN05 || !c.fast.enabled || !c.fast.fq2 || !p.fast.enabled || c.plan.perm != 32 || p.plan.perm != 32
-            || net->tensors[c.output].dtype != DT_I8)
-            continue;
-        // (slices of the upload: both or neither)
-        if (((int)ci < net->head_cells) != (c.chain_next < net->head_cells)) continue;
-        ConvGeom g = c.geom;
-        g.B = net->max_batch;
-        const char* why = "";
-        if (chain_make_plan(&c.chain, tensor_ptr(net, c.inputs[0], nullptr), c.d_weights, tensor_ptr(net, c.output, nullptr), tensor_ptr(net, c.residual, nullptr), g,
-                            net->tensors[c.inputs[0]].is_unsigned, p.d_weights, p.geom, net->tensors[c.output].is_unsigned, net->num_sms, &why))
-            continue;
-        c.chain_on = true;
+        if (!make_chain(net, c, tensor_ptr(net, c.inputs[0], nullptr), c.d_weights, tensor_ptr(net, c.output, nullptr), tensor_ptr(net, c.residual, nullptr),
+                        net->cells[c.chain_next].d_weights))
+            return fail(N2D2B_ERR_STATE, "internal: an expansion and the cell behind it without a plan");
         net->launches--;
     }
     return 0;
@@ -1297,9 +1445,6 @@ static bool dw3x3_faster(const ConvGeom& g, int batch)
 static bool use_dw3x3(const CellRec& c, int batch) { return c.d_dw3x3 && dw3x3_faster(c.geom, batch); }
 
 static int plan_dwpw(n2d2b_net* net, CellRec& c);
-static int plan_duals(n2d2b_net* net);
-static int plan_chains(n2d2b_net* net);
-
 int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
 {
     if (!net) return fail(N2D2B_ERR_INVALID, "net must not be NULL");
@@ -1316,8 +1461,8 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                    | N2D2B_FORCE_PAIR)))
         if (int rc = fuse_depthwise(net)) return rc;
     if (!(flags & (N2D2B_NO_FUSION | N2D2B_KEEP_ALL_OUTPUTS | N2D2B_FORCE_SIMT | N2D2B_EXACT64_EPILOGUE | N2D2B_FORCE_IM2COL | N2D2B_FORCE_PAIR))) {
-        mark_duals(net);
-        mark_chains(net);
+        if (int rc = settle_duals(net)) return rc;
+        if (int rc = settle_chains(net)) return rc;
     }
     net->head_limit = head_candidate_prefix(net);
     if (int rc = plan_buffers(net)) return rc;
@@ -1433,8 +1578,7 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
             gb.B = max_batch;
             const char* why = "";
             const void* in_ptr = tensor_ptr(net, c.inputs[0], nullptr);
-            static char dw_placeholder[16] __attribute__((aligned(16)));
-            const void* enc_ptr = in_ptr ? in_ptr : (const void*)dw_placeholder;
+            const void* enc_ptr = in_ptr ? in_ptr : placeholder();
             if (tensor && patch_eligible(gb)) {
                 std::vector<int8_t> arranged(patch_dw_weight_bytes(g));
                 if (int rc = alloc_blocks(arranged.size())) return rc;
@@ -1462,7 +1606,6 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                     c.plan.perm = pb;
                     if (int rc = upload_blocks(rows)) return rc;
                     c.engine = ENG_TCGEN05;
-                    c.has_plan = true;
                     c.plan_input = in_ptr;
                     continue;
                 }
@@ -1497,21 +1640,13 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
         CUDA_TRY(cudaMemset(c.d_weights, 0, c.d_weight_bytes + 256));
         if (!w4) CUDA_TRY(cudaMemcpy(c.d_weights, laid.data(), laid.size(), cudaMemcpyHostToDevice));
         if (igemm_shape) {
-            ConvGeom gb = gplan;
-            gb.B = max_batch;
             const char* why = "";
+            // the network input pointer is only known at forward time; its map is encoded again on first use
             const void* in_ptr = tensor_ptr(net, c.inputs[0], nullptr);
-            // the network input pointer is only known at forward time; plan against a placeholder
-            // that is re-encoded on first use
-            static char placeholder[16] __attribute__((aligned(16)));
-            const void* enc_ptr = in_ptr ? in_ptr : (const void*)placeholder;
-            const void* out_ptr = c.pad_O ? c.d_colpad
-                                : net->tensors[c.output].dtype == DT_I8 ? tensor_ptr(net, c.output, nullptr) : nullptr;
-            const void* res_ptr = c.residual == 0 ? (const void*)placeholder
-                                : c.residual > 0 ? tensor_ptr(net, c.residual, nullptr) : nullptr;
-            int planned = igemm_make_plan(&c.plan, enc_ptr, c.d_weights, out_ptr, res_ptr, gb, net->tensors[c.inputs[0]].is_unsigned,
-                                          (flags & N2D2B_FORCE_IM2COL) ? 1 : 0, 0, net->num_sms, &why,
-                                          (flags & N2D2B_FORCE_PAIR) ? 1 : 0, w4 ? 1 : 0);
+            const void* enc_ptr = in_ptr ? in_ptr : placeholder();
+            const void* out_ptr = c.pad_O ? c.d_colpad : net->tensors[c.output].dtype == DT_I8 ? tensor_or_placeholder(net, c.output) : nullptr;
+            const void* res_ptr = c.residual >= 0 ? tensor_or_placeholder(net, c.residual) : nullptr;
+            int planned = plan_dense(net, c, gplan, w4, enc_ptr, c.d_weights, out_ptr, res_ptr, &why);
             if (planned != 0 && w4) {
                 // no room for the packed variant: widen the weights after all
                 w4 = false;
@@ -1521,46 +1656,19 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
                 CUDA_TRY(cudaMalloc((void**)&c.d_weights, laid.size() + 256));
                 CUDA_TRY(cudaMemset(c.d_weights, 0, laid.size() + 256));
                 CUDA_TRY(cudaMemcpy(c.d_weights, laid.data(), laid.size(), cudaMemcpyHostToDevice));
-                planned = igemm_make_plan(&c.plan, enc_ptr, c.d_weights, out_ptr, res_ptr, gb, net->tensors[c.inputs[0]].is_unsigned,
-                                          (flags & N2D2B_FORCE_IM2COL) ? 1 : 0, 0, net->num_sms, &why,
-                                          (flags & N2D2B_FORCE_PAIR) ? 1 : 0, 0);
+                planned = plan_dense(net, c, gplan, w4, enc_ptr, c.d_weights, out_ptr, res_ptr, &why);
             }
             if (planned == 0) {
-                c.engine = ENG_TCGEN05;
-                c.has_plan = true;
+                if (int rc = choose_dense(net, c, w4, enc_ptr, c.d_weights)) return rc;
                 c.plan_input = in_ptr;  // nullptr = must be re-encoded with the real input
-                if (!(flags & N2D2B_EXACT64_EPILOGUE) && !c.pad_O) {
-                    // (the patch kernel's residual stage is not the dot-product form, nor is its sum with a projection)
-                    const bool res_i8 = c.residual >= 0 && net->tensors[c.residual].dtype == DT_I8 && (w4 || !patch_takes_residual(gb))
-                                        && !(c.dual_branch >= 0 && patch_takes_projection(net->cells[c.dual_branch].geom, g));
-                    if (int rc = upload_fast(c, net->tensors[c.output], res_i8,
-                                             c.residual >= 0 ? net->tensors[c.residual].is_unsigned : 0, w4))
-                        return rc;
-                }
-                // small-channel stride-1 layers read their input once, from a shared-memory patch
-                if (!w4 && !c.pad_O && c.fast.enabled && (c.residual < 0 || (patch_takes_residual(gb) && net->tensors[c.residual].dtype == DT_I8))
-                    && net->tensors[c.output].dtype == DT_I8
-                    && !(flags & (N2D2B_FORCE_IM2COL | N2D2B_EXACT64_EPILOGUE)) && patch_eligible(gb)
-                    && patch_make_plan(&c.patch, enc_ptr, c.d_weights, gb, net->tensors[c.inputs[0]].is_unsigned,
-                                       net->num_sms, &why) == 0)
-                    c.engine = ENG_PATCH;
-                // a cell that stays on the implicit-GEMM kernel with the 32-bit epilogue stores its weight rows in
-                // the permuted order that epilogue reads (see perm_block)
-                const bool permute = c.engine == ENG_TCGEN05
-                                     && igemm_uses_fast_epilogue(c.plan, c.fast, c.residual >= 0, net->tensors[c.output].dtype);
+                // weight rows in the permuted order that the 32-bit epilogue reads (see perm_block)
                 if (c.engine == ENG_PATCH) {
-                    // (the same order of rows as the implicit GEMM's, which small calls may take: patch_as_gemm)
-                    if (igemm_uses_fast_epilogue(c.plan, c.fast, c.residual >= 0, DT_I8) && igemm_perm_block(c.plan) == 32) c.plan.perm = 32;
                     std::vector<int8_t> rows(laid.size());
                     patch_permute_weights(laid.data(), rows.data(), g.O, (size_t)g.kH * g.kW * g.Cg);
                     CUDA_TRY(cudaMemcpy(c.d_weights, rows.data(), rows.size(), cudaMemcpyHostToDevice));
-                } else if (permute || w4) {
+                } else if (c.plan.perm || w4) {
                     std::vector<int8_t> rows = laid;
-                    if (permute) {
-                        const int pb = igemm_perm_block(c.plan);
-                        igemm_permute_weights(laid.data(), rows.data(), gplan.O, (size_t)g.kH * g.kW * g.Cg, pb);
-                        c.plan.perm = pb;
-                    }
+                    if (c.plan.perm) igemm_permute_weights(laid.data(), rows.data(), gplan.O, (size_t)g.kH * g.kW * g.Cg, c.plan.perm);
                     if (c.pad_O && !stores_rows(c, c.plan)) net->launches++;   // the copy that drops the padding
                     if (w4) rows = pack4(rows);
                     CUDA_TRY(cudaMemcpy(c.d_weights, rows.data(), rows.size(), cudaMemcpyHostToDevice));
@@ -1599,6 +1707,11 @@ int n2d2b_net_finalize(n2d2b_net* net, int max_batch, unsigned flags)
         }
         if (!sliceable || (int)ci >= net->head_limit) break;
         net->head_cells = (int)ci + 1;
+    }
+    // cells that share a kernel are in the head together or not at all
+    for (int ci = net->head_cells - 1; ci >= 0; --ci) {
+        const CellRec& c = net->cells[ci];
+        if (c.dual_sum >= net->head_cells || c.chain_next >= net->head_cells) net->head_cells = ci;
     }
     if (int rc = plan_duals(net)) return rc;
     if (int rc = plan_chains(net)) return rc;
@@ -1769,7 +1882,7 @@ static int run_igemm(n2d2b_net* net, const CellRec& c, IgemmPlan p, const Residu
 static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, cudaStream_t s, int img0 = 0)
 {
     if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], batch, net->call_batch)) return 0;   // computed by the cell that carries the sum
-    if (c.chain_prev >= 0 && net->cells[c.chain_prev].chain_on) return 0;   // written by the cell in front
+    if (c.chain_prev >= 0) return 0;   // written by the cell in front
     const void* in0 = tensor_ptr(net, c.inputs[0], d_input);
     void* out = tensor_ptr(net, c.output, d_input);
     const TensorRec& tin = net->tensors[c.inputs[0]];
@@ -1793,7 +1906,7 @@ static int run_cell(n2d2b_net* net, CellRec& c, const void* d_input, int batch, 
     // the maps and the loads of a residual start on 16 bytes; the network's input is the caller's buffer
     if (c.residual == 0 && mapped && ((uintptr_t)r.ptr & 15))
         return fail(N2D2B_ERR_INVALID, "a residual sum cannot read an input at %p: operands must be 16-byte aligned", r.ptr);
-    if (c.chain_on) {
+    if (c.chain_next >= 0) {
         const CellRec& p = net->cells[c.chain_next];
         const int pixels = c.geom.oH * c.geom.oW;
         CUDA_TRY(launch_chain(c.chain, batch * pixels, c.fast, r.is_unsigned, p.fast, tensor_ptr(net, p.output, d_input), img0 * pixels, net->d_status, s));
@@ -2292,8 +2405,8 @@ const char* n2d2b_net_cell_engine(const n2d2b_net* net, int cell)
     const CellRec& c = net->cells[cell];
     if (c.dual_sum >= 0 && use_dual(net, net->cells[c.dual_sum], net->max_batch, net->max_batch)) return "fused";
     if (c.dual_branch >= 0 && use_dual(net, c, net->max_batch, net->max_batch)) return c.dual_patch.proj_in ? "patch-tcgen05-dual" : "tcgen05-dual";
-    if (c.chain_prev >= 0 && net->cells[c.chain_prev].chain_on) return "fused";
-    if (c.chain_on) return "tcgen05-chain";
+    if (c.chain_prev >= 0) return "fused";
+    if (c.chain_next >= 0) return "tcgen05-chain";
     if (use_dw3x3(c, net->max_batch)) return "depthwise";
     if (use_widened(net, c, net->max_batch, net->max_batch)) return c.w8 == CellRec::W8_PATCH ? "patch-tcgen05-widened" : "tcgen05-widened";
     switch (c.engine) {

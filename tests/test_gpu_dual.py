@@ -88,3 +88,31 @@ def test_patch_branch_and_projection_with_packed_weights_and_slices():
         assert np.array_equal(qn.forward_host(x).astype(np.int64), ref)
     finally:
         qn.close()
+
+
+def _bytes_held(net, batch):
+    import torch
+    torch.zeros(1, device='cuda')
+    runtime.QuantizedNet(net, 1).close()   # (what the process itself takes)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    qn = runtime.QuantizedNet(net, batch)
+    torch.cuda.synchronize()
+    held = before - torch.cuda.mem_get_info()[0]
+    eng = qn.engines()
+    qn.close()
+    return held, eng
+
+
+# The branch's output has no buffer where the pair is one kernel in every call (packed weights: where a single image is enough to widen them); a pair
+# that stays two kernels (a 64-channel 3x3 branch whose projection reads 128 channels) does not keep the branch's input until the sum, which takes its place.
+@pytest.mark.parametrize('case, weight_bits, engine', [((256, 256, 256, 1), 8, ENGINE), ((256, 256, 256, 1), 4, ENGINE), ((128, 64, 64, 3), 8, None)],
+                         ids=['fused', 'packed', 'separate'])
+def test_only_what_is_stored_has_a_buffer(case, weight_bits, engine):
+    C, mid, O, k = case
+    images = 56 * 56 * 120
+    held, eng = _bytes_held(unit_net(C, mid, 56, 56, O, k, 1, 'fixed', weight_bits=weight_bits, clipped=weight_bits == 4), 120)
+    assert (ENGINE in eng) == (engine is not None)
+    # the front, the reduction and the sum, or the branch's output and the sum in place of the reduction; the staging of the host's calls (16 channels in, 32
+    # out); weights, constants and the steps of 2 MiB that the device hands out
+    assert held <= (C + mid + O + 16 + 32) * images + (24 << 20)
