@@ -56,6 +56,16 @@ def kernels_of(qn, batch):
     return names
 
 
+def kernels_of_host_call(qn, x):
+    """The output of a call on host buffers and the names of the kernels that ran for it."""
+    import torch
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        out = qn.forward_host(x)
+        torch.cuda.synchronize()
+    return out, [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+
+
 def compare_net(net, batch, flags=KEEP, flavour='i64', x=None, want_engine=None, slices=0, ref=None, kernels=False):
     """Returns (number of compared layers, engines), or with `kernels` the kernels that ran. Asserts bit-exact equality with the
     oracle."""

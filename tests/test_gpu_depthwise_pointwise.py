@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from gpu_common import compare_net
+from gpu_common import compare_net, kernels_of_host_call
 from n2d2_b200 import netdesc, runtime
 from oracle import oracle
 
@@ -49,7 +49,26 @@ def test_calls_of_any_size_on_one_network():
         assert qn.engines().count(ENGINE) == 13
         for batch in (40, 1, 7, 39, 2, 40):
             assert np.array_equal(qn.forward_host(x[:batch]).astype(np.int64), ref[:batch])
-        qn.set_slices(5)
-        assert np.array_equal(qn.forward_host(x).astype(np.int64), ref)
+    finally:
+        qn.close()
+
+
+# The leading cells of a host call run slice by slice while their outputs have 2048 pixels and more: one segment to a row and several, a patch of one tile
+# and of several, slices of one image and of three (weights 2, 2, 2, 1)
+@pytest.mark.parametrize('case', [(32, 56, 56, 64, 1), (64, 112, 112, 128, 2), (128, 48, 50, 160, 1), (32, 16, 260, 96, 1)], ids=lambda c: 'C%d_%dx%d_N%d_s%d' % c)
+@pytest.mark.parametrize('mode', ['single', 'float'])
+def test_slices_of_the_upload(case, mode):
+    C, H, W, N, s = case
+    net = pair_net(C, H, W, N, s, 1, mode)
+    x = netdesc.make_input(net, 11)
+    ref = oracle.run_net(net, x, 'i64')[-1].reshape(11, -1)
+    qn = runtime.QuantizedNet(net, 11)
+    try:
+        assert qn.engines()[2] == ENGINE
+        qn.set_slices(4)
+        for batch in (11, 7, 10):
+            out, kernels = kernels_of_host_call(qn, x[:batch])
+            assert sum('dwpw' in k for k in kernels) == 4
+            assert np.array_equal(out.astype(np.int64), ref[:batch])
     finally:
         qn.close()

@@ -10,14 +10,18 @@ pytestmark = pytest.mark.gpu
 ENGINE = 'tcgen05-dual'
 
 
-def unit_net(C, mid, H, W, O, k, stride, mode, unsigned_relu=True, clipped=False, act='linear', weight_bits=8, seed=5):
-    """A residual block's first unit: conv -> branch (k x k) beside a 1x1 projection of its input, their sum, and a cell that reads it."""
+def unit_net(C, mid, H, W, O, k, stride, mode, unsigned_relu=True, clipped=False, act='linear', weight_bits=8, seed=5, projection_first=False):
+    """A residual block's first unit: conv -> branch (k x k) beside a 1x1 projection of its input, their sum, and a cell that reads it.  The later one of
+    branch and projection carries the sum.  mid = 0: both read the same tensor."""
     dist = ('normal', 30) if weight_bits == 8 else ('uniform', 7)
     b = netdesc.NetBuilder('unit', 16, H, W, seed, mode, unsigned_relu=unsigned_relu, weight_dist=dist, clipped=clipped, weight_bits=weight_bits)
     x = b.conv(-1, C, 1, name='front')
-    y = b.conv(x, mid, 1, name='reduce')
+    y = b.conv(x, mid, 1, name='reduce') if mid else x
+    if projection_first:
+        p = b.conv(x, O, 1, stride=stride, act=act, name='projection')
     y = b.conv(y, O, k, stride=stride, pad=k // 2, act=act, name='branch')
-    p = b.conv(x, O, 1, stride=stride, act=act, name='projection')
+    if not projection_first:
+        p = b.conv(x, O, 1, stride=stride, act=act, name='projection')
     b.conv(b.sum([y, p], act='relu', name='sum'), 32, 1, name='reader')
     return b.net
 
@@ -29,20 +33,31 @@ CASES = [(64, 64, 13, 11, 256, 1, 1, 3), (64, 64, 28, 28, 256, 1, 1, 40), (256, 
          (32, 64, 20, 20, 96, 3, 1, 9), (96, 48, 15, 15, 160, 3, 2, 6), (32, 32, 5, 3, 32, 1, 1, 2), (64, 128, 28, 28, 128, 3, 1, 30),
          (512, 256, 14, 14, 1024, 1, 1, 110), (512, 512, 9, 7, 1120, 1, 2, 300), (256, 512, 7, 7, 288, 3, 1, 400), (64, 64, 30, 30, 480, 1, 1, 90)]
 
+# a 64-channel 3x3 branch whose projection reads other channels stays on the patch kernel
+SEPARATE = [(32, 64, 20, 20, 96, 3, 1, 9)]
+
 
 @pytest.mark.parametrize('case', CASES, ids=lambda c: 'C%d_%d_%dx%d_O%d_k%d_s%d_b%d' % c)
 @pytest.mark.parametrize('mode', ['double', 'fixed', 'float'])
 def test_branch_and_projection(case, mode):
     C, mid, H, W, O, k, s, batch = case
     n, eng = compare_net(unit_net(C, mid, H, W, O, k, s, mode), batch, flags=0)
-    if O % 64 == 0 and not (k == 3 and s == 1 and O <= 128):   # (narrow branches may keep the patch kernel)
-        assert ENGINE in eng
+    assert (ENGINE in eng) == (case not in SEPARATE), eng
 
 
 @pytest.mark.parametrize('mode, unsigned_relu, clipped, act', [('double', False, False, 'linear'), ('fixed', True, True, 'linear'), ('float', True, True, 'relu'),
                                                                ('single', True, False, 'relu'), ('fixed', False, False, 'linear')])
 def test_branch_and_projection_forms(mode, unsigned_relu, clipped, act):
     compare_net(unit_net(128, 64, 12, 10, 256, 1, 1, mode, unsigned_relu, clipped, act), 9, flags=0, want_engine=ENGINE)
+
+
+# The 3x3 layer carries the sum; a 3x3 and a 1x1 layer of one tensor; both
+@pytest.mark.parametrize('mid, projection_first', [(64, True), (0, False), (0, True)])
+@pytest.mark.parametrize('case', [(128, 14, 14, 256, 1, 5), (128, 15, 13, 160, 2, 40), (256, 7, 7, 512, 1, 90)], ids=lambda c: 'C%d_%dx%d_O%d_s%d_b%d' % c)
+@pytest.mark.parametrize('mode', ['double', 'fixed', 'float'])
+def test_order_and_inputs(case, mid, projection_first, mode):
+    C, H, W, O, s, batch = case
+    compare_net(unit_net(C, mid, H, W, O, 3, s, mode, projection_first=projection_first), batch, flags=0, want_engine=ENGINE)
 
 
 def test_packed_weights_and_calls_of_any_size_on_one_network():

@@ -10,15 +10,17 @@ from oracle import oracle
 pytestmark = pytest.mark.gpu
 
 
-# (H, W, outputs): 96 outputs leave a part of a tile; batches on both sides of the line of 148 tiles of 128 rows
+# (H, W, outputs): 96 outputs leave a part of a tile; batches on both sides of the line of a tile of 128 rows per multiprocessor
 @pytest.mark.parametrize('case', [(28, 28, 128), (13, 9, 96), (30, 31, 128)], ids=lambda c: '%dx%d_O%d' % c)
 @pytest.mark.parametrize('mode', ['double', 'fixed', 'float'])
 def test_both_kernels_on_one_network(case, mode):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
     H, W, O = case
     b = netdesc.NetBuilder('patch', 16, H, W, 17, mode, weight_dist=('normal', 30))
     b.conv(b.conv(-1, 128, 1, name='front'), O, 3, pad=1, name='c')
     net = b.net
-    line = 148 * 128 // (H * W)
+    line = sms * 128 // (H * W)   # images of one tile per multiprocessor
     capacity = min(line + 20, 200)
     x = netdesc.make_input(net, capacity)
     picks = sorted({0, 1, capacity // 2, capacity - 1})
