@@ -8,10 +8,12 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, 'csrc')
 OUT = os.path.join(HERE, 'libn2d2b.so')
-SOURCES = ['net.cu', 'simt_kernels.cu', 'depthwise3x3.cu', 'igemm_tcgen05.cu', 'igemm_w4.cu', 'igemm_dual.cu', 'igemm_chain.cu', 'stem_tcgen05.cu', 'patch_tcgen05.cu',
+SOURCES = ['net.cu', 'simt_kernels.cu', 'depthwise3x3.cu', 'igemm_tcgen05.cu', 'igemm_w4.cu', 'igemm_dual.cu', 'igemm_dual_float.cu', 'igemm_dual_any.cu',
+           'igemm_chain.cu', 'igemm_chain_float.cu', 'igemm_chain_any.cu', 'stem_tcgen05.cu', 'patch_tcgen05.cu', 'patch_float.cu', 'patch_wide.cu',
            'stem_s2d_tcgen05.cu', 'stem_s2d_pool.cu', 'stem_pool_tcgen05.cu', 'stem_pool_int.cu', 'stem_pool_float.cu',
            'stem_pool_wide.cu', 'small_net.cu', 'dwpw_tcgen05.cu', 'dwpw_forms.cu', 'probe_tcgen05.cu']
-HEADERS = ['common.cuh', 'kernels.h', 'tc_common.cuh', 'host_internal.h', 'igemm_kernel.cuh', 'stem_pool_kernel.cuh', 'stem_s2d_kernel.cuh',
+HEADERS = ['common.cuh', 'kernels.h', 'tc_common.cuh', 'host_internal.h', 'igemm_kernel.cuh', 'igemm_dual_kernel.cuh', 'igemm_chain_kernel.cuh',
+           'patch_kernel.cuh', 'stem_pool_kernel.cuh', 'stem_s2d_kernel.cuh',
            'dwpw_kernel.cuh', os.path.join('..', '..', 'include', 'n2d2b.h')]
 NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
               '-Xcompiler', '-fPIC', '-shared', '-diag-suppress', '550']
