@@ -240,9 +240,11 @@ int n2d2b_net_tensor_info(const n2d2b_net* net, int tensor_id, n2d2b_tensor_info
 /* Copies a tensor of the last forward (first `batch` images) to the host. */
 int n2d2b_net_read_tensor(n2d2b_net* net, int tensor_id, int batch, void* host_dst, size_t bytes);
 /* Bytes of weights the network keeps in HBM (*total_bytes), and how many of them are packed 4-bit weights
- * (*packed4_bytes: cells given weight_bits = 4 that run on the implicit-GEMM kernel, which expands them tile by
- * tile in shared memory; other cells hold int8).  A network that runs as one kernel holds its weights a second time, with its rescale
- * constants, as that kernel reads them.  Either pointer may be NULL. */
+ * (*packed4_bytes: cells given weight_bits = 4 that run on the implicit-GEMM kernel, other cells hold int8).
+ * Small calls expand packed weights tile by tile in shared memory; calls of 2^29 multiply-accumulates and more, and cells of many tiles, widen
+ * them to int8 first, into a block of twice their packed size (one byte a weight) that a network finalized for such calls holds beside
+ * *total_bytes.  A network that runs as one kernel holds its weights a second time, with its rescale constants, as that kernel reads them.
+ * Either pointer may be NULL. */
 int n2d2b_net_weight_bytes(const n2d2b_net* net, size_t* total_bytes, size_t* packed4_bytes);
 /* Number of kernel launches one n2d2b_net_forward of max_batch images issues. */
 int n2d2b_net_launches_per_forward(const n2d2b_net* net);

@@ -1075,21 +1075,25 @@ static bool patch_as_gemm(const n2d2b_net* net, const CellRec& c, int batch)
     return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) <= net->num_sms;
 }
 
-// Whether a call of `call` images widens the packed weights of all cells at its start, in one launch of 3 to 4 us.  The line is drawn where a call is large
-// enough to pay for it whatever its cells are (ResNet-18 at 224 x 224, 1.7 G multiply-accumulates an image: four images 217 us with the expansion in the
-// kernels, 182 widened cell by cell, 162 in one launch; 128 images 656 / 460 / 421: the expansion warps' shared-memory stores bound every layer of long
-// K, and the classifier, which has no 32-bit epilogue in that form, took 38 to 110 us).
+// Whether a call of `call` images widens packed weights at its start, in one launch of 3 to 4 us.  The line is drawn where a call is large enough to pay
+// for it (ResNet-18 at 224 x 224, 1.7 G multiply-accumulates an image: four images 217 us with the expansion in the kernels, 182 widened cell by cell, 162 in
+// one launch; 128 images 656 / 460 / 421: the expansion warps' shared-memory stores bound every layer of long K, and the classifier, which has no
+// 32-bit epilogue in that form, took 38 to 110 us).
 static bool widens_all(long long macs, int call) { return macs * call >= (1ll << 29); }
 static bool widen_all(const n2d2b_net* net, int call) { return widens_all(net->w8_macs, call); }
 
-// Whether a packed cell takes the widened form in a call of `call` images, `batch` of them at once.  In a smaller call a cell is widened by itself where a
-// CTA has more than two tiles, whose in-kernel expansions would repeat.
+// In a smaller call a cell is widened by itself where a CTA has more than two tiles, whose in-kernel expansions would repeat
+static bool widens_alone(const n2d2b_net* net, const CellRec& c, int batch)
+{
+    const long long m_tiles = ((long long)batch * c.geom.oH * c.geom.oW + 127) / 128;
+    return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) > 2ll * net->num_sms;
+}
+
+// Whether a packed cell takes the widened form in a call of `call` images, `batch` of them at once
 static bool use_widened(const n2d2b_net* net, const CellRec& c, int batch, int call)
 {
     if (c.w8 == CellRec::W8_NONE) return false;
-    if (widen_all(net, call)) return true;
-    const long long m_tiles = ((long long)batch * c.geom.oH * c.geom.oW + 127) / 128;
-    return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) > 2ll * net->num_sms;
+    return widen_all(net, call) || widens_alone(net, c, batch);
 }
 
 // The implicit-GEMM plan of a dense cell
@@ -1135,7 +1139,8 @@ static size_t widened_bytes(const CellRec& c)
     return (n + 255) & ~(size_t)255;
 }
 
-// Whether a packed cell has a widened form, whose plans are made over the given addresses (out == nullptr: a padded matrix of the cell's own)
+// Whether a packed cell has a widened form, whose plans are made over the given addresses (out: a matrix of padded rows where the outputs are no whole
+// blocks of 32 columns)
 static int plan_widened_cell(n2d2b_net* net, CellRec& c, const void* in, const int8_t* w, void* out, const void* res)
 {
     ConvGeom g = c.geom;
@@ -1150,11 +1155,7 @@ static int plan_widened_cell(n2d2b_net* net, CellRec& c, const void* in, const i
         c.w8 = CellRec::W8_PATCH;
         return 0;
     }
-    if (!out) {
-        g.O = c.w8_rows = (g.O + 31) & ~31;
-        CUDA_TRY(cudaMalloc(&c.d_w8_out, (size_t)net->max_batch * g.oH * g.oW * g.O + 256));
-        out = c.d_w8_out;
-    }
+    g.O = c.w8_rows = (g.O + 31) & ~31;
     if (igemm_make_plan(&c.plan8, in, w, out, res, g, in_u, 0, 0, net->num_sms, &why) || !igemm_uses_fast_epilogue(c.plan8, c.fast, res != nullptr, DT_I8)) return 0;
     c.plan8.late_weights = 1;
     c.plan8.perm = igemm_perm_block(c.plan8);
@@ -1165,36 +1166,44 @@ static int plan_widened_cell(n2d2b_net* net, CellRec& c, const void* in, const i
 
 static long long cell_macs(const CellRec& c) { return (long long)c.geom.oH * c.geom.oW * c.geom.O * c.geom.kH * c.geom.kW * c.geom.C; }
 
-// Plans the widened form of every packed cell.  The weights stay packed in HBM; a scratch block holds the int8 weights of the call that is running.
+// Plans the widened form of the packed cells that some call widens.  The weights stay packed in HBM; a scratch block of twice their size holds the int8
+// weights of the call that is running.
 static int plan_widened(n2d2b_net* net)
 {
-    // (not where the input or the residual is the caller's buffer, whose address only the forward pass knows)
-    auto eligible = [&](const CellRec& c) {
-        return !c.skipped && c.engine == ENG_TCGEN05 && c.plan.w4 && c.fast.enabled && c.inputs[0] != 0 && c.residual != 0;
+    auto plan = [&](CellRec& c, const int8_t* w, void* out) {
+        const void* res = c.residual >= 0 ? tensor_or_placeholder(net, c.residual) : nullptr;
+        return plan_widened_cell(net, c, c.plan_input, w, out, res);
     };
-    size_t total = 0;
     for (CellRec& c : net->cells) {
         c.w8 = CellRec::W8_NONE;
-        if (!eligible(c)) continue;
+        // (not where the input or the residual is the caller's buffer, whose address only the forward pass knows)
+        if (c.skipped || c.engine != ENG_TCGEN05 || !c.plan.w4 || !c.fast.enabled || c.inputs[0] == 0 || c.residual == 0) continue;
+        if (net->tensors[c.output].dtype != DT_I8 || (c.geom.O % 32 != 0 && c.residual >= 0)) continue;
+        if (int rc = plan(c, (const int8_t*)placeholder(), placeholder())) return rc;
+        if (c.w8 != CellRec::W8_NONE) net->w8_macs += cell_macs(c);
+    }
+    size_t total = 0;
+    for (CellRec& c : net->cells) {
+        if (!use_widened(net, c, net->max_batch, net->max_batch)) c.w8 = CellRec::W8_NONE;   // nor in a smaller call
+        if (c.w8 == CellRec::W8_NONE) continue;
         c.w8_offset = total;
         total += widened_bytes(c);
     }
     if (!total) return 0;
     CUDA_TRY(cudaMalloc(&net->d_w8, total + 256));
-    for (CellRec& c : net->cells) {
-        if (!eligible(c) || net->tensors[c.output].dtype != DT_I8) continue;
-        const void* res = c.residual >= 0 ? tensor_ptr(net, c.residual, nullptr) : nullptr;
-        if (c.residual >= 0 && !res) res = placeholder();
-        if (c.geom.O % 32 != 0 && res) continue;
-        if (int rc = plan_widened_cell(net, c, c.plan_input, (const int8_t*)net->d_w8 + c.w8_offset, c.geom.O % 32 ? nullptr : tensor_or_placeholder(net, c.output), res))
-            return rc;
-    }
-    for (const CellRec& c : net->cells)
-        if (c.w8 != CellRec::W8_NONE) net->w8_macs += cell_macs(c);
     const bool all = widen_all(net, net->max_batch);
     if (all) net->launches++;
-    for (const CellRec& c : net->cells)
-        if (use_widened(net, c, net->max_batch, net->max_batch)) net->launches += (all ? 0 : 1) + (c.d_w8_out && !stores_rows(c, c.plan8) ? 1 : 0);
+    for (CellRec& c : net->cells) {
+        if (c.w8 == CellRec::W8_NONE) continue;
+        void* out = tensor_or_placeholder(net, c.output);
+        if (c.geom.O % 32 != 0) {
+            CUDA_TRY(cudaMalloc(&c.d_w8_out, (size_t)net->max_batch * c.geom.oH * c.geom.oW * ((c.geom.O + 31) & ~31) + 256));
+            out = c.d_w8_out;
+        }
+        if (int rc = plan(c, (const int8_t*)net->d_w8 + c.w8_offset, out)) return rc;
+        if (c.w8 == CellRec::W8_NONE) return fail(N2D2B_ERR_STATE, "internal: a packed cell lost its widened form");
+        net->launches += (all ? 0 : 1) + (c.d_w8_out && !stores_rows(c, c.plan8) ? 1 : 0);
+    }
     return 0;
 }
 
@@ -1327,8 +1336,18 @@ static int settle_duals(n2d2b_net* net)
         if (int rc = probe_dense(net, c, &dense)) return rc;
         if (c.w8 != CellRec::W8_NONE) macs += cell_macs(c);
     }
-    for (CellRec& b : net->cells)
-        if (b.dual_branch >= 0 && widens_all(macs, 1)) b.dual_always = true;
+    for (CellRec& b : net->cells) {
+        if (b.dual_branch < 0 || !b.plan.w4) continue;
+        CellRec& a = net->cells[b.dual_branch];
+        auto both = [&](int call) { return widens_all(macs, call) || (widens_alone(net, a, call) && widens_alone(net, b, call)); };
+        if (both(1)) {
+            b.dual_always = true;
+        } else if (!both(net->max_batch)) {
+            a.dual_sum = b.dual_branch = -1;   // they never share a kernel: the branch's input dies with the branch
+            b.inputs.pop_back();
+            forget_probe(b);
+        }
+    }
     return 0;
 }
 

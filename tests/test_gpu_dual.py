@@ -131,3 +131,29 @@ def test_only_what_is_stored_has_a_buffer(case, weight_bits, engine):
     # the front, the reduction and the sum, or the branch's output and the sum in place of the reduction; the staging of the host's calls (16 channels in, 32
     # out); weights, constants and the steps of 2 MiB that the device hands out
     assert held <= (C + mid + O + 16 + 32) * images + (24 << 20)
+
+
+def _packed_layers():
+    b = netdesc.NetBuilder('packed', 64, 1, 1, 3, 'fixed', weight_dist=('uniform', 7), weight_bits=4, clipped=True)
+    x = b.conv(-1, 64, 1, name='front')
+    x = b.fc(x, 4096, act='relu', name='wide')
+    b.fc(x, 4096, act='relu', name='square')
+    return b.net
+
+
+# Widened weights (one byte each) are held where a call widens them: 2^29 multiply-accumulates are 32 images of this network
+@pytest.mark.parametrize('images, widened', [(4, False), (64, True)])
+def test_widened_weights_are_held_where_a_call_widens_them(images, widened):
+    net = _packed_layers()
+    weights = sum(l['weights'].size for l in net['layers'])
+    held, eng = _bytes_held(net, images)
+    assert ('tcgen05-widened' in eng) == widened
+    assert (held > weights * 1.25) == widened   # packed: half a byte a weight
+    compare_net(net, images, flags=0)
+
+
+def test_packed_pair_that_no_call_widens():
+    net = unit_net(256, 256, 8, 8, 256, 1, 1, 'fixed', weight_bits=4, clipped=True)
+    n, eng = compare_net(net, 3, flags=0)
+    assert ENGINE not in eng and 'tcgen05-widened' not in eng
+    compare_net(net, 60, flags=0, want_engine=ENGINE)
