@@ -1160,9 +1160,10 @@ cudaError_t launch_topn(const void* scores, int dtype, int is_unsigned, size_t p
     if (pixels == 0 || C == 0 || topN == 0) return cudaSuccess;
     const unsigned grid = (unsigned)std::min<size_t>(pixels, 16 * (size_t)current_sms());
     if (dtype != DT_I32 && C <= 1024) {
-#define N2D2B_TOPN_BYTES(T)                                                                                                                      \
-    (C <= 128 ? launch_pdl(topn_bytes_kernel<T, 4>, grid, 32, 0, s, (const T*)scores, pixels, hw, C, topN, labels, values)                      \
-              : launch_pdl(topn_bytes_kernel<T, 32>, grid, 32, 0, s, (const T*)scores, pixels, hw, C, topN, labels, values))
+#define N2D2B_TOPN_BYTES(T)                                                                                                  \
+    launch_pdl(C <= 128 ? topn_bytes_kernel<T, 4> : C <= 256 ? topn_bytes_kernel<T, 8> : C <= 512 ? topn_bytes_kernel<T, 16> \
+                                                                                                  : topn_bytes_kernel<T, 32>, \
+               grid, 32, 0, s, (const T*)scores, pixels, hw, C, topN, labels, values)
         return is_unsigned ? N2D2B_TOPN_BYTES(uint8_t) : N2D2B_TOPN_BYTES(int8_t);
 #undef N2D2B_TOPN_BYTES
     }
