@@ -917,13 +917,20 @@ static void igemm_grid(const IgemmPlan& plan, int* tiles, int* grid)
 // A launch of up to two tiles per CTA has the variant that stores from the registers (see DRY)
 static bool igemm_short(int tiles, int grid) { return tiles <= 2 * grid; }
 
+// (of a cell with the 32-bit epilogue)
+bool igemm_takes_clusters(const IgemmPlan& plan)
+{
+    int tiles, grid;
+    igemm_grid(plan, &tiles, &grid);
+    return !plan.w4 && !plan.grouped && plan.BN == SPLIT_BN && igemm_split(tiles, plan.taps * ((plan.Cin + plan.BK - 1) / plan.BK), plan.num_sms);
+}
+
 bool igemm_writes_rows(const IgemmPlan& plan, int columns)
 {
     int tiles, grid;
     igemm_grid(plan, &tiles, &grid);
-    const int num_kb = plan.taps * ((plan.Cin + plan.BK - 1) / plan.BK);
     return plan.perm && !plan.w4 && !plan.grouped && !plan.pair && plan.BN / plan.parts >= 32 && columns % 8 == 0 && igemm_short(tiles, grid)
-        && !(plan.BN == SPLIT_BN && igemm_split(tiles, num_kb, plan.num_sms));
+        && !igemm_takes_clusters(plan);
 }
 
 cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residual& r, const FastQuant& fast, void* out,
@@ -983,7 +990,7 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     igemm_grid(plan, &tiles, &grid);
     // Few tiles, long K: a cluster of CTAs per tile
     const int num_kb = plan.taps * ((plan.Cin + plan.BK - 1) / plan.BK);
-    if (use_fast && !plan.w4 && !plan.grouped && plan.BN == SPLIT_BN && igemm_split(tiles, num_kb, plan.num_sms)) {
+    if (use_fast && igemm_takes_clusters(plan)) {
         static SmemLimitSet split_limit;
         if (cudaError_t e = raise_smem_limit(igemm_split_tcgen05_kernel, split_limit)) return e;
         SplitArgs sa;

@@ -276,6 +276,8 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
 // Whether a launch of plan.M rows stores from the registers and so may write rows of `columns` bytes
 bool igemm_writes_rows(const IgemmPlan& plan, int columns);
 
+// Whether it runs on clusters of CTAs that share a tile
+bool igemm_takes_clusters(const IgemmPlan& plan);
 // ---- two convolutions and the sum of their outputs (igemm_dual.cu) ----
 struct DualPlan {
     IgemmPlan a, b;       // maps, extents and tiling of the branch and of the projection

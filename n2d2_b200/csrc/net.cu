@@ -1239,6 +1239,9 @@ static bool make_dual(n2d2b_net* net, CellRec& b, const void* in_a, const int8_t
             b.dual_patch.proj_in = nullptr;
             return false;
         }
+    // A branch of few tiles and long K runs on clusters that share a tile when it is a kernel of its own: 3x3, 512 channels of 7 x 7 beside a projection of 256, one
+    // and two images 16.6 us as two kernels, 17.9 and 18.5 as one; three images, no clusters, 20.0 / 18.7
+    if (packed ? a.w8 == CellRec::W8_IGEMM && igemm_takes_clusters(a.plan8) : a.engine == ENG_TCGEN05 && igemm_takes_clusters(a.plan)) return false;
         b.dual_patch.late_weights = packed ? 1 : 0;
         return true;
     }

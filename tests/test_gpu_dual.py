@@ -34,7 +34,8 @@ CASES = [(64, 64, 13, 11, 256, 1, 1, 3), (64, 64, 28, 28, 256, 1, 1, 40), (256, 
          (512, 256, 14, 14, 1024, 1, 1, 110), (512, 512, 9, 7, 1120, 1, 2, 300), (256, 512, 7, 7, 288, 3, 1, 400), (64, 64, 30, 30, 480, 1, 1, 90)]
 
 # a 64-channel 3x3 branch whose projection reads other channels stays on the patch kernel
-SEPARATE = [(32, 64, 20, 20, 96, 3, 1, 9)]
+# the clusters of a branch of few tiles and long K are faster by themselves
+SEPARATE = [(32, 64, 20, 20, 96, 3, 1, 9), (256, 512, 7, 7, 512, 3, 1, 1)]
 
 
 @pytest.mark.parametrize('case', CASES, ids=lambda c: 'C%d_%d_%dx%d_O%d_k%d_s%d_b%d' % c)
