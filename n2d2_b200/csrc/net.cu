@@ -1382,6 +1382,9 @@ static int settle_chains(n2d2b_net* net)
     }
     return 0;
 }
+        // (few row tiles: by themselves the two cells spread their columns over more multiprocessors.  64 -> 256 -> 64 channels with the sum behind them, 7 tiles 16.1
+        // us as two kernels, 17.3 as one; 13 16.0 / 17.5; 25 16.8 / 16.9, to 128 channels 18.8 / 17.2; 49 20.0 / 18.9)
+        if (((long long)net->max_batch * c.geom.oH * c.geom.oW + 127) / 128 * 7 < net->num_sms) continue;
 
 static int plan_duals(n2d2b_net* net)
 {
