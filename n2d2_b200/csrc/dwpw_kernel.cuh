@@ -35,14 +35,14 @@ static constexpr int DP_PARAM_BYTES = FAST_NP * 256 * 4;   // the 1x1 layer's co
 
 // How the constants of a cell are applied
 // (DPF_UNIT: 32-bit without clamps, every multiplier 1 - a single shift: the addend then starts the dot product)
-static constexpr int DPF_INT = 0, DPF_CLAMP = 1, DPF_FLOAT = 2, DPF_WIDE = 3, DPF_UNIT = 4;
-__host__ __device__ constexpr bool dpf_clamp(int f) { return f == DPF_CLAMP || f == DPF_FLOAT; }
+static constexpr int DPF_INT = 0, DPF_CLAMP = 1, DPF_WIDE = 2, DPF_UNIT = 3;
+__host__ __device__ constexpr bool dpf_clamp(int f) { return f == DPF_CLAMP; }
 // rows of the five of a FastQuant that the form reads
 __host__ __device__ constexpr int dpf_rows(int f)
 {
-    return f == DPF_INT ? 0x1c : (f == DPF_CLAMP ? 0x1f : (f == DPF_FLOAT ? 0x0f : (f == DPF_WIDE ? 0x1d : 0x18)));
+    return f == DPF_INT ? 0x1c : (f == DPF_CLAMP ? 0x1f : (f == DPF_WIDE ? 0x1d : 0x18));
 }
-__host__ __device__ constexpr int dpf_ef(int f) { return f == DPF_FLOAT ? EF_FLOAT : (f == DPF_WIDE ? EF_WIDE : 0); }
+__host__ __device__ constexpr int dpf_ef(int f) { return f == DPF_WIDE ? EF_WIDE : 0; }
 
 struct DwPwArgs {
     int C, N, kchunks, oH, oW, pT, pL;
@@ -555,6 +555,6 @@ dwpw_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 
 typedef void (*DwPwKernel)(const CUtensorMap, const CUtensorMap, const DwPwArgs, int);
 // [stride - 1]; the forms beside the 32-bit ones are an object of their own
-extern const DwPwKernel dwpw_float[2], dwpw_wide[2], dwpw_wide_1x1[2], dwpw_wide_depthwise[2];
+extern const DwPwKernel dwpw_wide[2], dwpw_wide_1x1[2], dwpw_wide_depthwise[2];
 
 }  // namespace n2d2b

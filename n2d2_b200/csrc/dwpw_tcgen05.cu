@@ -19,6 +19,23 @@ bool dwpw_eligible(const ConvGeom& d, const ConvGeom& p)
         && p.H == d.oH && p.W == d.oW && p.oH == d.oH && p.oW == d.oW && p.O % 32 == 0 && p.O <= 2048;
 }
 
+// Whether one kernel is faster than two in calls of up to `batch` images.  Measured as pairs of 32 to 1024 channels, maps of 2 to 112 pixels a side, 0.5 to 4 times
+// as many outputs, strides 1 and 2 and 1 to 256 images, in graphs of several passes; times as two kernels over times as one:
+//   - 6400 output pixels and more (of 32 channels 12800), up to two blocks of channels and twice as many outputs, or up to four blocks and as many: shift scalings
+//     0.96 to 1.28 (512 -> 512 at 14 x 14, 33 images: 21.2 us, 19.9), fixed-point ones 0.95 to 1.2
+//   - one or two blocks of 128 channels and few output rows (up to a third of the multiprocessors): a hand-over less, 1.00 to 1.08; from 56 rows on, which
+//     column ranges share and compute several times, 0.9
+//   - in between (2 rows a CTA) 0.86 to 0.95
+//   - more outputs, which take several passes over the operand, 0.78 to 1.05 (512 -> 1024, 14 x 14 to 7 x 7, 256 images: 34.7 us, 41.8)
+//   - more blocks, whose patches and operands do not fit beside one another, 0.37 to 0.9 (960 channels at 7 x 7)
+bool dwpw_faster(const ConvGeom& d, int N, int batch, int num_sms)
+{
+    const int blocks = d.C / block_channels(d.C);
+    if (blocks > 4 || N > (blocks > 2 ? 1 : 2) * d.C) return false;
+    const long long rows = (long long)batch * d.oH, pixels = rows * d.oW;
+    return pixels >= (d.C > 32 ? 6400 : 12800) || (blocks <= 2 && d.C >= 128 && rows <= num_sms / 3);
+}
+
 size_t dwpw_depthwise_words(const ConvGeom& d) { return (size_t)3 * d.C; }
 
 // [C][3][3] -> [3][C] words: bytes w(0, kx), w(1, kx), w(2, kx), 0
@@ -33,17 +50,16 @@ void dwpw_arrange_depthwise(const ConvGeom& d, const int8_t* w, uint32_t* dst)
 }
 
 // (the constants of a depthwise layer, see DPF_UNIT; of the 1x1 layer a unit multiplier saves nothing)
-static int form_of(const FastQuant& f) { return f.form == EF_WIDE ? DPF_WIDE : (f.form == EF_FLOAT ? DPF_FLOAT : (f.need_clamp ? DPF_CLAMP : DPF_INT)); }
+static int form_of(const FastQuant& f) { return f.form == EF_WIDE ? DPF_WIDE : (f.need_clamp ? DPF_CLAMP : DPF_INT); }
 
 static const DwPwKernel* kernels_for(const FastQuant& dw, const FastQuant& pw)
 {
     static const DwPwKernel plain[2] = {dwpw_i8_tcgen05_kernel<1, DPF_INT, DPF_INT>, dwpw_i8_tcgen05_kernel<2, DPF_INT, DPF_INT>};
     static const DwPwKernel unit[2] = {dwpw_i8_tcgen05_kernel<1, DPF_UNIT, DPF_INT>, dwpw_i8_tcgen05_kernel<2, DPF_UNIT, DPF_INT>};
     static const DwPwKernel clamped[2] = {dwpw_i8_tcgen05_kernel<1, DPF_CLAMP, DPF_CLAMP>, dwpw_i8_tcgen05_kernel<2, DPF_CLAMP, DPF_CLAMP>};
+    if (dw.form == EF_FLOAT || pw.form == EF_FLOAT) return nullptr;   // slower than two kernels (MobileNet, 1 / 16 / 256 images: 82 / 144 / 813 us, as one 92 / 162 / 875)
     const int a = form_of(dw), b = form_of(pw);
     if ((a == DPF_WIDE && dw.need_clamp) || (b == DPF_WIDE && pw.need_clamp)) return nullptr;
-    if ((a == DPF_FLOAT) != (b == DPF_FLOAT)) return nullptr;
-    if (a == DPF_FLOAT) return dwpw_float;
     if (a == DPF_WIDE) return b == DPF_WIDE ? dwpw_wide : dwpw_wide_depthwise;
     if (b == DPF_WIDE) return dwpw_wide_1x1;
     if (a == DPF_INT && b == DPF_INT) return dw.unit_multiplier ? unit : plain;
@@ -140,7 +156,7 @@ int dwpw_set_batch(DwPwPlan* plan, int batch)
         plan->nsplit = ns; plan->bn = bn; plan->passes = passes; plan->groups = groups; plan->rt = rt;
         plan->subs = subs; plan->a_sub = a_sub; plan->na = na; plan->dw_shared = shared; plan->patch_bytes = patch; plan->np = np; plan->b_bytes = b_bytes; plan->nb = nb;
         plan->smem_bytes = bytes;
-        // Work items: as long as they keep the twelve warps busy over the patches in flight (two columns of every item are read for
+        // Work items: as long as they keep the depthwise warps (eight or twelve) busy over the patches in flight (two columns of every item are read for
         // its neighbour).  Items of several lanes' groups start an odd number of pixels apart: in other banks
         const int groups_of_lanes = 32 / (bk / 4), flight = std::min(np, kch * ((tiles + subs - 1) / subs));
         int item = seg;
@@ -216,10 +232,9 @@ cudaError_t launch_dwpw(const DwPwPlan& plan, int n_base, const FastQuant& dw, c
     a.fq = pw.fq; a.cpad = pw.cpad; a.out_unsigned = pw.out_unsigned;
     a.out = (uint8_t*)out;
     a.status = status_word;
-    static SmemLimitSet limits[8][2];
+    static SmemLimitSet limits[6][2];
     const int v = dw.unit_multiplier && form_of(dw) == DPF_INT && form_of(pw) == DPF_INT ? 0
-                : (form_of(dw) == DPF_INT && form_of(pw) == DPF_INT ? 1 : (table == dwpw_float ? 2 : (table == dwpw_wide ? 3
-                : (table == dwpw_wide_1x1 ? 4 : (table == dwpw_wide_depthwise ? 5 : 6)))));
+                : (form_of(dw) == DPF_INT && form_of(pw) == DPF_INT ? 1 : (table == dwpw_wide ? 2 : (table == dwpw_wide_1x1 ? 3 : (table == dwpw_wide_depthwise ? 4 : 5))));
     const DwPwKernel kernel = table[d.sX - 1];
     if (cudaError_t e = raise_smem_limit(kernel, limits[v][d.sX - 1])) return e;
     return launch_pdl(kernel, dim3((unsigned)(plan.groups * plan.nsplit)), DP_THREADS, plan.smem_bytes, s, plan.tmA, plan.tmB, a, plan.bk);

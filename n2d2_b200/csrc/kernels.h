@@ -212,6 +212,7 @@ struct DwPwPlan {
     size_t smem_bytes;
 };
 bool dwpw_eligible(const ConvGeom& d, const ConvGeom& p);
+bool dwpw_faster(const ConvGeom& d, int N, int batch, int num_sms);
 bool dwpw_takes_forms(const FastQuant& dw, const FastQuant& pw);
 size_t dwpw_depthwise_words(const ConvGeom& d);
 void dwpw_arrange_depthwise(const ConvGeom& d, const int8_t* w, uint32_t* dst);
@@ -275,9 +276,9 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
                          void* out, int out_dtype, int m_base, int* status_word, cudaStream_t s, void* rows = nullptr, int columns = 0);
 // Whether a launch of plan.M rows stores from the registers and so may write rows of `columns` bytes
 bool igemm_writes_rows(const IgemmPlan& plan, int columns);
-
 // Whether it runs on clusters of CTAs that share a tile
 bool igemm_takes_clusters(const IgemmPlan& plan);
+
 // ---- two convolutions and the sum of their outputs (igemm_dual.cu) ----
 struct DualPlan {
     IgemmPlan a, b;       // maps, extents and tiling of the branch and of the projection

@@ -1817,6 +1817,7 @@ static int fuse_depthwise(n2d2b_net* net)
             for (CellRec* x : {&c, &p}) {
                 cudaFree(x->d_fast);
                 x->d_fast = nullptr;
+        if (!dwpw_faster(c.geom, p.geom.O, net->max_batch, net->num_sms)) continue;
                 x->fast = FastQuant{};
             }
             continue;
