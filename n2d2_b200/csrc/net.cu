@@ -1082,18 +1082,31 @@ static bool patch_as_gemm(const n2d2b_net* net, const CellRec& c, int batch)
 static bool widens_all(long long macs, int call) { return macs * call >= (1ll << 29); }
 static bool widen_all(const n2d2b_net* net, int call) { return widens_all(net->w8_macs, call); }
 
-// In a smaller call a cell is widened by itself where a CTA has more than two tiles, whose in-kernel expansions would repeat
-static bool widens_alone(const n2d2b_net* net, const CellRec& c, int batch)
+static long long packed_tiles(const CellRec& c, int batch)
 {
-    const long long m_tiles = ((long long)batch * c.geom.oH * c.geom.oW + 127) / 128;
-    return m_tiles * ((c.geom.O + c.plan.BN - 1) / c.plan.BN) > 2ll * net->num_sms;
+    return ((long long)batch * c.geom.oH * c.geom.oW + 127) / 128 * ((c.geom.O + c.plan.BN - 1) / c.plan.BN);
 }
 
-// Whether a packed cell takes the widened form in a call of `call` images, `batch` of them at once
+// In a smaller call a cell is widened by itself where a CTA has more than two tiles, whose in-kernel expansions would repeat
+static bool widens_alone(const n2d2b_net* net, const CellRec& c, int batch) { return packed_tiles(c, batch) > 2ll * net->num_sms; }
+
+// Which cells a large call widens.  The expansion costs a CTA about 0.14 us per K block and tile; widening moves 2.5 bytes a weight, 0.05 us per K block
+// and 1024 outputs.  So wide layers of a tile per CTA keep their packed weights, unless their epilogue is not the 32-bit one in that form.
+static bool worth_widening(const n2d2b_net* net, const CellRec& c, int call)
+{
+    const long long per_cta = (packed_tiles(c, call) + net->num_sms - 1) / net->num_sms;
+    return c.geom.O < 1024 * per_cta || widens_alone(net, c, call) || !igemm_uses_fast_epilogue(c.plan, c.fast, c.residual >= 0, DT_I8);
+}
+
+// Whether a packed cell takes the widened form in a call of `call` images, `batch` of them at once; macs: of the network's packed cells, per image
+static bool widens_in(const n2d2b_net* net, const CellRec& c, long long macs, int batch, int call)
+{
+    return (widens_all(macs, call) && worth_widening(net, c, call)) || widens_alone(net, c, batch);
+}
+
 static bool use_widened(const n2d2b_net* net, const CellRec& c, int batch, int call)
 {
-    if (c.w8 == CellRec::W8_NONE) return false;
-    return widen_all(net, call) || widens_alone(net, c, batch);
+    return c.w8 != CellRec::W8_NONE && widens_in(net, c, net->w8_macs, batch, call);
 }
 
 // The implicit-GEMM plan of a dense cell
@@ -1226,6 +1239,9 @@ static bool make_dual(n2d2b_net* net, CellRec& b, const void* in_a, const int8_t
     if (packed ? (a.w8 == CellRec::W8_NONE || b.w8 == CellRec::W8_NONE || a.w8_ng_dst != 4 || b.w8_ng_dst != 4)
                : (b.plan.perm != 32 || (a.engine == ENG_TCGEN05 && a.plan.perm != 32)))
         return false;
+    // A branch of few tiles and long K runs on clusters that share a tile when it is a kernel of its own: 3x3, 512 channels of 7 x 7 beside a projection of 256, one
+    // and two images 16.6 us as two kernels, 17.9 and 18.5 as one; three images, no clusters, 20.0 / 18.7
+    if (packed ? a.w8 == CellRec::W8_IGEMM && igemm_takes_clusters(a.plan8) : a.engine == ENG_TCGEN05 && igemm_takes_clusters(a.plan)) return false;
     ConvGeom ga = a.geom, gb = b.geom;
     ga.B = gb.B = net->max_batch;
     const char* why = "";
@@ -1239,9 +1255,6 @@ static bool make_dual(n2d2b_net* net, CellRec& b, const void* in_a, const int8_t
             b.dual_patch.proj_in = nullptr;
             return false;
         }
-    // A branch of few tiles and long K runs on clusters that share a tile when it is a kernel of its own: 3x3, 512 channels of 7 x 7 beside a projection of 256, one
-    // and two images 16.6 us as two kernels, 17.9 and 18.5 as one; three images, no clusters, 20.0 / 18.7
-    if (packed ? a.w8 == CellRec::W8_IGEMM && igemm_takes_clusters(a.plan8) : a.engine == ENG_TCGEN05 && igemm_takes_clusters(a.plan)) return false;
         b.dual_patch.late_weights = packed ? 1 : 0;
         return true;
     }
@@ -1342,7 +1355,7 @@ static int settle_duals(n2d2b_net* net)
     for (CellRec& b : net->cells) {
         if (b.dual_branch < 0 || !b.plan.w4) continue;
         CellRec& a = net->cells[b.dual_branch];
-        auto both = [&](int call) { return widens_all(macs, call) || (widens_alone(net, a, call) && widens_alone(net, b, call)); };
+        auto both = [&](int call) { return widens_in(net, a, macs, call, call) && widens_in(net, b, macs, call, call); };
         if (both(1)) {
             b.dual_always = true;
         } else if (!both(net->max_batch)) {
@@ -1369,6 +1382,9 @@ static int settle_chains(n2d2b_net* net)
         CellRec& p = net->cells[j];
         if (p.type != CELL_CONV || p.residual >= 0 || p.inputs.size() != 1 || p.inputs[0] != c.output || p.wbits != 8 || p.dual_sum >= 0) continue;
         if (!chain_eligible(c.geom, p.geom) || net->tensors[p.output].dtype != DT_I8) continue;
+        // (few row tiles: by themselves the two cells spread their columns over more multiprocessors.  64 -> 256 -> 64 channels with the sum behind them, 7 tiles 16.1
+        // us as two kernels, 17.3 as one; 13 16.0 / 17.5; 25 16.8 / 16.9, to 128 channels 18.8 / 17.2; 49 20.0 / 18.9)
+        if (((long long)net->max_batch * c.geom.oH * c.geom.oW + 127) / 128 * 7 < net->num_sms) continue;
         c.chain_next = (int)j;
         bool both = false;
         if (int rc = probe_dense(net, c, &both)) return rc;
@@ -1382,9 +1398,6 @@ static int settle_chains(n2d2b_net* net)
     }
     return 0;
 }
-        // (few row tiles: by themselves the two cells spread their columns over more multiprocessors.  64 -> 256 -> 64 channels with the sum behind them, 7 tiles 16.1
-        // us as two kernels, 17.3 as one; 13 16.0 / 17.5; 25 16.8 / 16.9, to 128 channels 18.8 / 17.2; 49 20.0 / 18.9)
-        if (((long long)net->max_batch * c.geom.oH * c.geom.oW + 127) / 128 * 7 < net->num_sms) continue;
 
 static int plan_duals(n2d2b_net* net)
 {
@@ -1804,6 +1817,7 @@ static int fuse_depthwise(n2d2b_net* net)
         if (pj < 0) continue;
         CellRec& p = net->cells[pj];
         if (p.type != CELL_CONV || p.residual >= 0 || p.wbits != 8 || net->tensors[p.output].dtype != DT_I8 || !dwpw_eligible(c.geom, p.geom)) continue;
+        if (!dwpw_faster(c.geom, p.geom.O, net->max_batch, net->num_sms)) continue;
         ConvGeom g = c.geom;
         g.B = net->max_batch;
         DwPwPlan probe{};
@@ -1817,7 +1831,6 @@ static int fuse_depthwise(n2d2b_net* net)
             for (CellRec* x : {&c, &p}) {
                 cudaFree(x->d_fast);
                 x->d_fast = nullptr;
-        if (!dwpw_faster(c.geom, p.geom.O, net->max_batch, net->num_sms)) continue;
                 x->fast = FastQuant{};
             }
             continue;
@@ -1865,14 +1878,14 @@ static bool depthwise_takes(const n2d2b_net* net, const CellRec& c, int batch, c
     return !block_form && (uintptr_t)in % depthwise_alignment(g, c.fast) == 0;
 }
 
-// Widens the packed weights of cell `c` into the scratch block, or in a large call those of every cell, once
+// Widens the packed weights of cell `c` into the scratch block, or in a large call those of every cell that takes the form, once
 static int widen_weights(n2d2b_net* net, const CellRec& c, cudaStream_t s)
 {
     const bool all = widen_all(net, net->call_batch);
     if (all && net->call_widened) return 0;
     std::vector<WidenJob> jobs;
     for (const CellRec& x : net->cells) {
-        if (x.w8 == CellRec::W8_NONE || (!all && &x != &c)) continue;
+        if (x.w8 == CellRec::W8_NONE || (all ? !worth_widening(net, x, net->call_batch) : &x != &c)) continue;
         WidenJob j;
         j.packed = (const uint8_t*)x.d_weights;
         j.dst = (int8_t*)net->d_w8 + x.w8_offset;

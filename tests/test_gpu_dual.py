@@ -137,8 +137,8 @@ def test_only_what_is_stored_has_a_buffer(case, weight_bits, engine):
 def _packed_layers():
     b = netdesc.NetBuilder('packed', 64, 1, 1, 3, 'fixed', weight_dist=('uniform', 7), weight_bits=4, clipped=True)
     x = b.conv(-1, 64, 1, name='front')
-    x = b.fc(x, 4096, act='relu', name='wide')
-    b.fc(x, 4096, act='relu', name='square')
+    x = b.fc(x, 16384, act='relu', name='wide')
+    b.fc(x, 960, act='relu', name='narrow')
     return b.net
 
 
