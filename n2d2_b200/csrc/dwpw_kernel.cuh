@@ -14,9 +14,9 @@
 // eight or twelve warps drain the accumulators beside the twelve or eight that fill the operand.  Rows of a tile beyond its pixels hold
 // whatever is there: their sums are not stored.
 //
-// What bounds it: the latency of the warps' instructions, six to eight cycles each at five working warps a scheduler (65 % of the issue slots); a
-// depthwise output takes eight to nine instructions and a 1x1 output four.  The same twenty warps doing both kinds of work in turn were slower
-// (MobileNet at 256 images 814 us against 685): every wait then stalls both.
+// What bounds it: up to 256 channels instructions (63 to 73 % of the issue slots; per 32 depthwise outputs 18 with as many 1x1 outputs behind them, 31 with
+// twice as many, their waits included); from 512 outputs on the waits for operand slots, which a tile of two passes hands back in the second (45 to 55 %).
+// The same twenty warps doing both kinds of work in turn were slower (MobileNet at 256 images 814 us against 685): every wait then stalls both.
 // As two kernels the depthwise output crosses L2 or HBM twice, and the pair costs two hand-overs between kernels of 1.3 to 2 us each:
 // 14 x 14 x 512 at 256 images 46 us as two launches by themselves, 33 as one.
 #pragma once

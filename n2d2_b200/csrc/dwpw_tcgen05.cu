@@ -82,7 +82,7 @@ static int dp_epilogue_warps(int bn) { return bn == 64 ? 12 : 8; }
 
 // How a call of `batch` images is split.  A CTA's work is, in cycles, the issue slots of its depthwise outputs and of its 1x1 outputs (about 9.5 and
 // 4 instructions each, four a cycle, three quarters of the slots used), its MMAs (full tiles of 128 rows whatever they hold) and the
-// weights it streams (about 60 bytes a cycle).  Column ranges of a tile go to several CTAs, which then repeat the depthwise part, only where
+// weights it streams (about 60 bytes a cycle).  It ranks the splits; launches take 1.2 to 2.4 times what it says (waits for operand slots).  Column ranges of a tile go to several CTAs, which then repeat the depthwise part, only where
 // there are fewer row segments than multiprocessors.
 int dwpw_set_batch(DwPwPlan* plan, int batch)
 {
