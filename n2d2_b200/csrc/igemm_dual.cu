@@ -11,6 +11,20 @@ static size_t dual_smem_bytes(int stages, int slot_bytes, size_t resident)
          + DUAL_SETS * FAST_NP * 256 * 4 + 64;
 }
 
+static long long dual_tiles_per_cta(const ConvGeom& g, int bn, int num_sms)
+{
+    const long long tiles = ((long long)g.B * g.oH * g.oW + BM - 1) / BM * ((g.O + bn - 1) / bn);
+    return (tiles + num_sms - 1) / num_sms;
+}
+
+// Whether the weights of a CTA's column block stay in shared memory: for a single tile they would all have to arrive before its first multiplication
+static bool dual_resident(const ConvGeom* g, int bn, int num_sms)
+{
+    long long weights = 0;
+    for (int s = 0; s < 2; ++s) weights += (long long)g[s].kH * g[s].kW * g[s].C * bn;
+    return weights <= 96 * 1024 && dual_tiles_per_cta(g[1], bn, num_sms) > 1;
+}
+
 // Columns of a tile by an estimate in cycles like igemm_tile_columns', for two multiplications and both rescales.  Tiles of 128 columns keep two
 // tiles' accumulators in TMEM: the longer of loads and epilogue, and 0.4 of the shorter.  Tiles of 256 keep one: each multiplication runs under the
 // epilogue of the other one, 0.4 of it the branch's.  An activation block then serves twice the columns, which pays where the operand loads bound
@@ -21,11 +35,10 @@ static int dual_tile_columns(const ConvGeom* g, const int* bk, const bool* im2co
 {
     const long long m_tiles = ((long long)g[1].B * g[1].oH * g[1].oW + BM - 1) / BM;
     auto cost = [&](int bn) {
-        const long long n_tiles = (g[1].O + bn - 1) / bn, tiles = m_tiles * n_tiles, per_cta = (tiles + num_sms - 1) / num_sms;
+        const long long tiles = m_tiles * ((g[1].O + bn - 1) / bn), per_cta = dual_tiles_per_cta(g[1], bn, num_sms);
         const double rate = tiles < num_sms ? 114.0 - 43.0 * tiles / num_sms : 71.0;
-        double weights = 0, k[2];
-        for (int s = 0; s < 2; ++s) weights += (double)g[s].kH * g[s].kW * g[s].C * bn;
-        const bool resident = bn < 256 && weights <= 96 * 1024 && per_cta > 1;
+        const bool resident = dual_resident(g, bn, num_sms);
+        double k[2];
         for (int s = 0; s < 2; ++s) {
             const double blocks = (double)g[s].kH * g[s].kW * ((g[s].C + bk[s] - 1) / bk[s]);
             const double load = bk[s] * (BM / (im2col[s] ? std::min(rate, 34.0) : rate) + (resident ? 0 : bn) / rate);
@@ -67,7 +80,7 @@ int dual_make_plan(DualPlan* plan, const void* in_a, const int8_t* w_a, const Co
         a_most = std::max(a_most, BM * p.BK);
         slot = std::max(slot, (BM + bn) * p.BK);
     }
-    plan->resident = weights <= 96 * 1024 ? 1 : 0;
+    plan->resident = dual_resident(g, bn, num_sms) ? 1 : 0;
     auto depth = [&] {
         int st = 8;
         while (st > 2 && dual_smem_bytes(st, plan->slot_bytes, plan->resident ? weights : 0) > 226 * 1024) --st;
