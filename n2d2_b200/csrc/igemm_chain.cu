@@ -61,7 +61,7 @@ cudaError_t launch_chain(const ChainPlan& plan, int M, const FastQuant& fast, in
     const bool t_unsigned = fast.dp4a ? fast.dp_t_unsigned : (fast.t_lo == 0);
     a.ef = (fast.out_unsigned ? EF_OUT_UNSIGNED : 0) | (res_unsigned ? EF_RES_UNSIGNED : 0) | (t_unsigned ? EF_T_UNSIGNED : 0)
          | (fast.dp_a_signed ? EF_DP_A_SIGNED : 0) | fast.form;
-    a.t_lo = fast.t_lo; a.t_hi = fast.t_hi; a.dp_xor = fast.dp_xor;
+    a.t_lo = fast.t_lo; a.t_hi = fast.t_hi;
     a.ef_next = (next.out_unsigned ? EF_OUT_UNSIGNED : 0) | next.form;
     a.clamp_next = next.need_clamp ? 1 : 0;
     a.out = (uint8_t*)out;

@@ -31,7 +31,6 @@ struct ChainArgs {
     const int *fq, *fq2, *fq_next;   // the expansion's rescale, the sum's, the next layer's
     int cpad, cpad_next;
     int ef, t_lo, t_hi;
-    unsigned dp_xor;
     int ef_next, clamp_next;
     uint8_t* out;
     int* status;
@@ -233,7 +232,7 @@ igemm_chain_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
         e.BN = 128; e.N = CH_N; e.M = m_end; e.wp = 64;
         // constants by column of y: a block of 128 columns is drained as columns cbase.. of its accumulator
         e.par_off = (unsigned)((unsigned char*)par - smem_raw) + (unsigned)(n * 128 * 4);
-        e.t_lo = a.t_lo; e.t_hi = a.t_hi; e.dp_xor = a.dp_xor;
+        e.t_lo = a.t_lo; e.t_hi = a.t_hi;
         const unsigned next_off = (unsigned)((unsigned char*)par - smem_raw) + 2u * FAST_NP * 1024u;
         const unsigned my_region = (unsigned)(regions - smem_raw) + (unsigned)(part4 * (BM * 64) + quad * REGION_BYTES);
         const unsigned my_rbar = rbar0 + 8u * CH_SLOTS_MAX * (unsigned)(warp - EPI_WARP0);

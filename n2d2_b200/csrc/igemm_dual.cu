@@ -29,8 +29,8 @@ static bool dual_resident(const ConvGeom* g, int bn, int num_sms)
 // tiles' accumulators in TMEM: the longer of loads and epilogue, and 0.4 of the shorter.  Tiles of 256 keep one: each multiplication runs under the
 // epilogue of the other one, 0.4 of it the branch's.  An activation block then serves twice the columns, which pays where the operand loads bound
 // the tile: 256 + 512 channels into 1024 at 1024 images of 14 x 14 go from 220 us to 172, 512 + 1024 into 2048 at 7 x 7 from 183 to 136 (at 128 images
-// from 31.3 to 26.9), but 64 + 64 into 256 at 55 x 55 and 128 images from 65.7 to 67.9.  Over 33 calls (4 to 1024 images) the choice is within 0.4 % of the
-// best of the three columns for each.
+// from 31.3 to 26.9), but 64 + 64 into 256 at 55 x 55 and 128 images from 65.7 to 67.9.  Fitted to 33 calls of
+// 4 to 1024 images.
 static int dual_tile_columns(const ConvGeom* g, const int* bk, const bool* im2col, int num_sms)
 {
     const long long m_tiles = ((long long)g[1].B * g[1].oH * g[1].oW + BM - 1) / BM;
@@ -133,7 +133,7 @@ cudaError_t launch_dual(const DualPlan& plan, const ConvGeom& gb, const FastQuan
     a.takers = (d.seg[0].num_kb + d.seg[1].num_kb) * 550 / (q.BN * 16) + 1;
     a.takers = std::min(a.takers, std::min(plan.stages, NUM_PRODUCERS));
     a.status = status_word;
-    a.fq = fb.fq; a.fq2 = fb.fq2; a.cpad = fb.cpad; a.t_lo = fb.t_lo; a.t_hi = fb.t_hi; a.dp_xor = fb.dp_xor;
+    a.fq = fb.fq; a.fq2 = fb.fq2; a.cpad = fb.cpad; a.t_lo = fb.t_lo; a.t_hi = fb.t_hi;
     const bool t_unsigned = fb.dp4a ? fb.dp_t_unsigned : (fb.t_lo == 0);
     a.ef = (fb.out_unsigned ? EF_OUT_UNSIGNED : 0) | (branch_unsigned ? EF_RES_UNSIGNED : 0) | (t_unsigned ? EF_T_UNSIGNED : 0)
          | (fb.dp_a_signed ? EF_DP_A_SIGNED : 0) | fb.form;

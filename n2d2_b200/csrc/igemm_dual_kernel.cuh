@@ -297,7 +297,7 @@ igemm_dual_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid
         pdl_wait();   // output stores touch a tensor that the previous kernel may read or write
         EpiTile e;
         e.BN = a.BN; e.N = a.N; e.M = a.m_base + a.M; e.n0 = n0; e.wp = wp;
-        e.t_lo = a.t_lo; e.t_hi = a.t_hi; e.dp_xor = a.dp_xor;
+        e.t_lo = a.t_lo; e.t_hi = a.t_hi;
         const unsigned par_off = (unsigned)((unsigned char*)par - smem_raw);
         const unsigned my_regions = (unsigned)(stage_out - smem_raw) + (unsigned)((warp - EPI_WARP0) * REGION_BYTES * DUAL_REGIONS);
         unsigned acc_it = 2u * (unsigned)group, mine = 0;

@@ -70,8 +70,7 @@ struct IgemmArgs {
     int cpad;
     int t_lo, t_hi;     // saturation range of the cell's own output (before the residual add)
     int out_unsigned;   // final 8-bit range: 1 = [0,255], 0 = [-128,127]
-    unsigned dp_xor;    // dot-product form of the residual stage: byte flips and operand signedness
-    int dp_a_signed;
+    int dp_a_signed;    // dot-product form of the residual stage: operand signedness
 };
 
 // Position of an output pixel in its image batch, walked without divisions
@@ -484,7 +483,7 @@ igemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                 e.tfull = tfull0 + 8u * as; e.tfull_parity = aph; e.tempty = tempty0 + 8u * as;
                 e.abort_flag = abort_flag; e.status = a.status; e.dry = dry;
                 e.ef = a.ef;
-                e.t_lo = a.t_lo; e.t_hi = a.t_hi; e.dp_xor = a.dp_xor;
+                e.t_lo = a.t_lo; e.t_hi = a.t_hi;
                 if (!fast_epilogue_tile<RES, CLAMP, DP, true, W4, DRY>(&tmO, &tmR, e, quad, part, lane, est)) { ok = false; break; }
                 if (dry) {
                     dry = false;

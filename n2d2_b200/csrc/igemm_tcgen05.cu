@@ -243,17 +243,17 @@ igemm_pair_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
                         tc_ld_2x16x256b_x4_wait(tbase + (unsigned)(32 * pass), va, vb);
                         const int pc = cbase + 32 * pass;
                         switch (a.ef & (EF_OUT_UNSIGNED | EF_WIDE | EF_FLOAT)) {
-                        case 0: perm_block<4, false, CLAMP, false, EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
+                        case 0: perm_block<4, false, CLAMP, false, EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0); break;
                         case EF_OUT_UNSIGNED:
-                            perm_block<4, false, CLAMP, false, EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
+                            perm_block<4, false, CLAMP, false, EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0);
                             break;
-                        case EF_WIDE: perm_block<4, false, CLAMP, false, EF_WIDE | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
+                        case EF_WIDE: perm_block<4, false, CLAMP, false, EF_WIDE | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0); break;
                         case EF_WIDE | EF_OUT_UNSIGNED:
-                            perm_block<4, false, CLAMP, false, EF_WIDE | EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
+                            perm_block<4, false, CLAMP, false, EF_WIDE | EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0);
                             break;
-                        case EF_FLOAT: perm_block<4, false, CLAMP, false, EF_FLOAT | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u); break;
+                        case EF_FLOAT: perm_block<4, false, CLAMP, false, EF_FLOAT | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0); break;
                         default:
-                            perm_block<4, false, CLAMP, false, EF_FLOAT | EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0, 0u);
+                            perm_block<4, false, CLAMP, false, EF_FLOAT | EF_OUT_UNSIGNED | EF_PERM>(va, vb, par_off, pc, region_off, rb, 0, lane, 0, 0);
                             break;
                         }
                     }
@@ -791,7 +791,6 @@ igemm_split_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid
                     unsigned a4;
                     if (sa.ef & EF_T_UNSIGNED) asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(a4) : "r"(y1), "r"(y0), "r"(rw));
                     else asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(a4) : "r"(y1), "r"(y0), "r"(rw));
-                    a4 ^= a.dp_xor;
                     // row 0 of the residual set holds the column-selecting multiplier words (see perm_block)
                     if (sa.ef & EF_DP_A_SIGNED) {
                         asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(y0) : "r"(a4), "r"(c2[0]), "r"(c2[3 * COLS]));
@@ -968,7 +967,6 @@ cudaError_t launch_igemm(const IgemmPlan& plan, const QuantDev& q, const Residua
     a.r = r;
     a.fq = fast.fq; a.fq2 = fast.fq2; a.cpad = fast.cpad; a.t_lo = fast.t_lo; a.t_hi = fast.t_hi;
     a.out_unsigned = fast.out_unsigned;
-    a.dp_xor = fast.dp_xor;
     a.dp_a_signed = fast.dp_a_signed;
     const bool t_unsigned = fast.dp4a ? fast.dp_t_unsigned : (fast.t_lo == 0);
     a.ef = (fast.out_unsigned ? EF_OUT_UNSIGNED : 0) | (r.is_unsigned ? EF_RES_UNSIGNED : 0)

@@ -87,7 +87,6 @@ struct FastQuant {
                                 // EF_FLOAT: floating-point scaling (both stages of a residual cell); 0: the 32-bit form
     bool dp4a = false;          // residual stage as a byte dot product (multipliers <= 255, native 8-bit ranges)
     bool dp_t_unsigned = false; //   the cell's own output is packed as unsigned bytes (natively, or shifted by +128)
-    unsigned dp_xor = 0;        //   bytes to flip from unsigned to signed (0x80 per byte)
     int dp_a_signed = 1;        //   signedness of the (t, r) byte vector
     bool unit_multiplier = false;   // every multiplier of the cell's own 32-bit rescale is 1
     bool monotone = false;      // no multiplier of the cell's own rescale is negative: it never decreases

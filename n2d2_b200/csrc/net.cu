@@ -522,7 +522,6 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
     // value is exactly 128 larger and the unsigned saturating pack clamps at the same places) and the second
     // addend drops 128 * m2.
     bool dp4a = false, dp_t_unsigned = false;
-    unsigned dp_xor = 0;
     int dp_a_signed = 1;
     if (with_res && !need_clamp && !wide && !flt && residual_dtype_i8) {
         const bool t_uns = (lo1 == 0 && hi1 == 255), t_sig = (lo1 == -128 && hi1 == 127);
@@ -569,7 +568,6 @@ static int upload_fast(CellRec& c, const TensorRec& tout, bool residual_dtype_i8
     c.fast.form = wide ? EF_WIDE : (flt ? EF_FLOAT : 0);
     c.fast.dp4a = dp4a;
     c.fast.dp_t_unsigned = dp_t_unsigned;
-    c.fast.dp_xor = dp_xor;
     c.fast.dp_a_signed = dp_a_signed;
     c.fast.monotone = true;   // (row 2: a multiplier, or a factor as the bits of a float)
     for (int ch = 0; ch < C; ++ch) c.fast.monotone = c.fast.monotone && f1[(size_t)2 * cpad + ch] >= 0;

@@ -105,7 +105,7 @@ __device__ __forceinline__ void s2d_drain(unsigned tbase, unsigned par_off, unsi
     for (int cb = 0; cb < BN; cb += 32) {
         unsigned va[16], vb[16];
         tc_ld_2x16x256b_x4_wait(tbase + (unsigned)cb, va, vb);
-        perm_block<4, false, CLAMP, false, EF | EF_PERM>(va, vb, par_off, cb, region_off, rb, cb, lane, 0, 0, 0u);
+        perm_block<4, false, CLAMP, false, EF | EF_PERM>(va, vb, par_off, cb, region_off, rb, cb, lane, 0, 0);
     }
 }
 

@@ -308,7 +308,7 @@ stem_conv_tcgen05_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
             e.tfull = tfull0 + 8u * as; e.tfull_parity = aph; e.tempty = tempty0 + 8u * as;
             e.abort_flag = abort_flag; e.status = a.status; e.dry = false;
             e.ef = (a.out_unsigned ? EF_OUT_UNSIGNED : 0) | a.form;
-            e.t_lo = 0; e.t_hi = 0; e.dp_xor = 0;
+            e.t_lo = 0; e.t_hi = 0;
             if (!fast_epilogue_tile<false, CLAMP, false>(&tmO, &tmO, e, quad, cp, lane, est)) break;
         }
         if (lane == 0) bulk_wait_all();

@@ -419,7 +419,6 @@ static constexpr int EF_RES_UNSIGNED = 2;   // residual operand is unsigned
 static constexpr int EF_T_UNSIGNED = 4;     // DP: the cell's own output saturates to [0,255]
 static constexpr int EF_DP_A_SIGNED = 8;    // DP: the packed (t, r) bytes are read as signed
 static constexpr int EF_WIDE = 16;          // first rescale in 64 bits: x * mult + (row 0 : row 3 as a 64-bit addend) >> shift
-static constexpr int EF_DP_XOR = 32;        // DP: some of the packed (t, r) bytes are flipped between unsigned and signed (dp_xor)
 static constexpr int EF_PERM = 64;          // weights stored with permuted output channels (perm_block)
 static constexpr int EF_FLOAT = 256;        // floating-point scaling: row 2 = factor, row 3 = bias, rows 0 and 1 = clamp of the converted value
 static constexpr int EF_W4 = 128;           // the accumulator holds 16 x the sum (packed 4-bit weights, see expand_int4_x16)
@@ -488,7 +487,7 @@ __device__ __forceinline__ int rescale(int x, int lo, int hi, int mult, int add,
 
 template <int NG, bool RES, bool CLAMP, bool DP, int EF>
 __device__ __forceinline__ void frag_block(const unsigned* vA, const unsigned* vB, unsigned par_off, int pcol0, unsigned region_off,
-                                           const unsigned* rb, int col0, int lane, int t_lo, int t_hi, unsigned dp_xor)
+                                           const unsigned* rb, int col0, int lane, int t_lo, int t_hi)
 {
     unsigned char* const sm = dyn_smem();
     constexpr int NK = 4;   // rows tr + 8k: k = 0, 1 from vA (TMEM lanes 0-15), k = 2, 3 from vB (lanes 16-31)
@@ -546,7 +545,6 @@ __device__ __forceinline__ void frag_block(const unsigned* vA, const unsigned* v
                 unsigned a4;
                 if (EF & EF_T_UNSIGNED) asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(a4) : "r"(y1), "r"(y0), "r"(rw));
                 else asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(a4) : "r"(y1), "r"(y0), "r"(rw));
-                a4 ^= dp_xor;
                 // lo2 row holds the column-selecting multiplier words, ad2 the (compensated) addends
                 int d0, d1;
                 if (EF & EF_DP_A_SIGNED) {
@@ -623,7 +621,7 @@ __device__ __forceinline__ unsigned pack4_sat(int y0, int y1, int y2, int y3, bo
 
 template <int NG, bool RES, bool CLAMP, bool DP, int EF>
 __device__ __forceinline__ void perm_block(const unsigned* vA, const unsigned* vB, unsigned par_off, int pcol0, unsigned region_off,
-                                           const unsigned* rb, int col0, int lane, int t_lo, int t_hi, unsigned dp_xor)
+                                           const unsigned* rb, int col0, int lane, int t_lo, int t_hi)
 {
     unsigned char* const sm = dyn_smem();
     constexpr int NK = 4;          // rows tr + 8k: k = 0, 1 from vA (TMEM lanes 0-15), k = 2, 3 from vB (lanes 16-31)
@@ -693,10 +691,6 @@ __device__ __forceinline__ void perm_block(const unsigned* vA, const unsigned* v
                 } else {
                     asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(a01) : "r"(y[1]), "r"(y[0]), "r"(rw));
                     asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(a23) : "r"(y[3]), "r"(y[2]), "r"(rw >> 16));
-                }
-                if (EF & EF_DP_XOR) {
-                    a01 ^= dp_xor;
-                    a23 ^= dp_xor;
                 }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -837,7 +831,6 @@ struct EpiTile {
     int* status;
     int ef;                 // EF_* switches of this cell
     int t_lo, t_hi;
-    unsigned dp_xor;
 };
 
 // Per-warp state carried from tile to tile.
@@ -858,16 +851,15 @@ __device__ __forceinline__ void epi_drain(const EpiTile& e, unsigned tbase, int 
             unsigned va[16], vb[16];
             tc_ld_2x16x256b_x4_wait(tbase + (unsigned)cb, va, vb);
             if (PERM)
-                perm_block<4, RES, CLAMP, DP, EF>(va, vb, e.par_off, cbase + cb, region_off, rb, cb, lane, e.t_lo, e.t_hi, e.dp_xor);
+                perm_block<4, RES, CLAMP, DP, EF>(va, vb, e.par_off, cbase + cb, region_off, rb, cb, lane, e.t_lo, e.t_hi);
             else
-                frag_block<4, RES, CLAMP, DP, EF>(va, vb, e.par_off, cbase + cb, region_off, rb, cb, lane, e.t_lo, e.t_hi,
-                                                  e.dp_xor);
+                frag_block<4, RES, CLAMP, DP, EF>(va, vb, e.par_off, cbase + cb, region_off, rb, cb, lane, e.t_lo, e.t_hi);
         }
     } else {
         unsigned va[8], vb[8];
         tc_ld_2x16x256b_x2_wait(tbase, va, vb);
-        if (PERM) perm_block<2, RES, CLAMP, DP, EF>(va, vb, e.par_off, cbase, region_off, rb, 0, lane, e.t_lo, e.t_hi, e.dp_xor);
-        else frag_block<2, RES, CLAMP, DP, EF>(va, vb, e.par_off, cbase, region_off, rb, 0, lane, e.t_lo, e.t_hi, e.dp_xor);
+        if (PERM) perm_block<2, RES, CLAMP, DP, EF>(va, vb, e.par_off, cbase, region_off, rb, 0, lane, e.t_lo, e.t_hi);
+        else frag_block<2, RES, CLAMP, DP, EF>(va, vb, e.par_off, cbase, region_off, rb, 0, lane, e.t_lo, e.t_hi);
     }
 }
 
