@@ -95,3 +95,8 @@ def test_resnet50_at_the_benchmark_batch():
 
 def test_resnet18_w4_at_the_benchmark_batch():
     _entry_points_agree(FULL['resnet18_w4_clipped_fixed'](), 2048)
+
+
+def test_mobilenet_at_the_benchmark_batch():
+    # 256 images: two upload slices through depthwise + 1x1 pairs, the deep layers as two kernels a pair
+    _entry_points_agree(FULL['mobilenet_single'](), 256)
