@@ -876,7 +876,7 @@ cudaError_t launch_widen_int4(const WidenJob* jobs, int count, cudaStream_t s)
         unsigned long long total = 0;
         for (; done < count && t.count < WIDEN_JOBS; ++done) {
             const unsigned long long words = (unsigned long long)jobs[done].rows * jobs[done].words;
-            if (words >= (1ull << 30)) return cudaErrorInvalidValue;
+            if (words >= (1ull << 31)) return cudaErrorInvalidValue;
             if (words == 0) continue;
             if (total + words >= (1ull << 31)) break;
             t.job[t.count] = jobs[done];
