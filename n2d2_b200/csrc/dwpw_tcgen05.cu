@@ -21,19 +21,22 @@ bool dwpw_eligible(const ConvGeom& d, const ConvGeom& p)
 
 // Whether one kernel is faster than two in calls of up to `batch` images.  Measured as pairs of 32 to 1024 channels, maps of 2 to 112 pixels a side, 0.5 to 4 times
 // as many outputs, strides 1 and 2 and 1 to 256 images, in graphs of several passes; times as two kernels over times as one:
-//   - 6400 output pixels and more (of 32 channels 12800), up to two blocks of channels and twice as many outputs, or up to four blocks and as many: shift scalings
+//   - 6400 output pixels and more (of 32 channels 12500), up to two blocks of channels and twice as many outputs, or up to four blocks and as many: shift scalings
 //     0.96 to 1.28 (512 -> 512 at 14 x 14, 33 images: 21.2 us, 19.9), fixed-point ones 0.95 to 1.2
-//   - one or two blocks of 128 channels and few output rows (up to a third of the multiprocessors): a hand-over less, 1.00 to 1.08; from 56 rows on, which
-//     column ranges share and compute several times, 0.9
+//   - one, two, four or eight blocks of 128 channels and few output rows (a third of the multiprocessors, fewer of more blocks; of one block and up to 128 outputs,
+//     more of which several CTAs would share and compute the depthwise part again, up to half): 0.97 to 1.1 and a launch less, which bounds a pass of so few
+//     pixels outside a graph (MobileNet, one image: 86.3 us with thirteen pairs, 90.3 with three; in a graph 81.1 and 79.0)
 //   - in between (2 rows a CTA) 0.86 to 0.95
 //   - more outputs, which take several passes over the operand, 0.78 to 1.05 (512 -> 1024, 14 x 14 to 7 x 7, 256 images: 34.7 us, 41.8)
 //   - more blocks, whose patches and operands do not fit beside one another, 0.37 to 0.9 (960 channels at 7 x 7)
 bool dwpw_faster(const ConvGeom& d, int N, int batch, int num_sms)
 {
-    const int blocks = d.C / block_channels(d.C);
-    if (blocks > 4 || N > (blocks > 2 ? 1 : 2) * d.C) return false;
+    const int bk = block_channels(d.C), blocks = d.C / bk;
     const long long rows = (long long)batch * d.oH, pixels = rows * d.oW;
-    return pixels >= (d.C > 32 ? 6400 : 12800) || (blocks <= 2 && d.C >= 128 && rows <= num_sms / 3);
+    if (N > 2 * d.C) return false;
+    if (bk == 128 && (blocks & (blocks - 1)) == 0 && rows <= num_sms / 3 && rows * blocks <= 64) return true;
+    if (blocks == 1 && d.C > 32 && N <= 128 && rows <= num_sms / 2) return true;
+    return blocks <= 4 && (blocks <= 2 || N <= d.C) && pixels >= (d.C > 32 ? 6400 : 12500);
 }
 
 size_t dwpw_depthwise_words(const ConvGeom& d) { return (size_t)3 * d.C; }

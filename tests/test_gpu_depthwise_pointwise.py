@@ -25,14 +25,13 @@ CASES = [(32, 112, 112, 64, 1, 1, 3), (64, 30, 30, 128, 2, 1, 5), (128, 28, 28, 
          (512, 14, 14, 512, 1, 1, 1), (512, 14, 14, 512, 1, 1, 150), (512, 14, 14, 1024, 2, 1, 37), (1024, 7, 7, 1024, 1, 1, 50), (1024, 7, 7, 1024, 1, 1, 1),
          (96, 9, 13, 32, 1, 1, 3), (192, 5, 7, 96, 2, 0, 9), (160, 3, 3, 160, 1, 2, 70), (256, 1, 1, 64, 1, 1, 300), (64, 1, 17, 64, 1, 1, 2),
          (32, 6, 300, 96, 1, 1, 2), (64, 5, 259, 128, 2, 1, 3), (128, 4, 127, 64, 1, 1, 3), (480, 6, 5, 576, 2, 2, 11),
-         (256, 14, 14, 512, 2, 1, 140), (96, 40, 41, 64, 1, 1, 5), (192, 33, 31, 96, 2, 0, 40), (256, 1, 1, 64, 1, 1, 45), (64, 7, 7, 32, 1, 1, 140),
-         (256, 13, 9, 160, 1, 1, 3), (512, 3, 3, 512, 1, 2, 300), (384, 9, 13, 384, 1, 1, 60), (128, 3, 3, 96, 1, 2, 9),
+         (256, 14, 14, 512, 2, 1, 140), (96, 40, 41, 64, 1, 1, 5), (192, 33, 31, 96, 2, 0, 40), (256, 1, 1, 64, 1, 1, 30), (64, 7, 7, 32, 1, 1, 140),
+         (256, 13, 9, 160, 1, 1, 2), (384, 5, 5, 384, 1, 1, 2), (512, 3, 3, 512, 1, 2, 300), (384, 9, 13, 384, 1, 1, 60), (128, 3, 3, 96, 1, 2, 9),
          (32, 6, 300, 64, 1, 1, 8), (64, 5, 259, 128, 2, 1, 20), (128, 28, 28, 128, 1, 1, 1), (64, 1, 97, 64, 1, 1, 70)]
 
-# two kernels are faster: a few rows per multiprocessor, many outputs, more than four K blocks
-SEPARATE = [(128, 28, 28, 128, 1, 1, 2), (64, 1, 17, 64, 1, 1, 2), (32, 6, 300, 96, 1, 1, 2), (64, 5, 259, 128, 2, 1, 3),
-            (64, 30, 30, 128, 2, 1, 5), (256, 14, 14, 512, 2, 1, 40), (512, 14, 14, 512, 1, 1, 1), (512, 14, 14, 1024, 2, 1, 37), (1024, 7, 7, 1024, 1, 1, 50),
-            (1024, 7, 7, 1024, 1, 1, 1), (96, 9, 13, 32, 1, 1, 3), (192, 5, 7, 96, 2, 0, 9), (160, 3, 3, 160, 1, 2, 70), (256, 1, 1, 64, 1, 1, 300), (480, 6, 5, 576, 2, 2, 11)]
+# two kernels are faster: a few rows per multiprocessor, many outputs, more than four K blocks or three of few rows
+SEPARATE = [(32, 6, 300, 96, 1, 1, 2), (64, 30, 30, 128, 2, 1, 5), (256, 14, 14, 512, 2, 1, 40), (512, 14, 14, 1024, 2, 1, 37),
+            (1024, 7, 7, 1024, 1, 1, 50), (96, 9, 13, 32, 1, 1, 3), (192, 5, 7, 96, 2, 0, 9), (160, 3, 3, 160, 1, 2, 70), (256, 1, 1, 64, 1, 1, 300), (480, 6, 5, 576, 2, 2, 11), (384, 5, 5, 384, 1, 1, 2)]
 
 
 @pytest.mark.parametrize('case', CASES, ids=lambda c: 'C%d_%dx%d_N%d_s%d_p%d_b%d' % c)
