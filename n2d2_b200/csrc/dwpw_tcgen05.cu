@@ -21,8 +21,9 @@ bool dwpw_eligible(const ConvGeom& d, const ConvGeom& p)
 
 // Whether one kernel is faster than two in calls of up to `batch` images.  Measured as pairs of 32 to 1024 channels, maps of 2 to 112 pixels a side, 0.5 to 4 times
 // as many outputs, strides 1 and 2 and 1 to 256 images, in graphs of several passes; times as two kernels over times as one:
-//   - 6400 output pixels and more (of 32 channels 12500), up to two blocks of channels and twice as many outputs, or up to four blocks and as many: shift scalings
-//     0.96 to 1.28 (512 -> 512 at 14 x 14, 33 images: 21.2 us, 19.9), fixed-point ones 0.95 to 1.2
+//   - 1500 output pixels and more of whole blocks of 128 channels (6200 of 64, 9000 of 32 channels, 6400 of three blocks), up to two blocks and twice as many outputs, or
+//     up to four blocks and as many: shift scalings 0.96 to 1.28 (512 -> 512 at 14 x 14, 33 images: 21.2 us, 19.9), fixed-point ones 0.95 to 1.2.  Outside a
+//     graph a hand-over costs about half a microsecond more than in one, so the lines lie a little below the points where the graphs are even
 //   - one, two, four or eight blocks of 128 channels and few output rows (a third of the multiprocessors, fewer of more blocks; of one block and up to 128 outputs,
 //     more of which several CTAs would share and compute the depthwise part again, up to half): 0.97 to 1.1 and a launch less, which bounds a pass of so few
 //     pixels outside a graph (MobileNet, one image: 86.3 us with thirteen pairs, 90.3 with three; in a graph 81.1 and 79.0)
@@ -36,7 +37,7 @@ bool dwpw_faster(const ConvGeom& d, int N, int batch, int num_sms)
     if (N > 2 * d.C) return false;
     if (bk == 128 && (blocks & (blocks - 1)) == 0 && rows <= num_sms / 3 && rows * blocks <= 64) return true;
     if (blocks == 1 && d.C > 32 && N <= 128 && rows <= num_sms / 2) return true;
-    return blocks <= 4 && (blocks <= 2 || N <= d.C) && pixels >= (d.C > 32 ? 6400 : 12500);
+    return blocks <= 4 && (blocks <= 2 || N <= d.C) && pixels >= (blocks == 3 ? 6400 : (d.C >= 128 ? 1500 : (d.C > 32 ? 6200 : 9000)));
 }
 
 size_t dwpw_depthwise_words(const ConvGeom& d) { return (size_t)3 * d.C; }
